@@ -164,6 +164,11 @@ int tc_orient(mc_dgraph *g, const int32_t *upload = nullptr);
 int clique_prepare(mc_dgraph *g, int pattern, bool *use, int64_t *dag_edges);
 int clique_launch(mc_dgraph *g, int pattern, int64_t dag_edges, int shard, int num_shards,
                   const unsigned long long *deadline, unsigned long long *stop_flag);
+// P1..P8 from motif sums (motifs.cu): whether a whole count of g takes that
+// route, and the count (synchronous; event ev[3] marks its last kernel).
+// MC_ERR_OOM when its scratch does not fit: the formula routes need less.
+bool motif_route(const mc_dgraph *g);
+int motif_count(mc_dgraph *g, int pattern, uint64_t *out);
 // Contract checks of the row offsets alone; sets max_degree.
 int validate_rowptr(mc_dgraph *g);
 int tc_partner_stats(mc_dgraph *g, unsigned long long *partner_edges, unsigned long long *work);

@@ -1,0 +1,1194 @@
+// P1..P8 from non-induced motif sums: the default route of whole counts.
+//
+// Reference: subgraph_matching/pattern_kernels.cuh (P1..P8) and the combine of
+// subgraph_matching/sm_multigpu.cu:206-232.  While no 32-bit product of those
+// formulas can wrap (maximum degree at most 46,340), each is a fixed multiple
+// of induced subgraph counts (claws, forks, K1,4, 4-paths, bulls, paws, darts,
+// K1,1,3, tailed K4).  An induced count is a signed sum of non-induced ones
+// over the graphs that contain the pattern on the same vertices, and every
+// non-induced count needed is a sum over vertices, edges, triangles, or pairs
+// at distance two of small polynomials in
+//   d   degrees,
+//   a   triangles on an edge,
+//   k   common neighbours of a triangle's three vertices,
+//   c   common neighbours of a vertex pair,
+// plus the numbers of K4, K5, 4-cycles (C4), 4-wheels (W4) and of K2,3 with
+// one edge in its side of three (X7).  So nothing is enumerated beyond
+// triangles and two-paths, where the per-edge formulas test every pair of an
+// edge's neighbours.
+//
+// What bounds it: latency of dependent gathers (row offsets, then columns,
+// then per-edge words) and, on small graphs, the launches.  On the Chung-Lu
+// graph of 100,000 vertices (mean 10, cap 200: m = 498,340, 84 k triangles,
+// 429 k triangle pairs on an edge, 81 M two-paths) the per-edge formulas
+// took P1..P8 1.9, 28.0, 9.7, 4.8, 11.1, 3.6, 0.95 and 3.6 ms per call on a
+// B200, and these sums take 0.36, 1.82, 0.46, 0.82, 1.74, 0.46, 0.37 and 0.37.
+// On the one of 60,000 (mean 20, cap 50,000, a hub of degree 17,215) P1, P4,
+// P7 and P8 took 74.7, 276, 25.9 and 26.1 ms, and take 0.94, 2.7, 1.5 and 1.5.
+//
+// Stages (each vertex pair ordered by (degree, id), written u < v below; an
+// "up" entry of the CSR is one with u < v):
+//   rows    entry -> row, degrees
+//   up      N+(u): the up entries of each row, compacted in place; the
+//           reverse entry of each edge
+//   tri     a of each entry: every pair (x, y) of N+(u) tested once in the
+//           row of the lower of the two, so sum of C(d+, 2) searches
+//   lists   per entry (u -> v) the entries (u -> w) of its common neighbours
+//           w, slot j of (u -> v) and slot j of (v -> u) holding the same w;
+//           edge and vertex sums
+//   tau     per u, bit rows of its up neighbours over N(u) and over N+(u):
+//           k is a popcount of two rows, K4 and K5 of two and three
+//   pairs   common neighbours c of pairs (s, t), counted per s in a table
+//           over t: C4, K2,3, X7
+//   wheel   4-cycles inside N(v), counted per (v, x) in a table over N(v)
+#include <algorithm>
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
+
+#include "device_common.cuh"
+#include "dgraph.cuh"
+#include "scan.cuh"
+
+namespace mc {
+namespace {
+
+using u64 = unsigned long long;
+
+// Sums over the graph, modulo 2^64.
+enum Sum : int {
+  kVd3, kVd4, kVt2, kVtd,                  // vertices: C(d,3), C(d,4), C(t,2), t d
+  kD, kC3, kEp4, kEfork, kEdart,           // edges
+  kT, kCricket, kBull, kLolli, kKite, kGem,  // triangles
+  kKd, kKa, kKk, kK4, kK5,                 // with common neighbours; cliques
+  kC4, kC4d, kC4a, kX7, kW4, kK23,         // 4-cycles and beyond
+  kSums
+};
+
+// Words of MotifArgs::counts: list lengths, then queue positions.
+enum Count : int {
+  kTauN, kMidN, kHashN, kHugeN, kBigN, kTauQueue, kMidQueue, kHashQueue, kBigQueue, kCounts
+};
+
+// What a pattern needs beyond a and the vertex and edge sums.
+enum Need : unsigned {
+  kNeedTau = 1u,    // triangle sums with k (else K4 alone)
+  kNeedD2 = 2u,     // sum of (d - 1) over each neighbourhood
+  kNeedT = 4u,      // C(t, 2) over the triangles per vertex
+  kNeedC4 = 8u,     // 4-cycles, each counted at its highest vertex
+  kNeedPairs = 16u, // every pair's common neighbours (C4 counted twice)
+  kNeedW4 = 32u,
+  kNeedK23 = 64u,   // with kNeedPairs: K2,3 and degrees on 4-cycles
+};
+
+__host__ __device__ constexpr unsigned needs_of(int pattern) {
+  return pattern == 1   ? 0u
+         : pattern == 2 ? kNeedTau | kNeedD2 | kNeedT | kNeedPairs | kNeedW4 | kNeedK23
+         : pattern == 3 ? kNeedTau | kNeedT | kNeedW4
+         : pattern == 4 ? kNeedC4
+         : pattern == 5 ? kNeedTau | kNeedPairs | kNeedW4
+         : pattern == 6 ? kNeedTau | kNeedW4
+                        : (unsigned)kNeedTau;
+}
+
+struct MotifArgs {
+  const int64_t *__restrict__ rp;
+  const int32_t *__restrict__ ci;
+  int n, nnz;
+  unsigned need;
+  int32_t *deg;    // n
+  int32_t *dp;     // n: |N+(v)|
+  int32_t *tv2;    // n: twice the triangles of v
+  u64 *d2;         // n: sum of (d - 1) over N(v)
+  u64 *walk;       // n: table entries the pairs stage visits for s = v
+  int32_t *src;    // nnz: row of an entry
+  int32_t *upe;    // nnz: rp[u] + i -> i-th up entry of u
+  int32_t *pos1;   // nnz: 1 + position in N+(row) of an up entry, else 0
+  int32_t *rev1;   // nnz: 1 + reverse entry, 0 if there is none
+  int32_t *a;      // nnz: triangles on the entry's edge
+  int32_t *cur;    // nnz: list slots taken, at the up entry
+  int64_t *off;    // nnz + 1: list offsets
+  int32_t *list;   // common-neighbour lists
+  int64_t list_cap;
+  u64 *acc;        // kSums
+  // Vertices too large for one warp.  pair_mid: the two hash classes, from the
+  // front and from the back of its n entries; pair_big: tables over all
+  // vertices, the longest walks from the front, so that they start first.
+  int32_t *tau_big, *pair_mid, *pair_big;
+  unsigned *counts;  // see Count
+  u64 mid_walk;      // pair_mid's front class ends here (kWarpWalk: none in it)
+  unsigned *slices;  // bit rows of the tau stage that exceed shared memory
+  int64_t slice_words;
+};
+
+constexpr int kThreads = 256;
+constexpr int kWarps = kThreads / kWarp;
+constexpr int kTauOut = 32;       // warp form of the tau stage: d+ and d at most
+constexpr int kTauDeg = 512;
+constexpr int kTauSmem = 96 << 10;  // bit rows of a CTA, two CTAs per SM
+// Classes of the pairs stage by table entries visited (a vertex's walk bounds
+// the keys of its table, which has at least twice as many slots): a warp, a
+// CTA of 128 and of 512 threads with a hash table, and a CTA of 1,024 with a
+// counter for every vertex.  With warps and 1,024-thread CTAs alone the stage
+// took 6.2 ms in P2 on the graph of 100,000 (one CTA per SM, three barriers
+// per vertex of some 1,000 entries); with the four classes it takes 1.4 ms.
+constexpr u64 kWarpWalk = 512, kMidWalk = 2048, kHashWalk = 8192;
+constexpr u64 kHugeWalk = 1 << 15;
+constexpr int kHashSlots = 1024;  // of a warp
+constexpr int kWheelDeg = 512;    // warp form of the wheel stage
+
+__device__ __forceinline__ u64 c2(u64 x) { return x * (x - 1) / 2; }  // 0 at 0 and 1
+__device__ __forceinline__ u64 c3(long long x) {
+  return x < 3 ? 0ull : (u64)x * (u64)(x - 1) / 2 * (u64)(x - 2) / 3;
+}
+// C(x, 4) below 2^64 for x up to 46,341: C(x, 3) (x - 3) is at most 8e17.
+__device__ __forceinline__ u64 c4(long long x) {
+  return x < 4 ? 0ull : c3(x) * (u64)(x - 3) / 4;
+}
+
+// (degree, id) order.
+__device__ __forceinline__ bool lower(int du, int u, int dv, int v) {
+  return du < dv || (du == dv && u < v);
+}
+
+// Index of x in the ascending ci[b, e), or -1.
+__device__ __forceinline__ int find_entry(const int32_t *__restrict__ ci, int b, int e, int x) {
+  while (b < e) {
+    const int mid = (b + e) >> 1;
+    const int y = __ldg(ci + mid);
+    if (y == x) return mid;
+    if (y < x) b = mid + 1;
+    else e = mid;
+  }
+  return -1;
+}
+
+// Per-block totals of the sums a kernel adds to.
+struct BlockSums {
+  u64 *s;
+  __device__ __forceinline__ void init() const {
+    for (int i = threadIdx.x; i < kSums; i += blockDim.x) s[i] = 0;
+    __syncthreads();
+  }
+  // Every lane of the warp takes part.
+  __device__ __forceinline__ void add(int which, u64 v) const {
+    v = warp_sum_u64(v);
+    if ((threadIdx.x & (kWarp - 1)) == 0 && v) atomicAdd(s + which, v);
+  }
+  __device__ __forceinline__ void flush(u64 *acc) const {
+    __syncthreads();
+    for (int i = threadIdx.x; i < kSums; i += blockDim.x)
+      if (s[i]) atomicAdd(acc + i, s[i]);
+  }
+};
+
+// The warp's 32 lists laid end to end: flat position f belongs to list l (the
+// first whose inclusive end exceeds f) at offset f - excl(l).
+struct FlatLists {
+  int incl, total;
+  __device__ __forceinline__ FlatLists(int len, int lane) {
+    incl = warp_inclusive_scan(len, lane);
+    total = __shfl_sync(kFull, incl, kWarp - 1);
+  }
+  // Every lane calls it; positions past the end give list 31.
+  __device__ __forceinline__ int owner(int f) const {
+    int l = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (__shfl_sync(kFull, incl, l + step - 1) <= f) l += step;
+    return min(l, kWarp - 1);
+  }
+};
+
+// ---- rows, up ---------------------------------------------------------------
+// Warp per row: src, deg, and the sums of degrees alone.
+__global__ void __launch_bounds__(kThreads) motif_rows_kernel(MotifArgs a) {
+  __shared__ u64 sm[kSums];
+  const BlockSums bs{sm};
+  bs.init();
+  const int lane = threadIdx.x & (kWarp - 1);
+  u64 d3 = 0, d4 = 0;
+  const int stride = gridDim.x * kWarps;
+  for (int v = blockIdx.x * kWarps + threadIdx.x / kWarp; v < a.n; v += stride) {
+    const int b = (int)__ldg(a.rp + v), e = (int)__ldg(a.rp + v + 1);
+    for (int i = b + lane; i < e; i += kWarp) a.src[i] = v;
+    if (lane == 0) {
+      a.deg[v] = e - b;
+      d3 += c3(e - b);
+      d4 += c4(e - b);
+    }
+  }
+  bs.add(kVd3, d3);
+  bs.add(kVd4, d4);
+  bs.flush(a.acc);
+}
+
+// Thread per entry.  Up entries are compacted per row with one atomic per
+// (row, warp) piece (their order within a row does not matter), and find
+// their reverse entry in the longer row.
+__global__ void __launch_bounds__(kThreads) motif_up_kernel(MotifArgs a) {
+  const int lane = threadIdx.x & (kWarp - 1);
+  const int64_t e64 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  const bool in = e64 < a.nnz;
+  const int e = in ? (int)e64 : a.nnz - 1;
+  const int u = a.src[e], v = __ldg(a.ci + e);
+  const int64_t bu = __ldg(a.rp + u);
+  const int du = a.deg[u], dv = a.deg[v];
+  int r = -1;
+  int bv = 0;
+  if (in && lower(du, u, dv, v)) {
+    bv = (int)__ldg(a.rp + v);
+    r = find_entry(a.ci, bv, bv + dv, u);
+  }
+  const bool up = r >= 0;
+  const unsigned ups = __ballot_sync(kFull, up);
+  // Lanes of the same row: from the last row head at or below this lane to
+  // the one before the next head.
+  const int u_prev = __shfl_up_sync(kFull, u, 1);
+  const unsigned heads = __ballot_sync(kFull, lane == 0 || u != u_prev);
+  const unsigned upto = kFull >> (kWarp - 1 - lane);
+  const int first = kWarp - 1 - __clz(heads & upto);
+  const unsigned later = heads & ~upto;
+  const unsigned row = (later ? (1u << (__ffs(later) - 1)) - 1u : kFull) & (kFull << first);
+  int base = 0;
+  if (lane == first && (ups & row)) base = atomicAdd(a.dp + u, __popc(ups & row));
+  base = __shfl_sync(kFull, base, first);
+  if (up) {
+    const int k = base + __popc(ups & row & ((1u << lane) - 1u));
+    a.upe[bu + k] = e;
+    a.pos1[e] = k + 1;
+    a.rev1[e] = r + 1;
+    a.rev1[r] = e + 1;
+    if (a.need & kNeedC4) {
+      atomicAdd(a.walk + v, (u64)du);  // s = v visits N(u)
+    } else if (a.need & kNeedPairs) {
+      atomicAdd(a.walk + u, (u64)(r - bv));
+      atomicAdd(a.walk + v, (u64)(e - (int)bu));
+    }
+    if (a.need & kNeedD2) {
+      atomicAdd(a.d2 + u, (u64)(dv - 1));
+      atomicAdd(a.d2 + v, (u64)(du - 1));
+    }
+  } else if (in) {
+    a.pos1[e] = 0;  // a down entry, or one with no reverse, which the up lists leave out
+  }
+}
+
+// ---- triangles --------------------------------------------------------------
+// A warp takes 32 consecutive slots of the compacted up lists; slot i of N+(u)
+// pairs with the later slots, and the pairs of all 32 are walked flat.
+// kFill: the counts are known and the lists are written; the edge and vertex
+// sums are added on the way.
+template <bool kFill>
+__global__ void __launch_bounds__(kThreads) motif_tri_kernel(MotifArgs a) {
+  __shared__ u64 sm[kSums];
+  const BlockSums bs{sm};
+  bs.init();
+  const int lane = threadIdx.x & (kWarp - 1);
+  if (kFill && a.off[a.nnz] > a.list_cap) return;  // the host sizes the lists and starts over
+  const int64_t s64 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  if (kFill && s64 < a.n) {
+    const int v = (int)s64;
+    const int d = a.deg[v], p = a.dp[v];
+    if (p >= 2 && (p > kTauOut || d > kTauDeg)) a.tau_big[atomicAdd(a.counts + kTauN, 1u)] = v;
+    if (a.need & (kNeedC4 | kNeedPairs)) {
+      const u64 w = a.walk[v];
+      if (w > kHugeWalk) a.pair_big[atomicAdd(a.counts + kHugeN, 1u)] = v;
+      else if (w > kHashWalk) a.pair_big[a.n - 1 - atomicAdd(a.counts + kBigN, 1u)] = v;
+      else if (w > a.mid_walk) a.pair_mid[a.n - 1 - atomicAdd(a.counts + kHashN, 1u)] = v;
+      else if (w > kWarpWalk) a.pair_mid[atomicAdd(a.counts + kMidN, 1u)] = v;
+    }
+  }
+  if (kFill && (a.need & kNeedT)) {
+    // Triangles per vertex from a: one atomic per (row, warp) piece.
+    const int v = s64 < a.nnz ? a.src[s64] : -1;
+    int sum = s64 < a.nnz ? a.a[s64] : 0;
+#pragma unroll
+    for (int o = 1; o < kWarp; o <<= 1) {
+      const int other = __shfl_up_sync(kFull, sum, o), ov = __shfl_up_sync(kFull, v, o);
+      if (lane >= o && ov == v) sum += other;
+    }
+    const int next = __shfl_down_sync(kFull, v, 1);
+    if (v >= 0 && sum && (lane == kWarp - 1 || next != v)) atomicAdd(a.tv2 + v, sum);
+  }
+  int slot = 0, len = 0, e_ux = 0, x = 0, dx = 0, i0 = 0;
+  u64 D = 0, C3 = 0, p4 = 0, fork = 0, dart = 0;
+  if (s64 < a.nnz) {
+    slot = (int)s64;
+    const int u = a.src[slot];
+    const int i = slot - (int)__ldg(a.rp + u), p = a.dp[u];
+    if (i < p) {
+      len = p - 1 - i;
+      i0 = slot + 1;
+      e_ux = a.upe[slot];
+      x = __ldg(a.ci + e_ux);
+      dx = a.deg[x];
+      if (kFill) {
+        const u64 t = (u64)a.a[e_ux], du = (u64)a.deg[u], dv = (u64)dx;
+        D = c2(t);
+        C3 = c3((long long)t);
+        p4 = (du - 1 - t) * (dv - 1 - t);
+        fork = c2(du - 1) * (dv - 1) + c2(dv - 1) * (du - 1) - t * (du + dv - 4);
+        dart = c2(t) * (du + dv - 6);
+      }
+    }
+  }
+  const FlatLists fl(len, lane);
+  u64 tri = 0, vtd = 0;
+  for (int base = 0; base < fl.total; base += kWarp) {
+    const int f = base + lane;
+    const int l = fl.owner(f);
+    const int o = f - (__shfl_sync(kFull, fl.incl, l) - __shfl_sync(kFull, len, l));
+    const int ys = __shfl_sync(kFull, i0, l) + o;
+    const int ex = __shfl_sync(kFull, e_ux, l);
+    const int vx = __shfl_sync(kFull, x, l), dvx = __shfl_sync(kFull, dx, l);
+    if (f >= fl.total) continue;
+    const int ey = a.upe[ys];
+    const int y = __ldg(a.ci + ey);
+    const int dy = a.deg[y];
+    const bool x_low = lower(dvx, vx, dy, y);
+    const int lo = x_low ? vx : y, hi = x_low ? y : vx;
+    const int b = (int)__ldg(a.rp + lo);
+    const int exy = find_entry(a.ci, b, b + (x_low ? dvx : dy), hi);
+    if (exy < 0 || a.rev1[exy] == 0) continue;
+    const int rx = a.rev1[ex] - 1, ry = a.rev1[ey] - 1, rxy = a.rev1[exy] - 1;
+    if (!kFill) {
+      atomicAdd(a.a + ex, 1);
+      atomicAdd(a.a + rx, 1);
+      atomicAdd(a.a + ey, 1);
+      atomicAdd(a.a + ry, 1);
+      atomicAdd(a.a + exy, 1);
+      atomicAdd(a.a + rxy, 1);
+      vtd += (u64)(a.deg[a.src[ex]] + dvx) + (u64)dy;
+      ++tri;
+    } else {
+      // Entries lo -> hi and hi -> lo, and those back to u.
+      const int r_lo = x_low ? rx : ry, r_hi = x_low ? ry : rx;
+      const int jx = atomicAdd(a.cur + ex, 1), jy = atomicAdd(a.cur + ey, 1),
+                jxy = atomicAdd(a.cur + exy, 1);
+      a.list[a.off[ex] + jx] = ey;
+      a.list[a.off[rx] + jx] = x_low ? exy : rxy;  // x -> y
+      a.list[a.off[ey] + jy] = ex;
+      a.list[a.off[ry] + jy] = x_low ? rxy : exy;  // y -> x
+      a.list[a.off[exy] + jxy] = r_lo;             // lo -> u
+      a.list[a.off[rxy] + jxy] = r_hi;             // hi -> u
+    }
+  }
+  __syncwarp();
+  if (!kFill) {
+    bs.add(kT, tri);
+    bs.add(kVtd, vtd);
+  } else {
+    bs.add(kD, D);
+    bs.add(kC3, C3);
+    bs.add(kEp4, p4);
+    bs.add(kEfork, fork);
+    bs.add(kEdart, dart);
+  }
+  bs.flush(a.acc);
+}
+
+// ---- triangles with their common neighbours -----------------------------------
+struct TauSums {
+  u64 cricket = 0, bull = 0, lolli = 0, kite = 0, gem = 0, kd = 0, ka = 0, kk = 0, K4 = 0, K5 = 0;
+  __device__ __forceinline__ void flush(const BlockSums &bs, bool tau) const {
+    if (tau) {
+      bs.add(kCricket, cricket);
+      bs.add(kBull, bull);
+      bs.add(kLolli, lolli);
+      bs.add(kKite, kite);
+      bs.add(kGem, gem);
+      bs.add(kKd, kd);
+      bs.add(kKa, ka);
+      bs.add(kKk, kk);
+    }
+    bs.add(kK4, K4);
+    bs.add(kK5, K5);
+  }
+};
+
+// Triangle (u, x, y): degrees, triangles on its edges, k common neighbours.
+__device__ __forceinline__ void tau_terms(const MotifArgs &a, TauSums &t, int u, int x, int y,
+                                          long long du, long long aux, long long auy,
+                                          long long axy, long long k) {
+  const long long dx = a.deg[x], dy = a.deg[y];
+  const long long sd = du + dx + dy, sa = aux + auy + axy;
+  t.cricket += c2((u64)(du - 2)) + c2((u64)(dx - 2)) + c2((u64)(dy - 2));
+  t.bull += (u64)((du - 2) * (dx - 2) + (du - 2) * (dy - 2) + (dx - 2) * (dy - 2) - sa + 3);
+  if (a.need & kNeedD2)
+    t.lolli += a.d2[u] + a.d2[x] + a.d2[y] - (u64)(2 * (sd - 3) + 2 * (sa - 3));
+  t.kite += (u64)((aux - 1) * (dy - 2) + (auy - 1) * (dx - 2) + (axy - 1) * (du - 2));
+  t.gem += (u64)((aux - 1) * (auy - 1) + (aux - 1) * (axy - 1) + (auy - 1) * (axy - 1));
+  t.kd += (u64)(k * sd);
+  t.ka += (u64)(k * sa);
+  t.kk += c2((u64)k);
+}
+
+// Bits above position j of a row's word w.
+__device__ __forceinline__ unsigned above(int j, int w) {
+  const int s = j + 1 - 32 * w;
+  return s <= 0 ? kFull : (s >= 32 ? 0u : kFull << s);
+}
+
+// Element q of the list of up entry i of u (row start b, entry e, reverse r):
+// when its neighbour is an up neighbour j > i, the triangle (u, i, j).  R:
+// rows over N(u) (wd words), M: rows over N+(u) (wp words).
+__device__ __forceinline__ void tau_element(const MotifArgs &a, TauSums &t, int u, int du, int i,
+                                            int e, int64_t q, int64_t rev_off, int idx,
+                                            const unsigned *R, int wd, const unsigned *M, int wp) {
+  const int j = a.pos1[idx] - 1;
+  if (j <= i) return;
+  if (a.need & kNeedTau) {
+    int k = 0;
+    for (int w = 0; w < wd; ++w) k += __popc(R[i * wd + w] & R[j * wd + w]);
+    tau_terms(a, t, u, __ldg(a.ci + e), __ldg(a.ci + idx), du, a.a[e], a.a[idx],
+              a.a[a.list[rev_off + q]], k);
+  }
+  for (int w = (j + 1) >> 5; w < wp; ++w) {
+    unsigned m = M[i * wp + w] & M[j * wp + w] & above(j, w);
+    t.K4 += __popc(m);
+    if (!(a.need & kNeedTau)) continue;
+    while (m) {
+      const int l = 32 * w + __ffs(m) - 1;
+      m &= m - 1;
+      for (int w2 = (l + 1) >> 5; w2 < wp; ++w2)
+        t.K5 += __popc(M[i * wp + w2] & M[j * wp + w2] & M[l * wp + w2] & above(l, w2));
+    }
+  }
+}
+
+// Warp per u with d+ <= 32 and d <= 512: lane i owns row i.
+__global__ void __launch_bounds__(kThreads) motif_tau_kernel(MotifArgs a) {
+  __shared__ u64 sm[kSums];
+  __shared__ unsigned s_r[kWarps][kTauOut * (kTauDeg / 32)];
+  __shared__ unsigned s_m[kWarps][kTauOut];
+  const BlockSums bs{sm};
+  bs.init();
+  if (a.off[a.nnz] > a.list_cap) return;
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  unsigned *R = s_r[warp], *M = s_m[warp];
+  TauSums t;
+  u64 vt2 = 0;
+  const int stride = gridDim.x * kWarps;
+  for (int u = blockIdx.x * kWarps + warp; u < a.n; u += stride) {
+    const int p = a.dp[u], d = a.deg[u];
+    if ((a.need & kNeedT) && lane == 0) vt2 += c2((u64)(a.tv2[u] >> 1));
+    if (p < 2 || p > kTauOut || d > kTauDeg) continue;
+    const int b = (int)__ldg(a.rp + u);
+    const int wd = (d + 31) >> 5;
+    int e = 0, na = 0;
+    int64_t off = 0, roff = 0;
+    if (lane < p) {
+      e = a.upe[b + lane];
+      na = a.a[e];
+    }
+    if (!__any_sync(kFull, na > 0)) continue;
+    unsigned mrow = 0;
+    if (lane < p) {
+      for (int w = 0; w < wd; ++w) R[lane * wd + w] = 0;
+      if (na > 0) {
+        off = a.off[e];
+        roff = a.off[a.rev1[e] - 1];
+      }
+      for (int q = 0; q < na; ++q) {
+        const int idx = a.list[off + q];
+        const int ps = idx - b, j1 = a.pos1[idx];
+        R[lane * wd + (ps >> 5)] |= 1u << (ps & 31);
+        if (j1) mrow |= 1u << (j1 - 1);
+      }
+    }
+    M[lane] = mrow;
+    __syncwarp();
+    for (int q = 0; q < na; ++q)
+      tau_element(a, t, u, d, lane, e, q, roff, a.list[off + q], R, wd, M, 1);
+    __syncwarp();
+  }
+  t.flush(bs, a.need & kNeedTau);
+  if (a.need & kNeedT) bs.add(kVt2, vt2);
+  bs.flush(a.acc);
+}
+
+// CTA per larger u (queue over tau_big): warp per row, lanes over its list.
+// The rows take p (wd + wp) words: p d <= nnz and p^2 <= nnz, since u's p up
+// neighbours have at least u's degree, so slice_words bounds them.
+__global__ void __launch_bounds__(kThreads) motif_tau_big_kernel(MotifArgs a, int smem_words) {
+  extern __shared__ unsigned s_rows[];
+  __shared__ u64 sm[kSums];
+  __shared__ int s_u;
+  const BlockSums bs{sm};
+  bs.init();
+  if (a.off[a.nnz] > a.list_cap) return;
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  TauSums t;
+  for (;;) {
+    if (threadIdx.x == 0) {
+      const unsigned i = atomicAdd(a.counts + kTauQueue, 1u);
+      s_u = i < a.counts[kTauN] ? a.tau_big[i] : -1;
+    }
+    __syncthreads();
+    const int u = s_u;
+    __syncthreads();
+    if (u < 0) break;
+    const int p = a.dp[u], d = a.deg[u], b = (int)__ldg(a.rp + u);
+    const int wd = (a.need & kNeedTau) ? (d + 31) >> 5 : 0, wp = (p + 31) >> 5;
+    const int64_t words = (int64_t)p * (wd + wp);
+    unsigned *R = words <= smem_words ? s_rows : a.slices + blockIdx.x * a.slice_words;
+    unsigned *M = R + (int64_t)p * wd;
+    for (int64_t i = threadIdx.x; i < words; i += kThreads) R[i] = 0;
+    __syncthreads();
+    for (int i = warp; i < p; i += kWarps) {
+      const int e = a.upe[b + i], na = a.a[e];
+      const int64_t off = a.off[e];
+      for (int q = lane; q < na; q += kWarp) {
+        const int idx = a.list[off + q];
+        const int ps = idx - b, j1 = a.pos1[idx];
+        if (wd) atomicOr(R + (int64_t)i * wd + (ps >> 5), 1u << (ps & 31));
+        if (j1) atomicOr(M + (int64_t)i * wp + ((j1 - 1) >> 5), 1u << ((j1 - 1) & 31));
+      }
+    }
+    __syncthreads();
+    for (int i = warp; i < p; i += kWarps) {
+      const int e = a.upe[b + i], na = a.a[e];
+      const int64_t off = a.off[e], roff = a.off[a.rev1[e] - 1];
+      for (int q = lane; q < na; q += kWarp)
+        tau_element(a, t, u, d, i, e, q, roff, a.list[off + q], R, wd, M, wp);
+    }
+    __syncthreads();
+  }
+  t.flush(bs, a.need & kNeedTau);
+  bs.flush(a.acc);
+}
+
+// ---- pairs at distance two -----------------------------------------------------
+// Per s, a table over t counts the two-paths s - v - t.  kOrdered: v and t
+// below s in (degree, id), so that a 4-cycle is counted once, at its highest
+// vertex (sum over edges of the smaller degree in entries).  Otherwise every
+// pair t < s by id: entries of N(v) before s, which the reverse entry ends
+// (half the two-paths).  An increment from c to c + 1 adds c to sum C(c, 2)
+// and C(c, 2) to sum C(c, 3).
+struct PairSums {
+  u64 c4 = 0, c4d = 0, c4a = 0, x7 = 0, k23 = 0;
+};
+
+// This warp's share of a row's 32-entry pieces among nwarps warps: whole
+// pieces when there are enough of them, else a part of one piece each.
+struct Share {
+  int first, step, part, parts;
+  __device__ __forceinline__ Share(int d, int warp, int nwarps) {
+    const int pieces = (d + kWarp - 1) / kWarp;
+    parts = pieces >= nwarps || pieces == 0 ? 1 : nwarps / pieces;
+    first = warp / parts;
+    step = max(pieces, nwarps / parts);  // parts > 1: one piece
+    if (parts == 1) step = nwarps;
+    part = warp % parts;
+  }
+};
+
+// Calls f(t, entry of v -> t, entry of s -> v, v) for this warp's share of the
+// two-paths from s.
+template <bool kOrdered, class F>
+__device__ __forceinline__ void walk_pairs(const MotifArgs &a, int s, int b, int d, const Share &sh,
+                                           int lane, F f) {
+  for (int c = sh.first; c * kWarp < d; c += sh.step) {
+    const int k = c * kWarp + lane;
+    int e = 0, v = 0, st = 0, len = 0;
+    if (k < d) {
+      e = b + k;
+      v = __ldg(a.ci + e);
+      const int r1 = a.rev1[e];
+      if (r1) {
+        st = (int)__ldg(a.rp + v);
+        if (kOrdered) {
+          const int dv = a.deg[v];
+          len = lower(dv, v, d, s) ? dv : 0;
+        } else {
+          len = r1 - 1 - st;
+        }
+      }
+    }
+    const FlatLists fl(len, lane);
+    constexpr int kU = 4;
+    for (int base = sh.part * kU * kWarp; base < fl.total; base += sh.parts * kU * kWarp) {
+      int q[kU], t[kU], l[kU];
+#pragma unroll
+      for (int i = 0; i < kU; ++i) {
+        const int g = base + i * kWarp + lane;
+        l[i] = fl.owner(g);
+        const int start = __shfl_sync(kFull, st - (fl.incl - len), l[i]);
+        q[i] = g < fl.total ? start + g : -1;
+        t[i] = q[i] >= 0 ? __ldg(a.ci + q[i]) : 0;
+      }
+      bool ok[kU];
+#pragma unroll
+      for (int i = 0; i < kU; ++i)
+        ok[i] = q[i] >= 0 && (!kOrdered || lower(a.deg[t[i]], t[i], d, s));
+#pragma unroll
+      for (int i = 0; i < kU; ++i) {
+        const int le = __shfl_sync(kFull, e, l[i]), lv = __shfl_sync(kFull, v, l[i]);
+        if (ok[i]) f(t[i], q[i], le, lv);
+      }
+    }
+  }
+}
+
+// All terms of one s with the table's operations: count(t) returns the count
+// before an increment, get(t) the count; sync() orders the phases among the
+// threads that share the table, which the caller clears afterwards.
+template <bool kOrdered, class Count, class Get, class Sync>
+__device__ __forceinline__ void pair_terms(const MotifArgs &a, PairSums &ps, int s, int b, int d,
+                                           const Share &sh, int lane, Count count, Get get,
+                                           Sync sync) {
+  const bool k23 = a.need & kNeedK23;
+  walk_pairs<kOrdered>(a, s, b, d, sh, lane, [&](int t, int, int, int) {
+    const u64 c = count(t);
+    ps.c4 += c;
+    if (!kOrdered && k23 && c) {
+      ps.c4d += c * (u64)(d + a.deg[t]);
+      ps.k23 += c2(c);
+    }
+  });
+  sync();
+  if (kOrdered) return;
+  walk_pairs<kOrdered>(a, s, b, d, sh, lane, [&](int t, int q, int e, int v) {
+    const u64 c = get(t);
+    if (c < 2) return;
+    ps.c4a += (c - 1) * (u64)(a.a[e] + a.a[q]);
+    if (k23) ps.c4d += (c - 1) * (u64)a.deg[v];
+  });
+  // X7: for each edge (p, r) inside N(s), the pairs (s, t) with t adjacent to
+  // p and r.
+  int nth = 0;
+  for (int c = sh.first; c * kWarp < d; c += sh.step) {
+    const int k = c * kWarp + lane;
+    const int e0 = b + (k < d ? k : 0);
+    unsigned with = __ballot_sync(kFull, k < d && a.a[e0] > 0);
+    while (with) {
+      const int src = __ffs(with) - 1;
+      with &= with - 1;
+      if (nth++ % sh.parts != sh.part) continue;
+      const int e = __shfl_sync(kFull, e0, src);
+      const int na = a.a[e];
+      const int64_t off = a.off[e], roff = a.off[a.rev1[e] - 1];
+      for (int j = lane; j < na; j += kWarp) {
+        if (a.list[off + j] <= e) continue;  // seen from the edge's other end
+        const int pr = a.list[roff + j];
+        const int64_t lo = a.off[pr], hi = a.off[pr + 1];
+        for (int64_t q = lo; q < hi; ++q) {
+          const int t = __ldg(a.ci + a.list[q]);
+          if (t < s) ps.x7 += get(t) - 2;
+        }
+      }
+    }
+  }
+  sync();
+}
+
+__device__ __forceinline__ void flush_pairs(const BlockSums &bs, const PairSums &ps, u64 *acc) {
+  bs.add(kC4, ps.c4);
+  bs.add(kC4d, ps.c4d);
+  bs.add(kC4a, ps.c4a);
+  bs.add(kX7, ps.x7);
+  bs.add(kK23, ps.k23);
+  bs.flush(acc);
+}
+
+// An open-addressing table of 2^lg slots: keys, and 16-bit counts two to a
+// word (a count is at most the maximum degree, 46,340).  Never more than half
+// full, so every probe ends.
+struct HashTable {
+  int *key;
+  unsigned *cnt;
+  int lg;
+  __device__ __forceinline__ void size_for(unsigned walk) {
+    lg = 6;
+    while ((1u << lg) < 2 * walk) ++lg;
+  }
+  __device__ __forceinline__ u64 count(int t) const {
+    const int mask = (1 << lg) - 1;
+    int sl = (int)hash_slot(t, 32 - lg);
+    for (;;) {
+      const int k = atomicCAS(key + sl, -1, t);
+      if (k == -1 || k == t) break;
+      sl = (sl + 1) & mask;
+    }
+    const int sh = (sl & 1) * 16;
+    return (u64)((atomicAdd(cnt + (sl >> 1), 1u << sh) >> sh) & 0xffffu);
+  }
+  __device__ __forceinline__ u64 get(int t) const {
+    const int mask = (1 << lg) - 1;
+    int sl = (int)hash_slot(t, 32 - lg);
+    for (;;) {
+      const int k = key[sl];
+      if (k == t) return (u64)((cnt[sl >> 1] >> ((sl & 1) * 16)) & 0xffffu);
+      if (k == -1) return 0;
+      sl = (sl + 1) & mask;
+    }
+  }
+  __device__ __forceinline__ void clear(int tid, int threads) const {
+    int4 *k4 = reinterpret_cast<int4 *>(key);
+    uint4 *c4 = reinterpret_cast<uint4 *>(cnt);
+    for (int i = tid; i < 1 << (lg - 2); i += threads) k4[i] = make_int4(-1, -1, -1, -1);
+    for (int i = tid; i < 1 << (lg - 3); i += threads) c4[i] = make_uint4(0, 0, 0, 0);
+  }
+};
+
+constexpr size_t hash_bytes(int slots) { return (sizeof(int) + 2) * (size_t)slots; }
+
+// Warp per s of at most kWarpWalk table entries.
+template <bool kOrdered>
+__global__ void __launch_bounds__(kThreads) motif_pairs_kernel(MotifArgs a) {
+  extern __shared__ __align__(16) int s_tab[];
+  __shared__ u64 sm[kSums];
+  const BlockSums bs{sm};
+  bs.init();
+  if (a.off[a.nnz] > a.list_cap) return;
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  int *mine = s_tab + warp * (kHashSlots + kHashSlots / 2);
+  HashTable tab{mine, reinterpret_cast<unsigned *>(mine + kHashSlots), 10};
+  tab.clear(lane, kWarp);
+  __syncwarp();
+  PairSums ps;
+  const int stride = gridDim.x * kWarps;
+  for (int s = blockIdx.x * kWarps + warp; s < a.n; s += stride) {
+    const u64 w = a.walk[s];
+    if (w < 2 || w > kWarpWalk) continue;
+    tab.size_for((unsigned)w);
+    const int b = (int)__ldg(a.rp + s), d = a.deg[s];
+    pair_terms<kOrdered>(
+        a, ps, s, b, d, Share(d, 0, 1), lane, [&](int t) { return tab.count(t); },
+        [&](int t) { return tab.get(t); }, [&]() { __syncwarp(); });
+    tab.clear(lane, kWarp);
+    __syncwarp();
+  }
+  flush_pairs(bs, ps, a.acc);
+}
+
+// CTA per s of the hash classes: kFront the front list of pair_mid, else the
+// back one; 2^kLg slots.
+template <bool kOrdered, bool kFront, int kT, int kLg>
+__global__ void __launch_bounds__(kT) motif_pairs_hash_kernel(MotifArgs a) {
+  extern __shared__ __align__(16) int s_tab[];
+  __shared__ u64 sm[kSums];
+  __shared__ int s_s;
+  const BlockSums bs{sm};
+  bs.init();
+  if (a.off[a.nnz] > a.list_cap) return;
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  HashTable tab{s_tab, reinterpret_cast<unsigned *>(s_tab + (1 << kLg)), kLg};
+  tab.clear(threadIdx.x, kT);
+  PairSums ps;
+  for (;;) {
+    if (threadIdx.x == 0) {
+      const unsigned i = atomicAdd(a.counts + (kFront ? kMidQueue : kHashQueue), 1u);
+      s_s = i < a.counts[kFront ? kMidN : kHashN] ? a.pair_mid[kFront ? i : a.n - 1 - i] : -1;
+    }
+    __syncthreads();
+    const int s = s_s;
+    if (s < 0) break;
+    tab.size_for((unsigned)a.walk[s]);
+    const int b = (int)__ldg(a.rp + s), d = a.deg[s];
+    pair_terms<kOrdered>(
+        a, ps, s, b, d, Share(d, warp, kT / kWarp), lane, [&](int t) { return tab.count(t); },
+        [&](int t) { return tab.get(t); }, [&]() { __syncthreads(); });
+    tab.clear(threadIdx.x, kT);
+  }
+  flush_pairs(bs, ps, a.acc);
+}
+
+constexpr int kPairThreads = 1024;
+
+// CTA per larger s (longest walks first): 16-bit counters over all vertices,
+// two to a word, in shared memory when n of them fit, else one slice of
+// `counters` per CTA.
+template <bool kOrdered, bool kShared>
+__global__ void __launch_bounds__(kPairThreads) motif_pairs_big_kernel(MotifArgs a,
+                                                                       unsigned *counters) {
+  extern __shared__ __align__(16) int s_tab[];
+  __shared__ u64 sm[kSums];
+  __shared__ int s_s;
+  const BlockSums bs{sm};
+  bs.init();
+  if (a.off[a.nnz] > a.list_cap) return;
+  const int words = (a.n + 1) >> 1;
+  unsigned *cnt = kShared ? reinterpret_cast<unsigned *>(s_tab)
+                          : counters + (int64_t)blockIdx.x * words;
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  bool clean = false;  // the counters are zero
+  PairSums ps;
+  for (;;) {
+    if (threadIdx.x == 0) {
+      const unsigned i = atomicAdd(a.counts + kBigQueue, 1u);
+      const unsigned huge = a.counts[kHugeN], big = a.counts[kBigN];
+      s_s = i < huge ? a.pair_big[i] : i - huge < big ? a.pair_big[a.n - 1 - (i - huge)] : -1;
+    }
+    __syncthreads();
+    const int s = s_s;
+    if (s < 0) break;
+    if (!clean) {
+      for (int i = threadIdx.x; i < words; i += kPairThreads) cnt[i] = 0;
+      __syncthreads();
+    }
+    const int b = (int)__ldg(a.rp + s), d = a.deg[s];
+    const Share sh(d, warp, kPairThreads / kWarp);
+    pair_terms<kOrdered>(
+        a, ps, s, b, d, sh, lane,
+        [&](int t) {
+          const int bit = (t & 1) * 16;
+          return (u64)((atomicAdd(cnt + (t >> 1), 1u << bit) >> bit) & 0xffffu);
+        },
+        [&](int t) { return (u64)((cnt[t >> 1] >> ((t & 1) * 16)) & 0xffffu); },
+        [&]() { __syncthreads(); });
+    // A walk much shorter than the table clears its words one by one (both
+    // counters of a word in this phase), a longer one leaves it to the sweep.
+    clean = a.walk[s] * 4 < (u64)words;
+    if (clean)
+      walk_pairs<kOrdered>(a, s, b, d, sh, lane, [&](int t, int, int, int) { cnt[t >> 1] = 0; });
+    __syncthreads();
+  }
+  flush_pairs(bs, ps, a.acc);
+}
+
+// ---- 4-wheels ---------------------------------------------------------------
+// Per entry (v -> x), the two-paths x - y - z inside N(v) with y and z before
+// x in v's row, counted in a table over N(v): a 4-cycle of N(v) is counted
+// once, at its last vertex.  Warp per entry of a row of at most kWheelDeg.
+__global__ void __launch_bounds__(kThreads) motif_wheel_kernel(MotifArgs a) {
+  __shared__ u64 sm[kSums];
+  __shared__ unsigned s_cnt[kWarps][kWheelDeg];
+  const BlockSums bs{sm};
+  bs.init();
+  if (a.off[a.nnz] > a.list_cap) return;
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  unsigned *cnt = s_cnt[warp];
+  for (int i = lane; i < kWheelDeg; i += kWarp) cnt[i] = 0;
+  __syncwarp();
+  u64 w4 = 0;
+  const int64_t stride = (int64_t)gridDim.x * kThreads;
+  for (int64_t base = (int64_t)blockIdx.x * kThreads + warp * kWarp; base < a.nnz; base += stride) {
+    const int64_t e64 = base + lane;
+    unsigned todo = __ballot_sync(
+        kFull, e64 < a.nnz && a.a[e64] >= 2 && a.deg[a.src[e64]] <= kWheelDeg);
+    while (todo) {
+      const int e = (int)base + __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int b = (int)__ldg(a.rp + a.src[e]);
+      const int na = a.a[e];
+      const int64_t off = a.off[e];
+      for (int j = lane; j < na; j += kWarp) {
+        const int y = a.list[off + j];
+        if (y >= e) continue;
+        const int64_t lo = a.off[y], hi = a.off[y + 1];
+        for (int64_t q = lo; q < hi; ++q) {
+          const int z = a.list[q];
+          if (z < e) w4 += atomicAdd(cnt + (z - b), 1u);
+        }
+      }
+      __syncwarp();
+      for (int j = lane; j < na; j += kWarp) {
+        const int y = a.list[off + j];
+        if (y >= e) continue;
+        const int64_t lo = a.off[y], hi = a.off[y + 1];
+        for (int64_t q = lo; q < hi; ++q) {
+          const int z = a.list[q];
+          if (z < e) cnt[z - b] = 0;
+        }
+      }
+      __syncwarp();
+    }
+  }
+  bs.add(kW4, w4);
+  bs.flush(a.acc);
+}
+
+// CTA per entry of a longer row: warp per y, lanes over y's list.
+__global__ void __launch_bounds__(kThreads) motif_wheel_big_kernel(MotifArgs a, int table) {
+  extern __shared__ unsigned s_cnt[];
+  __shared__ u64 sm[kSums];
+  __shared__ int s_e[kThreads], s_n;
+  const BlockSums bs{sm};
+  bs.init();
+  if (a.off[a.nnz] > a.list_cap) return;
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  for (int i = threadIdx.x; i < table; i += kThreads) s_cnt[i] = 0;
+  u64 w4 = 0;
+  const int64_t stride = (int64_t)gridDim.x * kThreads;
+  for (int64_t base = (int64_t)blockIdx.x * kThreads; base < a.nnz; base += stride) {
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    const int64_t e64 = base + threadIdx.x;
+    if (e64 < a.nnz && a.a[e64] >= 2 && a.deg[a.src[e64]] > kWheelDeg)
+      s_e[atomicAdd(&s_n, 1)] = (int)e64;
+    __syncthreads();
+    for (int i = 0; i < s_n; ++i) {
+      const int e = s_e[i];
+      const int b = (int)__ldg(a.rp + a.src[e]);
+      const int na = a.a[e];
+      const int64_t off = a.off[e];
+      for (int pass = 0; pass < 2; ++pass) {
+        for (int j = warp; j < na; j += kWarps) {
+          const int y = a.list[off + j];
+          if (y >= e) continue;
+          const int64_t lo = a.off[y], hi = a.off[y + 1];
+          for (int64_t q = lo + lane; q < hi; q += kWarp) {
+            const int z = a.list[q];
+            if (z >= e) continue;
+            if (pass == 0) w4 += atomicAdd(s_cnt + (z - b), 1u);
+            else s_cnt[z - b] = 0;
+          }
+        }
+        __syncthreads();
+      }
+    }
+    __syncthreads();
+  }
+  bs.add(kW4, w4);
+  bs.flush(a.acc);
+}
+
+// ---- host -------------------------------------------------------------------
+// The pattern's count from the sums, modulo 2^64: non-induced counts of the
+// subgraphs on five vertices that contain the pattern, each with the signed
+// number of the pattern's copies in it.
+u64 combine(int pattern, const u64 *s) {
+  const u64 K4 = s[kK4], K5 = s[kK5], D = s[kD], T = s[kT];
+  // C4 family: the ordered walk counts each cycle once, the pair walk twice.
+  const u64 ka = s[kKa] - 24 * K4;   // 2 x K5 minus a path of 3 vertices
+  const u64 kd = s[kKd] - 36 * K4;   // 3 x tailed K4
+  const u64 third = 0xaaaaaaaaaaaaaaabull;  // 1/3 modulo 2^64
+  const u64 tk4 = kd * third;
+  const u64 claw = s[kVd3] - s[kVtd] + 6 * T + 2 * D - 4 * K4;
+  const u64 gem = s[kGem] - 12 * K4, kite = s[kKite] - 12 * K4;
+  const u64 butterfly = s[kVt2] - 2 * D;
+  switch (pattern) {
+    case 1: return claw;
+    case 2:
+      // banner = C4d / 2 - 8 (C4 / 2) - 2 D and house = C4a / 2 - 4 D, with
+      // the doubled sums of the pair walk.
+      return s[kEfork] - 2 * s[kCricket] - 2 * s[kBull] - s[kLolli] - (s[kC4d] - 8 * s[kC4] - 4 * D) +
+             6 * s[kK23] + 5 * s[kEdart] + 4 * kite + (2 * s[kC4a] - 16 * D) + 4 * butterfly -
+             10 * gem - 10 * s[kX7] + 20 * s[kW4] - 3 * kd + 10 * ka - 12 * s[kC3] - 36 * s[kKk] +
+             60 * K5;
+    case 3: {
+      const u64 star = s[kVd4] - s[kCricket] + s[kEdart] + butterfly - gem + s[kW4] - tk4 -
+                       2 * s[kC3] - 3 * s[kKk] + 5 * K5;  // + 2 (K5 - P3), added below
+      return 4 * star + 4 * ka + 3 * claw;
+    }
+    case 4: return s[kEp4] - 4 * s[kC4] + 4 * D - 12 * K4;
+    case 5:
+      return 2 * s[kBull] - 4 * s[kEdart] - 4 * kite - (s[kC4a] - 8 * D) + 10 * gem + 8 * s[kX7] -
+             24 * s[kW4] + 4 * kd - 14 * ka + 12 * s[kC3] + 60 * s[kKk] - 120 * K5;
+    case 6: {
+      const u64 paw = s[kVtd] - 6 * T - 4 * (D - 6 * K4) - 12 * K4;
+      return 2 * paw + 2 * s[kEdart] - 4 * gem + 8 * s[kW4] - 2 * kd + 10 * ka - 12 * s[kC3] -
+             48 * s[kKk] + 120 * K5;
+    }
+    case 7: return 2 * s[kC3] - ka + 6 * s[kKk] - 20 * K5;
+    default: return kd - 3 * ka + 18 * s[kKk] - 60 * K5;
+  }
+}
+
+unsigned blocks(int64_t items, int per_block) {
+  return (unsigned)std::max<int64_t>(1, (items + per_block - 1) / per_block);
+}
+
+int resident(const void *kernel, int threads, size_t smem) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess)
+    per_sm = 1;
+  return std::max(per_sm, 1);
+}
+
+// Carves aligned arrays out of one allocation.
+struct Carver {
+  char *base = nullptr;
+  size_t used = 0;
+  template <typename T>
+  T *take(int64_t count) {
+    T *p = reinterpret_cast<T *>(base + used);
+    used += (sizeof(T) * (size_t)std::max<int64_t>(count, 1) + 255) & ~size_t(255);
+    return p;
+  }
+};
+
+// The pairs stage's classes that walks up to `longest` reach.
+template <bool kOrdered>
+int launch_pairs(mc_dgraph *g, const MotifArgs &a, int64_t longest, int big_grid, bool shared,
+                 size_t table_b, unsigned *counters) {
+  cudaStream_t s = g->stream;
+  auto launch = [&](auto kern, int threads, size_t smem, int64_t items) -> int {
+    MC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int64_t fit = (int64_t)g->num_sms * resident((const void *)kern, threads, smem);
+    kern<<<(unsigned)std::max<int64_t>(1, std::min(items, fit)), threads, smem, s>>>(a);
+    MC_CUDA_TRY(cudaGetLastError());
+    g->launches += 1;
+    return MC_OK;
+  };
+  int rc = launch(motif_pairs_kernel<kOrdered>, kThreads, kWarps * hash_bytes(kHashSlots),
+                  blocks(a.n, kWarps));
+  if (rc == MC_OK && longest > (int64_t)kWarpWalk && a.mid_walk > kWarpWalk)
+    rc = launch(motif_pairs_hash_kernel<kOrdered, true, 128, 12>, 128, hash_bytes(1 << 12), a.n);
+  if (rc == MC_OK && longest > (int64_t)a.mid_walk)
+    rc = launch(motif_pairs_hash_kernel<kOrdered, false, 512, 14>, 512, hash_bytes(1 << 14), a.n);
+  if (rc != MC_OK || longest <= (int64_t)kHashWalk) return rc;
+  auto big = shared ? motif_pairs_big_kernel<kOrdered, true> : motif_pairs_big_kernel<kOrdered, false>;
+  const size_t smem = shared ? table_b : 0;
+  MC_CUDA_TRY(cudaFuncSetAttribute(big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  big<<<big_grid, kPairThreads, smem, s>>>(a, counters);
+  MC_CUDA_TRY(cudaGetLastError());
+  g->launches += 1;
+  return MC_OK;
+}
+
+}  // namespace
+
+// Whether a whole count of this graph takes this route: not above the degree
+// at which the reference's 32-bit products could wrap (its counts are then no
+// subgraph counts), not with columns in host memory (the pairs stage reads
+// rows once per two-path), and not when the environment asks for another
+// route or its forms.
+bool motif_route(const mc_dgraph *g) {
+  if (g->n == 0 || g->nnz == 0 || g->batch.gid || g->col_host) return false;
+  if (g->max_degree > 46340 || g->nnz > (int64_t(1) << 30)) return false;
+  if (const char *env = std::getenv("MERCURY_MOTIF_ROUTE"))
+    if (std::atoi(env) == 0) return false;
+  for (const char *name : {"MERCURY_PATTERN_KERNEL", "MERCURY_CLIQUE_ROUTE", "MERCURY_PATTERN_SETS",
+                           "MERCURY_PATTERN_SLICE", "MERCURY_HUB_P1", "MERCURY_HOP_ROWS"})
+    if (std::getenv(name)) return false;
+  return true;
+}
+
+int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
+  NvtxRange range("motif_count");
+  cudaStream_t s = g->stream;
+  const int n = (int)g->n, nnz = (int)g->nnz;
+  const unsigned need = needs_of(pattern);
+  const bool pairs = need & (kNeedC4 | kNeedPairs), ordered = need & kNeedC4;
+  const bool wheel = need & kNeedW4;
+  // Shared-memory tables of the pairs stage: 16 bits per vertex.
+  const size_t table_b = sizeof(unsigned) * (size_t)((n + 1) / 2);
+  const bool table_shared = table_b <= (size_t(200) << 10);
+  const int pair_grid = table_shared ? g->num_sms
+                                     : (int)std::max<int64_t>(
+                                           1, std::min<int64_t>(2 * g->num_sms,
+                                                                (int64_t(2) << 30) / (int64_t)table_b));
+  // A vertex's walk is at most the entries of its neighbours' rows.  Where no
+  // walk exceeds the second hash class, that class takes the first's as well.
+  const int64_t longest = std::min<int64_t>(nnz, g->max_degree * g->max_degree);
+  const u64 mid_walk = longest <= (int64_t)kHashWalk ? kWarpWalk : kMidWalk;
+  const int64_t root = (int64_t)std::sqrt((double)nnz) + 1;
+  const int64_t slice_words = (2 * (int64_t)nnz + 64 * root) / 32 + 64;
+  const bool slices = slice_words * 4 > kTauSmem;
+  const int tau_grid = (int)std::max<int64_t>(
+      1, std::min<int64_t>(2 * g->num_sms, slices ? (int64_t(1) << 30) / (4 * slice_words) : 1 << 20));
+  int64_t list_cap = std::max<int64_t>(int64_t(16) << 20, 4 * (int64_t)nnz);
+  for (;;) {
+    MotifArgs a{};
+    a.rp = g->rowptr;
+    a.ci = g->col;
+    a.n = n;
+    a.nnz = nnz;
+    a.need = need;
+    a.list_cap = list_cap;
+    a.slice_words = slice_words;
+    a.mid_walk = mid_walk;
+    void *temp = nullptr;
+    unsigned *counters = nullptr;
+    size_t zeroed = 0;
+    auto lay_out = [&](Carver &c) {
+      // Zeroed before the first kernel.
+      a.acc = c.take<u64>(kSums);
+      a.counts = c.take<unsigned>(kCounts);
+      a.dp = c.take<int32_t>(n);
+      a.tv2 = c.take<int32_t>(need & kNeedT ? n : 0);
+      a.d2 = c.take<u64>(need & kNeedD2 ? n : 0);
+      a.walk = c.take<u64>(pairs ? n : 0);
+      a.rev1 = c.take<int32_t>(nnz);
+      a.a = c.take<int32_t>(nnz);
+      a.cur = c.take<int32_t>(nnz);
+      zeroed = c.used;
+      a.deg = c.take<int32_t>(n);
+      a.src = c.take<int32_t>(nnz);
+      a.upe = c.take<int32_t>(nnz);
+      a.pos1 = c.take<int32_t>(nnz);
+      a.off = c.take<int64_t>((int64_t)nnz + 1);
+      a.tau_big = c.take<int32_t>(n);
+      a.pair_mid = c.take<int32_t>(pairs ? n : 0);
+      a.pair_big = c.take<int32_t>(pairs ? n : 0);
+      temp = c.take<char>((int64_t)scan_temp_bytes(nnz));
+      a.slices = c.take<unsigned>(slices ? tau_grid * slice_words : 0);
+      counters = c.take<unsigned>(pairs && !table_shared ? pair_grid * (int64_t)(table_b / 4) : 0);
+      a.list = c.take<int32_t>(list_cap);
+    };
+    Carver size;
+    lay_out(size);
+    Carver c;
+    // Large scratch leaves half of the free memory alone; the caller then
+    // takes a formula route, as it does when the allocation fails.
+    if (size.used > size_t(1) << 30) {
+      size_t free_b = 0, total_b = 0;
+      MC_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+      if (size.used > free_b / 2) return MC_ERR_OOM;
+    }
+    MC_CUDA_TRY(dev_alloc(reinterpret_cast<void **>(&c.base), size.used, s));
+    lay_out(c);
+    u64 h[kSums];
+    int64_t total = 0;
+    auto run = [&]() -> int {
+      MC_CUDA_TRY(cudaMemsetAsync(c.base, 0, zeroed, s));
+      motif_rows_kernel<<<std::min(blocks(n, kWarps), 4096u), kThreads, 0, s>>>(a);
+      MC_CUDA_TRY(cudaGetLastError());
+      motif_up_kernel<<<blocks(nnz, kThreads), kThreads, 0, s>>>(a);
+      MC_CUDA_TRY(cudaGetLastError());
+      motif_tri_kernel<false><<<blocks(nnz, kThreads), kThreads, 0, s>>>(a);
+      MC_CUDA_TRY(cudaGetLastError());
+      MC_CUDA_TRY(exclusive_scan(a.a, a.off, nnz, temp, s));
+      motif_tri_kernel<true><<<blocks(std::max(n, nnz), kThreads), kThreads, 0, s>>>(a);
+      MC_CUDA_TRY(cudaGetLastError());
+      g->launches += 4 + scan_launches(nnz);
+      motif_tau_kernel<<<std::min(blocks(n, kWarps), (unsigned)(8 * g->num_sms)), kThreads, 0, s>>>(a);
+      MC_CUDA_TRY(cudaGetLastError());
+      MC_CUDA_TRY(cudaFuncSetAttribute(motif_tau_big_kernel,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kTauSmem));
+      motif_tau_big_kernel<<<tau_grid, kThreads, kTauSmem, s>>>(a, kTauSmem / 4);
+      MC_CUDA_TRY(cudaGetLastError());
+      g->launches += 2;
+      if (pairs) {
+        const int rcp = ordered ? launch_pairs<true>(g, a, longest, pair_grid, table_shared, table_b, counters)
+                                : launch_pairs<false>(g, a, longest, pair_grid, table_shared, table_b, counters);
+        if (rcp != MC_OK) return rcp;
+      }
+      if (wheel) {
+        motif_wheel_kernel<<<std::min(blocks(nnz, kThreads), (unsigned)(8 * g->num_sms)), kThreads, 0,
+                             s>>>(a);
+        MC_CUDA_TRY(cudaGetLastError());
+        g->launches += 1;
+        if (g->max_degree > kWheelDeg) {
+          const int table = (int)g->max_degree;
+          const size_t smem = sizeof(unsigned) * (size_t)table;
+          MC_CUDA_TRY(cudaFuncSetAttribute(motif_wheel_big_kernel,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+          const int per_sm = resident((const void *)motif_wheel_big_kernel, kThreads, smem);
+          motif_wheel_big_kernel<<<std::min(blocks(nnz, kThreads), (unsigned)(per_sm * g->num_sms)),
+                                   kThreads, smem, s>>>(a, table);
+          MC_CUDA_TRY(cudaGetLastError());
+          g->launches += 1;
+        }
+      }
+      MC_CUDA_TRY(cudaEventRecord(g->ev[3], s));
+      MC_CUDA_TRY(cudaMemcpyAsync(h, a.acc, sizeof(h), cudaMemcpyDeviceToHost, s));
+      MC_CUDA_TRY(cudaMemcpyAsync(&total, a.off + nnz, sizeof(total), cudaMemcpyDeviceToHost, s));
+      MC_CUDA_TRY(cudaStreamSynchronize(s));
+      return MC_OK;
+    };
+    const int rc = run();
+    dev_free(c.base, s);
+    if (rc != MC_OK) return rc;
+    if (total <= list_cap) {
+      *out = combine(pattern, h);
+      return MC_OK;
+    }
+    list_cap = total;  // more triangles than the first guess: once more, sized
+  }
+}
+
+}  // namespace mc

@@ -2165,6 +2165,27 @@ int pattern_count_body(mc_dgraph *g, int pattern, uint64_t *out, uint64_t *c12,
                        double *progress) {
   NvtxRange range("pattern_count");
   if (pattern < 1 || pattern > 8) return MC_ERR_ARG;
+  // Whole counts without a budget: motif sums (motifs.cu).  A shard's partial
+  // count, a budget's slices and the two counters stay with the routes below.
+  if (num_shards == 1 && budget_ms <= 0 && !c12 && motif_route(g)) {
+    const int64_t launches = g->launches;
+    MC_CUDA_TRY(cudaEventRecord(g->ev[0], g->stream));
+    const int rc = motif_count(g, pattern, out);
+    if (rc != MC_OK && rc != MC_ERR_OOM) return rc;
+    if (rc == MC_OK) {
+      if (progress) *progress = 1.0;
+      if (timing) {
+        std::memset(timing, 0, sizeof(*timing));
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, g->ev[0], g->ev[3]);
+        timing->count_ms = ms;
+        timing->total_ms = ms;
+        timing->launches = g->launches - launches;
+      }
+      return MC_OK;
+    }
+    cudaGetLastError();  // a failed allocation: the routes below need less scratch
+  }
   // P7 and P8 on graphs with hubs: by clique counts over the degree-ordered
   // DAG (cliques.cu), which is built first; its time counts as the pattern's.
   bool cliques = false;

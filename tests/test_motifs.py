@@ -1,0 +1,150 @@
+"""P1..P8 from motif sums (mercury_b200/csrc/motifs.cu).
+
+CPU: the identities themselves -- every pattern as a signed combination of
+sums over vertices, edges, triangles and vertex pairs -- restated in Python
+and checked against the oracle's counts.  GPU: the route at the sizes where
+its stages change form, against the oracle and against the formula routes.
+"""
+import math
+
+import numpy as np
+import pytest
+
+from brute import random_graph
+from conftest import csr_from_edges
+from mercury_b200 import DeviceGraph, Graph
+from oracle import oracle as orc
+
+
+def motif_sums(rp, col):
+    n = len(rp) - 1
+    N = [set(int(x) for x in col[rp[v]:rp[v + 1]]) for v in range(n)]
+    d = [len(s) for s in N]
+    a = {(u, v): len(N[u] & N[v]) for u in range(n) for v in N[u]}
+    t = [sum(a[v, x] for x in N[v]) // 2 for v in range(n)]
+    d2 = [sum(d[p] - 1 for p in N[v]) for v in range(n)]
+    C = math.comb
+    s = dict.fromkeys("d3 d4 t2 td D C3 p4 fork dart T cricket bull lolli kite gem kd ka kk "
+                      "K4 K5 C4 C4d C4a X7 W4 K23".split(), 0)
+    for v in range(n):
+        s["d3"] += C(d[v], 3)
+        s["d4"] += C(d[v], 4)
+        s["t2"] += C(t[v], 2)
+        s["td"] += t[v] * d[v]
+    for (u, v), x in a.items():
+        if u > v:
+            continue
+        s["D"] += C(x, 2)
+        s["C3"] += C(x, 3)
+        s["p4"] += (d[u] - 1 - x) * (d[v] - 1 - x)
+        s["fork"] += (C(d[u] - 1, 2) * (d[v] - 1) + C(d[v] - 1, 2) * (d[u] - 1)
+                      - x * (d[u] + d[v] - 4))
+        s["dart"] += C(x, 2) * (d[u] + d[v] - 6)
+        for z in (N[u] & N[v]):
+            if z < v:
+                continue
+            S = N[u] & N[v] & N[z]
+            k = len(S)
+            dd, aa = (d[u], d[v], d[z]), (a[v, z], a[u, z], a[u, v])  # aa[i] opposite dd[i]
+            s["T"] += 1
+            s["cricket"] += sum(C(q - 2, 2) for q in dd)
+            s["bull"] += sum((dd[i] - 2) * (dd[i - 1] - 2) for i in range(3)) - sum(aa) + 3
+            s["lolli"] += d2[u] + d2[v] + d2[z] - 2 * (sum(dd) - 3) - 2 * (sum(aa) - 3)
+            s["kite"] += sum((aa[i] - 1) * (dd[i] - 2) for i in range(3))
+            s["gem"] += sum((aa[i] - 1) * (aa[i - 1] - 1) for i in range(3))
+            s["kd"] += k * sum(dd)
+            s["ka"] += k * sum(aa)
+            s["kk"] += C(k, 2)
+            for w in (x for x in S if x > z):
+                s["K4"] += 1
+                s["K5"] += sum(1 for y in S & N[w] if y > w)
+    for x in range(n):
+        for y in range(x):
+            S = N[x] & N[y]
+            c = len(S)
+            s["C4"] += C(c, 2)  # twice the 4-cycles, as are C4d and C4a
+            s["K23"] += C(c, 3)
+            s["C4d"] += C(c, 2) * (d[x] + d[y]) + sum((c - 1) * d[v] for v in S)
+            s["C4a"] += sum((c - 1) * (a[x, v] + a[v, y]) for v in S)
+            s["X7"] += sum((c - 2) * len(N[p] & S) for p in S)
+            s["W4"] += sum(C(len(N[v] & S), 2) for v in S)
+    s["X7"] //= 2
+    s["W4"] //= 2
+    return s
+
+
+def counts(s):
+    ka, kd = s["ka"] - 24 * s["K4"], s["kd"] - 36 * s["K4"]
+    gem, kite = s["gem"] - 12 * s["K4"], s["kite"] - 12 * s["K4"]
+    claw = s["d3"] - s["td"] + 6 * s["T"] + 2 * s["D"] - 4 * s["K4"]
+    butterfly = s["t2"] - 2 * s["D"]
+    house2, banner2 = s["C4a"] - 8 * s["D"], s["C4d"] - 8 * s["C4"] - 4 * s["D"]
+    paw = s["td"] - 6 * s["T"] - 4 * (s["D"] - 6 * s["K4"]) - 12 * s["K4"]
+    star = (s["d4"] - s["cricket"] + s["dart"] + butterfly - gem + s["W4"] - kd // 3 + ka
+            - 2 * s["C3"] - 3 * s["kk"] + 5 * s["K5"])
+    return [
+        claw,
+        s["fork"] - 2 * s["cricket"] - 2 * s["bull"] - s["lolli"] - banner2 + 6 * s["K23"]
+        + 5 * s["dart"] + 4 * kite + 2 * house2 + 4 * butterfly - 10 * gem - 10 * s["X7"]
+        + 20 * s["W4"] - 3 * kd + 10 * ka - 12 * s["C3"] - 36 * s["kk"] + 60 * s["K5"],
+        4 * star + 3 * claw,
+        s["p4"] - 2 * s["C4"] + 4 * s["D"] - 12 * s["K4"],
+        2 * s["bull"] - 4 * s["dart"] - 4 * kite - house2 + 10 * gem + 8 * s["X7"] - 24 * s["W4"]
+        + 4 * kd - 14 * ka + 12 * s["C3"] + 60 * s["kk"] - 120 * s["K5"],
+        2 * paw + 2 * s["dart"] - 4 * gem + 8 * s["W4"] - 2 * kd + 10 * ka - 12 * s["C3"]
+        - 48 * s["kk"] + 120 * s["K5"],
+        2 * s["C3"] - ka + 6 * s["kk"] - 20 * s["K5"],
+        kd - 3 * ka + 18 * s["kk"] - 60 * s["K5"],
+    ]
+
+
+@pytest.mark.parametrize("n,p,seed", [(6, 1.0, 0), (12, 0.3, 1), (16, 0.5, 2), (14, 0.8, 3),
+                                      (25, 0.6, 4), (40, 0.1, 5), (30, 0.25, 6)])
+def test_identities_give_the_oracle_counts(n, p, seed):
+    rp, col = csr_from_edges(n, random_graph(n, p, seed))
+    assert counts(motif_sums(rp, col)) == [orc.pattern(rp, col, k) for k in range(1, 9)]
+
+
+def gpu_counts(rp, col):
+    with DeviceGraph(rp, col) as d:
+        return [d.pattern_count(k) for k in range(1, 9)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,p,seed", [
+    (1, 0.0, 0), (2, 1.0, 0), (3, 1.0, 0), (4, 1.0, 0), (5, 1.0, 0), (6, 0.0, 0),
+    (33, 1.0, 0), (34, 1.0, 0),    # d+ of 32 (one warp's rows) and of 33
+    (65, 1.0, 0), (70, 0.9, 1), (100, 0.3, 2), (180, 0.5, 3), (300, 0.02, 4)])
+def test_motif_route_vs_oracle(n, p, seed):
+    rp, col = csr_from_edges(n, random_graph(n, p, seed))
+    assert gpu_counts(rp, col) == [orc.pattern(rp, col, k) for k in range(1, 9)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("make", [
+    # Pair tables of every class (walks below 512 to above 32,768), degrees on
+    # both sides of 512; tables over all vertices in shared memory.
+    lambda: Graph.chung_lu(30001, 2.1, 12.0, 900.0, seed=7),
+    # More vertices than the shared tables hold.
+    lambda: Graph.chung_lu(150001, 2.1, 6.0, 3000.0, seed=3),
+    lambda: Graph.rmat(11, 16, seed=5),
+], ids=["classes", "global_tables", "rmat11"])
+def test_motif_route_equals_formula_routes(monkeypatch, make):
+    g = make()
+    with DeviceGraph(g) as d:
+        motif = [d.pattern_count(k) for k in range(1, 9)]
+        monkeypatch.setenv("MERCURY_MOTIF_ROUTE", "0")
+        assert motif == [d.pattern_count(k) for k in range(1, 9)]
+
+
+@pytest.mark.gpu
+def test_motif_route_sizes_its_lists_again():
+    """More common-neighbour entries (six per triangle) than the first guess
+    of 16 M: the count starts over with room for all.  A clique of n with one
+    vertex hung on vertex 0 holds C(n - 1, 2) induced paws and C(n - 1, 3)
+    induced tailed K4s, and none of the other subgraphs."""
+    n = 300  # 4,455,100 triangles, 26.7 M entries
+    rp, col = csr_from_edges(n + 1, [(i, j) for i in range(n) for j in range(i)] + [(0, n)])
+    want = [0] * 8
+    want[5], want[7] = 2 * math.comb(n - 1, 2), 3 * math.comb(n - 1, 3)
+    assert gpu_counts(rp, col) == want
