@@ -164,11 +164,25 @@ int tc_orient(mc_dgraph *g, const int32_t *upload = nullptr);
 int clique_prepare(mc_dgraph *g, int pattern, bool *use, int64_t *dag_edges);
 int clique_launch(mc_dgraph *g, int pattern, int64_t dag_edges, int shard, int num_shards,
                   const unsigned long long *deadline, unsigned long long *stop_flag);
-// P1..P8 from motif sums (motifs.cu): whether a whole count of g takes that
-// route, and the count (synchronous; event ev[3] marks its last kernel).
-// MC_ERR_OOM when its scratch does not fit: the formula routes need less.
-bool motif_route(const mc_dgraph *g);
+// P1..P8 from motif sums: over sparse stages (motifs.cu) or, for graphs of at
+// most kDenseMax vertices, from bit rows in shared memory (dense.cu).  The
+// counts are synchronous; event ev[3] marks their last kernel.  motif_count
+// returns MC_ERR_OOM when its scratch does not fit: the formula routes need
+// less.
+enum class PatternRoute { kFormula, kDense, kSparse };
+PatternRoute pattern_route(const mc_dgraph *g, int pattern);
+constexpr int kDenseMax = 1024;
 int motif_count(mc_dgraph *g, int pattern, uint64_t *out);
+int dense_count(mc_dgraph *g, int pattern, uint64_t *out);
+// Part `part` of `parts` of one pattern graph of a batch.
+struct DenseTask {
+  int64_t v0;
+  int n, graph, job, part, parts;
+};
+// acc: the motif sums of every batch graph (zeroed by the caller); largest:
+// the most vertices among the tasks' graphs.
+int dense_batch_launch(const int64_t *rp, const int32_t *ci, const DenseTask *tasks, int num_tasks,
+                       int largest, unsigned long long *acc, cudaStream_t s);
 // Contract checks of the row offsets alone; sets max_degree.
 int validate_rowptr(mc_dgraph *g);
 int tc_partner_stats(mc_dgraph *g, unsigned long long *partner_edges, unsigned long long *work);

@@ -22,21 +22,21 @@
 // graph of 100,000 vertices (mean 10, cap 200: m = 498,340, 84 k triangles,
 // 429 k triangle pairs on an edge, 81 M two-paths) the per-edge formulas
 // took P1..P8 1.9, 28.0, 9.7, 4.8, 11.1, 3.6, 0.95 and 3.6 ms per call on a
-// B200, and these sums take 0.36, 1.82, 0.46, 0.82, 1.74, 0.46, 0.37 and 0.37.
+// B200, and these sums take 0.28, 1.37, 0.39, 0.76, 1.25, 0.38, 0.31 and 0.31.
 // On the one of 60,000 (mean 20, cap 50,000, a hub of degree 17,215) P1, P4,
-// P7 and P8 took 74.7, 276, 25.9 and 26.1 ms, and take 0.94, 2.7, 1.5 and 1.5.
+// P7 and P8 took 74.7, 276, 25.9 and 26.1 ms, and take 0.82, 2.6, 1.3 and 1.3.
+// There the pairs of P2 and P5 take 0.24 s (544 M two-paths).
 //
 // Stages (each vertex pair ordered by (degree, id), written u < v below; an
 // "up" entry of the CSR is one with u < v):
 //   rows    entry -> row, degrees
 //   up      N+(u): the up entries of each row, compacted in place; the
-//           reverse entry of each edge
-//   tri     a of each entry: every pair (x, y) of N+(u) tested once in the
-//           row of the lower of the two, so sum of C(d+, 2) searches
-//   lists   per entry (u -> v) the entries (u -> w) of its common neighbours
-//           w, slot j of (u -> v) and slot j of (v -> u) holding the same w;
-//           edge and vertex sums
-//   tau     per u, bit rows of its up neighbours over N(u) and over N+(u):
+//           reverse entry of each edge; room for the edge's two lists below
+//   tri     every pair (x, y) of N+(u) tested once in the row of the lower of
+//           the two (sum of C(d+, 2) searches): a of each entry, and per entry
+//           (u -> v) a list of the entries (u -> w) of its common neighbours
+//           w, slot j of (u -> v) and slot j of (v -> u) holding the same w
+//   tau     edge sums; per u, bit rows of its up neighbours over N(u) and over N+(u):
 //           k is a popcount of two rows, K4 and K5 of two and three
 //   pairs   common neighbours c of pairs (s, t), counted per s in a table
 //           over t: C4, K2,3, X7
@@ -48,48 +48,15 @@
 
 #include "device_common.cuh"
 #include "dgraph.cuh"
-#include "scan.cuh"
+#include "motifs.cuh"
 
 namespace mc {
 namespace {
-
-using u64 = unsigned long long;
-
-// Sums over the graph, modulo 2^64.
-enum Sum : int {
-  kVd3, kVd4, kVt2, kVtd,                  // vertices: C(d,3), C(d,4), C(t,2), t d
-  kD, kC3, kEp4, kEfork, kEdart,           // edges
-  kT, kCricket, kBull, kLolli, kKite, kGem,  // triangles
-  kKd, kKa, kKk, kK4, kK5,                 // with common neighbours; cliques
-  kC4, kC4d, kC4a, kX7, kW4, kK23,         // 4-cycles and beyond
-  kSums
-};
 
 // Words of MotifArgs::counts: list lengths, then queue positions.
 enum Count : int {
   kTauN, kMidN, kHashN, kHugeN, kBigN, kTauQueue, kMidQueue, kHashQueue, kBigQueue, kCounts
 };
-
-// What a pattern needs beyond a and the vertex and edge sums.
-enum Need : unsigned {
-  kNeedTau = 1u,    // triangle sums with k (else K4 alone)
-  kNeedD2 = 2u,     // sum of (d - 1) over each neighbourhood
-  kNeedT = 4u,      // C(t, 2) over the triangles per vertex
-  kNeedC4 = 8u,     // 4-cycles, each counted at its highest vertex
-  kNeedPairs = 16u, // every pair's common neighbours (C4 counted twice)
-  kNeedW4 = 32u,
-  kNeedK23 = 64u,   // with kNeedPairs: K2,3 and degrees on 4-cycles
-};
-
-__host__ __device__ constexpr unsigned needs_of(int pattern) {
-  return pattern == 1   ? 0u
-         : pattern == 2 ? kNeedTau | kNeedD2 | kNeedT | kNeedPairs | kNeedW4 | kNeedK23
-         : pattern == 3 ? kNeedTau | kNeedT | kNeedW4
-         : pattern == 4 ? kNeedC4
-         : pattern == 5 ? kNeedTau | kNeedPairs | kNeedW4
-         : pattern == 6 ? kNeedTau | kNeedW4
-                        : (unsigned)kNeedTau;
-}
 
 struct MotifArgs {
   const int64_t *__restrict__ rp;
@@ -105,18 +72,19 @@ struct MotifArgs {
   int32_t *upe;    // nnz: rp[u] + i -> i-th up entry of u
   int32_t *pos1;   // nnz: 1 + position in N+(row) of an up entry, else 0
   int32_t *rev1;   // nnz: 1 + reverse entry, 0 if there is none
-  int32_t *a;      // nnz: triangles on the entry's edge
-  int32_t *cur;    // nnz: list slots taken, at the up entry
-  int64_t *off;    // nnz + 1: list offsets
+  int32_t *a;      // nnz: triangles on the entry's edge = length of its list
+  int32_t *cnt;    // nnz: the same at the up entry, counted ahead (null: not)
+  int64_t *off;    // nnz: list offsets
   int32_t *list;   // common-neighbour lists
   int64_t list_cap;
+  u64 *pool;       // list entries handed out (above list_cap: all later stages stop)
   u64 *acc;        // kSums
   // Vertices too large for one warp.  pair_mid: the two hash classes, from the
   // front and from the back of its n entries; pair_big: tables over all
   // vertices, the longest walks from the front, so that they start first.
   int32_t *tau_big, *pair_mid, *pair_big;
   unsigned *counts;  // see Count
-  u64 mid_walk;      // pair_mid's front class ends here (kWarpWalk: none in it)
+  u64 warp_walk, mid_walk;  // where the warp class and pair_mid's front class end
   unsigned *slices;  // bit rows of the tau stage that exceed shared memory
   int64_t slice_words;
 };
@@ -126,25 +94,19 @@ constexpr int kWarps = kThreads / kWarp;
 constexpr int kTauOut = 32;       // warp form of the tau stage: d+ and d at most
 constexpr int kTauDeg = 512;
 constexpr int kTauSmem = 96 << 10;  // bit rows of a CTA, two CTAs per SM
+constexpr int kTauBoth = 8 << 10;   // up to here the two forms share a launch
 // Classes of the pairs stage by table entries visited (a vertex's walk bounds
 // the keys of its table, which has at least twice as many slots): a warp, a
 // CTA of 128 and of 512 threads with a hash table, and a CTA of 1,024 with a
 // counter for every vertex.  With warps and 1,024-thread CTAs alone the stage
 // took 6.2 ms in P2 on the graph of 100,000 (one CTA per SM, three barriers
-// per vertex of some 1,000 entries); with the four classes it takes 1.4 ms.
+// per vertex of some 1,000 entries); with the four classes it takes 1.1 ms.
 constexpr u64 kWarpWalk = 512, kMidWalk = 2048, kHashWalk = 8192;
 constexpr u64 kHugeWalk = 1 << 15;
+constexpr u64 kFewWalk = 64;
+constexpr int kFewVertices = 16384;
 constexpr int kHashSlots = 1024;  // of a warp
 constexpr int kWheelDeg = 512;    // warp form of the wheel stage
-
-__device__ __forceinline__ u64 c2(u64 x) { return x * (x - 1) / 2; }  // 0 at 0 and 1
-__device__ __forceinline__ u64 c3(long long x) {
-  return x < 3 ? 0ull : (u64)x * (u64)(x - 1) / 2 * (u64)(x - 2) / 3;
-}
-// C(x, 4) below 2^64 for x up to 46,341: C(x, 3) (x - 3) is at most 8e17.
-__device__ __forceinline__ u64 c4(long long x) {
-  return x < 4 ? 0ull : c3(x) * (u64)(x - 3) / 4;
-}
 
 // (degree, id) order.
 __device__ __forceinline__ bool lower(int du, int u, int dv, int v) {
@@ -163,30 +125,11 @@ __device__ __forceinline__ int find_entry(const int32_t *__restrict__ ci, int b,
   return -1;
 }
 
-// Per-block totals of the sums a kernel adds to.
-struct BlockSums {
-  u64 *s;
-  __device__ __forceinline__ void init() const {
-    for (int i = threadIdx.x; i < kSums; i += blockDim.x) s[i] = 0;
-    __syncthreads();
-  }
-  // Every lane of the warp takes part.
-  __device__ __forceinline__ void add(int which, u64 v) const {
-    v = warp_sum_u64(v);
-    if ((threadIdx.x & (kWarp - 1)) == 0 && v) atomicAdd(s + which, v);
-  }
-  __device__ __forceinline__ void flush(u64 *acc) const {
-    __syncthreads();
-    for (int i = threadIdx.x; i < kSums; i += blockDim.x)
-      if (s[i]) atomicAdd(acc + i, s[i]);
-  }
-};
-
 // The warp's 32 lists laid end to end: flat position f belongs to list l (the
 // first whose inclusive end exceeds f) at offset f - excl(l).
 struct FlatLists {
   int incl, total;
-  __device__ __forceinline__ FlatLists(int len, int lane) {
+  __device__ __forceinline__ FlatLists(int len, int lane) {  // every lane calls it
     incl = warp_inclusive_scan(len, lane);
     total = __shfl_sync(kFull, incl, kWarp - 1);
   }
@@ -199,6 +142,42 @@ struct FlatLists {
     return min(l, kWarp - 1);
   }
 };
+
+// Calls f(entry, owner lane, place) for the entries of this warp's 32 lists
+// [lo, lo + len) of a.list, flat.
+template <class F>
+__device__ __forceinline__ void walk_lists(const MotifArgs &a, int64_t lo, int len, int lane, F f) {
+  const FlatLists fl(len, lane);
+  const int64_t start = lo - (fl.incl - len);
+  for (int base = 0; base < fl.total; base += kWarp) {
+    const int g = base + lane;
+    const int l = fl.owner(g);
+    const int64_t at = __shfl_sync(kFull, start, l) + g;
+    if (g < fl.total) f(a.list[at], l, at);
+  }
+}
+
+__device__ __forceinline__ bool lists_overrun(const MotifArgs &a) {
+  return *a.pool > (u64)a.list_cap;
+}
+
+// Offsets of the lists of this lane's up entry e and its reverse, `len` entries
+// each (0: none); one atomic per warp.
+__device__ __forceinline__ void take_lists(const MotifArgs &a, int e, int r, int len, int lane) {
+  u64 incl = 2 * (u64)len;
+#pragma unroll
+  for (int o = 1; o < kWarp; o <<= 1) {
+    const u64 x = __shfl_up_sync(kFull, incl, o);
+    if (lane >= o) incl += x;
+  }
+  u64 base = 0;
+  if (lane == kWarp - 1 && incl) base = atomicAdd(a.pool, incl);
+  base = __shfl_sync(kFull, base, kWarp - 1);
+  if (len > 0) {
+    a.off[e] = (int64_t)(base + incl - 2 * (u64)len);
+    a.off[r] = (int64_t)(base + incl - (u64)len);
+  }
+}
 
 // ---- rows, up ---------------------------------------------------------------
 // Warp per row: src, deg, and the sums of degrees alone.
@@ -272,65 +251,56 @@ __global__ void __launch_bounds__(kThreads) motif_up_kernel(MotifArgs a) {
   } else if (in) {
     a.pos1[e] = 0;  // a down entry, or one with no reverse, which the up lists leave out
   }
+  // Without counts: u's other neighbours bound the list.
+  if (!a.cnt) take_lists(a, e, r, up ? du - 1 : 0, lane);
+}
+
+// With counts: exactly sized lists.
+__global__ void __launch_bounds__(kThreads) motif_lists_kernel(MotifArgs a) {
+  const int64_t e64 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  const int e = (int)(e64 < a.nnz ? e64 : 0);
+  const bool up = e64 < a.nnz && a.pos1[e];
+  take_lists(a, e, up ? a.rev1[e] - 1 : 0, up ? a.cnt[e] : 0, threadIdx.x & (kWarp - 1));
 }
 
 // ---- triangles --------------------------------------------------------------
-// A warp takes 32 consecutive slots of the compacted up lists; slot i of N+(u)
-// pairs with the later slots, and the pairs of all 32 are walked flat.
-// kFill: the counts are known and the lists are written; the edge and vertex
-// sums are added on the way.
-template <bool kFill>
-__global__ void __launch_bounds__(kThreads) motif_tri_kernel(MotifArgs a) {
+// A warp takes `per` consecutive slots of the compacted up lists (32, fewer
+// on graphs that would leave warps idle: see spread()); slot i of N+(u) pairs
+// with the later slots, and the pairs of all of them are walked flat.
+// kCount: the list lengths alone.  Otherwise the lists, and the vertices of
+// the later stages' classes.
+template <bool kCount>
+__global__ void __launch_bounds__(kThreads) motif_tri_kernel(MotifArgs a, int per) {
   __shared__ u64 sm[kSums];
   const BlockSums bs{sm};
   bs.init();
   const int lane = threadIdx.x & (kWarp - 1);
-  if (kFill && a.off[a.nnz] > a.list_cap) return;  // the host sizes the lists and starts over
+  if (!kCount && lists_overrun(a)) return;  // the host makes room and starts over
   const int64_t s64 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (kFill && s64 < a.n) {
+  if (!kCount && s64 < a.n) {
     const int v = (int)s64;
     const int d = a.deg[v], p = a.dp[v];
-    if (p >= 2 && (p > kTauOut || d > kTauDeg)) a.tau_big[atomicAdd(a.counts + kTauN, 1u)] = v;
+    if (p > kTauOut || (p >= 2 && d > kTauDeg)) a.tau_big[atomicAdd(a.counts + kTauN, 1u)] = v;
     if (a.need & (kNeedC4 | kNeedPairs)) {
       const u64 w = a.walk[v];
       if (w > kHugeWalk) a.pair_big[atomicAdd(a.counts + kHugeN, 1u)] = v;
       else if (w > kHashWalk) a.pair_big[a.n - 1 - atomicAdd(a.counts + kBigN, 1u)] = v;
       else if (w > a.mid_walk) a.pair_mid[a.n - 1 - atomicAdd(a.counts + kHashN, 1u)] = v;
-      else if (w > kWarpWalk) a.pair_mid[atomicAdd(a.counts + kMidN, 1u)] = v;
+      else if (w > a.warp_walk) a.pair_mid[atomicAdd(a.counts + kMidN, 1u)] = v;
     }
   }
-  if (kFill && (a.need & kNeedT)) {
-    // Triangles per vertex from a: one atomic per (row, warp) piece.
-    const int v = s64 < a.nnz ? a.src[s64] : -1;
-    int sum = s64 < a.nnz ? a.a[s64] : 0;
-#pragma unroll
-    for (int o = 1; o < kWarp; o <<= 1) {
-      const int other = __shfl_up_sync(kFull, sum, o), ov = __shfl_up_sync(kFull, v, o);
-      if (lane >= o && ov == v) sum += other;
-    }
-    const int next = __shfl_down_sync(kFull, v, 1);
-    if (v >= 0 && sum && (lane == kWarp - 1 || next != v)) atomicAdd(a.tv2 + v, sum);
-  }
-  int slot = 0, len = 0, e_ux = 0, x = 0, dx = 0, i0 = 0;
-  u64 D = 0, C3 = 0, p4 = 0, fork = 0, dart = 0;
-  if (s64 < a.nnz) {
-    slot = (int)s64;
+  int slot = 0, len = 0, e_ux = 0, x = 0, dx = 0, du = 0;
+  const int64_t mine = s64 / kWarp * per + lane;
+  if (lane < per && mine < a.nnz) {
+    slot = (int)mine;
     const int u = a.src[slot];
     const int i = slot - (int)__ldg(a.rp + u), p = a.dp[u];
-    if (i < p) {
+    if (i < p - 1) {
       len = p - 1 - i;
-      i0 = slot + 1;
       e_ux = a.upe[slot];
       x = __ldg(a.ci + e_ux);
       dx = a.deg[x];
-      if (kFill) {
-        const u64 t = (u64)a.a[e_ux], du = (u64)a.deg[u], dv = (u64)dx;
-        D = c2(t);
-        C3 = c3((long long)t);
-        p4 = (du - 1 - t) * (dv - 1 - t);
-        fork = c2(du - 1) * (dv - 1) + c2(dv - 1) * (du - 1) - t * (du + dv - 4);
-        dart = c2(t) * (du + dv - 6);
-      }
+      du = a.deg[u];
     }
   }
   const FlatLists fl(len, lane);
@@ -338,10 +308,10 @@ __global__ void __launch_bounds__(kThreads) motif_tri_kernel(MotifArgs a) {
   for (int base = 0; base < fl.total; base += kWarp) {
     const int f = base + lane;
     const int l = fl.owner(f);
-    const int o = f - (__shfl_sync(kFull, fl.incl, l) - __shfl_sync(kFull, len, l));
-    const int ys = __shfl_sync(kFull, i0, l) + o;
+    const int ys = f + __shfl_sync(kFull, slot + 1 - (fl.incl - len), l);
     const int ex = __shfl_sync(kFull, e_ux, l);
     const int vx = __shfl_sync(kFull, x, l), dvx = __shfl_sync(kFull, dx, l);
+    const int dvu = __shfl_sync(kFull, du, l);
     if (f >= fl.total) continue;
     const int ey = a.upe[ys];
     const int y = __ldg(a.ci + ey);
@@ -351,47 +321,54 @@ __global__ void __launch_bounds__(kThreads) motif_tri_kernel(MotifArgs a) {
     const int b = (int)__ldg(a.rp + lo);
     const int exy = find_entry(a.ci, b, b + (x_low ? dvx : dy), hi);
     if (exy < 0 || a.rev1[exy] == 0) continue;
-    const int rx = a.rev1[ex] - 1, ry = a.rev1[ey] - 1, rxy = a.rev1[exy] - 1;
-    if (!kFill) {
-      atomicAdd(a.a + ex, 1);
-      atomicAdd(a.a + rx, 1);
-      atomicAdd(a.a + ey, 1);
-      atomicAdd(a.a + ry, 1);
-      atomicAdd(a.a + exy, 1);
-      atomicAdd(a.a + rxy, 1);
-      vtd += (u64)(a.deg[a.src[ex]] + dvx) + (u64)dy;
-      ++tri;
+    if (kCount) {
+      atomicAdd(a.cnt + ex, 1);
+      atomicAdd(a.cnt + ey, 1);
+      atomicAdd(a.cnt + exy, 1);
     } else {
-      // Entries lo -> hi and hi -> lo, and those back to u.
-      const int r_lo = x_low ? rx : ry, r_hi = x_low ? ry : rx;
-      const int jx = atomicAdd(a.cur + ex, 1), jy = atomicAdd(a.cur + ey, 1),
-                jxy = atomicAdd(a.cur + exy, 1);
+      const int rx = a.rev1[ex] - 1, ry = a.rev1[ey] - 1, rxy = a.rev1[exy] - 1;
+      const int jx = atomicAdd(a.a + ex, 1), jy = atomicAdd(a.a + ey, 1),
+                jxy = atomicAdd(a.a + exy, 1);
+      atomicAdd(a.a + rx, 1);
+      atomicAdd(a.a + ry, 1);
+      atomicAdd(a.a + rxy, 1);
       a.list[a.off[ex] + jx] = ey;
       a.list[a.off[rx] + jx] = x_low ? exy : rxy;  // x -> y
       a.list[a.off[ey] + jy] = ex;
       a.list[a.off[ry] + jy] = x_low ? rxy : exy;  // y -> x
-      a.list[a.off[exy] + jxy] = r_lo;             // lo -> u
-      a.list[a.off[rxy] + jxy] = r_hi;             // hi -> u
+      a.list[a.off[exy] + jxy] = x_low ? rx : ry;  // lo -> u
+      a.list[a.off[rxy] + jxy] = x_low ? ry : rx;  // hi -> u
+      vtd += (u64)(dvu + dvx) + (u64)dy;
+      ++tri;
     }
   }
   __syncwarp();
-  if (!kFill) {
+  if (!kCount) {
     bs.add(kT, tri);
     bs.add(kVtd, vtd);
-  } else {
+    bs.flush(a.acc);
+  }
+}
+
+// ---- triangles with their common neighbours -----------------------------------
+struct TauSums {
+  u64 D = 0, C3 = 0, p4 = 0, fork = 0, dart = 0, vt2 = 0;
+  u64 cricket = 0, bull = 0, lolli = 0, kite = 0, gem = 0, kd = 0, ka = 0, kk = 0, K4 = 0, K5 = 0;
+  // Up edge (u, v) with t triangles.
+  __device__ __forceinline__ void edge(u64 du, u64 dv, u64 t) {
+    D += c2(t);
+    C3 += c3((long long)t);
+    p4 += (du - 1 - t) * (dv - 1 - t);
+    fork += c2(du - 1) * (dv - 1) + c2(dv - 1) * (du - 1) - t * (du + dv - 4);
+    dart += c2(t) * (du + dv - 6);
+  }
+  __device__ __forceinline__ void flush(const BlockSums &bs, bool tau) const {
     bs.add(kD, D);
     bs.add(kC3, C3);
     bs.add(kEp4, p4);
     bs.add(kEfork, fork);
     bs.add(kEdart, dart);
-  }
-  bs.flush(a.acc);
-}
-
-// ---- triangles with their common neighbours -----------------------------------
-struct TauSums {
-  u64 cricket = 0, bull = 0, lolli = 0, kite = 0, gem = 0, kd = 0, ka = 0, kk = 0, K4 = 0, K5 = 0;
-  __device__ __forceinline__ void flush(const BlockSums &bs, bool tau) const {
+    bs.add(kVt2, vt2);
     if (tau) {
       bs.add(kCricket, cricket);
       bs.add(kBull, bull);
@@ -424,25 +401,20 @@ __device__ __forceinline__ void tau_terms(const MotifArgs &a, TauSums &t, int u,
   t.kk += c2((u64)k);
 }
 
-// Bits above position j of a row's word w.
-__device__ __forceinline__ unsigned above(int j, int w) {
-  const int s = j + 1 - 32 * w;
-  return s <= 0 ? kFull : (s >= 32 ? 0u : kFull << s);
-}
-
-// Element q of the list of up entry i of u (row start b, entry e, reverse r):
-// when its neighbour is an up neighbour j > i, the triangle (u, i, j).  R:
-// rows over N(u) (wd words), M: rows over N+(u) (wp words).
+// Element idx of the list of up entry i of u (entry e), the same slot of its
+// reverse list being at rev_at: when its neighbour is an up neighbour j > i,
+// the triangle (u, i, j).  R: rows over N(u) (wd words), M: rows over N+(u)
+// (wp words).
 __device__ __forceinline__ void tau_element(const MotifArgs &a, TauSums &t, int u, int du, int i,
-                                            int e, int64_t q, int64_t rev_off, int idx,
-                                            const unsigned *R, int wd, const unsigned *M, int wp) {
+                                            int e, int64_t rev_at, int idx, const unsigned *R,
+                                            int wd, const unsigned *M, int wp) {
   const int j = a.pos1[idx] - 1;
   if (j <= i) return;
   if (a.need & kNeedTau) {
     int k = 0;
     for (int w = 0; w < wd; ++w) k += __popc(R[i * wd + w] & R[j * wd + w]);
     tau_terms(a, t, u, __ldg(a.ci + e), __ldg(a.ci + idx), du, a.a[e], a.a[idx],
-              a.a[a.list[rev_off + q]], k);
+              a.a[a.list[rev_at]], k);
   }
   for (int w = (j + 1) >> 5; w < wp; ++w) {
     unsigned m = M[i * wp + w] & M[j * wp + w] & above(j, w);
@@ -457,76 +429,71 @@ __device__ __forceinline__ void tau_element(const MotifArgs &a, TauSums &t, int 
   }
 }
 
-// Warp per u with d+ <= 32 and d <= 512: lane i owns row i.
-__global__ void __launch_bounds__(kThreads) motif_tau_kernel(MotifArgs a) {
-  __shared__ u64 sm[kSums];
-  __shared__ unsigned s_r[kWarps][kTauOut * (kTauDeg / 32)];
-  __shared__ unsigned s_m[kWarps][kTauOut];
-  const BlockSums bs{sm};
-  bs.init();
-  if (a.off[a.nnz] > a.list_cap) return;
-  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
-  unsigned *R = s_r[warp], *M = s_m[warp];
-  TauSums t;
-  u64 vt2 = 0;
+// Warps over all u: vertex and edge sums, and the bit rows of u with d+ <= 32
+// and d <= 512, lane i owning row i.  R: kTauOut x kTauDeg bits, M: kTauOut.
+__device__ void tau_small(const MotifArgs &a, TauSums &t, unsigned *R, unsigned *M, int lane) {
   const int stride = gridDim.x * kWarps;
-  for (int u = blockIdx.x * kWarps + warp; u < a.n; u += stride) {
+  for (int u = blockIdx.x * kWarps + threadIdx.x / kWarp; u < a.n; u += stride) {
     const int p = a.dp[u], d = a.deg[u];
-    if ((a.need & kNeedT) && lane == 0) vt2 += c2((u64)(a.tv2[u] >> 1));
-    if (p < 2 || p > kTauOut || d > kTauDeg) continue;
     const int b = (int)__ldg(a.rp + u);
-    const int wd = (d + 31) >> 5;
+    if (a.need & kNeedT) {
+      int t2 = 0;
+      for (int i = b + lane; i < b + d; i += kWarp) t2 += a.a[i];
+      const u64 sum = warp_sum_u64((u64)t2);
+      if (lane == 0) t.vt2 += c2(sum >> 1);
+    }
+    if (p == 0 || p > kTauOut) continue;
     int e = 0, na = 0;
     int64_t off = 0, roff = 0;
     if (lane < p) {
       e = a.upe[b + lane];
       na = a.a[e];
+      t.edge((u64)d, (u64)a.deg[__ldg(a.ci + e)], (u64)na);
     }
-    if (!__any_sync(kFull, na > 0)) continue;
-    unsigned mrow = 0;
-    if (lane < p) {
-      for (int w = 0; w < wd; ++w) R[lane * wd + w] = 0;
-      if (na > 0) {
-        off = a.off[e];
-        roff = a.off[a.rev1[e] - 1];
-      }
-      for (int q = 0; q < na; ++q) {
-        const int idx = a.list[off + q];
-        const int ps = idx - b, j1 = a.pos1[idx];
-        R[lane * wd + (ps >> 5)] |= 1u << (ps & 31);
-        if (j1) mrow |= 1u << (j1 - 1);
-      }
+    if (p < 2 || d > kTauDeg || !__any_sync(kFull, na > 0)) continue;
+    const int wd = (a.need & kNeedTau) ? (d + 31) >> 5 : 0;
+    for (int w = lane; w < p * wd; w += kWarp) R[w] = 0;
+    M[lane] = 0;
+    if (na > 0) {
+      off = a.off[e];
+      roff = a.off[a.rev1[e] - 1];
     }
-    M[lane] = mrow;
     __syncwarp();
-    for (int q = 0; q < na; ++q)
-      tau_element(a, t, u, d, lane, e, q, roff, a.list[off + q], R, wd, M, 1);
+    walk_lists(a, off, na, lane, [&](int idx, int i, int64_t) {
+      const int ps = idx - b, j1 = a.pos1[idx];
+      if (wd) atomicOr(R + i * wd + (ps >> 5), 1u << (ps & 31));
+      if (j1) atomicOr(M + i, 1u << (j1 - 1));
+    });
+    __syncwarp();
+    // The up entry of the list's row, and where its reverse list starts
+    // against its own, by lane.
+    const int64_t shift = roff - off;
+    const FlatLists fl(na, lane);
+    const int64_t start = off - (fl.incl - na);
+    for (int base = 0; base < fl.total; base += kWarp) {
+      const int g = base + lane;
+      const int i = fl.owner(g);
+      const int64_t q = __shfl_sync(kFull, start, i) + g;
+      const int64_t sh = __shfl_sync(kFull, shift, i);
+      const int ei = __shfl_sync(kFull, e, i);
+      if (g < fl.total) tau_element(a, t, u, d, i, ei, q + sh, a.list[q], R, wd, M, 1);
+    }
     __syncwarp();
   }
-  t.flush(bs, a.need & kNeedTau);
-  if (a.need & kNeedT) bs.add(kVt2, vt2);
-  bs.flush(a.acc);
 }
 
 // CTA per larger u (queue over tau_big): warp per row, lanes over its list.
 // The rows take p (wd + wp) words: p d <= nnz and p^2 <= nnz, since u's p up
 // neighbours have at least u's degree, so slice_words bounds them.
-__global__ void __launch_bounds__(kThreads) motif_tau_big_kernel(MotifArgs a, int smem_words) {
-  extern __shared__ unsigned s_rows[];
-  __shared__ u64 sm[kSums];
-  __shared__ int s_u;
-  const BlockSums bs{sm};
-  bs.init();
-  if (a.off[a.nnz] > a.list_cap) return;
-  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
-  TauSums t;
+__device__ void tau_large(const MotifArgs &a, TauSums &t, unsigned *s_rows, int smem_words,
+                          int *s_u, int lane, int warp) {
   for (;;) {
     if (threadIdx.x == 0) {
       const unsigned i = atomicAdd(a.counts + kTauQueue, 1u);
-      s_u = i < a.counts[kTauN] ? a.tau_big[i] : -1;
+      *s_u = i < a.counts[kTauN] ? a.tau_big[i] : -1;
     }
     __syncthreads();
-    const int u = s_u;
+    const int u = *s_u;
     __syncthreads();
     if (u < 0) break;
     const int p = a.dp[u], d = a.deg[u], b = (int)__ldg(a.rp + u);
@@ -538,6 +505,8 @@ __global__ void __launch_bounds__(kThreads) motif_tau_big_kernel(MotifArgs a, in
     __syncthreads();
     for (int i = warp; i < p; i += kWarps) {
       const int e = a.upe[b + i], na = a.a[e];
+      if (p > kTauOut && lane == 0) t.edge((u64)d, (u64)a.deg[__ldg(a.ci + e)], (u64)na);
+      if (na == 0) continue;
       const int64_t off = a.off[e];
       for (int q = lane; q < na; q += kWarp) {
         const int idx = a.list[off + q];
@@ -549,12 +518,31 @@ __global__ void __launch_bounds__(kThreads) motif_tau_big_kernel(MotifArgs a, in
     __syncthreads();
     for (int i = warp; i < p; i += kWarps) {
       const int e = a.upe[b + i], na = a.a[e];
+      if (na == 0) continue;
       const int64_t off = a.off[e], roff = a.off[a.rev1[e] - 1];
       for (int q = lane; q < na; q += kWarp)
-        tau_element(a, t, u, d, i, e, q, roff, a.list[off + q], R, wd, M, wp);
+        tau_element(a, t, u, d, i, e, roff + q, a.list[off + q], R, wd, M, wp);
     }
     __syncthreads();
   }
+}
+
+// Both forms in one launch while the large form's rows leave the SM full of
+// CTAs, else one launch each.
+template <bool kLarge, bool kSmall>
+__global__ void __launch_bounds__(kThreads) motif_tau_kernel(MotifArgs a, int smem_words) {
+  extern __shared__ unsigned s_rows[];
+  __shared__ u64 sm[kSums];
+  __shared__ unsigned s_r[kSmall ? kWarps : 1][kSmall ? kTauOut * (kTauDeg / 32) : 1];
+  __shared__ unsigned s_m[kSmall ? kWarps : 1][kTauOut];
+  __shared__ int s_u;
+  const BlockSums bs{sm};
+  bs.init();
+  if (lists_overrun(a)) return;
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  TauSums t;
+  if (kLarge) tau_large(a, t, s_rows, smem_words, &s_u, lane, warp);
+  if (kSmall) tau_small(a, t, s_r[kSmall ? warp : 0], s_m[kSmall ? warp : 0], lane);
   t.flush(bs, a.need & kNeedTau);
   bs.flush(a.acc);
 }
@@ -656,28 +644,35 @@ __device__ __forceinline__ void pair_terms(const MotifArgs &a, PairSums &ps, int
     if (k23) ps.c4d += (c - 1) * (u64)a.deg[v];
   });
   // X7: for each edge (p, r) inside N(s), the pairs (s, t) with t adjacent to
-  // p and r.
-  int nth = 0;
+  // p and r: the lists of 32 p's are walked flat for 32 r's at a time, and
+  // those edges' lists flat again.
   for (int c = sh.first; c * kWarp < d; c += sh.step) {
     const int k = c * kWarp + lane;
-    const int e0 = b + (k < d ? k : 0);
-    unsigned with = __ballot_sync(kFull, k < d && a.a[e0] > 0);
-    while (with) {
-      const int src = __ffs(with) - 1;
-      with &= with - 1;
-      if (nth++ % sh.parts != sh.part) continue;
-      const int e = __shfl_sync(kFull, e0, src);
-      const int na = a.a[e];
-      const int64_t off = a.off[e], roff = a.off[a.rev1[e] - 1];
-      for (int j = lane; j < na; j += kWarp) {
-        if (a.list[off + j] <= e) continue;  // seen from the edge's other end
-        const int pr = a.list[roff + j];
-        const int64_t lo = a.off[pr], hi = a.off[pr + 1];
-        for (int64_t q = lo; q < hi; ++q) {
-          const int t = __ldg(a.ci + a.list[q]);
-          if (t < s) ps.x7 += get(t) - 2;
-        }
+    const int e = b + k;
+    const int na = k < d ? a.a[e] : 0;
+    int64_t off = 0, shift = 0;
+    if (na > 0) {
+      off = a.off[e];
+      shift = a.off[a.rev1[e] - 1] - off;
+    }
+    const FlatLists fl(na, lane);
+    const int64_t start = off - (fl.incl - na);
+    for (int base = sh.part * kWarp; base < fl.total; base += sh.parts * kWarp) {
+      const int g = base + lane;
+      const int l = fl.owner(g);
+      const int64_t at = __shfl_sync(kFull, start, l) + g, sft = __shfl_sync(kFull, shift, l);
+      const int ep = __shfl_sync(kFull, e, l);
+      int len = 0;
+      int64_t lo = 0;
+      if (g < fl.total && a.list[at] > ep) {  // each edge from one end
+        const int pr = a.list[at + sft];
+        lo = a.off[pr];
+        len = a.a[pr];
       }
+      walk_lists(a, lo, len, lane, [&](int idx, int, int64_t) {
+        const int t = __ldg(a.ci + idx);
+        if (t < s) ps.x7 += get(t) - 2;
+      });
     }
   }
   sync();
@@ -741,7 +736,7 @@ __global__ void __launch_bounds__(kThreads) motif_pairs_kernel(MotifArgs a) {
   __shared__ u64 sm[kSums];
   const BlockSums bs{sm};
   bs.init();
-  if (a.off[a.nnz] > a.list_cap) return;
+  if (lists_overrun(a)) return;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   int *mine = s_tab + warp * (kHashSlots + kHashSlots / 2);
   HashTable tab{mine, reinterpret_cast<unsigned *>(mine + kHashSlots), 10};
@@ -751,7 +746,7 @@ __global__ void __launch_bounds__(kThreads) motif_pairs_kernel(MotifArgs a) {
   const int stride = gridDim.x * kWarps;
   for (int s = blockIdx.x * kWarps + warp; s < a.n; s += stride) {
     const u64 w = a.walk[s];
-    if (w < 2 || w > kWarpWalk) continue;
+    if (w < 2 || w > a.warp_walk) continue;
     tab.size_for((unsigned)w);
     const int b = (int)__ldg(a.rp + s), d = a.deg[s];
     pair_terms<kOrdered>(
@@ -772,12 +767,11 @@ __global__ void __launch_bounds__(kT) motif_pairs_hash_kernel(MotifArgs a) {
   __shared__ int s_s;
   const BlockSums bs{sm};
   bs.init();
-  if (a.off[a.nnz] > a.list_cap) return;
+  if (lists_overrun(a)) return;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   HashTable tab{s_tab, reinterpret_cast<unsigned *>(s_tab + (1 << kLg)), kLg};
-  tab.clear(threadIdx.x, kT);
   PairSums ps;
-  for (;;) {
+  for (bool first = true;; first = false) {
     if (threadIdx.x == 0) {
       const unsigned i = atomicAdd(a.counts + (kFront ? kMidQueue : kHashQueue), 1u);
       s_s = i < a.counts[kFront ? kMidN : kHashN] ? a.pair_mid[kFront ? i : a.n - 1 - i] : -1;
@@ -785,12 +779,16 @@ __global__ void __launch_bounds__(kT) motif_pairs_hash_kernel(MotifArgs a) {
     __syncthreads();
     const int s = s_s;
     if (s < 0) break;
+    if (first) {
+      tab.clear(threadIdx.x, kT);
+      __syncthreads();
+    }
     tab.size_for((unsigned)a.walk[s]);
     const int b = (int)__ldg(a.rp + s), d = a.deg[s];
     pair_terms<kOrdered>(
         a, ps, s, b, d, Share(d, warp, kT / kWarp), lane, [&](int t) { return tab.count(t); },
         [&](int t) { return tab.get(t); }, [&]() { __syncthreads(); });
-    tab.clear(threadIdx.x, kT);
+    tab.clear(threadIdx.x, kT);  // as far as this walk's table went
   }
   flush_pairs(bs, ps, a.acc);
 }
@@ -808,7 +806,7 @@ __global__ void __launch_bounds__(kPairThreads) motif_pairs_big_kernel(MotifArgs
   __shared__ int s_s;
   const BlockSums bs{sm};
   bs.init();
-  if (a.off[a.nnz] > a.list_cap) return;
+  if (lists_overrun(a)) return;
   const int words = (a.n + 1) >> 1;
   unsigned *cnt = kShared ? reinterpret_cast<unsigned *>(s_tab)
                           : counters + (int64_t)blockIdx.x * words;
@@ -851,49 +849,43 @@ __global__ void __launch_bounds__(kPairThreads) motif_pairs_big_kernel(MotifArgs
 // ---- 4-wheels ---------------------------------------------------------------
 // Per entry (v -> x), the two-paths x - y - z inside N(v) with y and z before
 // x in v's row, counted in a table over N(v): a 4-cycle of N(v) is counted
-// once, at its last vertex.  Warp per entry of a row of at most kWheelDeg.
-__global__ void __launch_bounds__(kThreads) motif_wheel_kernel(MotifArgs a) {
+// once, at its last vertex.  Warp per entry of a row of at most kWheelDeg, a
+// warp taking `per` consecutive entries.
+__global__ void __launch_bounds__(kThreads) motif_wheel_kernel(MotifArgs a, int per) {
   __shared__ u64 sm[kSums];
   __shared__ unsigned s_cnt[kWarps][kWheelDeg];
   const BlockSums bs{sm};
   bs.init();
-  if (a.off[a.nnz] > a.list_cap) return;
+  if (lists_overrun(a)) return;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   unsigned *cnt = s_cnt[warp];
   for (int i = lane; i < kWheelDeg; i += kWarp) cnt[i] = 0;
   __syncwarp();
   u64 w4 = 0;
-  const int64_t stride = (int64_t)gridDim.x * kThreads;
-  for (int64_t base = (int64_t)blockIdx.x * kThreads + warp * kWarp; base < a.nnz; base += stride) {
+  const int64_t stride = (int64_t)gridDim.x * kWarps * per;
+  for (int64_t base = ((int64_t)blockIdx.x * kWarps + warp) * per; base < a.nnz; base += stride) {
     const int64_t e64 = base + lane;
     unsigned todo = __ballot_sync(
-        kFull, e64 < a.nnz && a.a[e64] >= 2 && a.deg[a.src[e64]] <= kWheelDeg);
+        kFull, lane < per && e64 < a.nnz && a.a[e64] >= 2 && a.deg[a.src[e64]] <= kWheelDeg);
     while (todo) {
       const int e = (int)base + __ffs(todo) - 1;
       todo &= todo - 1;
       const int b = (int)__ldg(a.rp + a.src[e]);
       const int na = a.a[e];
       const int64_t off = a.off[e];
-      for (int j = lane; j < na; j += kWarp) {
-        const int y = a.list[off + j];
-        if (y >= e) continue;
-        const int64_t lo = a.off[y], hi = a.off[y + 1];
-        for (int64_t q = lo; q < hi; ++q) {
-          const int z = a.list[q];
-          if (z < e) w4 += atomicAdd(cnt + (z - b), 1u);
+      for (int pass = 0; pass < 2; ++pass) {
+        for (int j0 = 0; j0 < na; j0 += kWarp) {
+          const int y = j0 + lane < na ? a.list[off + j0 + lane] : e;
+          const bool before = y < e;
+          walk_lists(a, before ? a.off[y] : 0, before ? a.a[y] : 0, lane,
+                     [&](int z, int, int64_t) {
+            if (z >= e) return;
+            if (pass == 0) w4 += atomicAdd(cnt + (z - b), 1u);
+            else cnt[z - b] = 0;
+          });
         }
+        __syncwarp();
       }
-      __syncwarp();
-      for (int j = lane; j < na; j += kWarp) {
-        const int y = a.list[off + j];
-        if (y >= e) continue;
-        const int64_t lo = a.off[y], hi = a.off[y + 1];
-        for (int64_t q = lo; q < hi; ++q) {
-          const int z = a.list[q];
-          if (z < e) cnt[z - b] = 0;
-        }
-      }
-      __syncwarp();
     }
   }
   bs.add(kW4, w4);
@@ -907,7 +899,7 @@ __global__ void __launch_bounds__(kThreads) motif_wheel_big_kernel(MotifArgs a, 
   __shared__ int s_e[kThreads], s_n;
   const BlockSums bs{sm};
   bs.init();
-  if (a.off[a.nnz] > a.list_cap) return;
+  if (lists_overrun(a)) return;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   for (int i = threadIdx.x; i < table; i += kThreads) s_cnt[i] = 0;
   u64 w4 = 0;
@@ -928,7 +920,7 @@ __global__ void __launch_bounds__(kThreads) motif_wheel_big_kernel(MotifArgs a, 
         for (int j = warp; j < na; j += kWarps) {
           const int y = a.list[off + j];
           if (y >= e) continue;
-          const int64_t lo = a.off[y], hi = a.off[y + 1];
+          const int64_t lo = a.off[y], hi = lo + a.a[y];
           for (int64_t q = lo + lane; q < hi; q += kWarp) {
             const int z = a.list[q];
             if (z >= e) continue;
@@ -946,49 +938,13 @@ __global__ void __launch_bounds__(kThreads) motif_wheel_big_kernel(MotifArgs a, 
 }
 
 // ---- host -------------------------------------------------------------------
-// The pattern's count from the sums, modulo 2^64: non-induced counts of the
-// subgraphs on five vertices that contain the pattern, each with the signed
-// number of the pattern's copies in it.
-u64 combine(int pattern, const u64 *s) {
-  const u64 K4 = s[kK4], K5 = s[kK5], D = s[kD], T = s[kT];
-  // C4 family: the ordered walk counts each cycle once, the pair walk twice.
-  const u64 ka = s[kKa] - 24 * K4;   // 2 x K5 minus a path of 3 vertices
-  const u64 kd = s[kKd] - 36 * K4;   // 3 x tailed K4
-  const u64 third = 0xaaaaaaaaaaaaaaabull;  // 1/3 modulo 2^64
-  const u64 tk4 = kd * third;
-  const u64 claw = s[kVd3] - s[kVtd] + 6 * T + 2 * D - 4 * K4;
-  const u64 gem = s[kGem] - 12 * K4, kite = s[kKite] - 12 * K4;
-  const u64 butterfly = s[kVt2] - 2 * D;
-  switch (pattern) {
-    case 1: return claw;
-    case 2:
-      // banner = C4d / 2 - 8 (C4 / 2) - 2 D and house = C4a / 2 - 4 D, with
-      // the doubled sums of the pair walk.
-      return s[kEfork] - 2 * s[kCricket] - 2 * s[kBull] - s[kLolli] - (s[kC4d] - 8 * s[kC4] - 4 * D) +
-             6 * s[kK23] + 5 * s[kEdart] + 4 * kite + (2 * s[kC4a] - 16 * D) + 4 * butterfly -
-             10 * gem - 10 * s[kX7] + 20 * s[kW4] - 3 * kd + 10 * ka - 12 * s[kC3] - 36 * s[kKk] +
-             60 * K5;
-    case 3: {
-      const u64 star = s[kVd4] - s[kCricket] + s[kEdart] + butterfly - gem + s[kW4] - tk4 -
-                       2 * s[kC3] - 3 * s[kKk] + 5 * K5;  // + 2 (K5 - P3), added below
-      return 4 * star + 4 * ka + 3 * claw;
-    }
-    case 4: return s[kEp4] - 4 * s[kC4] + 4 * D - 12 * K4;
-    case 5:
-      return 2 * s[kBull] - 4 * s[kEdart] - 4 * kite - (s[kC4a] - 8 * D) + 10 * gem + 8 * s[kX7] -
-             24 * s[kW4] + 4 * kd - 14 * ka + 12 * s[kC3] + 60 * s[kKk] - 120 * K5;
-    case 6: {
-      const u64 paw = s[kVtd] - 6 * T - 4 * (D - 6 * K4) - 12 * K4;
-      return 2 * paw + 2 * s[kEdart] - 4 * gem + 8 * s[kW4] - 2 * kd + 10 * ka - 12 * s[kC3] -
-             48 * s[kKk] + 120 * K5;
-    }
-    case 7: return 2 * s[kC3] - ka + 6 * s[kKk] - 20 * K5;
-    default: return kd - 3 * ka + 18 * s[kKk] - 60 * K5;
-  }
-}
-
 unsigned blocks(int64_t items, int per_block) {
   return (unsigned)std::max<int64_t>(1, (items + per_block - 1) / per_block);
+}
+
+// Entries a warp takes at once, so that some 64 warps per SM have work.
+int spread(int64_t entries, int num_sms) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(kWarp, entries / (64 * (int64_t)num_sms)));
 }
 
 int resident(const void *kernel, int threads, size_t smem) {
@@ -996,6 +952,16 @@ int resident(const void *kernel, int threads, size_t smem) {
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess)
     per_sm = 1;
   return std::max(per_sm, 1);
+}
+
+// Scratch blocks come in eight sizes per power of two: the pool hands a block
+// of the same size out again as it is, and maps memory anew for any other size
+// (about a millisecond per call when counts of similar graphs, or of several
+// patterns, alternated with sizes of their own).
+size_t block_bytes(size_t bytes) {
+  size_t step = size_t(1) << 20;
+  while (step * 16 < bytes) step *= 2;
+  return (bytes + step - 1) / step * step;
 }
 
 // Carves aligned arrays out of one allocation.
@@ -1017,7 +983,9 @@ int launch_pairs(mc_dgraph *g, const MotifArgs &a, int64_t longest, int big_grid
   cudaStream_t s = g->stream;
   auto launch = [&](auto kern, int threads, size_t smem, int64_t items) -> int {
     MC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int64_t fit = (int64_t)g->num_sms * resident((const void *)kern, threads, smem);
+    const int64_t fit = items <= g->num_sms
+                            ? items
+                            : (int64_t)g->num_sms * resident((const void *)kern, threads, smem);
     kern<<<(unsigned)std::max<int64_t>(1, std::min(items, fit)), threads, smem, s>>>(a);
     MC_CUDA_TRY(cudaGetLastError());
     g->launches += 1;
@@ -1025,7 +993,7 @@ int launch_pairs(mc_dgraph *g, const MotifArgs &a, int64_t longest, int big_grid
   };
   int rc = launch(motif_pairs_kernel<kOrdered>, kThreads, kWarps * hash_bytes(kHashSlots),
                   blocks(a.n, kWarps));
-  if (rc == MC_OK && longest > (int64_t)kWarpWalk && a.mid_walk > kWarpWalk)
+  if (rc == MC_OK && longest > (int64_t)a.warp_walk)
     rc = launch(motif_pairs_hash_kernel<kOrdered, true, 128, 12>, 128, hash_bytes(1 << 12), a.n);
   if (rc == MC_OK && longest > (int64_t)a.mid_walk)
     rc = launch(motif_pairs_hash_kernel<kOrdered, false, 512, 14>, 512, hash_bytes(1 << 14), a.n);
@@ -1041,27 +1009,57 @@ int launch_pairs(mc_dgraph *g, const MotifArgs &a, int64_t longest, int big_grid
 
 }  // namespace
 
-// Whether a whole count of this graph takes this route: not above the degree
-// at which the reference's 32-bit products could wrap (its counts are then no
-// subgraph counts), not with columns in host memory (the pairs stage reads
-// rows once per two-path), and not when the environment asks for another
-// route or its forms.
-bool motif_route(const mc_dgraph *g) {
-  if (g->n == 0 || g->nnz == 0 || g->batch.gid || g->col_host) return false;
-  if (g->max_degree > 46340 || g->nnz > (int64_t(1) << 30)) return false;
-  if (const char *env = std::getenv("MERCURY_MOTIF_ROUTE"))
-    if (std::atoi(env) == 0) return false;
+// The route of a whole count.  Not the motif sums: above the degree at which
+// the reference's 32-bit products could wrap (its counts are then no subgraph
+// counts), with columns in host memory (the pairs stage reads rows once per
+// two-path), and when the environment asks for another route or its forms.
+//
+// By size (measured on a B200, whole calls, formula / bit rows / sparse, ms):
+//  - bit rows take P2 and P5 up to 512 vertices (RMAT scale 8, edge factor 8:
+//    1.39 / 0.14 / 0.41 and 0.32 / 0.14 / 0.41; at 1,024 vertices the two
+//    differ by -15% to +50%), and every pattern up to 64, where the sparse
+//    stages are launches alone (RMAT 6, P6: 0.068 / 0.055 / 0.079);
+//  - the per-edge formulas, one launch against five or more, keep P4 to P8
+//    on small graphs of low degree (the limits below), where every set of an
+//    edge is a warp or two: Chung-Lu of 10,001 vertices, mean 4, cap 40 (39,942
+//    entries, degree 61), P4 to P8: 0.094, 0.093, 0.081, 0.081 and 0.094 against
+//    0.122, 0.139, 0.096, 0.091 and 0.091 sparse; of 30,001 (119,934 entries):
+//    0.172, 0.167, 0.146, 0.132 and 0.170 against 0.165, 0.165, 0.107, 0.097 and
+//    0.097.  Hubs turn it: 3,001 vertices, mean 4, cap 200 (11,186 entries,
+//    degree 165), P5 to P8: 0.52, 1.20, 0.33 and 0.71 against 0.37, 0.10, 0.09
+//    and 0.09.
+PatternRoute pattern_route(const mc_dgraph *g, int pattern) {
+  if (g->n == 0 || g->nnz == 0 || g->batch.gid || g->col_host) return PatternRoute::kFormula;
+  if (g->max_degree > 46340 || g->nnz > (int64_t(1) << 30)) return PatternRoute::kFormula;
   for (const char *name : {"MERCURY_PATTERN_KERNEL", "MERCURY_CLIQUE_ROUTE", "MERCURY_PATTERN_SETS",
                            "MERCURY_PATTERN_SLICE", "MERCURY_HUB_P1", "MERCURY_HOP_ROWS"})
-    if (std::getenv(name)) return false;
-  return true;
+    if (std::getenv(name)) return PatternRoute::kFormula;
+  const bool few = g->n <= kDenseMax;
+  // MERCURY_MOTIF_ROUTE=formula|dense|sparse (tests and timing comparisons).
+  if (const char *env = std::getenv("MERCURY_MOTIF_ROUTE")) {
+    if (std::strcmp(env, "formula") == 0) return PatternRoute::kFormula;
+    if (std::strcmp(env, "dense") == 0) return few ? PatternRoute::kDense : PatternRoute::kSparse;
+    if (std::strcmp(env, "sparse") == 0) return PatternRoute::kSparse;
+  }
+  if (g->n <= 64 && pattern != 4) return PatternRoute::kDense;
+  if (g->n <= 512 && (pattern == 2 || pattern == 5)) return PatternRoute::kDense;
+  struct Limit {
+    int64_t degree, entries;
+  };
+  constexpr Limit kFormulaUpTo[] = {{100, 65536}, {80, 98304}, {72, 49152}, {80, 65536}, {64, 16384}};
+  if (pattern >= 4) {
+    const Limit &up = kFormulaUpTo[pattern - 4];
+    if (g->max_degree <= up.degree && g->nnz <= up.entries) return PatternRoute::kFormula;
+    if (pattern == 4 && g->nnz <= 12288) return PatternRoute::kFormula;
+  }
+  return PatternRoute::kSparse;
 }
 
 int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
   NvtxRange range("motif_count");
   cudaStream_t s = g->stream;
   const int n = (int)g->n, nnz = (int)g->nnz;
-  const unsigned need = needs_of(pattern);
+  const unsigned need = motif_needs(pattern);
   const bool pairs = need & (kNeedC4 | kNeedPairs), ordered = need & kNeedC4;
   const bool wheel = need & kNeedW4;
   // Shared-memory tables of the pairs stage: 16 bits per vertex.
@@ -1071,16 +1069,19 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
                                      : (int)std::max<int64_t>(
                                            1, std::min<int64_t>(2 * g->num_sms,
                                                                 (int64_t(2) << 30) / (int64_t)table_b));
-  // A vertex's walk is at most the entries of its neighbours' rows.  Where no
-  // walk exceeds the second hash class, that class takes the first's as well.
+  // A vertex's walk is at most the entries of its neighbours' rows.
   const int64_t longest = std::min<int64_t>(nnz, g->max_degree * g->max_degree);
-  const u64 mid_walk = longest <= (int64_t)kHashWalk ? kWarpWalk : kMidWalk;
   const int64_t root = (int64_t)std::sqrt((double)nnz) + 1;
   const int64_t slice_words = (2 * (int64_t)nnz + 64 * root) / 32 + 64;
   const bool slices = slice_words * 4 > kTauSmem;
   const int tau_grid = (int)std::max<int64_t>(
       1, std::min<int64_t>(2 * g->num_sms, slices ? (int64_t(1) << 30) / (4 * slice_words) : 1 << 20));
-  int64_t list_cap = std::max<int64_t>(int64_t(16) << 20, 4 * (int64_t)nnz);
+  // Room for the lists: nnz x max_degree bounds what the up stage hands out.
+  // Where that exceeds the first guess, the count starts over with the room it
+  // asked for, or, above 2 GiB, with lists sized by a counting pass.
+  int64_t list_cap = std::min<int64_t>((int64_t)nnz * g->max_degree,
+                                       std::max<int64_t>(int64_t(16) << 20, 64 * (int64_t)nnz));
+  bool counted = false;
   for (;;) {
     MotifArgs a{};
     a.rp = g->rowptr;
@@ -1090,33 +1091,32 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
     a.need = need;
     a.list_cap = list_cap;
     a.slice_words = slice_words;
-    a.mid_walk = mid_walk;
-    void *temp = nullptr;
-    unsigned *counters = nullptr;
+    // Few vertices: a CTA for all but the shortest walks.
+    a.warp_walk = n <= kFewVertices ? kFewWalk : kWarpWalk;
+    a.mid_walk = kMidWalk;
     size_t zeroed = 0;
+    // The same layout for every pattern (see block_bytes).
     auto lay_out = [&](Carver &c) {
       // Zeroed before the first kernel.
-      a.acc = c.take<u64>(kSums);
+      a.acc = c.take<u64>(kSums + 1);
+      a.pool = a.acc + kSums;
       a.counts = c.take<unsigned>(kCounts);
       a.dp = c.take<int32_t>(n);
-      a.tv2 = c.take<int32_t>(need & kNeedT ? n : 0);
-      a.d2 = c.take<u64>(need & kNeedD2 ? n : 0);
-      a.walk = c.take<u64>(pairs ? n : 0);
+      a.d2 = c.take<u64>(n);
+      a.walk = c.take<u64>(n);
       a.rev1 = c.take<int32_t>(nnz);
       a.a = c.take<int32_t>(nnz);
-      a.cur = c.take<int32_t>(nnz);
+      if (counted) a.cnt = c.take<int32_t>(nnz);
       zeroed = c.used;
       a.deg = c.take<int32_t>(n);
       a.src = c.take<int32_t>(nnz);
       a.upe = c.take<int32_t>(nnz);
       a.pos1 = c.take<int32_t>(nnz);
-      a.off = c.take<int64_t>((int64_t)nnz + 1);
+      a.off = c.take<int64_t>(nnz);
       a.tau_big = c.take<int32_t>(n);
-      a.pair_mid = c.take<int32_t>(pairs ? n : 0);
-      a.pair_big = c.take<int32_t>(pairs ? n : 0);
-      temp = c.take<char>((int64_t)scan_temp_bytes(nnz));
+      a.pair_mid = c.take<int32_t>(n);
+      a.pair_big = c.take<int32_t>(n);
       a.slices = c.take<unsigned>(slices ? tau_grid * slice_words : 0);
-      counters = c.take<unsigned>(pairs && !table_shared ? pair_grid * (int64_t)(table_b / 4) : 0);
       a.list = c.take<int32_t>(list_cap);
     };
     Carver size;
@@ -1124,42 +1124,62 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
     Carver c;
     // Large scratch leaves half of the free memory alone; the caller then
     // takes a formula route, as it does when the allocation fails.
-    if (size.used > size_t(1) << 30) {
+    const size_t counters_b = pairs && !table_shared ? pair_grid * table_b : 0;
+    if (size.used + counters_b > size_t(1) << 30) {
       size_t free_b = 0, total_b = 0;
       MC_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-      if (size.used > free_b / 2) return MC_ERR_OOM;
+      if (size.used + counters_b > free_b / 2) return MC_ERR_OOM;
     }
-    MC_CUDA_TRY(dev_alloc(reinterpret_cast<void **>(&c.base), size.used, s));
+    MC_CUDA_TRY(dev_alloc(reinterpret_cast<void **>(&c.base), block_bytes(size.used), s));
     lay_out(c);
-    u64 h[kSums];
-    int64_t total = 0;
+    unsigned *counters = nullptr;
+    if (counters_b) {
+      const cudaError_t e = dev_alloc(reinterpret_cast<void **>(&counters), block_bytes(counters_b), s);
+      if (e != cudaSuccess) dev_free(c.base, s);
+      MC_CUDA_TRY(e);
+    }
+    u64 h[kSums + 1];
     auto run = [&]() -> int {
+      const int per = spread(nnz, g->num_sms);
+      const unsigned tri_grid = blocks(std::max<int64_t>(n, ((int64_t)nnz + per - 1) / per * kWarp),
+                                       kThreads);
       MC_CUDA_TRY(cudaMemsetAsync(c.base, 0, zeroed, s));
       motif_rows_kernel<<<std::min(blocks(n, kWarps), 4096u), kThreads, 0, s>>>(a);
       MC_CUDA_TRY(cudaGetLastError());
       motif_up_kernel<<<blocks(nnz, kThreads), kThreads, 0, s>>>(a);
       MC_CUDA_TRY(cudaGetLastError());
-      motif_tri_kernel<false><<<blocks(nnz, kThreads), kThreads, 0, s>>>(a);
+      if (counted) {
+        motif_tri_kernel<true><<<tri_grid, kThreads, 0, s>>>(a, per);
+        MC_CUDA_TRY(cudaGetLastError());
+        motif_lists_kernel<<<blocks(nnz, kThreads), kThreads, 0, s>>>(a);
+        MC_CUDA_TRY(cudaGetLastError());
+        g->launches += 2;
+      }
+      motif_tri_kernel<false><<<tri_grid, kThreads, 0, s>>>(a, per);
       MC_CUDA_TRY(cudaGetLastError());
-      MC_CUDA_TRY(exclusive_scan(a.a, a.off, nnz, temp, s));
-      motif_tri_kernel<true><<<blocks(std::max(n, nnz), kThreads), kThreads, 0, s>>>(a);
-      MC_CUDA_TRY(cudaGetLastError());
-      g->launches += 4 + scan_launches(nnz);
-      motif_tau_kernel<<<std::min(blocks(n, kWarps), (unsigned)(8 * g->num_sms)), kThreads, 0, s>>>(a);
-      MC_CUDA_TRY(cudaGetLastError());
-      MC_CUDA_TRY(cudaFuncSetAttribute(motif_tau_big_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kTauSmem));
-      motif_tau_big_kernel<<<tau_grid, kThreads, kTauSmem, s>>>(a, kTauSmem / 4);
-      MC_CUDA_TRY(cudaGetLastError());
-      g->launches += 2;
+      const unsigned tau_small_grid = std::min(blocks(n, kWarps), (unsigned)(8 * g->num_sms));
+      if (slice_words * 4 <= kTauBoth) {
+        motif_tau_kernel<true, true><<<tau_small_grid, kThreads, slice_words * 4, s>>>(
+            a, (int)slice_words);
+        MC_CUDA_TRY(cudaGetLastError());
+        g->launches += 4;
+      } else {
+        MC_CUDA_TRY(cudaFuncSetAttribute(motif_tau_kernel<true, false>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kTauSmem));
+        motif_tau_kernel<true, false><<<tau_grid, kThreads, kTauSmem, s>>>(a, kTauSmem / 4);
+        MC_CUDA_TRY(cudaGetLastError());
+        motif_tau_kernel<false, true><<<tau_small_grid, kThreads, 0, s>>>(a, 0);
+        MC_CUDA_TRY(cudaGetLastError());
+        g->launches += 5;
+      }
       if (pairs) {
         const int rcp = ordered ? launch_pairs<true>(g, a, longest, pair_grid, table_shared, table_b, counters)
                                 : launch_pairs<false>(g, a, longest, pair_grid, table_shared, table_b, counters);
         if (rcp != MC_OK) return rcp;
       }
       if (wheel) {
-        motif_wheel_kernel<<<std::min(blocks(nnz, kThreads), (unsigned)(8 * g->num_sms)), kThreads, 0,
-                             s>>>(a);
+        motif_wheel_kernel<<<std::min(blocks(nnz, kWarps * per), (unsigned)(8 * g->num_sms)), kThreads,
+                             0, s>>>(a, per);
         MC_CUDA_TRY(cudaGetLastError());
         g->launches += 1;
         if (g->max_degree > kWheelDeg) {
@@ -1176,18 +1196,23 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
       }
       MC_CUDA_TRY(cudaEventRecord(g->ev[3], s));
       MC_CUDA_TRY(cudaMemcpyAsync(h, a.acc, sizeof(h), cudaMemcpyDeviceToHost, s));
-      MC_CUDA_TRY(cudaMemcpyAsync(&total, a.off + nnz, sizeof(total), cudaMemcpyDeviceToHost, s));
       MC_CUDA_TRY(cudaStreamSynchronize(s));
       return MC_OK;
     };
     const int rc = run();
     dev_free(c.base, s);
+    if (counters) dev_free(counters, s);
     if (rc != MC_OK) return rc;
-    if (total <= list_cap) {
-      *out = combine(pattern, h);
+    const int64_t asked = (int64_t)h[kSums];
+    if (asked <= list_cap) {
+      *out = motif_combine(pattern, h);
       return MC_OK;
     }
-    list_cap = total;  // more triangles than the first guess: once more, sized
+    if (!counted && asked > int64_t(512) << 20) {
+      counted = true;  // six entries per triangle instead of two rows per edge
+    } else {
+      list_cap = asked;
+    }
   }
 }
 

@@ -2165,12 +2165,16 @@ int pattern_count_body(mc_dgraph *g, int pattern, uint64_t *out, uint64_t *c12,
                        double *progress) {
   NvtxRange range("pattern_count");
   if (pattern < 1 || pattern > 8) return MC_ERR_ARG;
-  // Whole counts without a budget: motif sums (motifs.cu).  A shard's partial
-  // count, a budget's slices and the two counters stay with the routes below.
-  if (num_shards == 1 && budget_ms <= 0 && !c12 && motif_route(g)) {
+  // Whole counts without a budget: motif sums (motifs.cu, dense.cu) where they
+  // apply and pay.  A shard's partial count, a budget's slices and the two
+  // counters stay with the routes below.
+  const PatternRoute route = num_shards == 1 && budget_ms <= 0 && !c12 ? pattern_route(g, pattern)
+                                                                        : PatternRoute::kFormula;
+  if (route != PatternRoute::kFormula) {
     const int64_t launches = g->launches;
     MC_CUDA_TRY(cudaEventRecord(g->ev[0], g->stream));
-    const int rc = motif_count(g, pattern, out);
+    const int rc = route == PatternRoute::kDense ? dense_count(g, pattern, out)
+                                                 : motif_count(g, pattern, out);
     if (rc != MC_OK && rc != MC_ERR_OOM) return rc;
     if (rc == MC_OK) {
       if (progress) *progress = 1.0;

@@ -113,9 +113,13 @@ def gpu_counts(rp, col):
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,p,seed", [
     (1, 0.0, 0), (2, 1.0, 0), (3, 1.0, 0), (4, 1.0, 0), (5, 1.0, 0), (6, 0.0, 0),
+    (31, 0.4, 5), (32, 0.4, 5),    # bit rows of one whole word and a part
     (33, 1.0, 0), (34, 1.0, 0),    # d+ of 32 (one warp's rows) and of 33
-    (65, 1.0, 0), (70, 0.9, 1), (100, 0.3, 2), (180, 0.5, 3), (300, 0.02, 4)])
-def test_motif_route_vs_oracle(n, p, seed):
+    (64, 0.3, 6), (65, 1.0, 0), (70, 0.9, 1), (100, 0.3, 2), (180, 0.5, 3), (300, 0.02, 4)])
+@pytest.mark.parametrize("route", ["default", "dense", "sparse"])
+def test_motif_routes_vs_oracle(monkeypatch, n, p, seed, route):
+    if route != "default":
+        monkeypatch.setenv("MERCURY_MOTIF_ROUTE", route)
     rp, col = csr_from_edges(n, random_graph(n, p, seed))
     assert gpu_counts(rp, col) == [orc.pattern(rp, col, k) for k in range(1, 9)]
 
@@ -128,23 +132,38 @@ def test_motif_route_vs_oracle(n, p, seed):
     # More vertices than the shared tables hold.
     lambda: Graph.chung_lu(150001, 2.1, 6.0, 3000.0, seed=3),
     lambda: Graph.rmat(11, 16, seed=5),
-], ids=["classes", "global_tables", "rmat11"])
+    # The largest graphs the bit rows take.
+    lambda: Graph.chung_lu(1024, 2.1, 12.0, 300.0, seed=5),
+], ids=["classes", "global_tables", "rmat11", "n1024"])
 def test_motif_route_equals_formula_routes(monkeypatch, make):
     g = make()
+    monkeypatch.setenv("MERCURY_MOTIF_ROUTE", "sparse")
     with DeviceGraph(g) as d:
         motif = [d.pattern_count(k) for k in range(1, 9)]
-        monkeypatch.setenv("MERCURY_MOTIF_ROUTE", "0")
+        if g.n <= 1024:
+            monkeypatch.setenv("MERCURY_MOTIF_ROUTE", "dense")
+            assert motif == [d.pattern_count(k) for k in range(1, 9)]
+        monkeypatch.setenv("MERCURY_MOTIF_ROUTE", "formula")
         assert motif == [d.pattern_count(k) for k in range(1, 9)]
 
 
 @pytest.mark.gpu
-def test_motif_route_sizes_its_lists_again():
-    """More common-neighbour entries (six per triangle) than the first guess
-    of 16 M: the count starts over with room for all.  A clique of n with one
-    vertex hung on vertex 0 holds C(n - 1, 2) induced paws and C(n - 1, 3)
-    induced tailed K4s, and none of the other subgraphs."""
-    n = 300  # 4,455,100 triangles, 26.7 M entries
-    rp, col = csr_from_edges(n + 1, [(i, j) for i in range(n) for j in range(i)] + [(0, n)])
+@pytest.mark.parametrize("n", [300, 700, 1200])
+def test_motif_route_on_a_clique_with_a_tail(monkeypatch, n):
+    """A clique of n with one vertex hung on vertex 0 holds C(n - 1, 2)
+    induced paws and C(n - 1, 3) induced tailed K4s, and none of the other
+    subgraphs.  At 700 the common-neighbour lists outgrow the first guess
+    (64 M entries): the count starts over with the room asked for; at 1,200
+    that is above 512 M entries, and a counting pass sizes them."""
+    monkeypatch.setenv("MERCURY_MOTIF_ROUTE", "sparse")
+    i, j = np.tril_indices(n, -1)
+    edges = np.stack([np.concatenate([i, [0]]), np.concatenate([j, [n]])], axis=1)
+    adj = np.zeros((n + 1, n + 1), dtype=bool)
+    adj[edges[:, 0], edges[:, 1]] = adj[edges[:, 1], edges[:, 0]] = True
+    rp = np.concatenate([[0], np.cumsum(adj.sum(axis=1))]).astype(np.int64)
+    col = np.nonzero(adj)[1].astype(np.int32)
+    patterns = range(1, 9) if n == 300 else (1, 8)
     want = [0] * 8
     want[5], want[7] = 2 * math.comb(n - 1, 2), 3 * math.comb(n - 1, 3)
-    assert gpu_counts(rp, col) == want
+    with DeviceGraph(rp, col) as d:
+        assert [d.pattern_count(k) for k in patterns] == [want[k - 1] for k in patterns]
