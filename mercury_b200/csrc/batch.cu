@@ -21,6 +21,7 @@
 
 #include "dgraph.cuh"
 #include "device_common.cuh"
+#include "motifs.cuh"
 
 namespace mc {
 namespace {
@@ -60,11 +61,20 @@ __global__ void check_within_graph_kernel(const int64_t *rowptr, const int32_t *
   if (col[b] < gptr[g] || col[e - 1] >= gptr[g + 1]) atomicOr(err, (unsigned)kErrIdRange);
 }
 
+// sums: the motif sums of the graphs marked dense (null: none), else the
+// pattern kernel's two counters.
 __global__ void combine_kernel(const int32_t *job, const unsigned long long *res, int num_graphs,
+                               const uint8_t *dense, unsigned long long *sums,
                                unsigned long long *out) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= num_graphs) return;
   const int j = job[g];
+  if (sums && dense[g]) {
+    unsigned long long *s = sums + (int64_t)g * kSums;
+    s[kX7] >>= 1;  // counted from both ends of its inner edge
+    out[g] = motif_combine(j, s);
+    return;
+  }
   const unsigned long long tc = res[g], c1 = res[num_graphs + g], c2 = res[2 * num_graphs + g];
   out[g] = j == 0 ? tc : ((j == 4 || j == 6) ? c1 : c1 - c2);
 }
@@ -96,7 +106,15 @@ struct mc_batch {
   unsigned long long *d_res = nullptr;   // 3 x num_graphs: triangles, c1, c2
   unsigned long long *d_out = nullptr;   // num_graphs
   unsigned long long *h_out = nullptr;   // pinned
-  bool has_tc = false, has_pat = false;
+  bool has_tc = false, has_pat = false;  // has_pat: graphs for the pattern kernel
+  // Pattern graphs of at most kDenseMax vertices: bit rows (dense.cu).
+  int dense_tasks = 0, dense_largest = 0;
+  mc::DenseTask *d_dense_tasks = nullptr;
+  uint8_t *d_dense = nullptr;                // per graph
+  unsigned long long *d_sums = nullptr;      // kSums per graph
+  // The bit rows run beside the triangle part, on a stream of their own.
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   mc::BatchPatternArgs pa{};
   int pat_grid = 0;
   int table_log2 = 8;
@@ -120,13 +138,17 @@ void batch_release(mc_batch *b) {
   if (b->graph) cudaGraphDestroy(b->graph);
   void *bufs[] = {b->d_gptr, b->d_gid, b->d_job, b->d_job_active, b->d_param, b->d_res, b->d_out,
                   (void *)b->pa.graph, (void *)b->pa.job, (void *)b->pa.v0, (void *)b->pa.v1,
-                  (void *)b->pa.star_off, (void *)b->pa.edge_off, b->pa.scratch, b->pa.queue};
+                  (void *)b->pa.star_off, (void *)b->pa.edge_off, b->pa.scratch, b->pa.queue,
+                  b->d_dense_tasks, b->d_dense, b->d_sums};
   if (b->g)
     for (void *p : bufs)
       if (p) dev_free(p, b->g->stream);
   delete[] b->h_out;
   if (b->e0) cudaEventDestroy(b->e0);
   if (b->e1) cudaEventDestroy(b->e1);
+  if (b->fork) cudaEventDestroy(b->fork);
+  if (b->join) cudaEventDestroy(b->join);
+  if (b->side) cudaStreamDestroy(b->side);
   if (b->g) mc_dgraph_free(b->g);
   delete b;
 }
@@ -149,6 +171,19 @@ int enqueue(mc_batch *b) {
   cudaStream_t s = g->stream;
   const int G = b->num_graphs;
   MC_CUDA_TRY(cudaMemsetAsync(b->d_res, 0, sizeof(unsigned long long) * 3 * G, s));
+  const bool side = b->side && b->dense_tasks > 0 && (b->has_tc || b->has_pat);
+  if (b->dense_tasks > 0) {
+    cudaStream_t ds = side ? b->side : s;
+    if (side) {
+      MC_CUDA_TRY(cudaEventRecord(b->fork, s));
+      MC_CUDA_TRY(cudaStreamWaitEvent(ds, b->fork, 0));
+    }
+    MC_CUDA_TRY(cudaMemsetAsync(b->d_sums, 0, sizeof(unsigned long long) * kSums * G, ds));
+    int rc = dense_batch_launch(g->rowptr, g->col, b->d_dense_tasks, b->dense_tasks,
+                                b->dense_largest, b->d_sums, ds);
+    if (rc != MC_OK) return rc;
+    g->launches += 1;
+  }
   if (b->has_tc) {
     g->batch.gid = b->d_gid;
     g->batch.job = b->d_job_active;
@@ -166,7 +201,12 @@ int enqueue(mc_batch *b) {
     if (rc != MC_OK) return rc;
     g->launches += 1;
   }
-  combine_kernel<<<blocks(G, 256), 256, 0, s>>>(b->d_job, b->d_res, G, b->d_out);
+  if (side) {
+    MC_CUDA_TRY(cudaEventRecord(b->join, b->side));
+    MC_CUDA_TRY(cudaStreamWaitEvent(s, b->join, 0));
+  }
+  combine_kernel<<<blocks(G, 256), 256, 0, s>>>(b->d_job, b->d_res, G, b->d_dense,
+                                                b->dense_tasks > 0 ? b->d_sums : nullptr, b->d_out);
   MC_CUDA_TRY(cudaGetLastError());
   g->launches += 1;
   return MC_OK;
@@ -270,6 +310,10 @@ int batch_create(const int64_t *rowptr, const int32_t *col, bool device_csr, int
   int64_t pat_cap = 1;
   std::vector<int32_t> pg_graph, pg_job;
   std::vector<int64_t> pg_v0, pg_v1, star_off(1, 0), edge_off(1, 0);
+  std::vector<DenseTask> dense;
+  std::vector<uint8_t> is_dense(G, 0);
+  const char *route = std::getenv("MERCURY_MOTIF_ROUTE");
+  const bool use_dense = !(route && std::strcmp(route, "formula") == 0);
   for (int i = 0; i < G; ++i) {
     const int64_t md = gmaxdeg[i];
     const int64_t gnnz = gnnz_of[i];
@@ -277,6 +321,13 @@ int batch_create(const int64_t *rowptr, const int32_t *col, bool device_csr, int
       b->has_tc = true;
       b->bucket[i] = degree_bucket(md);
       b->dplus_bound[i] = std::min<int64_t>(md, (int64_t)std::sqrt((double)gnnz) + 1);
+    } else if (use_dense && graph_vptr[i + 1] - graph_vptr[i] <= kDenseMax) {
+      const int gn = (int)(graph_vptr[i + 1] - graph_vptr[i]);
+      const int parts = dense_parts(gn, gnnz, md);
+      for (int p = 0; p < parts; ++p)
+        dense.push_back(DenseTask{graph_vptr[i], gn, i, jobs[i], p, parts});
+      is_dense[i] = 1;
+      b->dense_largest = std::max(b->dense_largest, gn);
     } else {
       b->has_pat = true;
       pat_cap = std::max(pat_cap, md);
@@ -323,6 +374,23 @@ int batch_create(const int64_t *rowptr, const int32_t *col, bool device_csr, int
       g->batch.gid = b->d_gid;  // a batch handle: no degree ranks (see tc_alloc)
       rc = tc_alloc(g);
       if (rc != MC_OK) return fail(rc);
+    }
+    if (!dense.empty()) {
+      // Longest parts first: they then do not end the launch.
+      std::stable_sort(dense.begin(), dense.end(), [](const DenseTask &x, const DenseTask &y) {
+        return x.parts > y.parts;
+      });
+      b->dense_tasks = (int)dense.size();
+      MC_CUDA_TRY(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking));
+      MC_CUDA_TRY(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+      MC_CUDA_TRY(cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming));
+      MC_BALLOC(b->d_dense_tasks, sizeof(DenseTask) * dense.size());
+      MC_BALLOC(b->d_dense, sizeof(uint8_t) * G);
+      MC_BALLOC(b->d_sums, sizeof(unsigned long long) * kSums * G);
+      MC_CUDA_TRY(cudaMemcpyAsync(b->d_dense_tasks, dense.data(), sizeof(DenseTask) * dense.size(),
+                                  cudaMemcpyHostToDevice, s));
+      MC_CUDA_TRY(cudaMemcpyAsync(b->d_dense, is_dense.data(), sizeof(uint8_t) * G,
+                                  cudaMemcpyHostToDevice, s));
     }
     if (b->has_pat) {
       const int Gp = (int)pg_graph.size();
@@ -437,7 +505,9 @@ int mc_batch_autotune(mc_batch_t *b, int32_t *choice) {
     MC_CUDA_TRY(cudaMemcpyAsync(b->d_job_active, active.data(), sizeof(int32_t) * G,
                                 cudaMemcpyHostToDevice, s));
     const bool had_pat = b->has_pat;
+    const int had_dense = b->dense_tasks;
     b->has_pat = false;  // time the triangle part of this bucket alone
+    b->dense_tasks = 0;
     float best = 1e30f;
     for (int leaf : kLeafChoices) {
       for (int slots : kSlotChoices) {
@@ -463,11 +533,13 @@ int mc_batch_autotune(mc_batch_t *b, int32_t *choice) {
         }
         if (rc != MC_OK) {
           b->has_pat = had_pat;
+          b->dense_tasks = had_dense;
           return rc;
         }
       }
     }
     b->has_pat = had_pat;
+    b->dense_tasks = had_dense;
   }
   for (int i = 0; i < G; ++i)
     if (b->job[i] == 0 && b->tuned[b->bucket[i]][0] > 0)

@@ -8,7 +8,9 @@
 // two rows; each common neighbour v adds popcounts of v's row against them,
 // so the work is n^2 / 2 row ANDs plus one per two-path.  RMAT scale 8 (256
 // vertices, 1,297 edges), all eight patterns: the per-edge kernels took 6.1
-// ms (P2 1.39), the sparse motif stages 1.3 (P2 0.41), these 0.84 (P2 0.14).
+// ms (P2 1.39), the sparse motif stages 1.3 (P2 0.41), these 0.7 (P2 0.13).
+// In a batch, 455 such graphs took the persistent per-edge kernel some 5 ms,
+// and take 0.75 ms, beside the triangle jobs.
 #include <algorithm>
 #include <cstdlib>
 
@@ -20,6 +22,7 @@ namespace mc {
 namespace {
 
 constexpr int kDenseThreads = 512;
+constexpr int kBatchThreads = 256;
 
 // One graph: vertices [v0, v0 + n) of the CSR.
 struct DenseGraph {
@@ -29,18 +32,23 @@ struct DenseGraph {
   int n;
 };
 
-// Rows of W words at an odd stride, so that lanes reading the same word of
-// consecutive rows hit distinct banks; then n + 1 row offsets.
-__host__ __device__ constexpr int dense_words(int n) { return (n + 31) / 32; }
+// Rows of W words (1, 2, 4, 8 or above 256 vertices what n takes: the loops
+// over a row's words are unrolled up to 8) at an odd stride, so that lanes
+// reading the same word of consecutive rows hit distinct banks; then n + 1 row
+// offsets.
+__host__ __device__ constexpr int dense_words(int n) {
+  return n <= 32 ? 1 : n <= 64 ? 2 : n <= 128 ? 4 : n <= 256 ? 8 : (n + 31) / 32;
+}
 __host__ __device__ constexpr int dense_stride(int n) { return dense_words(n) | 1; }
 size_t dense_bytes(int n) { return sizeof(int) * ((size_t)n * dense_stride(n) + n + 1); }
 
 // Adds this part's share of the graph's sums: warp tasks of (vertex) and of
 // (vertex t, 32 vertices s below it), dealt round-robin over the warps of all
-// parts.  need: Need bits; smem: dense_bytes(n).
-__device__ void dense_sums(const DenseGraph &g, unsigned need, int part, int parts,
-                           unsigned *smem, const BlockSums &bs) {
-  const int n = g.n, W = dense_words(n), P = dense_stride(n);
+// parts.  need: Need bits; kW: words of a row, 0 above 8; smem: dense_bytes(n).
+template <unsigned need, int kW>
+__device__ __forceinline__ void dense_sums(const DenseGraph &g, int part, int parts, unsigned *smem,
+                                           const BlockSums &bs) {
+  const int n = g.n, W = kW > 0 ? kW : dense_words(n), P = W | 1;
   unsigned *bits = smem;
   int *off = reinterpret_cast<int *>(smem + (size_t)n * P);
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
@@ -62,8 +70,8 @@ __device__ void dense_sums(const DenseGraph &g, unsigned need, int part, int par
   __syncthreads();
   auto deg = [&](int v) { return (u64)(off[v + 1] - off[v]); };
   const int gw = part * (blockDim.x / kWarp) + warp, step = parts * (blockDim.x / kWarp);
-  const bool tau = need & kNeedTau, pairs = need & kNeedPairs, wheel = need & kNeedW4;
-  const bool k23 = need & kNeedK23;
+  constexpr bool tau = need & kNeedTau, pairs = need & kNeedPairs, wheel = need & kNeedW4;
+  constexpr bool k23 = need & kNeedK23;
 
   u64 d3 = 0, d4 = 0, vt2 = 0, lolli = 0;
   for (int v = gw; v < n; v += step) {
@@ -226,18 +234,43 @@ __device__ void dense_sums(const DenseGraph &g, unsigned need, int part, int par
   }
 }
 
+template <unsigned need>
+__device__ __forceinline__ void dense_words_of(const DenseGraph &g, int part, int parts,
+                                               unsigned *smem, const BlockSums &bs) {
+  switch (dense_words(g.n)) {
+    case 1: return dense_sums<need, 1>(g, part, parts, smem, bs);
+    case 2: return dense_sums<need, 2>(g, part, parts, smem, bs);
+    case 4: return dense_sums<need, 4>(g, part, parts, smem, bs);
+    case 8: return dense_sums<need, 8>(g, part, parts, smem, bs);
+    default: return dense_sums<need, 0>(g, part, parts, smem, bs);
+  }
+}
+
+__device__ __forceinline__ void dense_pattern(const DenseGraph &g, int pattern, int part, int parts,
+                                              unsigned *smem, const BlockSums &bs) {
+  switch (pattern) {
+    case 1: return dense_words_of<motif_needs(1)>(g, part, parts, smem, bs);
+    case 2: return dense_words_of<motif_needs(2)>(g, part, parts, smem, bs);
+    case 3: return dense_words_of<motif_needs(3)>(g, part, parts, smem, bs);
+    case 4: return dense_words_of<motif_needs(4)>(g, part, parts, smem, bs);
+    case 5: return dense_words_of<motif_needs(5)>(g, part, parts, smem, bs);
+    case 6: return dense_words_of<motif_needs(6)>(g, part, parts, smem, bs);
+    default: return dense_words_of<motif_needs(7)>(g, part, parts, smem, bs);  // 7 and 8 alike
+  }
+}
+
 __global__ void __launch_bounds__(kDenseThreads) dense_kernel(DenseGraph g, int pattern, u64 *acc) {
   extern __shared__ unsigned smem[];
   __shared__ u64 sm[kSums];
   const BlockSums bs{sm};
   bs.init();
-  dense_sums(g, motif_needs(pattern), blockIdx.x, gridDim.x, smem, bs);
+  dense_pattern(g, pattern, blockIdx.x, gridDim.x, smem, bs);
   bs.flush(acc);
 }
 
 // A batch's small pattern graphs: one CTA per part (task) of a graph; acc
 // holds kSums per batch graph.
-__global__ void __launch_bounds__(kDenseThreads) dense_batch_kernel(
+__global__ void __launch_bounds__(kBatchThreads) dense_batch_kernel(
     const int64_t *__restrict__ rp, const int32_t *__restrict__ ci,
     const DenseTask *__restrict__ tasks, u64 *acc) {
   extern __shared__ unsigned smem[];
@@ -245,7 +278,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_batch_kernel(
   const BlockSums bs{sm};
   bs.init();
   const DenseTask t = tasks[blockIdx.x];
-  dense_sums(DenseGraph{rp, ci, t.v0, t.n}, motif_needs(t.job), t.part, t.parts, smem, bs);
+  dense_pattern(DenseGraph{rp, ci, t.v0, t.n}, t.job, t.part, t.parts, smem, bs);
   bs.flush(acc + (int64_t)t.graph * kSums);
 }
 
@@ -281,12 +314,23 @@ int dense_count(mc_dgraph *g, int pattern, uint64_t *out) {
   return rc;
 }
 
+// Parts of one graph of a batch: about 1 M row words each (pairs, and three
+// rows per two-path, bounded through the largest degree), so that a batch's
+// largest graphs do not end it on one SM, while few CTAs build a matrix again.
+// 512 graphs (57 triangle jobs, 455 patterns on RMAT scale 5 to 8), whole
+// batch: 1.50, 1.42, 1.33, 1.28, 1.24 and 1.23 ms at 2^15 to 2^20 words, 2.8 ms
+// with one part per graph.
+int dense_parts(int64_t n, int64_t nnz, int64_t max_degree) {
+  const int64_t words = dense_words((int)n) * (n * n / 2 + 3 * nnz * max_degree / 2);
+  return (int)std::max<int64_t>(1, std::min<int64_t>(64, words >> 20));
+}
+
 int dense_batch_launch(const int64_t *rp, const int32_t *ci, const DenseTask *tasks, int num_tasks,
                        int largest, unsigned long long *acc, cudaStream_t s) {
   const size_t smem = dense_bytes(largest);
   MC_CUDA_TRY(cudaFuncSetAttribute(dense_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)dense_bytes(kDenseMax)));
-  dense_batch_kernel<<<num_tasks, kDenseThreads, smem, s>>>(rp, ci, tasks, acc);
+  dense_batch_kernel<<<num_tasks, kBatchThreads, smem, s>>>(rp, ci, tasks, acc);
   MC_CUDA_TRY(cudaGetLastError());
   return MC_OK;
 }

@@ -181,6 +181,7 @@ struct DenseTask {
 };
 // acc: the motif sums of every batch graph (zeroed by the caller); largest:
 // the most vertices among the tasks' graphs.
+int dense_parts(int64_t n, int64_t nnz, int64_t max_degree);
 int dense_batch_launch(const int64_t *rp, const int32_t *ci, const DenseTask *tasks, int num_tasks,
                        int largest, unsigned long long *acc, cudaStream_t s);
 // Contract checks of the row offsets alone; sets max_degree.

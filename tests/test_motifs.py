@@ -12,7 +12,7 @@ import pytest
 
 from brute import random_graph
 from conftest import csr_from_edges
-from mercury_b200 import DeviceGraph, Graph
+from mercury_b200 import Batch, DeviceGraph, Graph
 from oracle import oracle as orc
 
 
@@ -167,3 +167,27 @@ def test_motif_route_on_a_clique_with_a_tail(monkeypatch, n):
     want[5], want[7] = 2 * math.comb(n - 1, 2), 3 * math.comb(n - 1, 3)
     with DeviceGraph(rp, col) as d:
         assert [d.pattern_count(k) for k in patterns] == [want[k - 1] for k in patterns]
+
+
+@pytest.mark.gpu
+def test_batch_bit_rows_at_word_edges(monkeypatch):
+    """Every pattern of graphs at the edges of the bit rows' words and of
+    their largest size (1,024 vertices), beside a triangle job and a larger
+    pattern graph: the batch's counts are the formula routes'."""
+    sizes = [1, 2, 31, 32, 33, 64, 65, 128, 129, 256, 257, 700, 1024, 1025]
+    graphs, jobs = [], []
+    for i, n in enumerate(sizes):
+        g = (Graph.chung_lu(n, 2.1, 8.0, 60.0, seed=i + 1) if n > 8 else
+             Graph.from_csr(*csr_from_edges(n, random_graph(n, 1.0, i))))
+        graphs += [g] * 9
+        jobs += list(range(9))
+    with Batch(graphs, jobs) as b:
+        got = b.count().tolist()
+        b.autotune()
+        assert b.count().tolist() == got
+    monkeypatch.setenv("MERCURY_MOTIF_ROUTE", "formula")
+    want = []
+    for g in graphs[::9]:
+        with DeviceGraph(g) as d:
+            want += [d.tc_count()] + [d.pattern_count(k) for k in range(1, 9)]
+    assert got == want
