@@ -30,6 +30,7 @@ struct DenseGraph {
   const int32_t *__restrict__ ci;
   int64_t v0;
   int n;
+  int64_t nnz = 0;  // entries the caller gave (checked loads only)
 };
 
 // Rows of W words (1, 2, 4, 8 or above 256 vertices what n takes: the loops
@@ -42,6 +43,61 @@ __host__ __device__ constexpr int dense_words(int n) {
 __host__ __device__ constexpr int dense_stride(int n) { return dense_words(n) | 1; }
 size_t dense_bytes(int n) { return sizeof(int) * ((size_t)n * dense_stride(n) + n + 1); }
 
+// The last row starting at or before entry e.
+__device__ __forceinline__ int row_of(const int *off, int n, int e) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (off[mid] <= e) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+// The graph's matrix and row offsets into shared memory, by the whole CTA.
+// kCheck: a whole CSR against its contract, what breaks it in *err; false
+// (on every thread) when the offsets do, and then no entry is read.  An id
+// outside the graph sets nothing.
+template <bool kCheck>
+__device__ __forceinline__ bool load_matrix(const DenseGraph &g, unsigned *bits, int *off, int P,
+                                            unsigned *err) {
+  const int n = g.n;
+  const int64_t base = kCheck ? 0 : __ldg(g.rp + g.v0);
+  int bad_rows = 0;
+  for (int i = threadIdx.x; i <= n; i += blockDim.x) {
+    const int64_t a = __ldg(g.rp + g.v0 + i);
+    if (kCheck)
+      bad_rows |= a < 0 || a > g.nnz || (i == 0 && a != 0) || (i == n && a != g.nnz) ||
+                  (i < n && __ldg(g.rp + i + 1) < a);
+    off[i] = (int)(a - base);
+  }
+  for (int i = threadIdx.x; i < n * P; i += blockDim.x) bits[i] = 0;
+  if (kCheck) {
+    if (__syncthreads_or(bad_rows)) {
+      if (threadIdx.x == 0) atomicOr(err, (unsigned)kErrRowptr);
+      return false;
+    }
+  } else {
+    __syncthreads();
+  }
+  const int nnz = off[n];
+  for (int e = threadIdx.x; e < nnz; e += blockDim.x) {
+    const int64_t id = (int64_t)__ldg(g.ci + base + e) - g.v0;
+    const int r = row_of(off, n, e), x = (int)id;
+    if (kCheck) {
+      unsigned bad = 0;
+      if (id < 0 || id >= n) bad |= kErrIdRange;
+      if (id == r) bad |= kErrSelfLoop;
+      if (e > off[r] && __ldg(g.ci + e - 1) >= id) bad |= kErrUnsorted;
+      if (bad) atomicOr(err, bad);
+      if (bad & kErrIdRange) continue;
+    }
+    atomicOr(bits + r * P + (x >> 5), 1u << (x & 31));
+  }
+  __syncthreads();
+  return true;
+}
+
 // Adds this part's share of the graph's sums: warp tasks of (vertex) and of
 // (vertex t, 32 vertices s below it), dealt round-robin over the warps of all
 // parts.  need: Need bits; kW: words of a row, 0 above 8; smem: dense_bytes(n).
@@ -52,22 +108,7 @@ __device__ __forceinline__ void dense_sums(const DenseGraph &g, int part, int pa
   unsigned *bits = smem;
   int *off = reinterpret_cast<int *>(smem + (size_t)n * P);
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
-  const int64_t base = __ldg(g.rp + g.v0);
-  for (int i = threadIdx.x; i <= n; i += blockDim.x) off[i] = (int)(__ldg(g.rp + g.v0 + i) - base);
-  for (int i = threadIdx.x; i < n * P; i += blockDim.x) bits[i] = 0;
-  __syncthreads();
-  const int nnz = off[n];
-  for (int e = threadIdx.x; e < nnz; e += blockDim.x) {
-    const int x = (int)(__ldg(g.ci + base + e) - g.v0);
-    int lo = 0, hi = n - 1;  // the last row starting at or before e
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (off[mid] <= e) lo = mid;
-      else hi = mid - 1;
-    }
-    atomicOr(bits + lo * P + (x >> 5), 1u << (x & 31));
-  }
-  __syncthreads();
+  load_matrix<false>(g, bits, off, P, nullptr);
   auto deg = [&](int v) { return (u64)(off[v + 1] - off[v]); };
   const int gw = part * (blockDim.x / kWarp) + warp, step = parts * (blockDim.x / kWarp);
   constexpr bool tau = need & kNeedTau, pairs = need & kNeedPairs, wheel = need & kNeedW4;
@@ -282,7 +323,53 @@ __global__ void __launch_bounds__(kBatchThreads) dense_batch_kernel(
   bs.flush(acc + (int64_t)t.graph * kSums);
 }
 
+// Triangles: for each entry (s -> t) with s < t, the common neighbours above t.
+template <bool kCheck>
+__global__ void __launch_bounds__(kDenseThreads) dense_triangles_kernel(DenseGraph g, u64 *count,
+                                                                        unsigned *err) {
+  extern __shared__ unsigned smem[];
+  __shared__ u64 s_total;
+  if (threadIdx.x == 0) s_total = 0;
+  const int n = g.n, W = dense_words(n), P = W | 1;
+  int *off = reinterpret_cast<int *>(smem + (size_t)n * P);
+  if (!load_matrix<kCheck>(g, smem, off, P, err)) return;
+  const int nnz = off[n];
+  u64 hits = 0;
+  for (int e = blockIdx.x * kDenseThreads + threadIdx.x; e < nnz; e += gridDim.x * kDenseThreads) {
+    const int t = __ldg(g.ci + __ldg(g.rp + g.v0) + e) - (int)g.v0;
+    const int s = row_of(off, n, e);
+    if (t <= s || (kCheck && t >= n)) continue;
+    const unsigned *rs = smem + s * P, *rt = smem + t * P;
+    for (int w = t >> 5; w < W; ++w) hits += __popc(rs[w] & rt[w] & above(t, w));
+  }
+  hits = warp_sum_u64(hits);
+  if ((threadIdx.x & (kWarp - 1)) == 0 && hits) atomicAdd(&s_total, hits);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_total) atomicAdd(count, s_total);
+}
+
 }  // namespace
+
+// Triangles of g (at most kDenseMax vertices) into counters[0]; check: a CSR
+// that nothing has looked at yet, its contract errors in the low half of
+// counters[1].  Asynchronous.
+int dense_triangles(mc_dgraph *g, bool check) {
+  cudaStream_t s = g->stream;
+  const int n = (int)g->n;
+  const size_t smem = dense_bytes(n);
+  auto kern = check ? dense_triangles_kernel<true> : dense_triangles_kernel<false>;
+  MC_CUDA_TRY(cudaMemsetAsync(g->counters, 0, 2 * sizeof(u64), s));
+  if (smem > (size_t(40) << 10))
+    MC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // About 2^16 row words per CTA: each builds the matrix for itself.
+  const int64_t words = g->nnz * dense_words(n) / 2;
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(g->num_sms, words >> 16));
+  kern<<<grid, kDenseThreads, smem, s>>>(DenseGraph{g->rowptr, g->col, 0, n, g->nnz}, g->counters,
+                                         reinterpret_cast<unsigned *>(g->counters + 1));
+  MC_CUDA_TRY(cudaGetLastError());
+  g->launches += 1;
+  return MC_OK;
+}
 
 int dense_count(mc_dgraph *g, int pattern, uint64_t *out) {
   cudaStream_t s = g->stream;

@@ -88,6 +88,8 @@ struct mc_dgraph {
 
   // ---- triangle-count scratch, allocated on the first mc_tc_count -------
   bool tc_ready = false;
+  bool counted = false;      // mc_tc_count has run (by either route)
+  bool dag_built = false;    // the DAG and task lists are this graph's
   int2 *key = nullptr;            // n      {symmetric degree, DAG out-degree}
   // n: {d+, rank (INT_MAX without ranks), DAG row start low, high}: what a
   // hub task needs of a neighbour, in one 16-byte load.
@@ -174,6 +176,7 @@ PatternRoute pattern_route(const mc_dgraph *g, int pattern);
 constexpr int kDenseMax = 1024;
 int motif_count(mc_dgraph *g, int pattern, uint64_t *out);
 int dense_count(mc_dgraph *g, int pattern, uint64_t *out);
+int dense_triangles(mc_dgraph *g, bool check);
 // Part `part` of `parts` of one pattern graph of a batch.
 struct DenseTask {
   int64_t v0;

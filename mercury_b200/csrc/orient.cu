@@ -829,6 +829,7 @@ int tc_orient(mc_dgraph *g, const int32_t *upload) {
   cudaStream_t s = g->stream;
   MC_CUDA_TRY(cudaMemsetAsync(g->counters, 0, sizeof(unsigned long long) * 7, s));
   g->core_used = 0;
+  g->dag_built = false;
   if (n == 0) return MC_OK;
   const int64_t tiles = (nnz + kTileEdges - 1) / kTileEdges;
   // The degrees alone, for pass A's gathers, in mega_cnt (unused until the
@@ -907,6 +908,7 @@ int tc_orient(mc_dgraph *g, const int32_t *upload) {
                                                     g->hub_tasks, g->leaf_tasks, g->mega_tasks);
   MC_CUDA_TRY(cudaGetLastError());
   g->launches += 2 + 3 * scan_launches(n);
+  g->dag_built = true;
   return MC_OK;
 }
 
