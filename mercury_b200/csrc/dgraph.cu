@@ -27,9 +27,9 @@ void release(mc_dgraph *g) {
   cudaSetDevice(g->device);
   void *bufs[] = {g->rowptr,     g->col,        g->key,      g->dag_rowptr,
                   g->dag_col,    g->keep,       g->tile_counts, g->tile_offsets,
-                  g->hub_cnt,    g->leaf_cnt,   g->hub_off,  g->leaf_off,  g->hub_tasks,
+                  g->deg,        g->list_len,   g->task_status, g->hub_tasks,
                   g->leaf_tasks, g->scan_temp,  g->counters, g->err, g->pat_scratch,
-                  g->mega_cnt,   g->mega_off,   g->mega_tasks, g->rank,
+                  g->mega_tasks, g->rank,
                   g->dag_rank,   g->rank_keys,  g->rank_counts, g->rank_offsets,
                   g->center_scratch, g->stage, g->chunk_offsets, g->core_bits, g->pinfo,
                   g->hop_scratch, g->hub_bits, g->vlabels, g->tile_rows};
@@ -257,8 +257,7 @@ int tc_stats(mc_dgraph *g, mc_tc_stats_t *st) {
   const int drc = ensure_dag(g);
   if (drc != MC_OK) return drc;
   int64_t v[4] = {0, 0, 0, 0};
-  const int64_t *src[4] = {g->dag_rowptr + g->n, g->hub_off + g->n, g->leaf_off + g->n,
-                           g->mega_off + g->n};
+  const int64_t *src[4] = {g->dag_rowptr + g->n, g->list_len, g->list_len + 1, g->list_len + 2};
   for (int i = 0; i < 4; ++i)
     MC_CUDA_TRY(cudaMemcpyAsync(&v[i], src[i], sizeof(int64_t), cudaMemcpyDeviceToHost, g->stream));
   unsigned long long maxd = 0;
@@ -501,16 +500,22 @@ int tc_count_impl(mc_dgraph_t *g, int shard, int num_shards, uint64_t *count,
   rc = tc_orient(g, upload);
   if (rc != MC_OK) return rc;
   MC_CUDA_TRY(cudaEventRecord(g->ev[1], s));
-  // The hub table size follows the largest DAG out-degree (load <= 1/4).
-  MC_CUDA_TRY(cudaMemcpyAsync(g->h_counters + 3, g->counters + 3, sizeof(unsigned long long),
-                              cudaMemcpyDeviceToHost, s));
-  MC_CUDA_TRY(cudaMemcpyAsync(g->h_err, g->err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-  MC_CUDA_TRY(cudaStreamSynchronize(s));
-  // An exact-size DAG (host columns) that the rows overran (the input is not
-  // symmetric), or a streamed chunk that failed its contract checks: the DAG
-  // was left unwritten.
-  if (*g->h_err & (kErrDagCapacity | kErrContract)) return MC_ERR_FORMAT;
-  const long long maxd = (long long)g->h_counters[3];
+  // The hub table size follows the largest DAG out-degree (load <= 1/4): the
+  // device's, or, while tables for the bound on it cost no occupancy (they fit
+  // the shared memory every hub CTA has), the bound, which needs no wait.
+  long long maxd = g->max_out_bound;
+  const bool wait = upload || g->col_host || 4 * sizeof(int) * maxd > (size_t)kHubBitmapBytes;
+  if (wait) {
+    MC_CUDA_TRY(cudaMemcpyAsync(g->h_counters + 3, g->counters + 3, sizeof(unsigned long long),
+                                cudaMemcpyDeviceToHost, s));
+    MC_CUDA_TRY(cudaMemcpyAsync(g->h_err, g->err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    MC_CUDA_TRY(cudaStreamSynchronize(s));
+    // An exact-size DAG (host columns) that the rows overran (the input is not
+    // symmetric), or a streamed chunk that failed its contract checks: the DAG
+    // was left unwritten.
+    if (*g->h_err & (kErrDagCapacity | kErrContract)) return MC_ERR_FORMAT;
+    maxd = (long long)g->h_counters[3];
+  }
   // MERCURY_TC_TABLE_LOG2_MAX (8..15) lowers the shared-memory table cap;
   // owners whose list no longer fits are then probed by binary search in
   // global memory (tests use it to reach that path on small graphs).

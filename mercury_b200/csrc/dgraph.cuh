@@ -107,6 +107,8 @@ struct mc_dgraph {
   int64_t *rank_offsets = nullptr;
   const unsigned long long *rank_sorted = nullptr;  // rank p -> key of vertex (see orient.cu)
   unsigned *core_bits = nullptr;  // core_offset(core_ranks) words
+  bool ranked = false;            // this graph's ranks are set (it may have hub owners)
+  int64_t max_out_bound = 0;      // no d+ exceeds it
   int core_ranks = 0;             // capacity: core_offset(core_ranks) words
   int core_used = 0;              // ranks [0, core_used) have core bitmaps (<= n)
   int dense_factor = 2;           // AND when its words <= factor x list entries
@@ -120,8 +122,9 @@ struct mc_dgraph {
   int32_t *pin_slot[2] = {nullptr, nullptr};
   int64_t pin_entries = 0;
   cudaEvent_t pin_done[2] = {nullptr, nullptr};
-  int32_t *hub_cnt = nullptr, *leaf_cnt = nullptr, *mega_cnt = nullptr;    // n
-  int64_t *hub_off = nullptr, *leaf_off = nullptr, *mega_off = nullptr;    // n + 1
+  int32_t *deg = nullptr;         // n      degrees alone
+  int64_t *list_len = nullptr;    // 3      lengths of the hub, leaf and mega lists
+  unsigned long long *task_status = nullptr;  // chained scans of the task lists
   uint64_t *hub_tasks = nullptr, *leaf_tasks = nullptr, *mega_tasks = nullptr;  // capacity
   int64_t task_capacity = 0;
   // Host columns: two DMA staging buffers of stage_edges entries each, the

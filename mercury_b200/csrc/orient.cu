@@ -21,13 +21,15 @@
 //   B  DAG entries and row offsets written from the keep masks
 // Each vertex's (degree, d+) pair is one 8-byte word (key[]).
 #include <algorithm>
-#include <cstring>
 #include <climits>
+#include <cmath>
+#include <cstring>
 #include <cstdio>
 #include <cstdlib>
 
 #include "dgraph.cuh"
 #include "device_common.cuh"
+#include "lookback.cuh"
 #include "radix.cuh"
 #include "scan.cuh"
 
@@ -443,20 +445,12 @@ __global__ void core_bits_kernel(const unsigned long long *__restrict__ sorted, 
   }
 }
 
-// pinfo[v] = {d+(v), rank(v) (INT_MAX without ranks), dag_rowptr[v]}.
-__global__ void partner_info_kernel(const int2 *__restrict__ key, const int32_t *__restrict__ rank,
-                                    const int64_t *__restrict__ dag_rowptr, int64_t n,
-                                    int4 *__restrict__ pinfo) {
-  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n) return;
-  const long long st = dag_rowptr[v];
-  pinfo[v] = make_int4(key[v].y, rank ? rank[v] : INT_MAX, (int)(unsigned)(st & 0xffffffffll),
-                       (int)(st >> 32));
-}
-
 // key[v] = {degree, 0}; deg[v] = degree alone (4 bytes per gather in pass A).
-__global__ void init_key_kernel(const int64_t *rowptr, int64_t n, int2 *key, int32_t *deg) {
+// The first `words` words of status are cleared (words <= n + 4).
+__global__ void init_key_kernel(const int64_t *rowptr, int64_t n, int2 *key, int32_t *deg,
+                                unsigned long long *status, int64_t words) {
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v < words) status[v] = 0;
   if (v < n) {
     const int d = (int)(rowptr[v + 1] - rowptr[v]);
     key[v] = make_int2(d, 0);
@@ -464,17 +458,51 @@ __global__ void init_key_kernel(const int64_t *rowptr, int64_t n, int2 *key, int
   }
 }
 
-// Tasks each owner contributes to the hub, large-table hub and leaf queues
-// (chunks of its symmetric row), and the largest DAG out-degree.
-__global__ void task_count_kernel(const int2 *key, int64_t n, int32_t *hub_cnt,
-                                  int32_t *leaf_cnt, int32_t *mega_cnt,
-                                  unsigned long long *max_out, BatchView bv) {
-  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int32_t d = 0;
-  if (v < n) {
+struct TaskLists {
+  int64_t *hub_end, *leaf_end, *mega_end;  // receive the lists' lengths
+  uint64_t *hub, *leaf, *mega;
+  // One running sum per list and block (kTaskThreads x kTaskItems vertices), a
+  // ticket; cleared by init_key_kernel.
+  unsigned long long *status;
+  int64_t blocks;
+};
+constexpr int kTaskThreads = 256, kTaskItems = 4;  // vertices per thread
+
+// pinfo[v] = {d+(v), rank(v) (INT_MAX without ranks), dag_rowptr[v]}; the
+// largest d+; and the tasks of each owner (chunks of its symmetric row; a task
+// word is the owner in the high half, the chunk in the low half), appended to
+// the hub, leaf and large-table hub lists in vertex order: shards name tasks
+// by position, and the leaf kernel took 849 instead of 632 us on a Chung-Lu
+// graph of 2 M vertices with the blocks' tasks in order of arrival.  One launch
+// with a chained scan per list; a counting kernel, three scans and a filling
+// kernel took 188 us there and 64 us at RMAT scale 16.
+__global__ void __launch_bounds__(kTaskThreads) partner_tasks_kernel(
+    const int2 *__restrict__ key, const int32_t *__restrict__ rank,
+    const int64_t *__restrict__ dag_rowptr, int64_t n, int4 *__restrict__ pinfo, TaskLists t,
+    unsigned long long *max_out, BatchView bv, unsigned *err) {
+  constexpr int kW = kTaskThreads / kWarp;
+  __shared__ int s_warp[3][kW];
+  __shared__ int s_max[kW];
+  __shared__ int64_t s_base[3], s_block;
+  if (threadIdx.x == 0) s_block = (int64_t)atomicAdd(t.status + 3 * t.blocks, 1ull);
+  __syncthreads();
+  const int64_t block = s_block;
+  const int64_t v0 = (block * kTaskThreads + threadIdx.x) * kTaskItems;
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  int dmax = 0, c[3] = {0, 0, 0};  // hub, leaf, mega
+  int own[kTaskItems], chunks[kTaskItems];  // each vertex's list (-1: none) and tasks
+#pragma unroll
+  for (int i = 0; i < kTaskItems; ++i) {
+    const int64_t v = v0 + i;
+    own[i] = -1;
+    chunks[i] = 0;
+    if (v >= n) continue;
     const int2 kv = key[v];
-    d = kv.y;
-    int32_t h = 0, l = 0, m = 0;
+    const int d = kv.y;
+    dmax = max(dmax, d);
+    const long long st = dag_rowptr[v];
+    pinfo[v] = make_int4(d, rank ? rank[v] : INT_MAX, (int)(unsigned)(st & 0xffffffffll),
+                         (int)(st >> 32));
     int leaf_max = kLeafMaxOut;
     bool counted = true;
     if (bv.gid) {  // batch: only triangle jobs get tasks, with their graph's threshold
@@ -484,30 +512,52 @@ __global__ void task_count_kernel(const int2 *key, int64_t n, int32_t *hub_cnt,
     }
     // Owners need d+ >= 1; every neighbour of the row may be a partner.
     if (counted && d >= 1) {
-      if (d <= leaf_max) l = (kv.x + kLeafChunk - 1) / kLeafChunk;
-      else if (d <= kHubSmallMaxOut) h = (kv.x + kHubChunk - 1) / kHubChunk;
-      else m = (kv.x + kHubChunk - 1) / kHubChunk;
-    }
-    hub_cnt[v] = h;
-    leaf_cnt[v] = l;
-    mega_cnt[v] = m;
-  }
+      own[i] = d <= leaf_max ? 1 : d <= kHubSmallMaxOut ? 0 : 2;
+      const int per = own[i] == 1 ? kLeafChunk : kHubChunk;
+      chunks[i] = (kv.x + per - 1) / per;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) d = max(d, __shfl_down_sync(kFull, d, o));
-  if ((threadIdx.x & 31) == 0 && d > 0) atomicMax(max_out, (unsigned long long)d);
-}
-
-// Task word: owner id in the high half, chunk index in the low half.
-__global__ void task_fill_kernel(const int32_t *hub_cnt, const int64_t *hub_off,
-                                 const int32_t *leaf_cnt, const int64_t *leaf_off,
-                                 const int32_t *mega_cnt, const int64_t *mega_off, int64_t n,
-                                 uint64_t *hub_tasks, uint64_t *leaf_tasks, uint64_t *mega_tasks) {
-  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n) return;
-  const uint64_t hi = (uint64_t)v << 32;
-  for (int32_t c = 0, h = hub_cnt[v]; c < h; ++c) hub_tasks[hub_off[v] + c] = hi | (uint32_t)c;
-  for (int32_t c = 0, l = leaf_cnt[v]; c < l; ++c) leaf_tasks[leaf_off[v] + c] = hi | (uint32_t)c;
-  for (int32_t c = 0, m = mega_cnt[v]; c < m; ++c) mega_tasks[mega_off[v] + c] = hi | (uint32_t)c;
+      for (int k = 0; k < 3; ++k) c[k] += own[i] == k ? chunks[i] : 0;
+    }
+  }
+  int incl[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) incl[k] = warp_inclusive_scan(c[k], lane);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dmax = max(dmax, __shfl_xor_sync(kFull, dmax, o));
+  if (lane == kWarp - 1) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) s_warp[k][warp] = incl[k];
+    s_max[warp] = dmax;
+  }
+  __syncthreads();
+  if (warp < 3) {  // warp k: list k
+    unsigned long long sum = 0;
+    for (int w = 0; w < kW; ++w) sum += (unsigned)s_warp[warp][w];
+    const unsigned long long before = tile_prefix(t.status + warp * t.blocks, block, sum, lane, err);
+    if (lane == 0) {
+      s_base[warp] = (int64_t)before;
+      if (block == t.blocks - 1)
+        *(warp == 0 ? t.hub_end : warp == 1 ? t.leaf_end : t.mega_end) = (int64_t)(before + sum);
+    }
+  } else if (warp == 3 && lane == 0) {
+    int m = 0;
+    for (int w = 0; w < kW; ++w) m = max(m, s_max[w]);
+    if (m > 0) atomicMax(max_out, (unsigned long long)m);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (c[k] == 0) continue;
+    uint64_t *out = k == 0 ? t.hub : k == 1 ? t.leaf : t.mega;
+    int64_t at = s_base[k] + incl[k] - c[k];
+    for (int w = 0; w < warp; ++w) at += s_warp[k][w];
+#pragma unroll
+    for (int i = 0; i < kTaskItems; ++i) {
+      if (own[i] != k) continue;
+      const uint64_t hi = (uint64_t)(v0 + i) << 32;
+      for (int j = 0; j < chunks[i]; ++j) out[at++] = hi | (uint32_t)j;
+    }
+  }
 }
 
 // Partner edges (owner rule) and their streamed-list work, for statistics:
@@ -629,10 +679,13 @@ int64_t stage_capacity(int64_t nnz) {
   return std::min(stage, std::max<int64_t>((nnz + kTileEdges - 1) / kTileEdges, 1) * kTileEdges);
 }
 
-// Ranks with core bitmaps: kCoreRanks, or MERCURY_TC_CORE_RANKS (0 turns
-// them off; tests move the boundary with it), at most n.
+// Ranks with core bitmaps: kCoreRanks, on small graphs a sixteenth of the
+// vertices (clearing 67 MB of bitmaps and filling them cost more than the hub
+// kernel gained there: 521 -> 499 us per count at RMAT scale 16, 0.944 -> 0.933
+// ms at 18), or MERCURY_TC_CORE_RANKS (0 turns them off; tests move the
+// boundary with it), at most n.
 int core_rank_count(int64_t n) {
-  int64_t k = kCoreRanks;
+  int64_t k = std::min<int64_t>(kCoreRanks, n / 16);
   if (const char *env = std::getenv("MERCURY_TC_CORE_RANKS")) {
     const long long v = std::atoll(env);
     if (v >= 0) k = std::min<long long>(v, 1 << 18);
@@ -644,11 +697,10 @@ int64_t tc_device_bytes(int64_t n, int64_t nnz, bool col_host, bool dag_host) {
   const int64_t cap = std::max<int64_t>(nnz, 1);
   const int64_t tiles = std::max<int64_t>((nnz + kTileEdges - 1) / kTileEdges, 1);
   const int64_t tasks = n + cap / std::min(kHubChunk, kLeafChunk) + 1;
-  const int64_t scan = (int64_t)std::max(std::max(scan_temp_bytes(n + 1), scan_temp_bytes(tiles + 1)),
-                                         radix_temp_bytes(n));
+  const int64_t scan = (int64_t)std::max(scan_temp_bytes(tiles + 1), radix_temp_bytes(n));
   const int64_t staging =
       col_host ? 2 * 4 * stage_capacity(nnz) + 8 * (stage_capacity(nnz) / kTileEdges + 1) : 0;
-  return (n + 1) * (8 + 16 + 8 + 3 * 4 + 3 * 8 + 4 + 16) + 3 * 8 * tasks +
+  return (n + 1) * (8 + 16 + 8 + 4 + 4 + 16) + n / 8 + 3 * 8 * tasks +
          (dag_host ? 0 : 2 * 4 * (dag_capacity(nnz, col_host) + 4)) +
          tiles * (2 * kTileThreads + 28) +
          2 * 12 * (radix_entries(n) + 1) + scan + staging + 4 * core_offset(core_rank_count(n));
@@ -661,7 +713,7 @@ int tc_alloc(mc_dgraph *g) {
   g->dag_cap = dag_capacity(g->nnz, g->col_host);
   // Each owner contributes ceil(deg / chunk) <= 1 + deg / chunk tasks.
   g->task_capacity = n + cap / std::min(kHubChunk, kLeafChunk) + 1;
-  g->scan_temp_size = std::max(scan_temp_bytes(n + 1), scan_temp_bytes(tiles + 1));
+  g->scan_temp_size = scan_temp_bytes(tiles + 1);
   const bool ranked = g->batch.gid == nullptr;
   if (ranked) g->scan_temp_size = std::max(g->scan_temp_size, radix_temp_bytes(n));
 #define MC_ALLOC(ptr, count) \
@@ -684,14 +736,11 @@ int tc_alloc(mc_dgraph *g) {
   MC_ALLOC(g->tile_counts, tiles);
   MC_ALLOC(g->tile_offsets, tiles + 1);
   MC_ALLOC(g->tile_rows, 2 * tiles);
-  MC_ALLOC(g->hub_cnt, n + 1);
-  MC_ALLOC(g->leaf_cnt, n + 1);
-  MC_ALLOC(g->hub_off, n + 1);
-  MC_ALLOC(g->leaf_off, n + 1);
+  MC_ALLOC(g->deg, n + 1);
+  MC_ALLOC(g->list_len, 3);
+  MC_ALLOC(g->task_status, n / kTaskThreads + 4);  // at least 3 per block of 1,024, and a ticket
   MC_ALLOC(g->hub_tasks, g->task_capacity);
   MC_ALLOC(g->leaf_tasks, g->task_capacity);
-  MC_ALLOC(g->mega_cnt, n + 1);
-  MC_ALLOC(g->mega_off, n + 1);
   MC_ALLOC(g->mega_tasks, g->task_capacity);
   if (ranked) {
     MC_ALLOC(g->rank, n + 1);
@@ -814,8 +863,8 @@ static int staged_dag_passes(mc_dgraph *g, const int32_t *deg, const int32_t *sr
     (stage_dag_writes() ? dag_pass_kernel<true, true> : dag_pass_kernel<true, false>)
         <<<(unsigned)ct, kTileThreads, 0, s>>>(
         g->rowptr, cc, deg, n, nnz, g->key, g->keep, nullptr, g->tile_offsets, g->dag_rowptr,
-        g->dag_col, g->rank, g->dag_rank, g->tile_offsets + tb + ct, g->dag_cap, stop,
-        g->tile_rows);
+        g->dag_col, g->ranked ? g->rank : nullptr, g->ranked ? g->dag_rank : nullptr,
+        g->tile_offsets + tb + ct, g->dag_cap, stop, g->tile_rows);
     MC_CUDA_TRY(cudaGetLastError());
     MC_CUDA_TRY(cudaEventRecord(drained[slot], s));
     g->launches += 3 + scan_launches(ct);
@@ -832,13 +881,19 @@ int tc_orient(mc_dgraph *g, const int32_t *upload) {
   g->dag_built = false;
   if (n == 0) return MC_OK;
   const int64_t tiles = (nnz + kTileEdges - 1) / kTileEdges;
-  // The degrees alone, for pass A's gathers, in mega_cnt (unused until the
-  // task counts are written after pass B).
-  int32_t *deg = g->mega_cnt;
-  init_key_kernel<<<grid_for(n, 256), 256, 0, s>>>(g->rowptr, n, g->key, deg);
+  // The degrees alone, for pass A's gathers.
+  int32_t *deg = g->deg;
+  // d+(v)^2 <= nnz (v's out-neighbours have at least its degree), so without
+  // room for a hub owner nothing reads the ranks.
+  g->max_out_bound = std::min<int64_t>(g->max_degree, (int64_t)std::sqrt((double)nnz) + 1);
+  const bool ranked = g->rank && !g->batch.gid && g->max_out_bound > kLeafMaxOut;
+  g->ranked = ranked;
+  const int64_t task_blocks = (n + kTaskThreads * kTaskItems - 1) / (kTaskThreads * kTaskItems);
+  init_key_kernel<<<grid_for(n + 4, 256), 256, 0, s>>>(g->rowptr, n, g->key, deg, g->task_status,
+                                                       3 * task_blocks + 1);
   MC_CUDA_TRY(cudaGetLastError());
   g->launches += 1;
-  if (g->rank && !g->batch.gid) {
+  if (ranked) {
     // Degree ranks (the hub kernel's bitmaps are indexed by them).
     rank_keys_kernel<<<grid_for(n, 256), 256, 0, s>>>(g->key, n, (int)g->max_degree, g->rank_keys);
     MC_CUDA_TRY(cudaGetLastError());
@@ -878,36 +933,28 @@ int tc_orient(mc_dgraph *g, const int32_t *upload) {
     (stage_dag_writes() ? dag_pass_kernel<true, true> : dag_pass_kernel<true, false>)
         <<<grid, kTileThreads, 0, s>>>(
         g->rowptr, all, deg, n, nnz, g->key, g->keep, nullptr, g->tile_offsets, g->dag_rowptr,
-        g->dag_col, g->batch.gid ? nullptr : g->rank, g->batch.gid ? nullptr : g->dag_rank,
-        nullptr, 0, nullptr, g->tile_rows);
+        g->dag_col, ranked ? g->rank : nullptr, ranked ? g->dag_rank : nullptr, nullptr, 0, nullptr,
+        g->tile_rows);
     MC_CUDA_TRY(cudaGetLastError());
     g->launches += 2 + scan_launches(tiles);
   }
   // A handle reused for a smaller graph keeps its capacity: only the ranks
   // of this graph get core bitmaps.
-  if (g->core_bits && g->rank_sorted && !g->batch.gid) {
-    g->core_used = (int)std::min<int64_t>(g->core_ranks, n);
+  if (g->core_bits && ranked) {
+    g->core_used = std::min(g->core_ranks, core_rank_count(n));
     MC_CUDA_TRY(cudaMemsetAsync(g->core_bits, 0, sizeof(unsigned) * core_offset(g->core_used), s));
     core_bits_kernel<<<grid_for((int64_t)g->core_used * kWarp, 256), 256, 0, s>>>(
         g->rank_sorted, n, g->core_used, g->dag_rowptr, g->dag_rank, g->core_bits, g->err);
     MC_CUDA_TRY(cudaGetLastError());
     g->launches += 1;
   }
-  partner_info_kernel<<<grid_for(n, 256), 256, 0, s>>>(
-      g->key, g->batch.gid ? nullptr : g->rank, g->dag_rowptr, n, g->pinfo);
+  partner_tasks_kernel<<<(unsigned)task_blocks, kTaskThreads, 0, s>>>(
+      g->key, ranked ? g->rank : nullptr, g->dag_rowptr, n, g->pinfo,
+      TaskLists{g->list_len, g->list_len + 1, g->list_len + 2, g->hub_tasks, g->leaf_tasks,
+                g->mega_tasks, g->task_status, task_blocks},
+      g->counters + 3, g->batch, g->err);
   MC_CUDA_TRY(cudaGetLastError());
   g->launches += 1;
-  task_count_kernel<<<grid_for(n, 256), 256, 0, s>>>(g->key, n, g->hub_cnt, g->leaf_cnt,
-                                                     g->mega_cnt, g->counters + 3, g->batch);
-  MC_CUDA_TRY(cudaGetLastError());
-  MC_CUDA_TRY(exclusive_scan(g->hub_cnt, g->hub_off, n, g->scan_temp, s));
-  MC_CUDA_TRY(exclusive_scan(g->leaf_cnt, g->leaf_off, n, g->scan_temp, s));
-  MC_CUDA_TRY(exclusive_scan(g->mega_cnt, g->mega_off, n, g->scan_temp, s));
-  task_fill_kernel<<<grid_for(n, 256), 256, 0, s>>>(g->hub_cnt, g->hub_off, g->leaf_cnt,
-                                                    g->leaf_off, g->mega_cnt, g->mega_off, n,
-                                                    g->hub_tasks, g->leaf_tasks, g->mega_tasks);
-  MC_CUDA_TRY(cudaGetLastError());
-  g->launches += 2 + 3 * scan_launches(n);
   g->dag_built = true;
   return MC_OK;
 }

@@ -907,14 +907,17 @@ __global__ void __launch_bounds__(kCountThreads) tc_leaf_kernel(CountArgs a) {
   const CuckooProbe probe{tab, 32 - lg};
   const int64_t ntasks = shard_tasks(a);
   unsigned long long hits = 0;
-  // Tasks are claimed kLeafClaim at a time: one queue atomic per 16 tasks
-  // instead of per task (millions of them contend on one address).
-  constexpr unsigned long long kLeafClaim = 16;
-  unsigned long long batch = 0, used = kLeafClaim;
+  // Tasks are claimed up to 16 at a time: one queue atomic per 16 tasks
+  // instead of per task (millions of them contend on one address), fewer while
+  // that would leave warps without any (RMAT scale 16: 49,877 tasks on 7,104
+  // warps, 128 us at 16 a claim).
+  const unsigned long long claim = (unsigned long long)max(
+      1ll, min(16ll, (long long)ntasks / (4ll * gridDim.x * (kCountThreads / kWarp))));
+  unsigned long long batch = 0, used = claim;
   auto next_ticket = [&]() {
-    if (used == kLeafClaim) {
+    if (used == claim) {
       unsigned long long b = 0;
-      if (lane == 0) b = atomicAdd(a.queue, kLeafClaim);
+      if (lane == 0) b = atomicAdd(a.queue, claim);
       batch = __shfl_sync(kFull, b, 0);
       used = 0;
     }
@@ -1022,7 +1025,7 @@ int tc_count_launch(mc_dgraph *g, cudaEvent_t after_hub, int shard, int num_shar
   const int big_lg = std::max(kHubSmallTableLog2, g->hub_table_log2);
   const size_t small_smem = std::max<size_t>(sizeof(int) << small_lg, kHubBitmapBytes);
   const size_t big_smem = std::max<size_t>(sizeof(int) << big_lg, kHubBitmapBytes);
-  const bool ranked = g->rank != nullptr && g->batch.gid == nullptr;
+  const bool ranked = g->ranked && g->batch.gid == nullptr;
   a.rank = ranked ? g->rank : nullptr;
   a.dag_rank = ranked ? g->dag_rank : nullptr;
   a.core = ranked && g->core_used > 0 ? g->core_bits : nullptr;
@@ -1056,31 +1059,40 @@ int tc_count_launch(mc_dgraph *g, cudaEvent_t after_hub, int shard, int num_shar
                                    (int)(big_smem + extra)));
   a.table_log2_max = small_lg;
   a.tasks = g->hub_tasks;
-  a.ntasks = g->hub_off + g->n;
+  a.ntasks = g->list_len;
   a.queue = g->counters + 1;
   // (One quad of each bitmap's shared memory is the probe's zero word.)
   a.bitmap_bits = (int)std::min<size_t>(small_smem * 8 - 128, (size_t)g->bitmap_bits_cap);
   a.stage_off = (int)(small_smem / sizeof(int));
+  // Launches whose tasks the bound on d+ rules out are left out (a batch's
+  // thresholds are its own).
+  const int64_t most = g->batch.gid ? INT_MAX : g->max_out_bound;
   const int small_grid =
       g->num_sms * resident_blocks((const void *)kern, kCountThreads, small_smem + extra);
-  kern<<<small_grid, kCountThreads, small_smem + extra, g->stream>>>(a);
-  MC_CUDA_TRY(cudaGetLastError());
+  if (most > kLeafMaxOut) {
+    kern<<<small_grid, kCountThreads, small_smem + extra, g->stream>>>(a);
+    MC_CUDA_TRY(cudaGetLastError());
+    g->launches += 1;
+  }
   a.table_log2_max = big_lg;
   a.tasks = g->mega_tasks;
-  a.ntasks = g->mega_off + g->n;
+  a.ntasks = g->list_len + 2;
   a.queue = g->counters + 6;
   a.bitmap_bits = (int)std::min<size_t>(big_smem * 8 - 128, (size_t)g->bitmap_bits_cap);
   a.stage_off = (int)(big_smem / sizeof(int));
   const int big_grid =
       g->num_sms * resident_blocks((const void *)kern, kCountThreads, big_smem + extra);
-  kern<<<big_grid, kCountThreads, big_smem + extra, g->stream>>>(a);
-  MC_CUDA_TRY(cudaGetLastError());
-  g->launches += 3;
+  if (most > kHubSmallMaxOut) {
+    kern<<<big_grid, kCountThreads, big_smem + extra, g->stream>>>(a);
+    MC_CUDA_TRY(cudaGetLastError());
+    g->launches += 1;
+  }
+  g->launches += 1;
   if (after_hub) MC_CUDA_TRY(cudaEventRecord(after_hub, g->stream));
 
   const int leaf_grid = g->num_sms * resident_blocks((const void *)tc_leaf_kernel, kCountThreads, 0);
   a.tasks = g->leaf_tasks;
-  a.ntasks = g->leaf_off + g->n;
+  a.ntasks = g->list_len + 1;
   a.queue = g->counters + 2;
   tc_leaf_kernel<<<leaf_grid, kCountThreads, 0, g->stream>>>(a);
   MC_CUDA_TRY(cudaGetLastError());
