@@ -5,7 +5,7 @@
 // 1. Each pair (u, v) becomes two packed keys (u << col_bits | v) and
 //    (v << col_bits | u); a self-loop becomes two "dead" keys whose row field
 //    is n, so they sort after every real entry.
-// 2. An LSD radix sort orders the keys, 8 bits per pass, over exactly the
+// 2. An LSD radix sort orders the keys over exactly the
 //    bits the packing uses (2 * ceil(log2 n) + 1 bits).
 // 3. One pass drops the dead keys and the duplicates, writes the column array
 //    and adds each row's entry count into a degree array; a scan of the
@@ -179,8 +179,9 @@ struct CsrBuild {
   int32_t *own_src = nullptr, *own_dst = nullptr;
   u64 *keys[2] = {nullptr, nullptr};
   int cur = 0;                       // keys[cur] holds the sorted keys
-  int32_t *counts = nullptr;         // kRadixBins * tiles (then tiles) counters
+  int32_t *counts = nullptr;         // distinct entries per tile
   int64_t *offsets = nullptr;        // their exclusive scan
+  void *work = nullptr;              // sort scratch
   void *temp = nullptr;              // scan scratch
   u64 *deg = nullptr;                // n entry counts
   unsigned *flags = nullptr;         // [0] error bits, [2..3] max degree (u64)
@@ -213,11 +214,11 @@ int csr_build_create(int64_t m, int64_t n, cudaStream_t s, CsrBuild **out) {
   if (b->count > 0) {
     MC_CUDA_TRY(dev_alloc((void **)&b->keys[0], sizeof(u64) * (size_t)b->count, s));
     MC_CUDA_TRY(dev_alloc((void **)&b->keys[1], sizeof(u64) * (size_t)b->count, s));
-    const int64_t entries = (int64_t)kRadixBins * b->tiles;
-    MC_CUDA_TRY(dev_alloc((void **)&b->counts, sizeof(int32_t) * (size_t)entries, s));
-    MC_CUDA_TRY(dev_alloc((void **)&b->offsets, sizeof(int64_t) * (size_t)(entries + 1), s));
+    MC_CUDA_TRY(dev_alloc((void **)&b->counts, sizeof(int32_t) * (size_t)b->tiles, s));
+    MC_CUDA_TRY(dev_alloc((void **)&b->offsets, sizeof(int64_t) * (size_t)(b->tiles + 1), s));
+    MC_CUDA_TRY(dev_alloc(&b->work, radix_work_bytes(b->count, b->key_bits), s));
   }
-  const int64_t scan_max = std::max<int64_t>((int64_t)kRadixBins * b->tiles, n);
+  const int64_t scan_max = std::max<int64_t>(b->tiles, n);
   MC_CUDA_TRY(dev_alloc(&b->temp, scan_temp_bytes(scan_max), s));
   return MC_OK;
 }
@@ -253,8 +254,8 @@ int csr_build_sort(CsrBuild *b, int64_t *nnz) {
   ++b->launches;
   b->cur = 0;
   u64 *sorted = nullptr;
-  MC_CUDA_TRY(radix_sort_u64(b->keys[0], b->keys[1], b->count, 0, b->key_bits, b->counts,
-                             b->offsets, b->temp, s, &sorted, &b->launches));
+  MC_CUDA_TRY(radix_sort_u64(b->keys[0], b->keys[1], b->count, 0, b->key_bits, b->work, b->flags, s,
+                             &sorted, &b->launches));
   b->cur = sorted == b->keys[0] ? 0 : 1;
   const unsigned grid = (unsigned)b->tiles;
   unique_count_kernel<<<grid, kSortThreads, 0, s>>>(b->keys[b->cur], b->count, dead, b->counts);
@@ -266,6 +267,7 @@ int csr_build_sort(CsrBuild *b, int64_t *nnz) {
                               cudaMemcpyDeviceToHost, s));
   MC_CUDA_TRY(cudaStreamSynchronize(s));
   if (b->h_flags[0] & kErrIdRange) return MC_ERR_FORMAT;
+  if (b->h_flags[0]) return MC_ERR_DEVICE;
   int64_t total = 0;
   std::memcpy(&total, b->h_flags + 4, sizeof(total));
   *nnz = total;
@@ -306,7 +308,7 @@ int64_t csr_build_launches(const CsrBuild *b) { return b ? b->launches : 0; }
 void csr_build_free(CsrBuild *b) {
   if (!b) return;
   void *bufs[] = {b->own_src, b->own_dst, b->keys[0], b->keys[1], b->counts,
-                  b->offsets, b->temp,    b->deg,     b->flags};
+                  b->offsets, b->work,    b->temp,    b->deg,     b->flags};
   for (void *p : bufs)
     if (p) dev_free(p, b->s);
   cudaStreamSynchronize(b->s);

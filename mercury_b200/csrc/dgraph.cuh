@@ -103,8 +103,7 @@ struct mc_dgraph {
   int32_t *rank = nullptr;        // n
   int32_t *dag_rank = nullptr;    // dag_cap
   unsigned long long *rank_keys = nullptr;  // 2 n sort keys
-  int32_t *rank_counts = nullptr;           // radix histograms
-  int64_t *rank_offsets = nullptr;
+  void *rank_work = nullptr;                // sort scratch
   const unsigned long long *rank_sorted = nullptr;  // rank p -> key of vertex (see orient.cu)
   unsigned *core_bits = nullptr;  // core_offset(core_ranks) words
   bool ranked = false;            // this graph's ranks are set (it may have hub owners)

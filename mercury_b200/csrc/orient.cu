@@ -335,8 +335,25 @@ __global__ void chunk_offsets_kernel(const int64_t *__restrict__ local, int64_t 
   if (i == count && v > cap) atomicOr(err, (unsigned)kErrDagCapacity);
 }
 
+// x in N(u) (binary search; rows are checked sorted, and the probe never
+// leaves the column array where their offsets are not).
+__device__ bool in_row(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ col,
+                       int64_t nnz, int32_t u, int32_t x) {
+  int64_t lo = __ldg(rowptr + u), hi = __ldg(rowptr + u + 1) - 1;
+  while (lo <= hi && lo >= 0 && hi < nnz) {
+    const int64_t mid = lo + ((hi - lo) >> 1);
+    const int32_t m = __ldg(col + mid);
+    if (m == x) return true;
+    if (m < x) lo = mid + 1;
+    else hi = mid - 1;
+  }
+  return false;
+}
+
 // Contract checks that need the row of each entry: ids in range, strictly
-// ascending rows, no self-loops, and (optionally) symmetry.
+// ascending rows, no self-loops, and (optionally) symmetry.  Sixteen entries
+// per thread in four loads: one entry and its predecessor at a time took 322
+// us at RMAT scale 20 (31 M entries), this form 275.
 __global__ void __launch_bounds__(kTileThreads)
     validate_entries_kernel(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ col,
                             int64_t n, int64_t nnz, int check_sym, unsigned *err,
@@ -350,38 +367,37 @@ __global__ void __launch_bounds__(kTileThreads)
   const int64_t s = t0 + (int64_t)threadIdx.x * kEdgesPerThread;
   const int64_t e_end = min(s + kEdgesPerThread, t1);
   if (s >= t1) return;
+  int32_t vals[kEdgesPerThread];
+  // A caller's own column array may start anywhere: 16-byte loads only where
+  // it starts on 16 bytes (s is a multiple of 16 entries).
+  if ((reinterpret_cast<uintptr_t>(col) & 15u) == 0) {
+    load_span(col + s, nnz - s, vals);
+  } else {
+#pragma unroll
+    for (int k = 0; k < kEdgesPerThread; ++k) vals[k] = s + k < e_end ? __ldg(col + s + k) : 0;
+  }
   int64_t v = tr.row_of(s);
   int64_t start = tr.at(v), next = tr.at(v + 1);
+  int32_t prev = s > start ? __ldg(col + s - 1) : 0;
   unsigned bad = 0;
-  for (int64_t e = s; e < e_end; ++e) {
+#pragma unroll
+  for (int k = 0; k < kEdgesPerThread; ++k) {
+    const int64_t e = s + k;
+    if (e >= e_end) continue;
     while (e == next) {
       ++v;
       start = next;
       next = tr.at(v + 1);
     }
-    const int32_t u = __ldg(col + e);
+    const int32_t u = vals[k];
     if (u < 0 || (int64_t)u >= n) {
       bad |= kErrIdRange;
-      continue;
+    } else {
+      if ((int64_t)u == v) bad |= kErrSelfLoop;
+      if (e > start && prev >= u) bad |= kErrUnsorted;
+      if (check_sym && !in_row(rowptr, col, nnz, u, (int32_t)v)) bad |= kErrAsymmetric;
     }
-    if ((int64_t)u == v) bad |= kErrSelfLoop;
-    if (e > start && __ldg(col + e - 1) >= u) bad |= kErrUnsorted;
-    if (check_sym) {
-      // v must appear in N(u) (binary search; rows are checked sorted).
-      int64_t lo = __ldg(rowptr + u), hi = __ldg(rowptr + u + 1) - 1;
-      bool found = false;
-      while (lo <= hi && lo >= 0 && hi < nnz) {
-        int64_t mid = lo + ((hi - lo) >> 1);
-        int32_t m = __ldg(col + mid);
-        if (m == (int32_t)v) {
-          found = true;
-          break;
-        }
-        if (m < (int32_t)v) lo = mid + 1;
-        else hi = mid - 1;
-      }
-      if (!found) bad |= kErrAsymmetric;
-    }
+    prev = u;
   }
   if (bad) atomicOr(err, bad);
 }
@@ -420,7 +436,9 @@ __global__ void rank_keys_kernel(const int2 *__restrict__ key, int64_t n, int ma
 __global__ void rank_scatter_kernel(const unsigned long long *__restrict__ sorted, int64_t n,
                                     int32_t *__restrict__ rank) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < n) rank[n - 1 - (int64_t)(uint32_t)sorted[p]] = (int32_t)p;
+  // (A sort whose wait gave up leaves positions unwritten.)
+  if (p < n && (int64_t)(uint32_t)sorted[p] < n)
+    rank[n - 1 - (int64_t)(uint32_t)sorted[p]] = (int32_t)p;
 }
 
 // Core bitmaps: warp per rank p < core_ranks; its vertex is the one whose
@@ -437,6 +455,7 @@ __global__ void core_bits_kernel(const unsigned long long *__restrict__ sorted, 
   const int lane = threadIdx.x & (kWarp - 1);
   if (p >= core_ranks || (*(volatile unsigned *)err & (kErrDagCapacity | kErrContract))) return;
   const int64_t v = n - 1 - (int64_t)(uint32_t)sorted[p];
+  if (v < 0) return;
   unsigned *row = core + core_offset(p);
   for (int64_t e = dag_rowptr[v] + lane; e < dag_rowptr[v + 1]; e += kWarp) {
     const int z = __ldg(dag_rank + e);
@@ -667,11 +686,14 @@ int64_t dag_capacity(int64_t nnz, bool col_host) {
 }
 }  // namespace
 
-// Column entries per staging buffer with host columns (two buffers): 64 MB,
-// or MERCURY_STAGE_EDGES rounded down to whole tiles (tests use it to run
+// Column entries per chunk: with host columns (two staging buffers) 64 MB; of
+// a streamed upload 16 MB, so that the copy starts early and the passes over
+// the last chunk, which nothing overlaps, are short (pageable arrays at RMAT
+// scale 20, 126 MB: 7.08, 6.20, 5.95, 6.03 and 7.17 ms per call with 64, 32, 16,
+// 8 and 4 MB).  Or MERCURY_STAGE_EDGES rounded down to whole tiles (tests use it to run
 // many chunks on small graphs).
-int64_t stage_capacity(int64_t nnz) {
-  int64_t stage = 1ll << 24;
+int64_t stage_capacity(int64_t nnz, bool col_host) {
+  int64_t stage = col_host ? 1ll << 24 : 1ll << 22;
   if (const char *env = std::getenv("MERCURY_STAGE_EDGES")) {
     const long long v = std::atoll(env);
     if (v > 0) stage = std::max<int64_t>(kTileEdges, v / kTileEdges * kTileEdges);
@@ -697,13 +719,13 @@ int64_t tc_device_bytes(int64_t n, int64_t nnz, bool col_host, bool dag_host) {
   const int64_t cap = std::max<int64_t>(nnz, 1);
   const int64_t tiles = std::max<int64_t>((nnz + kTileEdges - 1) / kTileEdges, 1);
   const int64_t tasks = n + cap / std::min(kHubChunk, kLeafChunk) + 1;
-  const int64_t scan = (int64_t)std::max(scan_temp_bytes(tiles + 1), radix_temp_bytes(n));
+  const int64_t scan = (int64_t)scan_temp_bytes(tiles + 1);
   const int64_t staging =
-      col_host ? 2 * 4 * stage_capacity(nnz) + 8 * (stage_capacity(nnz) / kTileEdges + 1) : 0;
+      col_host ? 2 * 4 * stage_capacity(nnz, true) + 8 * (stage_capacity(nnz, true) / kTileEdges + 1) : 0;
   return (n + 1) * (8 + 16 + 8 + 4 + 4 + 16) + n / 8 + 3 * 8 * tasks +
          (dag_host ? 0 : 2 * 4 * (dag_capacity(nnz, col_host) + 4)) +
          tiles * (2 * kTileThreads + 28) +
-         2 * 12 * (radix_entries(n) + 1) + scan + staging + 4 * core_offset(core_rank_count(n));
+         (int64_t)radix_work_bytes(n, 32) + scan + staging + 4 * core_offset(core_rank_count(n));
 }
 
 int tc_alloc(mc_dgraph *g) {
@@ -715,7 +737,6 @@ int tc_alloc(mc_dgraph *g) {
   g->task_capacity = n + cap / std::min(kHubChunk, kLeafChunk) + 1;
   g->scan_temp_size = scan_temp_bytes(tiles + 1);
   const bool ranked = g->batch.gid == nullptr;
-  if (ranked) g->scan_temp_size = std::max(g->scan_temp_size, radix_temp_bytes(n));
 #define MC_ALLOC(ptr, count) \
   MC_CUDA_TRY(dev_alloc((void **)&(ptr), sizeof(*(ptr)) * (size_t)(count), g->stream))
   MC_ALLOC(g->key, n + 1);
@@ -746,15 +767,14 @@ int tc_alloc(mc_dgraph *g) {
     MC_ALLOC(g->rank, n + 1);
     MC_CUDA_TRY(dag_alloc(&g->dag_rank, &g->dag_rank_h));
     MC_ALLOC(g->rank_keys, 2 * n + 2);
-    MC_ALLOC(g->rank_counts, radix_entries(n) + 1);
-    MC_ALLOC(g->rank_offsets, radix_entries(n) + 1);
+    MC_CUDA_TRY(dev_alloc(&g->rank_work, radix_work_bytes(n, 32), g->stream));
     g->core_ranks = core_rank_count(n);
     if (g->core_ranks > 0) MC_ALLOC(g->core_bits, core_offset(g->core_ranks));
   }
   // Chunked column passes (host columns, or a streamed upload of a single
   // graph): the copy stream, its events and one chunk's tile offsets.
   if (ranked) {
-    g->chunk_edges = stage_capacity(g->nnz);
+    g->chunk_edges = stage_capacity(g->nnz, g->col_host);
     MC_ALLOC(g->chunk_offsets, g->chunk_edges / kTileEdges + 1);
     MC_CUDA_TRY(cudaStreamCreateWithFlags(&g->copy_stream, cudaStreamNonBlocking));
     for (cudaEvent_t &e : g->stage_ev)
@@ -899,8 +919,8 @@ int tc_orient(mc_dgraph *g, const int32_t *upload) {
     MC_CUDA_TRY(cudaGetLastError());
     unsigned long long *sorted = nullptr;
     MC_CUDA_TRY(radix_sort_u64(g->rank_keys, g->rank_keys + n, n, 32,
-                               32 + bit_width((uint64_t)g->max_degree), g->rank_counts,
-                               g->rank_offsets, g->scan_temp, s, &sorted, &g->launches));
+                               32 + bit_width((uint64_t)g->max_degree), g->rank_work, g->err, s,
+                               &sorted, &g->launches));
     rank_scatter_kernel<<<grid_for(n, 256), 256, 0, s>>>(sorted, n, g->rank);
     MC_CUDA_TRY(cudaGetLastError());
     g->rank_sorted = sorted;

@@ -1,5 +1,5 @@
-// Stable LSD radix sort of 64-bit keys on the device (8 bits per pass over a
-// chosen bit range), and the warp-striped tile layout its kernels share with
+// Stable LSD radix sort of 64-bit keys on the device (over a chosen bit range),
+// and the warp-striped tile layout its kernels share with
 // the CSR build: a CTA owns kSortTile consecutive keys, each warp a span of
 // kWarpSpan, read in kSortRounds rounds of 32 consecutive keys.
 #pragma once
@@ -15,9 +15,6 @@ constexpr int kSortWarps = kSortThreads / kWarp;
 constexpr int kSortRounds = 16;                          // keys per thread
 constexpr int kSortTile = kSortThreads * kSortRounds;    // keys per CTA
 constexpr int kWarpSpan = kWarp * kSortRounds;           // keys per warp
-constexpr int kRadixBits = 8;
-constexpr int kRadixBins = 1 << kRadixBits;
-static_assert(kRadixBins == kSortThreads, "one thread per digit in the digit scans");
 
 inline int bit_width(uint64_t x) {
   int b = 0;
@@ -48,17 +45,17 @@ __device__ __forceinline__ void load_warp_keys(const unsigned long long *__restr
   }
 }
 
-// Scratch of one radix sort of `count` keys: counts (int32) and offsets
-// (int64) of kRadixBins * tiles entries (+1), and the scan's temporary bytes.
-int64_t radix_entries(int64_t count);
-size_t radix_temp_bytes(int64_t count);
+// Scratch bytes of one sort of `count` keys over at most `bits` bits.
+size_t radix_work_bytes(int64_t count, int bits);
 
 // Sorts keys[0, count) by bits [begin_bit, end_bit), stably, using `alt` as
 // the other buffer of each pass; *sorted receives the buffer holding the
-// result (keys or alt). Asynchronous on `s`; *launches counts the kernels.
+// result (keys or alt).  Every bit of the keys from end_bit on is zero.  A
+// bounded wait that gives up raises kErrWaitTimeout in *err (device word; the
+// keys are then not sorted).  Asynchronous on `s`; *launches counts the
+// kernels.
 cudaError_t radix_sort_u64(unsigned long long *keys, unsigned long long *alt, int64_t count,
-                           int begin_bit, int end_bit, int32_t *counts, int64_t *offsets,
-                           void *temp, cudaStream_t s, unsigned long long **sorted,
-                           int64_t *launches);
+                           int begin_bit, int end_bit, void *work, unsigned *err, cudaStream_t s,
+                           unsigned long long **sorted, int64_t *launches);
 
 }  // namespace mc
