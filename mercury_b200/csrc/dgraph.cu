@@ -465,7 +465,7 @@ bool tc_dense_route(const mc_dgraph *g) {
   for (const char *name : {"MERCURY_TC_TABLE_LOG2_MAX", "MERCURY_TC_BITMAP_BITS",
                            "MERCURY_TC_DENSE_FACTOR", "MERCURY_TC_CORE_RANKS", "MERCURY_TC_TMA",
                            "MERCURY_TC_ROW_STAGE", "MERCURY_TC_SHORT_RANGES",
-                           "MERCURY_TC_LONG_CLASSES", "MERCURY_DAG_STAGE", "MERCURY_STAGE_EDGES"})
+                           "MERCURY_TC_LONG_CLASSES", "MERCURY_STAGE_EDGES"})
     if (std::getenv(name)) return false;
   const char *env = std::getenv("MERCURY_TC_BITS");  // 0: every graph by the DAG
   return !(env && std::atoi(env) == 0);

@@ -7,7 +7,7 @@
 // Tunables of the triangle-count schedule (task classes and chunk sizes).
 namespace mc {
 constexpr int kTileThreads = 256;          // threads per orientation tile
-constexpr int kEdgesPerThread = 16;        // consecutive CSR entries per thread
+constexpr int kEdgesPerThread = 16;        // CSR entries per thread
 constexpr int64_t kTileEdges = (int64_t)kTileThreads * kEdgesPerThread;
 constexpr int kLeafMaxOut = 64;            // d+(owner) <= this: warp task
 constexpr int kLeafSlots = 256;            // per-warp hash slots for leaf owners
@@ -111,7 +111,7 @@ struct mc_dgraph {
   int core_ranks = 0;             // capacity: core_offset(core_ranks) words
   int core_used = 0;              // ranks [0, core_used) have core bitmaps (<= n)
   int dense_factor = 2;           // AND when its words <= factor x list entries
-  uint16_t *keep = nullptr;       // one DAG keep mask per orientation thread
+  unsigned *keep = nullptr;       // one DAG keep bit per entry, kTileEdges / 32 words per tile
   int32_t *tile_counts = nullptr; // tiles
   int64_t *tile_offsets = nullptr;// tiles + 1
   int64_t *tile_rows = nullptr;   // 2 x tiles: first and last row of each tile

@@ -15,8 +15,8 @@
 // symmetric row, so no partner CSR is written.  Routing is per owner
 // (d+ <= kLeafMaxOut: warp task, else CTA task).
 //
-// Passes (each CTA owns a tile of kTileEdges consecutive CSR entries and
-// stages the tile's row offsets in shared memory):
+// Passes (each CTA owns a tile of kTileEdges consecutive CSR entries, each warp
+// 512 of them in rounds of 32, one entry per lane):
 //   A  DAG keep masks, per-tile DAG counts, d+ of every row by atomics
 //   B  DAG entries and row offsets written from the keep masks
 // Each vertex's (degree, d+) pair is one 8-byte word (key[]).
@@ -36,158 +36,63 @@
 namespace mc {
 namespace {
 
-constexpr int kSegMax = 2048;  // row offsets of a tile kept in shared memory
+constexpr int kTileWarps = kTileThreads / kWarp;
+constexpr int kTileRounds = kEdgesPerThread;                // 32-entry rounds per warp
+constexpr int kTileWords = (int)(kTileEdges / kWarp);       // keep words per tile
 
-// The span's entries from p (16-byte aligned), `avail` of them valid.
-__device__ __forceinline__ void load_span(const int32_t *__restrict__ p32, int64_t avail,
-                                          int32_t (&vals)[kEdgesPerThread]) {
-  if (avail >= kEdgesPerThread) {
-    const int4 *p = reinterpret_cast<const int4 *>(p32);
-#pragma unroll
-    for (int k = 0; k < kEdgesPerThread / 4; ++k) {
-      int4 q = __ldg(p + k);
-      vals[4 * k] = q.x;
-      vals[4 * k + 1] = q.y;
-      vals[4 * k + 2] = q.z;
-      vals[4 * k + 3] = q.w;
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < kEdgesPerThread; ++k) vals[k] = k < avail ? __ldg(p32 + k) : 0;
-  }
-}
-
-// Row offsets of one tile: rows [lo, hi] hold the tile's entries; when the
-// segment rowptr[lo .. hi+1] fits it is read from shared memory.
-struct TileRows {
-  const int64_t *g;
-  const int64_t *s;
-  int64_t lo, hi;
-  __device__ __forceinline__ int64_t at(int64_t r) const { return s ? s[r - lo] : __ldg(g + r); }
-  // Largest r in [lo, hi] with rowptr[r] <= key.
-  __device__ __forceinline__ int64_t row_of(int64_t key) const {
-    int64_t a = lo, b = hi;
-    while (a < b) {
-      int64_t mid = a + ((b - a + 1) >> 1);
-      if (at(mid) <= key) a = mid;
-      else b = mid - 1;
-    }
-    return a;
-  }
-  // Smallest r in [a, b] with rowptr[r] >= key (rowptr[b] >= key).
-  __device__ __forceinline__ int64_t first_at(int64_t a, int64_t b, int64_t key) const {
-    while (a < b) {
-      int64_t mid = a + ((b - a) >> 1);
-      if (at(mid) >= key) b = mid;
-      else a = mid + 1;
-    }
-    return a;
-  }
+// The rows of a tile's entries.  Every non-empty row that starts inside the
+// tile marks its first entry with its number from the tile's first row on; an
+// entry's row is the nearest mark at or before it, which a ballot finds within
+// a round, and a carry across rounds.  No lane ever walks rows (sixteen
+// consecutive entries per lane, each lane stepping over its rows' offsets,
+// diverged on every row boundary and empty row: 322 us for checks at RMAT scale 20; at scale 22 pass A took 1.08 ms and takes
+// 0.79, pass B 1.13 and 0.36; the checks at scale 20 take 157 us).
+struct TileMarks {
+  int64_t lo;      // row of the tile's first entry
+  bool at_start;   // that row starts at the tile
+  int carry;       // this warp's row before its first round
+  int m[kTileRounds];
 };
 
 // rows (optional): {first row, last row} of this tile, precomputed by
-// tile_rows_kernel; without it two threads binary-search rowptr (22
-// dependent loads at n = 4 M, which the rest of the CTA waits for).
-__device__ __forceinline__ TileRows load_tile_rows(const int64_t *rowptr, int64_t n, int64_t t0,
-                                                   int64_t t1, int64_t *seg,
-                                                   const int64_t *rows = nullptr) {
-  __shared__ int64_t sh[2];
+// tile_rows_kernel; without it two threads binary-search rowptr.
+__device__ __forceinline__ TileMarks tile_marks(const int64_t *__restrict__ rowptr, int64_t n,
+                                                int64_t t0, int64_t t1,
+                                                const int64_t *__restrict__ rows) {
+  __shared__ __align__(16) int s_mark[kTileEdges];
+  __shared__ int64_t s_rows[2];
+  __shared__ int s_max[kTileWarps];
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   if (rows) {
-    if (threadIdx.x < 2) sh[threadIdx.x] = __ldg(rows + threadIdx.x);
+    if (threadIdx.x < 2) s_rows[threadIdx.x] = __ldg(rows + threadIdx.x);
   } else {
-    if (threadIdx.x == 0) sh[0] = upper_row(rowptr, 0, n - 1, t0);
-    if (threadIdx.x == kTileThreads - 1) sh[1] = upper_row(rowptr, 0, n - 1, t1 - 1);
+    if (threadIdx.x == 0) s_rows[0] = upper_row(rowptr, 0, n - 1, t0);
+    if (threadIdx.x == kTileThreads - 1) s_rows[1] = upper_row(rowptr, 0, n - 1, t1 - 1);
+  }
+  int4 *m4 = reinterpret_cast<int4 *>(s_mark);
+  for (int i = threadIdx.x; i < kTileEdges / 4; i += kTileThreads) m4[i] = make_int4(0, 0, 0, 0);
+  __syncthreads();
+  TileMarks t;
+  t.lo = s_rows[0];
+  const int64_t hi = s_rows[1];
+  t.at_start = __ldg(rowptr + t.lo) == t0;
+  for (int64_t r = t.lo + 1 + threadIdx.x; r <= hi; r += kTileThreads) {
+    const int64_t b = __ldg(rowptr + r);
+    if (b < __ldg(rowptr + r + 1)) s_mark[b - t0] = (int)(r - t.lo);
   }
   __syncthreads();
-  TileRows tr{rowptr, nullptr, sh[0], sh[1]};
-  const int64_t len = tr.hi - tr.lo + 2;
-  if (len <= kSegMax) {
-    for (int64_t i = threadIdx.x; i < len; i += kTileThreads) seg[i] = __ldg(rowptr + tr.lo + i);
-    __syncthreads();
-    tr.s = seg;
-  }
-  return tr;
-}
-
-__device__ __forceinline__ int block_sum_int(int v) {
-  __shared__ int ws[kTileThreads / kWarp];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int mx = 0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(kFull, v, o);
-  if (lane == 0) ws[wid] = v;
+  for (int k = 0; k < kTileRounds; ++k) {
+    t.m[k] = s_mark[(warp * kTileRounds + k) * kWarp + lane];
+    mx = max(mx, t.m[k]);
+  }
+  mx = __reduce_max_sync(kFull, mx);
+  if (lane == 0) s_max[warp] = mx;
   __syncthreads();
-  int t = 0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < kTileThreads / kWarp; ++i) t += ws[i];
+  t.carry = 0;
+  for (int w = 0; w < warp; ++w) t.carry = max(t.carry, s_max[w]);
   return t;
-}
-
-// Exclusive prefix of v over the block; *total receives the block sum.
-__device__ __forceinline__ int block_exclusive_int(int v, int *total) {
-  __shared__ int ws[kTileThreads / kWarp];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int x = warp_inclusive_scan(v, lane);
-  if (lane == 31) ws[wid] = x;
-  __syncthreads();
-  if (wid == 0) {
-    int w = lane < kTileThreads / kWarp ? ws[lane] : 0;
-    w = warp_inclusive_scan(w, lane);
-    if (lane < kTileThreads / kWarp) ws[lane] = w;
-  }
-  __syncthreads();
-  *total = ws[kTileThreads / kWarp - 1];
-  return (wid ? ws[wid - 1] : 0) + x - v;
-}
-
-// Writes the kept entries of this thread's span [s, e_end) (row r holds s)
-// from position pos on, and out_rowptr[q] = position for every row q that
-// starts inside the span.  Rows starting at nnz are written by the caller.
-// kStage: the entries go to stage[pos - stage_base] in shared memory (the
-// caller copies the tile's range out, coalesced, and gathers the ranks
-// there); otherwise straight to out_col / out_rank.
-template <bool kStage>
-__device__ __forceinline__ void write_span(const TileRows &tr, const int64_t *rowptr, int64_t t0,
-                                           int64_t s, int64_t e_end, int64_t r,
-                                           const int32_t (&vals)[kEdgesPerThread], unsigned keep,
-                                           int64_t pos, int64_t *out_rowptr, int32_t *out_col,
-                                           const int32_t *__restrict__ rank, int32_t *out_rank,
-                                           int32_t *stage, int64_t stage_base) {
-  if (tr.at(r) == s) {
-    // Rows starting exactly at s: row r and the empty rows just before it.
-    // For s > t0 they all lie in the staged range; the tile's first span may
-    // share its start with rows before the range.
-    const int64_t rf = s == t0 ? lower_row(rowptr, 0, r, s) : tr.first_at(tr.lo, r, s);
-    for (int64_t q = rf; q <= r; ++q) out_rowptr[q] = pos;
-  }
-  // The ranks of the kept entries, gathered before the row walk so that
-  // they are all in flight at once.
-  int32_t ranks[kEdgesPerThread];
-  if (!kStage) {
-#pragma unroll
-    for (int k = 0; k < kEdgesPerThread; ++k)
-      ranks[k] = out_rank && (keep & (1u << k)) ? __ldg(rank + vals[k]) : 0;
-  }
-  int64_t next = tr.at(r + 1);
-#pragma unroll
-  for (int k = 0; k < kEdgesPerThread; ++k) {
-    const int64_t e = s + k;
-    if (e < e_end) {
-      while (e == next) {
-        ++r;
-        out_rowptr[r] = pos;
-        next = tr.at(r + 1);
-      }
-      if (keep & (1u << k)) {
-        if (kStage) {
-          stage[pos - stage_base] = vals[k];
-        } else {
-          out_col[pos] = vals[k];
-          if (out_rank) out_rank[pos] = ranks[k];
-        }
-        ++pos;
-      }
-    }
-  }
 }
 
 // Where a pass finds its tiles' column entries: the whole array (col_base
@@ -199,109 +104,185 @@ struct ColumnChunk {
   int64_t tile_base;
 };
 
-// Pass A (kWrite == false): DAG entries of every thread's span as a 16-bit
-// mask in keep[], per-tile counts, and d+ of every row by atomics on
-// key[].y (which starts at 0).  Pass B (kWrite == true): the kept entries
-// compacted into out_col (and, when rank is given, their ranks into
-// out_rank) and out_rowptr[r] = kept entries before rowptr[r].  With
-// chunk_end given, pass B writes nothing when *chunk_end (the DAG entries
-// up to the end of this chunk) exceeds cap; with stop given, neither pass
-// does anything once a contract bit is set there.
-template <bool kWrite, bool kStage = false>
+// x in N(u) (binary search; rows are checked sorted, and the probe never
+// leaves the column array where their offsets are not).
+__device__ bool in_row(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ col,
+                       int64_t nnz, int32_t u, int32_t x) {
+  int64_t lo = __ldg(rowptr + u), hi = __ldg(rowptr + u + 1) - 1;
+  while (lo <= hi && lo >= 0 && hi < nnz) {
+    const int64_t mid = lo + ((hi - lo) >> 1);
+    const int32_t m = __ldg(col + mid);
+    if (m == x) return true;
+    if (m < x) lo = mid + 1;
+    else hi = mid - 1;
+  }
+  return false;
+}
+
+// Pass A (kKeep): the DAG entries as one bit per entry in keep[] (kTileWords
+// words per tile), per-tile counts, and d+ of every row by one atomic per row
+// and round on key[].y (which starts at 0).  kCheck: the entries against the
+// CSR contract (ids in range, strictly ascending rows, no self-loops and, with
+// check_sym, symmetry), what breaks it into *err; an id out of range is then
+// never gathered with.  With stop given, nothing runs once a contract bit is
+// set there.
+template <bool kKeep, bool kCheck>
 __global__ void __launch_bounds__(kTileThreads)
-    dag_pass_kernel(const int64_t *__restrict__ rowptr, ColumnChunk cc,
+    dag_keep_kernel(const int64_t *__restrict__ rowptr, ColumnChunk cc,
                     const int32_t *__restrict__ deg, int64_t n, int64_t nnz, int2 *key,
-                    uint16_t *keep_masks, int32_t *counts_out,
-                    const int64_t *__restrict__ offs_in, int64_t *out_rowptr, int32_t *out_col,
-                    const int32_t *__restrict__ rank, int32_t *out_rank,
-                    const int64_t *chunk_end, int64_t cap, const unsigned *stop,
-                    const int64_t *__restrict__ tile_rows) {
-  __shared__ int64_t seg[kSegMax];
-  // Both checks read one word, the same for the whole CTA.  `stop`: the
-  // contract checks of a chunk validated just before found a bad entry, so
-  // no id is gathered or written.
+                    unsigned *keep, int32_t *counts_out, const unsigned *stop, int check_sym,
+                    unsigned *err, const int64_t *__restrict__ tile_rows) {
+  // One word, the same for the whole CTA: the checks of an earlier chunk found
+  // a bad entry.
   if (stop && (*(volatile const unsigned *)stop & kErrContract)) return;
-  if (kWrite && chunk_end && *chunk_end > cap) return;
+  __shared__ int s_count[kTileWarps];
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   const int64_t tile = cc.tile_base + blockIdx.x;
   const int64_t t0 = tile * kTileEdges;
   const int64_t t1 = min(t0 + kTileEdges, nnz);
-  const TileRows tr =
-      load_tile_rows(rowptr, n, t0, t1, seg, tile_rows ? tile_rows + 2 * tile : nullptr);
-  const int64_t s = t0 + (int64_t)threadIdx.x * kEdgesPerThread;
-  const int64_t e_end = min(s + kEdgesPerThread, t1);
-  const int64_t slot = tile * kTileThreads + threadIdx.x;
-  int32_t vals[kEdgesPerThread];
-  unsigned keep = 0;
-  int64_t r = 0;
-  if (s < t1) {
-    load_span(cc.col + (s - cc.col_base), nnz - s, vals);
-    r = tr.row_of(s);
-    if (!kWrite) {
-      // All sixteen degree gathers are issued before the row walk below
-      // (whose loop would otherwise serialise them); entries past the span
-      // hold id 0, a valid vertex.
-      int du[kEdgesPerThread];
+  const int64_t e0 = t0 + (int64_t)warp * kTileRounds * kWarp + lane;  // round 0
+  int u[kTileRounds], du[kTileRounds];
 #pragma unroll
-      for (int k = 0; k < kEdgesPerThread; ++k) du[k] = __ldg(deg + vals[k]);
-      int64_t v = r, next = tr.at(r + 1);
-      int dv = __ldg(deg + v);
-      int run = 0;  // DAG entries of row v seen in this span
+  for (int k = 0; k < kTileRounds; ++k) {
+    const int64_t e = e0 + k * kWarp;
+    u[k] = e < t1 ? __ldg(cc.col + (e - cc.col_base)) : 0;
+  }
+  if (kKeep) {
+    // All sixteen degree gathers in flight before the rows are known.
 #pragma unroll
-      for (int k = 0; k < kEdgesPerThread; ++k) {
-        const int64_t e = s + k;
-        if (e < e_end) {
-          while (e == next) {
-            if (run) {
-              atomicAdd(&key[v].y, run);
-              run = 0;
-            }
-            ++v;
-            next = tr.at(v + 1);
-            dv = __ldg(deg + v);
-          }
-          const int u = vals[k];
-          if (du[k] > dv || (du[k] == dv && u > (int)v)) {
-            keep |= 1u << k;
-            ++run;
-          }
+    for (int k = 0; k < kTileRounds; ++k)
+      du[k] = !kCheck || (u[k] >= 0 && u[k] < n) ? __ldg(deg + u[k]) : 0;
+  }
+  const TileMarks tm = tile_marks(rowptr, n, t0, t1, tile_rows ? tile_rows + 2 * tile : nullptr);
+  int carry = tm.carry, count = 0;
+  unsigned bad = 0, mine = 0;
+  const unsigned upto = kFull >> (kWarp - 1 - lane);
+  // The entry before this warp's first (checks of a row that goes on).
+  int last = 0;
+  if (kCheck && lane == 0 && e0 > 0 && e0 < t1) last = __ldg(cc.col + (e0 - 1 - cc.col_base));
+  last = kCheck ? __shfl_sync(kFull, last, 0) : 0;
+#pragma unroll
+  for (int k = 0; k < kTileRounds; ++k) {
+    const int64_t e = e0 + k * kWarp;
+    const bool in = e < t1;
+    const unsigned starts = __ballot_sync(kFull, tm.m[k] > 0);
+    const unsigned before = starts & upto;
+    int row = __shfl_sync(kFull, tm.m[k], before ? kWarp - 1 - __clz(before) : 0);
+    if (!before) row = carry;
+    if (starts) carry = __shfl_sync(kFull, tm.m[k], kWarp - 1 - __clz(starts));
+    const int64_t v = tm.lo + row;
+    if (kCheck) {
+      int prev = __shfl_up_sync(kFull, u[k], 1);
+      if (lane == 0) prev = last;
+      last = __shfl_sync(kFull, u[k], kWarp - 1);
+      if (in) {
+        if (u[k] < 0 || (int64_t)u[k] >= n) {
+          bad |= kErrIdRange;
+        } else {
+          const bool first = tm.m[k] > 0 || (e == t0 && tm.at_start);
+          if ((int64_t)u[k] == v) bad |= kErrSelfLoop;
+          if (!first && prev >= u[k]) bad |= kErrUnsorted;
+          if (check_sym && !in_row(rowptr, cc.col - cc.col_base, nnz, u[k], (int32_t)v))
+            bad |= kErrAsymmetric;
         }
       }
-      if (run) atomicAdd(&key[v].y, run);
-      keep_masks[slot] = (uint16_t)keep;
-    } else {
-      keep = keep_masks[slot];
+    }
+    if (kKeep) {
+      const int dv = __ldg(deg + v);
+      const bool up = in && (du[k] > dv || (du[k] == dv && u[k] > (int)v));
+      const unsigned word = __ballot_sync(kFull, up);
+      if (lane == k) mine = word;
+      count += __popc(word);
+      // The row's entries of this round, at its first lane.
+      if ((lane == 0 || tm.m[k] > 0) && word) {
+        const unsigned later = starts & ~upto;
+        const unsigned seg = (later ? (1u << (__ffs(later) - 1)) - 1u : kFull) & (kFull << lane);
+        const int c = __popc(word & seg);
+        if (c) atomicAdd(&key[v].y, c);
+      }
     }
   }
-  if (!kWrite) {
-    const int t = block_sum_int(__popc(keep));
-    if (threadIdx.x == 0) counts_out[tile] = t;
-    return;
-  }
-  int total = 0;
-  const int64_t base = offs_in[tile];
-  const int64_t pos = base + block_exclusive_int(__popc(keep), &total);
-  if (kStage) {
-    // The tile's DAG entries are the range [base, base + total): staged in
-    // shared memory, then written with whole-line stores, the rank gathers
-    // issued four per thread at a time.
-    __shared__ int32_t stage[kTileEdges];
-    if (s < t1)
-      write_span<true>(tr, rowptr, t0, s, e_end, r, vals, keep, pos, out_rowptr, nullptr,
-                       nullptr, nullptr, stage, base);
+  if (kCheck && bad) atomicOr(err, bad);
+  if (kKeep) {
+    if (lane < kTileRounds) keep[tile * kTileWords + warp * kTileRounds + lane] = mine;
+    if (lane == 0) s_count[warp] = count;
     __syncthreads();
-#pragma unroll 4
-    for (int i = threadIdx.x; i < total; i += kTileThreads) {
-      const int32_t c = stage[i];
-      out_col[base + i] = c;
-      if (out_rank) out_rank[base + i] = __ldg(rank + c);
+    if (threadIdx.x == 0) {
+      int t = 0;
+      for (int w = 0; w < kTileWarps; ++w) t += s_count[w];
+      counts_out[tile] = t;
     }
-  } else if (s < t1) {
-    write_span<false>(tr, rowptr, t0, s, e_end, r, vals, keep, pos, out_rowptr, out_col, rank,
-                      out_rank, nullptr, 0);
   }
-  // Rows after the last entry (trailing empty rows and q == n) start at nnz.
-  if (t1 == nnz)
-    for (int64_t q = tr.hi + 1 + threadIdx.x; q <= n; q += kTileThreads) out_rowptr[q] = base + total;
+}
+
+// Pass B: the kept entries compacted into out_col (and, when rank is given,
+// their ranks into out_rank), and out_rowptr[r] = kept entries before
+// rowptr[r] for the rows that start in the tile, empty ones included.  With
+// chunk_end given, nothing is written when *chunk_end (the DAG entries up to
+// the end of this chunk) exceeds cap; stop as in pass A.
+__global__ void __launch_bounds__(kTileThreads)
+    dag_write_kernel(const int64_t *__restrict__ rowptr, ColumnChunk cc, int64_t n, int64_t nnz,
+                     const unsigned *__restrict__ keep, const int64_t *__restrict__ offs_in,
+                     int64_t *out_rowptr, int32_t *out_col, const int32_t *__restrict__ rank,
+                     int32_t *out_rank, const int64_t *chunk_end, int64_t cap,
+                     const unsigned *stop, const int64_t *__restrict__ tile_rows) {
+  if (stop && (*(volatile const unsigned *)stop & kErrContract)) return;
+  if (chunk_end && *chunk_end > cap) return;
+  static_assert(kTileWords <= kTileThreads, "one thread per keep word");
+  __shared__ unsigned s_word[kTileWords];
+  __shared__ int s_pre[kTileWords], s_sum[kTileWarps];
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  const int64_t tile = cc.tile_base + blockIdx.x;
+  const int64_t t0 = tile * kTileEdges;
+  const int64_t t1 = min(t0 + kTileEdges, nnz);
+  const unsigned word = threadIdx.x < kTileWords ? keep[tile * kTileWords + threadIdx.x] : 0u;
+  const int incl = warp_inclusive_scan(__popc(word), lane);
+  if (lane == kWarp - 1) s_sum[warp] = incl;
+  __syncthreads();
+  int pre = incl - __popc(word);
+  for (int w = 0; w < warp; ++w) pre += s_sum[w];
+  if (threadIdx.x < kTileWords) {
+    s_word[threadIdx.x] = word;
+    s_pre[threadIdx.x] = pre;
+  }
+  __syncthreads();
+  const int64_t base = offs_in[tile];
+  const unsigned lt = (1u << lane) - 1u;
+  const int64_t e0 = t0 + (int64_t)warp * kTileRounds * kWarp + lane;
+  constexpr int kU = 8;
+#pragma unroll
+  for (int k0 = 0; k0 < kTileRounds; k0 += kU) {
+    int u[kU], rk[kU];
+    unsigned wd[kU];
+#pragma unroll
+    for (int i = 0; i < kU; ++i) {
+      wd[i] = s_word[warp * kTileRounds + k0 + i];
+      const bool kept = (wd[i] >> lane) & 1u;
+      u[i] = kept ? __ldg(cc.col + (e0 + (k0 + i) * kWarp - cc.col_base)) : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < kU; ++i)
+      rk[i] = out_rank && ((wd[i] >> lane) & 1u) ? __ldg(rank + u[i]) : 0;
+#pragma unroll
+    for (int i = 0; i < kU; ++i) {
+      if (!((wd[i] >> lane) & 1u)) continue;
+      const int64_t to = base + s_pre[warp * kTileRounds + k0 + i] + __popc(wd[i] & lt);
+      out_col[to] = u[i];
+      if (out_rank) out_rank[to] = rk[i];
+    }
+  }
+  // Rows that start here: those after the previous tile's last row.  Rows
+  // after the last entry (trailing empty rows and row n) start at nnz.
+  const int64_t first = tile > 0 ? __ldg(tile_rows + 2 * tile - 1) + 1 : 0;
+  const int64_t last = t1 == nnz ? n : __ldg(tile_rows + 2 * tile + 1);
+  const int end_pre = s_pre[kTileWords - 1] + __popc(s_word[kTileWords - 1]);
+  for (int64_t r = first + threadIdx.x; r <= last; r += kTileThreads) {
+    const int64_t at = __ldg(rowptr + r) - t0;
+    const int w = (int)(at / kWarp);
+    out_rowptr[r] =
+        base + (w < kTileWords ? s_pre[w] + __popc(s_word[w] & ((1u << (at & (kWarp - 1))) - 1u))
+                               : end_pre);
+  }
 }
 
 // rows[2t] / rows[2t + 1] = the rows holding the first and the last entry of
@@ -333,73 +314,6 @@ __global__ void chunk_offsets_kernel(const int64_t *__restrict__ local, int64_t 
   const int64_t v = base + local[i];
   offs[i] = v;
   if (i == count && v > cap) atomicOr(err, (unsigned)kErrDagCapacity);
-}
-
-// x in N(u) (binary search; rows are checked sorted, and the probe never
-// leaves the column array where their offsets are not).
-__device__ bool in_row(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ col,
-                       int64_t nnz, int32_t u, int32_t x) {
-  int64_t lo = __ldg(rowptr + u), hi = __ldg(rowptr + u + 1) - 1;
-  while (lo <= hi && lo >= 0 && hi < nnz) {
-    const int64_t mid = lo + ((hi - lo) >> 1);
-    const int32_t m = __ldg(col + mid);
-    if (m == x) return true;
-    if (m < x) lo = mid + 1;
-    else hi = mid - 1;
-  }
-  return false;
-}
-
-// Contract checks that need the row of each entry: ids in range, strictly
-// ascending rows, no self-loops, and (optionally) symmetry.  Sixteen entries
-// per thread in four loads: one entry and its predecessor at a time took 322
-// us at RMAT scale 20 (31 M entries), this form 275.
-__global__ void __launch_bounds__(kTileThreads)
-    validate_entries_kernel(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ col,
-                            int64_t n, int64_t nnz, int check_sym, unsigned *err,
-                            int64_t tile_base, const int64_t *__restrict__ tile_rows = nullptr) {
-  __shared__ int64_t seg[kSegMax];
-  const int64_t tile = tile_base + blockIdx.x;
-  const int64_t t0 = tile * kTileEdges;
-  const int64_t t1 = min(t0 + kTileEdges, nnz);
-  const TileRows tr =
-      load_tile_rows(rowptr, n, t0, t1, seg, tile_rows ? tile_rows + 2 * tile : nullptr);
-  const int64_t s = t0 + (int64_t)threadIdx.x * kEdgesPerThread;
-  const int64_t e_end = min(s + kEdgesPerThread, t1);
-  if (s >= t1) return;
-  int32_t vals[kEdgesPerThread];
-  // A caller's own column array may start anywhere: 16-byte loads only where
-  // it starts on 16 bytes (s is a multiple of 16 entries).
-  if ((reinterpret_cast<uintptr_t>(col) & 15u) == 0) {
-    load_span(col + s, nnz - s, vals);
-  } else {
-#pragma unroll
-    for (int k = 0; k < kEdgesPerThread; ++k) vals[k] = s + k < e_end ? __ldg(col + s + k) : 0;
-  }
-  int64_t v = tr.row_of(s);
-  int64_t start = tr.at(v), next = tr.at(v + 1);
-  int32_t prev = s > start ? __ldg(col + s - 1) : 0;
-  unsigned bad = 0;
-#pragma unroll
-  for (int k = 0; k < kEdgesPerThread; ++k) {
-    const int64_t e = s + k;
-    if (e >= e_end) continue;
-    while (e == next) {
-      ++v;
-      start = next;
-      next = tr.at(v + 1);
-    }
-    const int32_t u = vals[k];
-    if (u < 0 || (int64_t)u >= n) {
-      bad |= kErrIdRange;
-    } else {
-      if ((int64_t)u == v) bad |= kErrSelfLoop;
-      if (e > start && prev >= u) bad |= kErrUnsorted;
-      if (check_sym && !in_row(rowptr, col, nnz, u, (int32_t)v)) bad |= kErrAsymmetric;
-    }
-    prev = u;
-  }
-  if (bad) atomicOr(err, bad);
 }
 
 // Offsets monotone with the right ends; *max_deg receives the largest row.
@@ -628,8 +542,9 @@ int validate_graph(mc_dgraph *g, unsigned flags) {
   const int64_t tiles = (g->nnz + kTileEdges - 1) / kTileEdges;
   g->launches += 1 + (tiles > 0 ? 1 : 0);
   if (tiles > 0) {
-    validate_entries_kernel<<<(unsigned)tiles, kTileThreads, 0, g->stream>>>(
-        g->rowptr, g->col, g->n, g->nnz, (flags & MC_VALIDATE_SYMMETRY) ? 1 : 0, g->err, 0);
+    dag_keep_kernel<false, true><<<(unsigned)tiles, kTileThreads, 0, g->stream>>>(
+        g->rowptr, ColumnChunk{g->col, 0, 0}, nullptr, g->n, g->nnz, nullptr, nullptr, nullptr,
+        nullptr, (flags & MC_VALIDATE_SYMMETRY) ? 1 : 0, g->err, nullptr);
     MC_CUDA_TRY(cudaGetLastError());
   }
   MC_CUDA_TRY(cudaMemcpyAsync(g->h_err, g->err, sizeof(unsigned), cudaMemcpyDeviceToHost, g->stream));
@@ -668,8 +583,9 @@ int validate_csr_words(const int64_t *rowptr, const int32_t *col, int64_t n, int
   if (h_err) return MC_ERR_FORMAT;  // the entry walk needs monotone offsets
   const int64_t tiles = (nnz + kTileEdges - 1) / kTileEdges;
   if (tiles > 0) {
-    validate_entries_kernel<<<(unsigned)tiles, kTileThreads, 0, s>>>(rowptr, col, n, nnz, 0, d_err,
-                                                                   0);
+    dag_keep_kernel<false, true><<<(unsigned)tiles, kTileThreads, 0, s>>>(
+        rowptr, ColumnChunk{col, 0, 0}, nullptr, n, nnz, nullptr, nullptr, nullptr, nullptr, 0, d_err,
+        nullptr);
     MC_CUDA_TRY(cudaGetLastError());
     MC_CUDA_TRY(cudaMemcpyAsync(&h_err, d_err, sizeof(h_err), cudaMemcpyDeviceToHost, s));
     MC_CUDA_TRY(cudaStreamSynchronize(s));
@@ -753,7 +669,7 @@ int tc_alloc(mc_dgraph *g) {
     return cudaHostGetDevicePointer((void **)dev, *host, 0);
   };
   MC_CUDA_TRY(dag_alloc(&g->dag_col, &g->dag_col_h));
-  MC_ALLOC(g->keep, tiles * kTileThreads);
+  MC_ALLOC(g->keep, tiles * kTileWords);
   MC_ALLOC(g->tile_counts, tiles);
   MC_ALLOC(g->tile_offsets, tiles + 1);
   MC_ALLOC(g->tile_rows, 2 * tiles);
@@ -809,19 +725,12 @@ static void parallel_copy(int32_t *dst, const int32_t *src, int64_t count) {
 //  * host columns (in_place false): chunks go to two staging buffers; the
 //    columns were validated when the handle was made;
 //  * streamed upload (in_place true): chunks land in the handle's own device
-//    column array, and each chunk's contract checks run before its passes,
-//    which do nothing once a check has failed (no gather of an unchecked id).
+//    column array, and pass A checks each chunk against the contract on the
+//    way (no gather with an id out of range); once a check has failed, the
+//    later passes do nothing.
 // The DAG holds dag_cap entries; a chunk that would end past it raises
 // kErrDagCapacity and writes nothing.  The caller reads the flags before
 // counting.
-// Pass B stages each tile's DAG entries in shared memory and writes them
-// out with whole-line stores (MERCURY_DAG_STAGE=0: each thread writes its
-// own kept entries directly).
-static bool stage_dag_writes() {
-  const char *env = std::getenv("MERCURY_DAG_STAGE");
-  return env ? std::atoi(env) != 0 : true;
-}
-
 static int staged_dag_passes(mc_dgraph *g, const int32_t *deg, const int32_t *src, bool in_place) {
   const int64_t n = g->n, nnz = g->nnz;
   cudaStream_t s = g->stream, cs = g->copy_stream;
@@ -864,27 +773,20 @@ static int staged_dag_passes(mc_dgraph *g, const int32_t *deg, const int32_t *sr
     }
     MC_CUDA_TRY(cudaEventRecord(copied[slot], cs));
     MC_CUDA_TRY(cudaStreamWaitEvent(s, copied[slot], 0));
-    if (in_place) {
-      validate_entries_kernel<<<(unsigned)ct, kTileThreads, 0, s>>>(g->rowptr, g->col, n, nnz, 0,
-                                                                    g->err, tb, g->tile_rows);
-      MC_CUDA_TRY(cudaGetLastError());
-      g->launches += 1;
-    }
     const ColumnChunk cc = in_place ? ColumnChunk{g->col, 0, tb} : ColumnChunk{buf, e0, tb};
-    dag_pass_kernel<false><<<(unsigned)ct, kTileThreads, 0, s>>>(
-        g->rowptr, cc, deg, n, nnz, g->key, g->keep, g->tile_counts, nullptr, nullptr, nullptr,
-        nullptr, nullptr, nullptr, 0, stop, g->tile_rows);
+    (in_place ? dag_keep_kernel<true, true> : dag_keep_kernel<true, false>)
+        <<<(unsigned)ct, kTileThreads, 0, s>>>(g->rowptr, cc, deg, n, nnz, g->key, g->keep,
+                                               g->tile_counts, stop, 0, g->err, g->tile_rows);
     MC_CUDA_TRY(cudaGetLastError());
     MC_CUDA_TRY(exclusive_scan(g->tile_counts + tb, g->chunk_offsets, ct, g->scan_temp, s));
     chunk_offsets_kernel<<<grid_for(ct + 1, 256), 256, 0, s>>>(g->chunk_offsets, ct,
                                                                g->tile_offsets + tb, g->dag_cap,
                                                                g->err);
     MC_CUDA_TRY(cudaGetLastError());
-    (stage_dag_writes() ? dag_pass_kernel<true, true> : dag_pass_kernel<true, false>)
-        <<<(unsigned)ct, kTileThreads, 0, s>>>(
-        g->rowptr, cc, deg, n, nnz, g->key, g->keep, nullptr, g->tile_offsets, g->dag_rowptr,
-        g->dag_col, g->ranked ? g->rank : nullptr, g->ranked ? g->dag_rank : nullptr,
-        g->tile_offsets + tb + ct, g->dag_cap, stop, g->tile_rows);
+    dag_write_kernel<<<(unsigned)ct, kTileThreads, 0, s>>>(
+        g->rowptr, cc, n, nnz, g->keep, g->tile_offsets, g->dag_rowptr, g->dag_col,
+        g->ranked ? g->rank : nullptr, g->ranked ? g->dag_rank : nullptr, g->tile_offsets + tb + ct,
+        g->dag_cap, stop, g->tile_rows);
     MC_CUDA_TRY(cudaGetLastError());
     MC_CUDA_TRY(cudaEventRecord(drained[slot], s));
     g->launches += 3 + scan_launches(ct);
@@ -945,15 +847,14 @@ int tc_orient(mc_dgraph *g, const int32_t *upload) {
   } else {
     const unsigned grid = (unsigned)tiles;
     const ColumnChunk all{g->col, 0, 0};
-    dag_pass_kernel<false><<<grid, kTileThreads, 0, s>>>(
-        g->rowptr, all, deg, n, nnz, g->key, g->keep, g->tile_counts, nullptr, nullptr, nullptr,
-        nullptr, nullptr, nullptr, 0, nullptr, g->tile_rows);
+    dag_keep_kernel<true, false><<<grid, kTileThreads, 0, s>>>(
+        g->rowptr, all, deg, n, nnz, g->key, g->keep, g->tile_counts, nullptr, 0, g->err,
+        g->tile_rows);
     MC_CUDA_TRY(cudaGetLastError());
     MC_CUDA_TRY(exclusive_scan(g->tile_counts, g->tile_offsets, tiles, g->scan_temp, s));
-    (stage_dag_writes() ? dag_pass_kernel<true, true> : dag_pass_kernel<true, false>)
-        <<<grid, kTileThreads, 0, s>>>(
-        g->rowptr, all, deg, n, nnz, g->key, g->keep, nullptr, g->tile_offsets, g->dag_rowptr,
-        g->dag_col, ranked ? g->rank : nullptr, ranked ? g->dag_rank : nullptr, nullptr, 0, nullptr,
+    dag_write_kernel<<<grid, kTileThreads, 0, s>>>(
+        g->rowptr, all, n, nnz, g->keep, g->tile_offsets, g->dag_rowptr, g->dag_col,
+        ranked ? g->rank : nullptr, ranked ? g->dag_rank : nullptr, nullptr, 0, nullptr,
         g->tile_rows);
     MC_CUDA_TRY(cudaGetLastError());
     g->launches += 2 + scan_launches(tiles);
