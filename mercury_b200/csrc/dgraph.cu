@@ -457,18 +457,36 @@ int mc_tc_count(mc_dgraph_t *g, uint64_t *count, mc_timing_t *timing) {
 
 namespace mc {
 namespace {
-// Bit rows for the triangle count: at most kDenseMax vertices, columns in
-// device memory, and no setting of the hub kernel or the orientation that a
-// caller wants to see at work.
-bool tc_dense_route(const mc_dgraph *g) {
-  if (g->n > kDenseMax || g->n == 0 || g->col_host || g->dag_host) return false;
+// How a whole triangle count runs: over the DAG's tasks; on small graphs from
+// bit rows, or from pairs of up neighbours in three launches.  The DAG's dozen
+// launches are what those save, so a setting of the hub kernel or the
+// orientation that a caller wants to see at work keeps the DAG.
+enum class TriangleRoute { kDag, kBits, kPairs };
+// Whole calls on a B200, us, bits / pairs / DAG: RMAT scale 10, edge factor 16:
+// 74 / 49 / 144; scale 13, 16 (203,886 entries): - / 144 / 189; scale 13, 32
+// (365,688): - / 336 / 195; Chung-Lu of 100,000, mean 5 (499,200): - / 78 / 190;
+// mean 20 (1,960,194): - / 323 / 284.  The pairs grow with the square of the
+// out-degrees, so beyond 2^18 entries they keep sparse graphs only.
+// Bits win while one pass over the CSR is all there is (RMAT 8, edge factors 4,
+// 16 and 64: 37 / 46 / 98, 47 / 45 / 135 and 62 / 47 / 137).
+constexpr int64_t kBitVertices = 256, kBitEntries = 4096;
+bool pairs_pay(const mc_dgraph *g) {
+  return g->nnz <= 1 << 18 || (g->nnz <= 1 << 19 && g->nnz <= 16 * g->n);
+}
+TriangleRoute triangle_route(const mc_dgraph *g) {
+  if (g->n == 0 || g->nnz == 0 || g->col_host || g->dag_host) return TriangleRoute::kDag;
+  if (g->n > kDenseMax && !pairs_pay(g)) return TriangleRoute::kDag;
   for (const char *name : {"MERCURY_TC_TABLE_LOG2_MAX", "MERCURY_TC_BITMAP_BITS",
                            "MERCURY_TC_DENSE_FACTOR", "MERCURY_TC_CORE_RANKS", "MERCURY_TC_TMA",
                            "MERCURY_TC_ROW_STAGE", "MERCURY_TC_SHORT_RANGES",
-                           "MERCURY_TC_LONG_CLASSES", "MERCURY_STAGE_EDGES"})
-    if (std::getenv(name)) return false;
-  const char *env = std::getenv("MERCURY_TC_BITS");  // 0: every graph by the DAG
-  return !(env && std::atoi(env) == 0);
+                           "MERCURY_TC_LONG_CLASSES", "MERCURY_DAG_STAGE", "MERCURY_STAGE_EDGES"})
+    if (std::getenv(name)) return TriangleRoute::kDag;
+  if (const char *env = std::getenv("MERCURY_TC_ROUTE"))  // dag, bits or pairs
+    return std::strcmp(env, "bits") == 0 && g->n <= kDenseMax ? TriangleRoute::kBits
+           : std::strcmp(env, "pairs") == 0                   ? TriangleRoute::kPairs
+                                                              : TriangleRoute::kDag;
+  if (g->n <= kBitVertices && g->nnz <= kBitEntries) return TriangleRoute::kBits;
+  return pairs_pay(g) ? TriangleRoute::kPairs : TriangleRoute::kBits;
 }
 
 // The triangle count of a handle; upload (host memory, or null) streams the
@@ -480,19 +498,28 @@ int tc_count_impl(mc_dgraph_t *g, int shard, int num_shards, uint64_t *count,
   MC_CUDA_TRY(cudaSetDevice(g->device));
   cudaStream_t s = g->stream;
   const int64_t launches_before = g->launches;
-  // Small graphs, whole: bit rows in one launch (RMAT scale 8, edge factor 8:
-  // the 20 launches and two waits below took 195 us per call).  A shard counts
-  // the tasks of the lists built below.
-  if (num_shards == 1 && !upload && tc_dense_route(g)) {
+  // Small graphs, whole (a shard counts the tasks of the lists built below).
+  // RMAT scale 8, edge factor 8: the 20 launches and two waits of the DAG took
+  // 195 us per call.
+  const TriangleRoute route =
+      num_shards == 1 && !upload ? triangle_route(g) : TriangleRoute::kDag;
+  if (route != TriangleRoute::kDag) {
     MC_CUDA_TRY(cudaEventRecord(g->ev[0], s));
-    int rc = dense_triangles(g, false);
+    int rc = MC_OK;
+    if (route == TriangleRoute::kPairs) {
+      rc = motif_triangles(g, count);
+    } else {
+      rc = dense_triangles(g, false);
+      if (rc == MC_OK) {
+        MC_CUDA_TRY(cudaEventRecord(g->ev[3], s));
+        MC_CUDA_TRY(cudaMemcpyAsync(g->h_counters, g->counters, sizeof(unsigned long long),
+                                    cudaMemcpyDeviceToHost, s));
+        MC_CUDA_TRY(cudaStreamSynchronize(s));
+        *count = (uint64_t)g->h_counters[0];
+      }
+    }
     if (rc != MC_OK) return rc;
-    MC_CUDA_TRY(cudaEventRecord(g->ev[3], s));
-    MC_CUDA_TRY(cudaMemcpyAsync(g->h_counters, g->counters, sizeof(unsigned long long),
-                                cudaMemcpyDeviceToHost, s));
-    MC_CUDA_TRY(cudaStreamSynchronize(s));
     g->counted = true;
-    *count = (uint64_t)g->h_counters[0];
     if (timing) {
       std::memset(timing, 0, sizeof(*timing));
       timing->count_ms = timing->total_ms = mc::elapsed(g->ev[0], g->ev[3]);
@@ -654,8 +681,10 @@ int mc_tc_count_host(const int64_t *rowptr, const int32_t *col, int64_t n, int64
   g->dag_built = false;
   // Pageable arrays (the reference loader's new[] arrays) cross the link
   // through pinned slots that the host threads fill (see staged_dag_passes).
-  const bool bit_rows = mc::tc_dense_route(g);
-  const bool pageable = !bit_rows && !g->col_host && nnz > 0 && mc::is_pageable(col);
+  const mc::TriangleRoute route = mc::triangle_route(g);
+  const bool bit_rows = route != mc::TriangleRoute::kDag && n <= mc::kDenseMax;
+  const bool pairs = route == mc::TriangleRoute::kPairs && !bit_rows;
+  const bool pageable = !bit_rows && !pairs && !g->col_host && nnz > 0 && mc::is_pageable(col);
   g->pin_slot[0] = g->pin_slot[1] = nullptr;
   g->pin_entries = 0;
   if (pageable) {
@@ -728,6 +757,16 @@ int mc_tc_count_host(const int64_t *rowptr, const int32_t *col, int64_t n, int64
         timing->launches = g->launches;
       }
       return MC_OK;
+    };
+    rc = whole();
+  } else if (pairs) {
+    // Too small for chunks: copied whole, checked, counted.
+    auto whole = [&]() -> int {
+      MC_CUDA_TRY(cudaMemcpyAsync(g->col, col, sizeof(int32_t) * (size_t)nnz,
+                                  cudaMemcpyHostToDevice, g->stream));
+      const int vrc = mc::validate_graph(g, 0);
+      validate_launches = g->launches;
+      return vrc == MC_OK ? mc_tc_count(g, count, timing) : vrc;
     };
     rc = whole();
   } else if (g->col_host) {

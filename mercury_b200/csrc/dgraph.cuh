@@ -179,6 +179,9 @@ constexpr int kDenseMax = 1024;
 int motif_count(mc_dgraph *g, int pattern, uint64_t *out);
 int dense_count(mc_dgraph *g, int pattern, uint64_t *out);
 int dense_triangles(mc_dgraph *g, bool check);
+// Triangles from pairs of up neighbours (motifs.cu): three launches.
+// Synchronous; event ev[3] marks its last kernel.
+int motif_triangles(mc_dgraph *g, uint64_t *out);
 // Part `part` of `parts` of one pattern graph of a batch.
 struct DenseTask {
   int64_t v0;

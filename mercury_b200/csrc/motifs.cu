@@ -157,6 +157,21 @@ __device__ __forceinline__ void walk_lists(const MotifArgs &a, int64_t lo, int l
   }
 }
 
+// The lanes of a warp that hold entries of the same row u (rows in order): from
+// the last row head at or below this lane to the one before the next head.
+struct RowLanes {
+  int first;
+  unsigned mask;
+  __device__ __forceinline__ RowLanes(int u, int lane) {  // every lane calls it
+    const int prev = __shfl_up_sync(kFull, u, 1);
+    const unsigned heads = __ballot_sync(kFull, lane == 0 || u != prev);
+    const unsigned upto = kFull >> (kWarp - 1 - lane);
+    const unsigned later = heads & ~upto;
+    first = kWarp - 1 - __clz(heads & upto);
+    mask = (later ? (1u << (__ffs(later) - 1)) - 1u : kFull) & (kFull << first);
+  }
+};
+
 __device__ __forceinline__ bool lists_overrun(const MotifArgs &a) {
   return *a.pool > (u64)a.list_cap;
 }
@@ -221,14 +236,9 @@ __global__ void __launch_bounds__(kThreads) motif_up_kernel(MotifArgs a) {
   }
   const bool up = r >= 0;
   const unsigned ups = __ballot_sync(kFull, up);
-  // Lanes of the same row: from the last row head at or below this lane to
-  // the one before the next head.
-  const int u_prev = __shfl_up_sync(kFull, u, 1);
-  const unsigned heads = __ballot_sync(kFull, lane == 0 || u != u_prev);
-  const unsigned upto = kFull >> (kWarp - 1 - lane);
-  const int first = kWarp - 1 - __clz(heads & upto);
-  const unsigned later = heads & ~upto;
-  const unsigned row = (later ? (1u << (__ffs(later) - 1)) - 1u : kFull) & (kFull << first);
+  const RowLanes rl(u, lane);
+  const int first = rl.first;
+  const unsigned row = rl.mask;
   int base = 0;
   if (lane == first && (ups & row)) base = atomicAdd(a.dp + u, __popc(ups & row));
   base = __shfl_sync(kFull, base, first);
@@ -348,6 +358,63 @@ __global__ void __launch_bounds__(kThreads) motif_tri_kernel(MotifArgs a, int pe
     bs.add(kVtd, vtd);
     bs.flush(a.acc);
   }
+}
+
+// Triangles alone, in three launches (rows, up, pairs) where the DAG's
+// orientation takes a dozen: the up neighbours of each row compacted in place
+// (upe holds vertices here), then the pairs of motif_tri_kernel, counted.
+__global__ void __launch_bounds__(kThreads) tri_up_kernel(MotifArgs a) {
+  const int lane = threadIdx.x & (kWarp - 1);
+  const int64_t e64 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  const bool in = e64 < a.nnz;
+  const int e = in ? (int)e64 : a.nnz - 1;
+  const int u = a.src[e], v = __ldg(a.ci + e);
+  const bool up = in && lower(a.deg[u], u, a.deg[v], v);
+  const unsigned ups = __ballot_sync(kFull, up);
+  const RowLanes rl(u, lane);
+  int base = 0;
+  if (lane == rl.first && (ups & rl.mask)) base = atomicAdd(a.dp + u, __popc(ups & rl.mask));
+  base = __shfl_sync(kFull, base, rl.first);
+  if (up) a.upe[__ldg(a.rp + u) + base + __popc(ups & rl.mask & ((1u << lane) - 1u))] = v;
+}
+
+__global__ void __launch_bounds__(kThreads) tri_pairs_kernel(MotifArgs a, int per) {
+  __shared__ u64 s_total;
+  if (threadIdx.x == 0) s_total = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & (kWarp - 1);
+  const int64_t s64 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  const int64_t mine = s64 / kWarp * per + lane;
+  int slot = 0, len = 0, x = 0, dx = 0;
+  if (lane < per && mine < a.nnz) {
+    slot = (int)mine;
+    const int u = a.src[slot];
+    const int i = slot - (int)__ldg(a.rp + u), p = a.dp[u];
+    if (i < p - 1) {
+      len = p - 1 - i;
+      x = a.upe[slot];
+      dx = a.deg[x];
+    }
+  }
+  const FlatLists fl(len, lane);
+  u64 hits = 0;
+  for (int base = 0; base < fl.total; base += kWarp) {
+    const int f = base + lane;
+    const int l = fl.owner(f);
+    const int ys = f + __shfl_sync(kFull, slot + 1 - (fl.incl - len), l);
+    const int vx = __shfl_sync(kFull, x, l), dvx = __shfl_sync(kFull, dx, l);
+    if (f >= fl.total) continue;
+    const int y = a.upe[ys];
+    const int dy = a.deg[y];
+    const bool x_low = lower(dvx, vx, dy, y);
+    const int b = (int)__ldg(a.rp + (x_low ? vx : y));
+    hits += find_entry(a.ci, b, b + (x_low ? dvx : dy), x_low ? y : vx) >= 0;
+  }
+  __syncwarp();
+  hits = warp_sum_u64(hits);
+  if (lane == 0 && hits) atomicAdd(&s_total, hits);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_total) atomicAdd(a.acc + kT, s_total);
 }
 
 // ---- triangles with their common neighbours -----------------------------------
@@ -1053,6 +1120,50 @@ PatternRoute pattern_route(const mc_dgraph *g, int pattern) {
     if (pattern == 4 && g->nnz <= 12288) return PatternRoute::kFormula;
   }
   return PatternRoute::kSparse;
+}
+
+int motif_triangles(mc_dgraph *g, uint64_t *out) {
+  NvtxRange range("motif_triangles");
+  cudaStream_t s = g->stream;
+  const int n = (int)g->n, nnz = (int)g->nnz;
+  MotifArgs a{};
+  a.rp = g->rowptr;
+  a.ci = g->col;
+  a.n = n;
+  a.nnz = nnz;
+  size_t zeroed = 0;
+  auto lay_out = [&](Carver &c) {
+    a.acc = c.take<u64>(kSums);
+    a.dp = c.take<int32_t>(n);
+    zeroed = c.used;
+    a.deg = c.take<int32_t>(n);
+    a.src = c.take<int32_t>(nnz);
+    a.upe = c.take<int32_t>(nnz);
+  };
+  Carver size, c;
+  lay_out(size);
+  MC_CUDA_TRY(dev_alloc(reinterpret_cast<void **>(&c.base), block_bytes(size.used), s));
+  lay_out(c);
+  u64 total = 0;
+  auto run = [&]() -> int {
+    MC_CUDA_TRY(cudaMemsetAsync(c.base, 0, zeroed, s));
+    motif_rows_kernel<<<std::min(blocks(n, kWarps), 4096u), kThreads, 0, s>>>(a);
+    MC_CUDA_TRY(cudaGetLastError());
+    tri_up_kernel<<<blocks(nnz, kThreads), kThreads, 0, s>>>(a);
+    MC_CUDA_TRY(cudaGetLastError());
+    const int per = spread(nnz, g->num_sms);
+    tri_pairs_kernel<<<blocks(((int64_t)nnz + per - 1) / per * kWarp, kThreads), kThreads, 0, s>>>(a, per);
+    MC_CUDA_TRY(cudaGetLastError());
+    g->launches += 3;
+    MC_CUDA_TRY(cudaEventRecord(g->ev[3], s));
+    MC_CUDA_TRY(cudaMemcpyAsync(&total, a.acc + kT, sizeof(total), cudaMemcpyDeviceToHost, s));
+    MC_CUDA_TRY(cudaStreamSynchronize(s));
+    return MC_OK;
+  };
+  const int rc = run();
+  dev_free(c.base, s);
+  if (rc == MC_OK) *out = total;
+  return rc;
 }
 
 int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {

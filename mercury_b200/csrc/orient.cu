@@ -45,8 +45,9 @@ constexpr int kTileWords = (int)(kTileEdges / kWarp);       // keep words per ti
 // entry's row is the nearest mark at or before it, which a ballot finds within
 // a round, and a carry across rounds.  No lane ever walks rows (sixteen
 // consecutive entries per lane, each lane stepping over its rows' offsets,
-// diverged on every row boundary and empty row: 322 us for checks at RMAT scale 20; at scale 22 pass A took 1.08 ms and takes
-// 0.79, pass B 1.13 and 0.36; the checks at scale 20 take 157 us).
+// diverged on every row boundary and empty row: 322 us for the checks at RMAT
+// scale 20, against 157; at scale 22, 1.08 ms for pass A and 1.13 for pass B,
+// against 0.79 and 0.36).
 struct TileMarks {
   int64_t lo;      // row of the tile's first entry
   bool at_start;   // that row starts at the tile
