@@ -28,7 +28,7 @@ void release(mc_dgraph *g) {
   void *bufs[] = {g->rowptr,     g->col,        g->key,      g->dag_rowptr,
                   g->dag_col,    g->keep,       g->tile_counts, g->tile_offsets,
                   g->deg,        g->list_len,   g->task_status, g->hub_tasks,
-                  g->leaf_tasks, g->scan_temp,  g->counters, g->err, g->pat_scratch,
+                  g->leaf_tasks, g->scan_temp,  g->counters, g->pat_scratch,
                   g->mega_tasks, g->rank,
                   g->dag_rank,   g->rank_keys,  g->rank_work,
                   g->center_scratch, g->stage, g->chunk_offsets, g->core_bits, g->pinfo,
@@ -37,6 +37,7 @@ void release(mc_dgraph *g) {
   if (g->dag_host)  // DAG entries and ranks: pinned host memory, freed below
     for (void *&p : bufs)
       if (p == g->dag_col || p == g->dag_rank) p = nullptr;
+  if (g->copy_stream) cudaStreamSynchronize(g->copy_stream);
   // Stream-ordered frees: no device-wide synchronisation, so other handles'
   // work keeps running while this one is released.
   for (void *p : bufs)
@@ -156,8 +157,9 @@ int create_common(int64_t n, int64_t nnz, void *stream, mc_dgraph **out, mc_dgra
   } else {
     MC_CUDA_TRY(dev_alloc((void **)&g->col, col_bytes, g->stream));
   }
-  MC_CUDA_TRY(dev_alloc((void **)&g->counters, sizeof(unsigned long long) * 8, g->stream));
-  MC_CUDA_TRY(dev_alloc((void **)&g->err, sizeof(unsigned), g->stream));
+  // The error word follows the counters: one copy brings both back.
+  MC_CUDA_TRY(dev_alloc((void **)&g->counters, sizeof(unsigned long long) * 9, g->stream));
+  g->err = reinterpret_cast<unsigned *>(g->counters + 8);
   // Host mirror of the counters (read after a stream synchronisation).
   g->h_counters = new (std::nothrow) unsigned long long[16]();
   if (!g->h_counters) return MC_ERR_OOM;
@@ -578,9 +580,9 @@ int tc_count_impl(mc_dgraph_t *g, int shard, int num_shards, uint64_t *count,
   rc = mc::tc_count_launch(g, g->ev[2], shard, num_shards);
   if (rc != MC_OK) return rc;
   MC_CUDA_TRY(cudaEventRecord(g->ev[3], s));
-  MC_CUDA_TRY(cudaMemcpyAsync(g->h_counters, g->counters, sizeof(unsigned long long) * 8,
+  MC_CUDA_TRY(cudaMemcpyAsync(g->h_counters, g->counters,
+                              sizeof(unsigned long long) * 8 + sizeof(unsigned),
                               cudaMemcpyDeviceToHost, s));
-  MC_CUDA_TRY(cudaMemcpyAsync(g->h_err, g->err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   MC_CUDA_TRY(cudaStreamSynchronize(s));
   if (*g->h_err) return MC_ERR_DEVICE;
   g->counted = true;
