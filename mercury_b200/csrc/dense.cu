@@ -375,30 +375,24 @@ int dense_count(mc_dgraph *g, int pattern, uint64_t *out) {
   cudaStream_t s = g->stream;
   const int n = (int)g->n;
   const size_t smem = dense_bytes(n);
-  u64 *acc = nullptr;
-  MC_CUDA_TRY(dev_alloc(reinterpret_cast<void **>(&acc), sizeof(u64) * kSums, s));
+  u64 *acc = g->sums;
   u64 h[kSums];
-  auto run = [&]() -> int {
-    MC_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(u64) * kSums, s));
-    MC_CUDA_TRY(cudaFuncSetAttribute(dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
-    // A CTA per SM at most: each builds the matrix, which costs as much as
-    // its share of the tasks.
-    const int tasks = n * dense_words(n), warps = kDenseThreads / kWarp;
-    dense_kernel<<<std::min(g->num_sms, (tasks + warps - 1) / warps), kDenseThreads, smem, s>>>(
-        DenseGraph{g->rowptr, g->col, 0, n}, pattern, acc);
-    MC_CUDA_TRY(cudaGetLastError());
-    g->launches += 1;
-    MC_CUDA_TRY(cudaEventRecord(g->ev[3], s));
-    MC_CUDA_TRY(cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, s));
-    MC_CUDA_TRY(cudaStreamSynchronize(s));
-    return MC_OK;
-  };
-  const int rc = run();
-  dev_free(acc, s);
+  MC_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(u64) * kSums, s));
+  MC_CUDA_TRY(cudaFuncSetAttribute(dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)smem));
+  // A CTA per SM at most: each builds the matrix, which costs as much as
+  // its share of the tasks.
+  const int tasks = n * dense_words(n), warps = kDenseThreads / kWarp;
+  dense_kernel<<<std::min(g->num_sms, (tasks + warps - 1) / warps), kDenseThreads, smem, s>>>(
+      DenseGraph{g->rowptr, g->col, 0, n}, pattern, acc);
+  MC_CUDA_TRY(cudaGetLastError());
+  g->launches += 1;
+  MC_CUDA_TRY(cudaEventRecord(g->ev[3], s));
+  MC_CUDA_TRY(cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, s));
+  MC_CUDA_TRY(cudaStreamSynchronize(s));
   h[kX7] >>= 1;  // counted from both ends of its inner edge
-  if (rc == MC_OK) *out = motif_combine(pattern, h);
-  return rc;
+  *out = motif_combine(pattern, h);
+  return MC_OK;
 }
 
 // Parts of one graph of a batch: about 1 M row words each (pairs, and three

@@ -59,10 +59,20 @@ struct NvtxRange {
 // calls reuse their buffers. The pool stays private to this process.
 void retain_pool_memory(int device);
 
-inline cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s) {
-  return cudaMallocAsync(p, bytes < 8 ? 8 : bytes, s);
-}
+cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s);
 inline void dev_free(void *p, cudaStream_t s) { cudaFreeAsync(p, s); }
+
+// Scratch of one count (scratch.cu).  scratch_take returns a block of at least
+// `bytes` (its size in *got); scratch_give takes it back once no work that
+// uses it is in flight (dev_free instead where some may be).
+// scratch_flush returns all kept blocks to the pool (false: there were none);
+// scratch_attach/detach count the device's graph handles.
+cudaError_t scratch_take(void **p, size_t bytes, size_t *got, int device, cudaStream_t s);
+void scratch_give(void *p, size_t bytes, int device, cudaStream_t s);
+bool scratch_flush(int device, cudaStream_t s);
+size_t scratch_kept(int device);
+void scratch_attach(int device);
+void scratch_detach(int device, cudaStream_t s);
 
 __device__ __forceinline__ int warp_inclusive_scan(int v, int lane) {
 #pragma unroll

@@ -7,6 +7,7 @@
 
 #include "dgraph.cuh"
 #include "device_common.cuh"
+#include "motifs.cuh"
 #include "scan.cuh"
 
 namespace mc {
@@ -42,6 +43,7 @@ void release(mc_dgraph *g) {
   // work keeps running while this one is released.
   for (void *p : bufs)
     if (p) dev_free(p, g->stream);
+  if (g->attached) scratch_detach(g->device, g->stream);
   if (g->stream) cudaStreamSynchronize(g->stream);
   if (g->col_host && g->col_h) cudaFreeHost(g->col_h);
   if (g->dag_col_h) cudaFreeHost(g->dag_col_h);
@@ -72,6 +74,7 @@ int device_bytes_available(int device, int64_t *avail) {
         reserved > used)
       a += (int64_t)(reserved - used);
   }
+  a += (int64_t)scratch_kept(device);
   if (const char *env = std::getenv("MERCURY_DEVICE_BYTES")) {
     const long long v = std::atoll(env);
     if (v > 0) a = v;
@@ -139,6 +142,8 @@ int create_common(int64_t n, int64_t nnz, void *stream, mc_dgraph **out, mc_dgra
   MC_CUDA_TRY(cudaGetDevice(&g->device));
   MC_CUDA_TRY(cudaDeviceGetAttribute(&g->num_sms, cudaDevAttrMultiProcessorCount, g->device));
   retain_pool_memory(g->device);
+  scratch_attach(g->device);
+  g->attached = true;
   if (stream) {
     g->stream = static_cast<cudaStream_t>(stream);
   } else {
@@ -158,8 +163,9 @@ int create_common(int64_t n, int64_t nnz, void *stream, mc_dgraph **out, mc_dgra
     MC_CUDA_TRY(dev_alloc((void **)&g->col, col_bytes, g->stream));
   }
   // The error word follows the counters: one copy brings both back.
-  MC_CUDA_TRY(dev_alloc((void **)&g->counters, sizeof(unsigned long long) * 9, g->stream));
+  MC_CUDA_TRY(dev_alloc((void **)&g->counters, sizeof(unsigned long long) * (16 + kSums), g->stream));
   g->err = reinterpret_cast<unsigned *>(g->counters + 8);
+  g->sums = g->counters + 16;
   // Host mirror of the counters (read after a stream synchronisation).
   g->h_counters = new (std::nothrow) unsigned long long[16]();
   if (!g->h_counters) return MC_ERR_OOM;

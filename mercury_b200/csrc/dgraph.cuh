@@ -59,6 +59,7 @@ struct mc_dgraph {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  bool attached = false;  // counted among the handles that share scratch (scratch.cu)
   int num_sms = 0;
   int64_t n = 0, nnz = 0;
   int64_t max_degree = 0;     // set by validation on upload
@@ -140,6 +141,7 @@ struct mc_dgraph {
   // 0: result, 1: hub queue, 2: leaf queue, 3: max d+, 4-5: partner
   // statistics, 6: large-table hub queue, 7: max degree (validation)
   unsigned long long *counters = nullptr;
+  unsigned long long *sums = nullptr;  // motif sums of the bit-row route, behind the counters
   unsigned *err = nullptr;
   // pinned host mirror of counters + err
   unsigned long long *h_counters = nullptr;

@@ -1021,16 +1021,6 @@ int resident(const void *kernel, int threads, size_t smem) {
   return std::max(per_sm, 1);
 }
 
-// Scratch blocks come in eight sizes per power of two: the pool hands a block
-// of the same size out again as it is, and maps memory anew for any other size
-// (about a millisecond per call when counts of similar graphs, or of several
-// patterns, alternated with sizes of their own).
-size_t block_bytes(size_t bytes) {
-  size_t step = size_t(1) << 20;
-  while (step * 16 < bytes) step *= 2;
-  return (bytes + step - 1) / step * step;
-}
-
 // Carves aligned arrays out of one allocation.
 struct Carver {
   char *base = nullptr;
@@ -1142,7 +1132,8 @@ int motif_triangles(mc_dgraph *g, uint64_t *out) {
   };
   Carver size, c;
   lay_out(size);
-  MC_CUDA_TRY(dev_alloc(reinterpret_cast<void **>(&c.base), block_bytes(size.used), s));
+  size_t got = 0;
+  MC_CUDA_TRY(scratch_take(reinterpret_cast<void **>(&c.base), size.used, &got, g->device, s));
   lay_out(c);
   u64 total = 0;
   auto run = [&]() -> int {
@@ -1161,7 +1152,8 @@ int motif_triangles(mc_dgraph *g, uint64_t *out) {
     return MC_OK;
   };
   const int rc = run();
-  dev_free(c.base, s);
+  if (rc == MC_OK) scratch_give(c.base, got, g->device, s);
+  else dev_free(c.base, s);
   if (rc == MC_OK) *out = total;
   return rc;
 }
@@ -1206,7 +1198,7 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
     a.warp_walk = n <= kFewVertices ? kFewWalk : kWarpWalk;
     a.mid_walk = kMidWalk;
     size_t zeroed = 0;
-    // The same layout for every pattern (see block_bytes).
+    // The same layout for every pattern (so that each finds the last one's block).
     auto lay_out = [&](Carver &c) {
       // Zeroed before the first kernel.
       a.acc = c.take<u64>(kSums + 1);
@@ -1241,11 +1233,13 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
       MC_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
       if (size.used + counters_b > free_b / 2) return MC_ERR_OOM;
     }
-    MC_CUDA_TRY(dev_alloc(reinterpret_cast<void **>(&c.base), block_bytes(size.used), s));
+    size_t got = 0, got_counters = 0;
+    MC_CUDA_TRY(scratch_take(reinterpret_cast<void **>(&c.base), size.used, &got, g->device, s));
     lay_out(c);
     unsigned *counters = nullptr;
     if (counters_b) {
-      const cudaError_t e = dev_alloc(reinterpret_cast<void **>(&counters), block_bytes(counters_b), s);
+      const cudaError_t e = scratch_take(reinterpret_cast<void **>(&counters), counters_b,
+                                         &got_counters, g->device, s);
       if (e != cudaSuccess) dev_free(c.base, s);
       MC_CUDA_TRY(e);
     }
@@ -1311,9 +1305,13 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
       return MC_OK;
     };
     const int rc = run();
-    dev_free(c.base, s);
-    if (counters) dev_free(counters, s);
-    if (rc != MC_OK) return rc;
+    if (rc != MC_OK) {  // work may be in flight: freed in the stream's order
+      dev_free(c.base, s);
+      if (counters) dev_free(counters, s);
+      return rc;
+    }
+    scratch_give(c.base, got, g->device, s);
+    scratch_give(counters, got_counters, g->device, s);
     const int64_t asked = (int64_t)h[kSums];
     if (asked <= list_cap) {
       *out = motif_combine(pattern, h);

@@ -1804,8 +1804,7 @@ int launch_center(mc_dgraph *g, const CenterArgs &a, int num_sms, int64_t total,
       if (g->hop_scratch) dev_free(g->hop_scratch, g->stream);
       g->hop_scratch = nullptr;
       g->hop_scratch_bytes = 0;
-      MC_CUDA_TRY(dev_alloc(&g->hop_scratch, bytes, g->stream));
-      g->hop_scratch_bytes = bytes;
+      MC_CUDA_TRY(scratch_take(&g->hop_scratch, bytes, &g->hop_scratch_bytes, g->device, g->stream));
     }
     ha.hop = per_group > 0 ? static_cast<unsigned *>(g->hop_scratch) : nullptr;
     ha.hop_words = per_group;
@@ -1991,8 +1990,7 @@ int center_path(mc_dgraph *g, int pattern, PatArgs a, int grid, Slicer *sl) {
     if (g->center_scratch) dev_free(g->center_scratch, s);
     g->center_scratch = nullptr;
     g->center_scratch_bytes = 0;
-    MC_CUDA_TRY(dev_alloc(&g->center_scratch, need, s));
-    g->center_scratch_bytes = need;
+    MC_CUDA_TRY(scratch_take(&g->center_scratch, need, &g->center_scratch_bytes, g->device, s));
   }
   char *base = static_cast<char *>(g->center_scratch);
   int32_t *lists = reinterpret_cast<int32_t *>(base);
@@ -2078,8 +2076,7 @@ int center_path(mc_dgraph *g, int pattern, PatArgs a, int grid, Slicer *sl) {
       if (g->hub_bits) dev_free(g->hub_bits, s);
       g->hub_bits = nullptr;
       g->hub_bits_bytes = 0;
-      MC_CUDA_TRY(dev_alloc(&g->hub_bits, bits_b, s));
-      g->hub_bits_bytes = bits_b;
+      MC_CUDA_TRY(scratch_take(&g->hub_bits, bits_b, &g->hub_bits_bytes, g->device, s));
     }
     MC_CUDA_TRY(cudaMemsetAsync(g->hub_bits, 0, bits_b, s));
     HubP1Args ha{g->rowptr, g->col, n, chunk_off, static_cast<unsigned *>(g->hub_bits),
@@ -2136,15 +2133,16 @@ int pattern_count_body(mc_dgraph *g, int pattern, uint64_t *out, uint64_t *c12,
                        double *progress);
 
 // The pattern scratch (frontier lists, center classes, two-hop rows, hub
-// bitmaps) goes back to the stream-ordered pool after every count: a later
-// count on any handle reuses it from the pool, and a process that keeps
-// thousands of small graphs resident holds their CSRs only.
-void release_pattern_scratch(mc_dgraph *g) {
+// bitmaps) is given back after every count (scratch.cu): a later count on any
+// handle reuses it, and a process that keeps thousands of small graphs
+// resident holds their CSRs only.
+void release_pattern_scratch(mc_dgraph *g, bool idle) {
   void **bufs[] = {&g->pat_scratch, &g->center_scratch, &g->hop_scratch, &g->hub_bits};
   size_t *sizes[] = {&g->pat_scratch_bytes, &g->center_scratch_bytes, &g->hop_scratch_bytes,
                      &g->hub_bits_bytes};
   for (int i = 0; i < 4; ++i) {
-    if (*bufs[i]) dev_free(*bufs[i], g->stream);
+    if (*bufs[i] && idle) scratch_give(*bufs[i], *sizes[i], g->device, g->stream);
+    else if (*bufs[i]) dev_free(*bufs[i], g->stream);
     *bufs[i] = nullptr;
     *sizes[i] = 0;
   }
@@ -2155,7 +2153,8 @@ int pattern_count(mc_dgraph *g, int pattern, uint64_t *out, uint64_t *c12, mc_ti
                   int shard, int num_shards, double budget_ms, double *progress) {
   const int rc = pattern_count_body(g, pattern, out, c12, timing, shard, num_shards, budget_ms,
                                     progress);
-  release_pattern_scratch(g);
+  // A count that ended well has waited for its stream.
+  release_pattern_scratch(g, rc == MC_OK);
   return rc;
 }
 
@@ -2220,8 +2219,7 @@ int pattern_count_body(mc_dgraph *g, int pattern, uint64_t *out, uint64_t *c12,
     if (g->pat_scratch) dev_free(g->pat_scratch, s);
     g->pat_scratch = nullptr;
     g->pat_scratch_bytes = 0;
-    MC_CUDA_TRY(dev_alloc(&g->pat_scratch, need, s));
-    g->pat_scratch_bytes = need;
+    MC_CUDA_TRY(scratch_take(&g->pat_scratch, need, &g->pat_scratch_bytes, g->device, s));
   }
   PatArgs a{g->rowptr, g->col, g->n, g->nnz, static_cast<int32_t *>(g->pat_scratch), cap,
             g->counters + 0, g->counters + 2};

@@ -1,0 +1,39 @@
+"""Scratch shared by the counts of many handles: blocks of other sizes, from
+other streams and threads, kept and given back."""
+from concurrent.futures import ThreadPoolExecutor
+
+import numpy as np
+import pytest
+
+from mercury_b200 import DeviceGraph, Graph
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("threads", [1, 4])
+def test_counts_of_interleaved_handles(threads):
+    """Handles of several sizes (bit rows, sparse sums, formulas; scratch from
+    the smallest block to 80 MB), each on its own stream, counted in turn and
+    from several threads: every count stays its graph's own, also after all
+    handles are gone and new ones take the blocks again."""
+    specs = [(60, 6.0, 20.0), (300, 8.0, 60.0), (1500, 8.0, 90.0), (6000, 6.0, 120.0),
+             (20000, 5.0, 60.0)]
+    graphs = [Graph.chung_lu(n, 2.1, mean, cap, seed=n) for n, mean, cap in specs]
+    arrays = [(np.array(g.rowptr), np.array(g.col)) for g in graphs]
+    want = [[orc.tc(rp, col)] + [orc.pattern(rp, col, p) for p in (1, 4, 7, 8)]
+            for rp, col in arrays]
+
+    def work(d):
+        return [d.tc_count()] + [d.pattern_count(p) for p in (1, 4, 7, 8)]
+
+    for _ in range(2):
+        handles = [DeviceGraph(rp, col) for rp, col in arrays for _ in range(threads)]
+        try:
+            with ThreadPoolExecutor(threads) as pool:
+                for _ in range(3):
+                    got = list(pool.map(work, handles))
+                    assert got == [w for w in want for _ in range(threads)]
+        finally:
+            for d in handles:
+                d.close()
