@@ -360,7 +360,7 @@ int dense_triangles(mc_dgraph *g, bool check) {
   auto kern = check ? dense_triangles_kernel<true> : dense_triangles_kernel<false>;
   MC_CUDA_TRY(cudaMemsetAsync(g->counters, 0, 2 * sizeof(u64), s));
   if (smem > (size_t(40) << 10))
-    MC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MC_CUDA_TRY(allow_smem((const void *)kern, smem));
   // About 2^16 row words per CTA: each builds the matrix for itself.
   const int64_t words = g->nnz * dense_words(n) / 2;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(g->num_sms, words >> 16));
@@ -378,8 +378,7 @@ int dense_count(mc_dgraph *g, int pattern, uint64_t *out) {
   u64 *acc = g->sums;
   u64 h[kSums];
   MC_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(u64) * kSums, s));
-  MC_CUDA_TRY(cudaFuncSetAttribute(dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
+  MC_CUDA_TRY(allow_smem((const void *)dense_kernel, smem));
   // A CTA per SM at most: each builds the matrix, which costs as much as
   // its share of the tasks.
   const int tasks = n * dense_words(n), warps = kDenseThreads / kWarp;
@@ -409,8 +408,7 @@ int dense_parts(int64_t n, int64_t nnz, int64_t max_degree) {
 int dense_batch_launch(const int64_t *rp, const int32_t *ci, const DenseTask *tasks, int num_tasks,
                        int largest, unsigned long long *acc, cudaStream_t s) {
   const size_t smem = dense_bytes(largest);
-  MC_CUDA_TRY(cudaFuncSetAttribute(dense_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)dense_bytes(kDenseMax)));
+  MC_CUDA_TRY(allow_smem((const void *)dense_batch_kernel, dense_bytes(kDenseMax)));
   dense_batch_kernel<<<num_tasks, kBatchThreads, smem, s>>>(rp, ci, tasks, acc);
   MC_CUDA_TRY(cudaGetLastError());
   return MC_OK;

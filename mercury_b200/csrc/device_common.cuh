@@ -62,6 +62,12 @@ void retain_pool_memory(int device);
 cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s);
 inline void dev_free(void *p, cudaStream_t s) { cudaFreeAsync(p, s); }
 
+// Lets launches of kern use up to `bytes` of dynamic shared memory.  The limit
+// belongs to the function, not to the launch: it only grows here, so that a
+// thread with a smaller table does not lower it between another thread's call
+// and its launch (which then failed as an invalid argument).
+cudaError_t allow_smem(const void *kern, size_t bytes);
+
 // Scratch of one count (scratch.cu).  scratch_take returns a block of at least
 // `bytes` (its size in *got); scratch_give takes it back once no work that
 // uses it is in flight (dev_free instead where some may be).

@@ -3,6 +3,8 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <new>
 
 #include "dgraph.cuh"
@@ -229,6 +231,15 @@ thread_local HostCache t_cache;
 
 void set_last_cuda_error(cudaError_t e) { t_last_cuda = e; }
 cudaError_t last_cuda_error() { return t_last_cuda; }
+
+cudaError_t allow_smem(const void *kern, size_t bytes) {
+  static std::mutex mu;
+  static std::map<const void *, size_t> *limits = new std::map<const void *, size_t>;
+  std::lock_guard<std::mutex> lock(mu);
+  size_t &limit = (*limits)[kern];
+  limit = std::max(limit, bytes);
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+}
 
 void retain_pool_memory(int device) {
   static std::atomic<unsigned long long> done{0};  // one bit per device (first 64)

@@ -1039,7 +1039,7 @@ int launch_pairs(mc_dgraph *g, const MotifArgs &a, int64_t longest, int big_grid
                  size_t table_b, unsigned *counters) {
   cudaStream_t s = g->stream;
   auto launch = [&](auto kern, int threads, size_t smem, int64_t items) -> int {
-    MC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MC_CUDA_TRY(allow_smem((const void *)kern, smem));
     const int64_t fit = items <= g->num_sms
                             ? items
                             : (int64_t)g->num_sms * resident((const void *)kern, threads, smem);
@@ -1057,7 +1057,7 @@ int launch_pairs(mc_dgraph *g, const MotifArgs &a, int64_t longest, int big_grid
   if (rc != MC_OK || longest <= (int64_t)kHashWalk) return rc;
   auto big = shared ? motif_pairs_big_kernel<kOrdered, true> : motif_pairs_big_kernel<kOrdered, false>;
   const size_t smem = shared ? table_b : 0;
-  MC_CUDA_TRY(cudaFuncSetAttribute(big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  MC_CUDA_TRY(allow_smem((const void *)big, smem));
   big<<<big_grid, kPairThreads, smem, s>>>(a, counters);
   MC_CUDA_TRY(cudaGetLastError());
   g->launches += 1;
@@ -1269,8 +1269,7 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
         MC_CUDA_TRY(cudaGetLastError());
         g->launches += 4;
       } else {
-        MC_CUDA_TRY(cudaFuncSetAttribute(motif_tau_kernel<true, false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kTauSmem));
+        MC_CUDA_TRY(allow_smem((const void *)motif_tau_kernel<true, false>, kTauSmem));
         motif_tau_kernel<true, false><<<tau_grid, kThreads, kTauSmem, s>>>(a, kTauSmem / 4);
         MC_CUDA_TRY(cudaGetLastError());
         motif_tau_kernel<false, true><<<tau_small_grid, kThreads, 0, s>>>(a, 0);
@@ -1290,8 +1289,7 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
         if (g->max_degree > kWheelDeg) {
           const int table = (int)g->max_degree;
           const size_t smem = sizeof(unsigned) * (size_t)table;
-          MC_CUDA_TRY(cudaFuncSetAttribute(motif_wheel_big_kernel,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+          MC_CUDA_TRY(allow_smem((const void *)motif_wheel_big_kernel, smem));
           const int per_sm = resident((const void *)motif_wheel_big_kernel, kThreads, smem);
           motif_wheel_big_kernel<<<std::min(blocks(nnz, kThreads), (unsigned)(per_sm * g->num_sms)),
                                    kThreads, smem, s>>>(a, table);

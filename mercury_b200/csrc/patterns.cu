@@ -1777,7 +1777,7 @@ int launch_center(mc_dgraph *g, const CenterArgs &a, int num_sms, int64_t total,
   constexpr int G = center_group(W);
   const size_t smem = center_group_bytes(P, W) * (kPatThreads / kWarp / G);
   auto kern = center_kernel<P, W>;
-  MC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  MC_CUDA_TRY(allow_smem((const void *)kern, smem));
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPatThreads, smem) != cudaSuccess ||
       per_sm < 1)

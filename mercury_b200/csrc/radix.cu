@@ -263,7 +263,7 @@ cudaError_t sort_passes(u64 *keys, u64 *alt, int64_t count, int begin_bit, int p
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   auto kern = radix_pass_kernel<kBits, S>;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem<kBits>());
+  e = allow_smem((const void *)kern, pass_smem<kBits>());
   if (e != cudaSuccess) return e;
   u64 *buf[2] = {keys, alt};
   int cur = 0;

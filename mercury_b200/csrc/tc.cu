@@ -1055,8 +1055,7 @@ int tc_count_launch(mc_dgraph *g, cudaEvent_t after_hub, int shard, int num_shar
   auto kern = staged ? tc_hub_kernel<true, false>
                      : (row_stage ? tc_hub_kernel<false, true> : tc_hub_kernel<false, false>);
   const size_t extra = staged ? kStageBytes : 0;
-  MC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(big_smem + extra)));
+  MC_CUDA_TRY(allow_smem((const void *)kern, big_smem + extra));
   a.table_log2_max = small_lg;
   a.tasks = g->hub_tasks;
   a.ntasks = g->list_len;

@@ -37,3 +37,19 @@ def test_counts_of_interleaved_handles(threads):
         finally:
             for d in handles:
                 d.close()
+
+
+def test_triangle_counts_of_different_table_sizes_in_threads(monkeypatch):
+    """The hub kernel's shared-memory limit belongs to the function: a thread
+    with small tables must not lower it under another thread's launch."""
+    monkeypatch.setenv("MERCURY_TC_ROUTE", "dag")
+    graphs = [Graph.rmat(15, 16, seed=3), Graph.rmat(10, 8, seed=4)]
+    want = [orc.tc(np.array(g.rowptr), np.array(g.col)) for g in graphs]
+
+    def work(i):
+        with DeviceGraph(graphs[i]) as d:
+            return [d.tc_count() for _ in range(400)]
+
+    with ThreadPoolExecutor(2) as pool:
+        for got, w in zip(pool.map(work, [0, 1]), want):
+            assert set(got) == {w}
