@@ -254,7 +254,9 @@ int mc_tc_count(mc_dgraph_t *g, uint64_t *count, mc_timing_t *timing);
  * tc_multigpu/tc_challenge_multigpu.cu:198-206). */
 int mc_tc_count_shard(mc_dgraph_t *g, int shard, int num_shards,
                       uint64_t *partial, mc_timing_t *timing);
-/* Preprocessing sizes of the last mc_tc_count on this handle. */
+/* Preprocessing sizes of the last mc_tc_count on this handle.  Small graphs
+ * are counted without the DAG; this call and mc_dgraph_export_dag then build
+ * it. */
 int mc_tc_stats(const mc_dgraph_t *g, mc_tc_stats_t *stats);
 /* Copies the device-built DAG (after mc_tc_count) to host arrays of n+1
  * and dag_edges entries, for parity checks of the orientation.  With
@@ -266,8 +268,12 @@ int mc_dgraph_export_dag(const mc_dgraph_t *g, int64_t *rowptr_out,
  * single-rank path of SMSolverMultiGPU (subgraph_matching/sm_multigpu.cu:97,
  * kernels in subgraph_matching/pattern_kernels.cuh, combine at
  * sm_multigpu.cu:206-232): the same quantities over all 2m directed edges,
- * bit-exact, without MPI.  Uses per-warp frontier scratch of max_degree
- * entries per list, grown on first use and kept by the handle.  P7 and P8
+ * bit-exact, without MPI.  Whole counts come from sums over vertices,
+ * edges, triangles and vertex pairs wherever those apply and are faster
+ * (MERCURY_MOTIF_ROUTE=formula / dense / sparse forces a route); otherwise
+ * the formulas are evaluated edge by edge, with per-warp frontier scratch of
+ * max_degree entries per list.  Scratch is taken for the call and shared by
+ * the device's handles.  Shards and budgets of P7 and P8
  * on a graph with a vertex of degree above 4,096 (and none above 46,340,
  * where the reference's 32-bit products could wrap) are counted from the
  * triangles, K4s and K5s of the degree-ordered DAG instead of the per-edge

@@ -3,9 +3,10 @@
 // union: graph g owns vertices [gptr[g], gptr[g+1]) and no edge crosses
 // graphs).  One pass runs the device orientation over the union, the
 // triangle kernels on the triangle graphs (each task adds its hits to its
-// own graph), one persistent pattern kernel over every pattern graph's
-// tasks, and a combine step -- captured once as a CUDA graph and replayed
-// per count.  An autotuner picks, per degree bucket of the triangle graphs,
+// own graph), the motif sums of pattern graphs of at most 1,024 vertices from
+// bit rows on a second stream (dense.cu), one persistent pattern kernel over
+// the tasks of the larger ones, and a combine step -- captured once as a CUDA
+// graph and replayed per count.  An autotuner picks, per degree bucket of the triangle graphs,
 // the warp/CTA threshold on the owner's out-degree and the table slots per
 // key.
 //

@@ -1,7 +1,8 @@
 // P7 and P8 by clique counts: a second device route for the reference's P7
 // and P8 (subgraph_matching/pattern_kernels.cuh:352-459 and :461-572,
 // combined as in subgraph_matching/sm_multigpu.cu:206-232) on graphs whose
-// hubs make the per-edge formulas cubic in a hub's degree.
+// hubs make the per-edge formulas cubic in a hub's degree.  Whole counts take
+// the motif sums of motifs.cu; this route serves shards and budgets.
 //
 // P7.  Per directed edge (v0, v1) the formula counts I3(A), the pairwise
 // non-adjacent triples of A = N(v0) & N(v1).  By inclusion-exclusion over

@@ -5,9 +5,12 @@
 // subgraph_matching/sm_multigpu.cu:206-232.  Every count is a sum over the
 // 2m directed edges (v0, v1) of the symmetric CSR (graph.cc:336-365), plus
 // P1's sum over vertices, of two 64-bit counters; the result is counters[1]
-// for P4/P6 and counters[1] - counters[2] otherwise.  Two routes compute the
-// same per-edge terms (each pattern takes the faster; see
-// pattern_uses_centers):
+// for P4/P6 and counters[1] - counters[2] otherwise.  Whole counts take the
+// motif sums (motifs.cu, dense.cu) wherever those apply and are faster
+// (pattern_route); the two routes below, which compute the reference's own
+// per-edge terms, serve shards, budgets, host columns, degrees above 46,340,
+// small graphs of low degree and scratch that does not fit.  Each pattern
+// takes the faster of the two (pattern_uses_centers):
 //  * warp per directed edge: the frontier lists of the pattern materialised
 //    in a per-warp slice of global scratch, membership by binary search or,
 //    for the dominant terms of P4, P5, P6 and P8, by a per-warp hash set in
