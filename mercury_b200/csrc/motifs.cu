@@ -24,7 +24,7 @@
 // took P1..P8 1.9, 28.0, 9.7, 4.8, 11.1, 3.6, 0.95 and 3.6 ms per call on a
 // B200, and these sums take 0.28, 1.37, 0.39, 0.76, 1.25, 0.38, 0.31 and 0.31.
 // On the one of 60,000 (mean 20, cap 50,000, a hub of degree 17,215) P1, P4,
-// P7 and P8 took 74.7, 276, 25.9 and 26.1 ms, and take 0.82, 2.6, 1.3 and 1.3.
+// P7 and P8 took 74.7, 276, 25.9 and 26.1 ms, and take 0.82, 1.66, 1.3 and 1.3.
 // There the pairs of P2 and P5 take 0.24 s (544 M two-paths).
 //
 // Stages (each vertex pair ordered by (degree, id), written u < v below; an
@@ -55,7 +55,7 @@ namespace {
 
 // Words of MotifArgs::counts: list lengths, then queue positions.
 enum Count : int {
-  kTauN, kMidN, kHashN, kHugeN, kBigN, kTauQueue, kMidQueue, kHashQueue, kBigQueue, kCounts
+  kTauN, kMidN, kHashN, kHugeN, kBigN, kSplitN, kTauQueue, kMidQueue, kHashQueue, kBigQueue, kCounts
 };
 
 struct MotifArgs {
@@ -84,6 +84,11 @@ struct MotifArgs {
   // vertices, the longest walks from the front, so that they start first.
   int32_t *tau_big, *pair_mid, *pair_big;
   unsigned *counts;  // see Count
+  // Parts of the longest walks: split_cap entries (s, part, parts) at most (0:
+  // none); num_sms and the sum of walk place the line.
+  int4 *split;
+  int split_cap, num_sms;
+  u64 *walk_total;
   u64 warp_walk, mid_walk;  // where the warp class and pair_mid's front class end
   unsigned *slices;  // bit rows of the tau stage that exceed shared memory
   int64_t slice_words;
@@ -103,6 +108,15 @@ constexpr int kTauBoth = 8 << 10;   // up to here the two forms share a launch
 // per vertex of some 1,000 entries); with the four classes it takes 1.1 ms.
 constexpr u64 kWarpWalk = 512, kMidWalk = 2048, kHashWalk = 8192;
 constexpr u64 kHugeWalk = 1 << 15;
+// Ordered walks above this, and above an SM's share of all of them, go in parts
+// of the table's range, a CTA each: a CTA alone with the largest (677 k entries
+// of 27.7 M on the Chung-Lu graph of 60,000 vertices, cap 50,000) lasted 1.5 ms
+// of P4's 2.6 ms, which takes 1.66 so; 100,000 vertices of mean 60: 17.7 -> 14.5
+// ms.  Counters in L2 that all warps share were slower there (25.3 ms: atomics
+// on one address), and the sum of the walks by an atomic per warp of the up
+// stage cost 0.04 ms at 1 M entries.
+constexpr u64 kSplitWalk = 1 << 16;
+constexpr int kSplitMax = 1024;
 constexpr u64 kFewWalk = 64;
 constexpr int kFewVertices = 16384;
 constexpr int kHashSlots = 1024;  // of a warp
@@ -287,6 +301,10 @@ __global__ void __launch_bounds__(kThreads) motif_tri_kernel(MotifArgs a, int pe
   const int lane = threadIdx.x & (kWarp - 1);
   if (!kCount && lists_overrun(a)) return;  // the host makes room and starts over
   const int64_t s64 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  if (!kCount && a.split_cap > 0 && s64 - lane < a.n) {
+    const u64 w = warp_sum_u64(s64 < a.n ? a.walk[s64] : 0);
+    if (lane == 0 && w) atomicAdd(a.walk_total, w);
+  }
   if (!kCount && s64 < a.n) {
     const int v = (int)s64;
     const int d = a.deg[v], p = a.dp[v];
@@ -596,6 +614,24 @@ __device__ void tau_large(const MotifArgs &a, TauSums &t, unsigned *s_rows, int 
 
 // Both forms in one launch while the large form's rows leave the SM full of
 // CTAs, else one launch each.
+// Between the sum of all walks and the pairs stage: the walks to take in parts
+// leave the list of the huge ones (-1).
+__device__ __forceinline__ void split_walks(const MotifArgs &a) {
+  const int huge = (int)a.counts[kHugeN];
+  const u64 share = *a.walk_total / (u64)a.num_sms;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < huge; i += gridDim.x * blockDim.x) {
+    const int s = a.pair_big[i];
+    const u64 w = a.walk[s];
+    if (w <= kSplitWalk || w <= share) continue;
+    const int parts = (int)min(min(w >> 15, (u64)8), 2 * (w / (share + 1) + 1));
+    const int at = (int)atomicAdd(a.counts + kSplitN, (unsigned)parts);
+    const bool fits = at + parts <= a.split_cap;
+    for (int k = 0; k < parts && at + k < a.split_cap; ++k)
+      a.split[at + k] = make_int4(fits ? s : -1, k, parts, 0);
+    if (fits) a.pair_big[i] = -1;
+  }
+}
+
 template <bool kLarge, bool kSmall>
 __global__ void __launch_bounds__(kThreads) motif_tau_kernel(MotifArgs a, int smem_words) {
   extern __shared__ unsigned s_rows[];
@@ -608,6 +644,7 @@ __global__ void __launch_bounds__(kThreads) motif_tau_kernel(MotifArgs a, int sm
   if (lists_overrun(a)) return;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   TauSums t;
+  if (kLarge && a.split_cap > 0) split_walks(a);
   if (kLarge) tau_large(a, t, s_rows, smem_words, &s_u, lane, warp);
   if (kSmall) tau_small(a, t, s_r[kSmall ? warp : 0], s_m[kSmall ? warp : 0], lane);
   t.flush(bs, a.need & kNeedTau);
@@ -639,11 +676,21 @@ struct Share {
   }
 };
 
+// First entry of the ascending ci[b, e) that is at least x, or e.
+__device__ __forceinline__ int first_entry(const int32_t *__restrict__ ci, int b, int e, int x) {
+  while (b < e) {
+    const int mid = (b + e) >> 1;
+    if (__ldg(ci + mid) < x) b = mid + 1;
+    else e = mid;
+  }
+  return b;
+}
+
 // Calls f(t, entry of v -> t, entry of s -> v, v) for this warp's share of the
-// two-paths from s.
-template <bool kOrdered, class F>
+// two-paths from s (kRanged: of those with t in [t0, t1)).
+template <bool kOrdered, bool kRanged = false, class F>
 __device__ __forceinline__ void walk_pairs(const MotifArgs &a, int s, int b, int d, const Share &sh,
-                                           int lane, F f) {
+                                           int lane, F f, int t0 = 0, int t1 = 0) {
   for (int c = sh.first; c * kWarp < d; c += sh.step) {
     const int k = c * kWarp + lane;
     int e = 0, v = 0, st = 0, len = 0;
@@ -656,6 +703,11 @@ __device__ __forceinline__ void walk_pairs(const MotifArgs &a, int s, int b, int
         if (kOrdered) {
           const int dv = a.deg[v];
           len = lower(dv, v, d, s) ? dv : 0;
+          if (kRanged && len > 0) {
+            const int end = st + dv;
+            st = first_entry(a.ci, st, end, t0);
+            len = first_entry(a.ci, st, end, t1) - st;
+          }
         } else {
           len = r1 - 1 - st;
         }
@@ -862,6 +914,17 @@ __global__ void __launch_bounds__(kT) motif_pairs_hash_kernel(MotifArgs a) {
 
 constexpr int kPairThreads = 1024;
 
+// First row that starts at or after entry e; n if none does.
+__device__ int row_at(const int64_t *__restrict__ rp, int n, int64_t e) {
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (__ldg(rp + mid) < e) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
 // CTA per larger s (longest walks first): 16-bit counters over all vertices,
 // two to a word, in shared memory when n of them fit, else one slice of
 // `counters` per CTA.
@@ -870,7 +933,8 @@ __global__ void __launch_bounds__(kPairThreads) motif_pairs_big_kernel(MotifArgs
                                                                        unsigned *counters) {
   extern __shared__ __align__(16) int s_tab[];
   __shared__ u64 sm[kSums];
-  __shared__ int s_s;
+  __shared__ int2 s_item;
+  __shared__ int s_range[2];
   const BlockSums bs{sm};
   bs.init();
   if (lists_overrun(a)) return;
@@ -878,23 +942,52 @@ __global__ void __launch_bounds__(kPairThreads) motif_pairs_big_kernel(MotifArgs
   unsigned *cnt = kShared ? reinterpret_cast<unsigned *>(s_tab)
                           : counters + (int64_t)blockIdx.x * words;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  constexpr int kEnd = -2;
   bool clean = false;  // the counters are zero
   PairSums ps;
+  const int splits = kOrdered ? (int)min(a.counts[kSplitN], (unsigned)a.split_cap) : 0;
   for (;;) {
     if (threadIdx.x == 0) {
-      const unsigned i = atomicAdd(a.counts + kBigQueue, 1u);
+      unsigned i = atomicAdd(a.counts + kBigQueue, 1u);
       const unsigned huge = a.counts[kHugeN], big = a.counts[kBigN];
-      s_s = i < huge ? a.pair_big[i] : i - huge < big ? a.pair_big[a.n - 1 - (i - huge)] : -1;
+      int4 item = make_int4(kEnd, 0, 1, 0);
+      if ((int)i < splits) {
+        item = a.split[i];
+        // Parts of about the same number of entries: t's place in the CSR.
+        for (int k = 0; k < 2; ++k)
+          s_range[k] = row_at(a.rp, a.n, (int64_t)a.nnz * (item.y + k) / item.z);
+      } else if (i - (unsigned)splits < huge + big) {
+        i -= (unsigned)splits;
+        item.x = i < huge ? a.pair_big[i] : a.pair_big[a.n - 1 - (i - huge)];
+      }
+      s_item = make_int2(item.x, item.z);
     }
     __syncthreads();
-    const int s = s_s;
-    if (s < 0) break;
+    const int s = s_item.x, parts = s_item.y;
+    const int t0 = s_range[0], t1 = s_range[1];
+    if (s == kEnd) break;
+    if (s < 0) {  // a walk taken in parts, or room that no walk's parts fitted
+      __syncthreads();
+      continue;
+    }
     if (!clean) {
       for (int i = threadIdx.x; i < words; i += kPairThreads) cnt[i] = 0;
       __syncthreads();
     }
     const int b = (int)__ldg(a.rp + s), d = a.deg[s];
     const Share sh(d, warp, kPairThreads / kWarp);
+    if (kOrdered && parts > 1) {
+      walk_pairs<kOrdered, true>(
+          a, s, b, d, sh, lane,
+          [&](int t, int, int, int) {
+            const int bit = (t & 1) * 16;
+            ps.c4 += (u64)((atomicAdd(cnt + (t >> 1), 1u << bit) >> bit) & 0xffffu);
+          },
+          t0, t1);
+      clean = false;
+      __syncthreads();
+      continue;
+    }
     pair_terms<kOrdered>(
         a, ps, s, b, d, sh, lane,
         [&](int t) {
@@ -1197,12 +1290,15 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
     // Few vertices: a CTA for all but the shortest walks.
     a.warp_walk = n <= kFewVertices ? kFewWalk : kWarpWalk;
     a.mid_walk = kMidWalk;
+    a.num_sms = g->num_sms;
+    a.split_cap = ordered && longest > (int64_t)kSplitWalk ? kSplitMax : 0;
     size_t zeroed = 0;
     // The same layout for every pattern (so that each finds the last one's block).
     auto lay_out = [&](Carver &c) {
       // Zeroed before the first kernel.
-      a.acc = c.take<u64>(kSums + 1);
+      a.acc = c.take<u64>(kSums + 2);
       a.pool = a.acc + kSums;
+      a.walk_total = a.pool + 1;
       a.counts = c.take<unsigned>(kCounts);
       a.dp = c.take<int32_t>(n);
       a.d2 = c.take<u64>(n);
@@ -1211,6 +1307,7 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
       a.a = c.take<int32_t>(nnz);
       if (counted) a.cnt = c.take<int32_t>(nnz);
       zeroed = c.used;
+      a.split = c.take<int4>(kSplitMax);
       a.deg = c.take<int32_t>(n);
       a.src = c.take<int32_t>(nnz);
       a.upe = c.take<int32_t>(nnz);

@@ -191,3 +191,21 @@ def test_batch_bit_rows_at_word_edges(monkeypatch):
         with DeviceGraph(g) as d:
             want += [d.tc_count()] + [d.pattern_count(k) for k in range(1, 9)]
     assert got == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,cap,ids", [(5000, 5000.0, "hubs first"), (12000, 12000.0, "hubs last"),
+                                       (12000, 12000.0, "shuffled")])
+def test_walks_in_parts(n, cap, ids):
+    """Hubs whose walks outlast an SM's share of all walks (ordered pairs, in
+    parts of the table's range), with the hubs at either end of the ids, isolated
+    vertices at both, and shuffled."""
+    g = Graph.chung_lu(n, 2.1, 30.0, cap, seed=n)
+    rp, col = np.array(g.rowptr), np.array(g.col)
+    src = np.repeat(np.arange(n), np.diff(rp))
+    perm = {"hubs first": np.arange(n), "hubs last": np.arange(n)[::-1],
+            "shuffled": np.random.default_rng(n).permutation(n)}[ids]
+    keep = src < col
+    rp, col = csr_from_edges(n + 20, np.stack([perm[src[keep]] + 7, perm[col[keep]] + 7], 1))
+    with DeviceGraph(rp, col) as d:
+        assert d.pattern_count(4) == orc.pattern_fast(rp, col, 4)
