@@ -280,6 +280,7 @@ int clique_prepare(mc_dgraph *g, int pattern, bool *use, int64_t *dag_edges) {
                               cudaMemcpyDeviceToHost, s));
   MC_CUDA_TRY(cudaStreamSynchronize(s));
   if (*g->h_err & (kErrDagCapacity | kErrContract)) return MC_ERR_FORMAT;
+  if (*g->h_err) return MC_ERR_DEVICE;
   *use = g->h_counters[3] <= (unsigned long long)kCliqueMaxOut && edges > 0;
   *dag_edges = edges;
   return MC_OK;

@@ -22,6 +22,7 @@ enum DeviceError : unsigned {
   kErrRank = 1u << 7,         // an out-list entry not ranked below its owner
   kErrDagCapacity = 1u << 8,  // more DAG entries than an exact-size DAG holds
   kErrWaitTimeout = 1u << 9,  // a bounded wait for an asynchronous copy gave up
+  kErrScanTimeout = 1u << 10, // a bounded wait of a chained scan gave up
 };
 // Bits of the CSR contract checks.
 constexpr unsigned kErrContract = kErrIdRange | kErrUnsorted | kErrSelfLoop | kErrRowptr |

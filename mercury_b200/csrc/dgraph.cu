@@ -264,7 +264,10 @@ int ensure_dag(mc_dgraph *g) {
   if (rc != MC_OK) return rc;
   MC_CUDA_TRY(cudaMemcpyAsync(g->h_err, g->err, sizeof(unsigned), cudaMemcpyDeviceToHost, g->stream));
   MC_CUDA_TRY(cudaStreamSynchronize(g->stream));
-  return *g->h_err ? MC_ERR_FORMAT : MC_OK;
+  if (*g->h_err & (kErrDagCapacity | kErrContract)) return MC_ERR_FORMAT;
+  if (*g->h_err) return MC_ERR_DEVICE;
+  g->dag_built = true;
+  return MC_OK;
 }
 }  // namespace
 
@@ -566,6 +569,7 @@ int tc_count_impl(mc_dgraph_t *g, int shard, int num_shards, uint64_t *count,
     // symmetric), or a streamed chunk that failed its contract checks: the DAG
     // was left unwritten.
     if (*g->h_err & (kErrDagCapacity | kErrContract)) return MC_ERR_FORMAT;
+    if (*g->h_err) return MC_ERR_DEVICE;
     maxd = (long long)g->h_counters[3];
   }
   // MERCURY_TC_TABLE_LOG2_MAX (8..15) lowers the shared-memory table cap;
@@ -602,6 +606,7 @@ int tc_count_impl(mc_dgraph_t *g, int shard, int num_shards, uint64_t *count,
                               cudaMemcpyDeviceToHost, s));
   MC_CUDA_TRY(cudaStreamSynchronize(s));
   if (*g->h_err) return MC_ERR_DEVICE;
+  g->dag_built = true;
   g->counted = true;
   *count = (uint64_t)g->h_counters[0];
   if (timing) {

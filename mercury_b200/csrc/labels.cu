@@ -275,6 +275,7 @@ int mc_tc_count_by_label(mc_dgraph_t *g, uint64_t *counts, mc_timing_t *timing) 
   mc::dev_free(d, s);
   MC_CUDA_TRY(cudaStreamSynchronize(s));
   if (*g->h_err & (mc::kErrDagCapacity | mc::kErrContract)) return MC_ERR_FORMAT;
+  if (*g->h_err) return MC_ERR_DEVICE;
   if (timing) {
     std::memset(timing, 0, sizeof(*timing));
     timing->orient_ms = mc::ms_between(g->ev[0], g->ev[1]);

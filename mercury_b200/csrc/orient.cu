@@ -368,7 +368,8 @@ __global__ void core_bits_kernel(const unsigned long long *__restrict__ sorted, 
                                  unsigned *err) {
   const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
   const int lane = threadIdx.x & (kWarp - 1);
-  if (p >= core_ranks || (*(volatile unsigned *)err & (kErrDagCapacity | kErrContract))) return;
+  if (p >= core_ranks || (*(volatile unsigned *)err & (kErrDagCapacity | kErrContract | kErrScanTimeout)))
+    return;
   const int64_t v = n - 1 - (int64_t)(uint32_t)sorted[p];
   if (v < 0) return;
   unsigned *row = core + core_offset(p);
@@ -380,10 +381,12 @@ __global__ void core_bits_kernel(const unsigned long long *__restrict__ sorted, 
 }
 
 // key[v] = {degree, 0}; deg[v] = degree alone (4 bytes per gather in pass A).
-// The first `words` words of status are cleared (words <= n + 4).
+// The first `words` words of status are cleared (words <= n + 4), and so are
+// the waits that gave up in an earlier orientation or count.
 __global__ void init_key_kernel(const int64_t *rowptr, int64_t n, int2 *key, int32_t *deg,
-                                unsigned long long *status, int64_t words) {
+                                unsigned long long *status, int64_t words, unsigned *err) {
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v == 0) atomicAnd(err, ~(unsigned)(kErrScanTimeout | kErrWaitTimeout));
   if (v < words) status[v] = 0;
   if (v < n) {
     const int d = (int)(rowptr[v + 1] - rowptr[v]);
@@ -413,7 +416,7 @@ constexpr int kTaskThreads = 256, kTaskItems = 4;  // vertices per thread
 __global__ void __launch_bounds__(kTaskThreads) partner_tasks_kernel(
     const int2 *__restrict__ key, const int32_t *__restrict__ rank,
     const int64_t *__restrict__ dag_rowptr, int64_t n, int4 *__restrict__ pinfo, TaskLists t,
-    unsigned long long *max_out, BatchView bv, unsigned *err) {
+    unsigned long long *max_out, BatchView bv, int max_polls, unsigned *err) {
   constexpr int kW = kTaskThreads / kWarp;
   __shared__ int s_warp[3][kW];
   __shared__ int s_max[kW];
@@ -467,7 +470,8 @@ __global__ void __launch_bounds__(kTaskThreads) partner_tasks_kernel(
   if (warp < 3) {  // warp k: list k
     unsigned long long sum = 0;
     for (int w = 0; w < kW; ++w) sum += (unsigned)s_warp[warp][w];
-    const unsigned long long before = tile_prefix(t.status + warp * t.blocks, block, sum, lane, err);
+    const unsigned long long before =
+        tile_prefix(t.status + warp * t.blocks, block, sum, lane, max_polls, err);
     if (lane == 0) {
       s_base[warp] = (int64_t)before;
       if (block == t.blocks - 1)
@@ -813,7 +817,7 @@ int tc_orient(mc_dgraph *g, const int32_t *upload) {
   g->ranked = ranked;
   const int64_t task_blocks = (n + kTaskThreads * kTaskItems - 1) / (kTaskThreads * kTaskItems);
   init_key_kernel<<<grid_for(n + 4, 256), 256, 0, s>>>(g->rowptr, n, g->key, deg, g->task_status,
-                                                       3 * task_blocks + 1);
+                                                       3 * task_blocks + 1, g->err);
   MC_CUDA_TRY(cudaGetLastError());
   g->launches += 1;
   if (ranked) {
@@ -874,10 +878,9 @@ int tc_orient(mc_dgraph *g, const int32_t *upload) {
       g->key, ranked ? g->rank : nullptr, g->dag_rowptr, n, g->pinfo,
       TaskLists{g->list_len, g->list_len + 1, g->list_len + 2, g->hub_tasks, g->leaf_tasks,
                 g->mega_tasks, g->task_status, task_blocks},
-      g->counters + 3, g->batch, g->err);
+      g->counters + 3, g->batch, wait_polls(), g->err);
   MC_CUDA_TRY(cudaGetLastError());
   g->launches += 1;
-  g->dag_built = true;
   return MC_OK;
 }
 

@@ -17,7 +17,9 @@
 // ranking (312 us a pass), and finding a digit's lanes by atomicOr masks in
 // shared memory (310 us: 82% of its bandwidth).
 #include <algorithm>
+#include <cstdlib>
 
+#include "lookback.cuh"
 #include "radix.cuh"
 
 namespace mc {
@@ -87,8 +89,6 @@ struct TileWord {
   static constexpr S kValue = kSum - 1;
 };
 
-constexpr int kRadixPolls = 1 << 22;
-
 template <int kBits>
 constexpr size_t pass_smem() {
   return sizeof(u64) * kSortTile + (sizeof(long long) + sizeof(int) * kSortWarps) * (1 << kBits);
@@ -109,7 +109,8 @@ __device__ __forceinline__ int block_exclusive(int v, int *s_warp, int lane, int
 template <int kBits, class S>
 __global__ void __launch_bounds__(kSortThreads, 4) radix_pass_kernel(
     const u64 *__restrict__ keys_in, u64 *__restrict__ keys_out, int64_t count, int shift,
-    const u64 *__restrict__ hist, volatile S *status, unsigned *ticket, unsigned *err) {
+    const u64 *__restrict__ hist, volatile S *status, unsigned *ticket, int max_polls,
+    unsigned *err) {
   constexpr int kBins = 1 << kBits, kPer = (kBins + kSortThreads - 1) / kSortThreads;
   using W = TileWord<S>;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -204,6 +205,10 @@ __global__ void __launch_bounds__(kSortThreads, 4) radix_pass_kernel(
     int polls = 0;
     bool done = tile == 0;
     for (int64_t t = tile - 1; !done;) {
+      if (polls == max_polls) {  // the output of this sort is then not used
+        atomicOr(err, (unsigned)kErrScanTimeout);
+        break;
+      }
       // A window of predecessors at once: their loads overlap.
       constexpr int kWindow = 8;
       S v[kWindow];
@@ -219,10 +224,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) radix_pass_kernel(
         ++used;
       }
       t -= used;
-      if (used == 0 && ++polls == kRadixPolls) {  // the output of this sort is then not used
-        atomicOr(err, (unsigned)kErrWaitTimeout);
-        done = true;
-      }
+      polls += used == 0;
     }
     if (tile > 0) status[tile * kBins + d0 + i] = W::kTotal | (before + (S)tot[i]);
     bin_dest[d0 + i] = base + below[i] + (long long)before - starts[i];
@@ -265,6 +267,7 @@ cudaError_t sort_passes(u64 *keys, u64 *alt, int64_t count, int begin_bit, int p
   auto kern = radix_pass_kernel<kBits, S>;
   e = allow_smem((const void *)kern, pass_smem<kBits>());
   if (e != cudaSuccess) return e;
+  const int polls = wait_polls();
   u64 *buf[2] = {keys, alt};
   int cur = 0;
   for (int p = 0; p < passes; ++p) {
@@ -275,7 +278,7 @@ cudaError_t sort_passes(u64 *keys, u64 *alt, int64_t count, int begin_bit, int p
     }
     kern<<<(unsigned)tiles, kSortThreads, pass_smem<kBits>(), s>>>(
         buf[cur], buf[cur ^ 1], count, begin_bit + p * kBits, hist + p * kRadixBinsMax, st,
-        tickets + p, err);
+        tickets + p, polls, err);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     cur ^= 1;
@@ -286,6 +289,11 @@ cudaError_t sort_passes(u64 *keys, u64 *alt, int64_t count, int begin_bit, int p
 }
 
 }  // namespace
+
+int wait_polls() {
+  const char *env = std::getenv("MERCURY_WAIT_POLLS");
+  return env ? std::max(0, std::atoi(env)) : 1 << 22;
+}
 
 size_t radix_work_bytes(int64_t count, int bits) {
   const size_t one = word_bytes(count) * (size_t)sort_tiles(count) << kRadixBitsMax;

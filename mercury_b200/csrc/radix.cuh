@@ -51,7 +51,7 @@ size_t radix_work_bytes(int64_t count, int bits);
 // Sorts keys[0, count) by bits [begin_bit, end_bit), stably, using `alt` as
 // the other buffer of each pass; *sorted receives the buffer holding the
 // result (keys or alt).  Every bit of the keys from end_bit on is zero.  A
-// bounded wait that gives up raises kErrWaitTimeout in *err (device word; the
+// bounded wait that gives up raises kErrScanTimeout in *err (device word; the
 // keys are then not sorted).  Asynchronous on `s`; *launches counts the
 // kernels.
 cudaError_t radix_sort_u64(unsigned long long *keys, unsigned long long *alt, int64_t count,

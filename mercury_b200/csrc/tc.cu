@@ -75,7 +75,9 @@ __device__ __forceinline__ void flush_task(const CountArgs &a, int x, unsigned l
 }
 
 // Tasks of this shard: queue position t maps to task t * num_shards + shard.
+// None when the ranks or the lists are not complete.
 __device__ __forceinline__ int64_t shard_tasks(const CountArgs &a) {
+  if (*a.err & kErrScanTimeout) return 0;
   const int64_t total = *a.ntasks;
   return total > a.shard ? (total - a.shard + a.num_shards - 1) / a.num_shards : 0;
 }
