@@ -479,25 +479,13 @@ int mc_tc_count(mc_dgraph_t *g, uint64_t *count, mc_timing_t *timing) {
 
 namespace mc {
 namespace {
-// How a whole triangle count runs: over the DAG's tasks; on small graphs from
-// bit rows, or from pairs of up neighbours in three launches.  The DAG's dozen
-// launches are what those save, so a setting of the hub kernel or the
+// The route of a whole triangle count: by sizes (routes.h).  The DAG's dozen
+// launches are what the others save, so a setting of the hub kernel or the
 // orientation that a caller wants to see at work keeps the DAG.
-enum class TriangleRoute { kDag, kBits, kPairs };
-// Whole calls on a B200, us, bits / pairs / DAG: RMAT scale 10, edge factor 16:
-// 74 / 49 / 144; scale 13, 16 (203,886 entries): - / 144 / 189; scale 13, 32
-// (365,688): - / 336 / 195; Chung-Lu of 100,000, mean 5 (499,200): - / 78 / 190;
-// mean 20 (1,960,194): - / 323 / 284.  The pairs grow with the square of the
-// out-degrees, so beyond 2^18 entries they keep sparse graphs only.
-// Bits win while one pass over the CSR is all there is (RMAT 8, edge factors 4,
-// 16 and 64: 37 / 46 / 98, 47 / 45 / 135 and 62 / 47 / 137).
-constexpr int64_t kBitVertices = 256, kBitEntries = 4096;
-bool pairs_pay(const mc_dgraph *g) {
-  return g->nnz <= 1 << 18 || (g->nnz <= 1 << 19 && g->nnz <= 16 * g->n);
-}
 TriangleRoute triangle_route(const mc_dgraph *g) {
-  if (g->n == 0 || g->nnz == 0 || g->col_host || g->dag_host) return TriangleRoute::kDag;
-  if (g->n > kDenseMax && !pairs_pay(g)) return TriangleRoute::kDag;
+  const TriangleRoute by_size = triangle_route_by_size(g->n, g->nnz);
+  if (!motif_range(g->n, g->nnz) || g->col_host || g->dag_host) return TriangleRoute::kDag;
+  if (g->n > kDenseMax && by_size == TriangleRoute::kDag) return TriangleRoute::kDag;
   for (const char *name : {"MERCURY_TC_TABLE_LOG2_MAX", "MERCURY_TC_BITMAP_BITS",
                            "MERCURY_TC_DENSE_FACTOR", "MERCURY_TC_CORE_RANKS", "MERCURY_TC_TMA",
                            "MERCURY_TC_ROW_STAGE", "MERCURY_TC_SHORT_RANGES",
@@ -507,8 +495,7 @@ TriangleRoute triangle_route(const mc_dgraph *g) {
     return std::strcmp(env, "bits") == 0 && g->n <= kDenseMax ? TriangleRoute::kBits
            : std::strcmp(env, "pairs") == 0                   ? TriangleRoute::kPairs
                                                               : TriangleRoute::kDag;
-  if (g->n <= kBitVertices && g->nnz <= kBitEntries) return TriangleRoute::kBits;
-  return pairs_pay(g) ? TriangleRoute::kPairs : TriangleRoute::kBits;
+  return by_size;
 }
 
 // The triangle count of a handle; upload (host memory, or null) streams the

@@ -3,6 +3,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "mercury.h"
+#include "routes.h"
 
 // Tunables of the triangle-count schedule (task classes and chunk sizes).
 namespace mc {
@@ -175,9 +176,7 @@ int clique_launch(mc_dgraph *g, int pattern, int64_t dag_edges, int shard, int n
 // counts are synchronous; event ev[3] marks their last kernel.  motif_count
 // returns MC_ERR_OOM when its scratch does not fit: the formula routes need
 // less.
-enum class PatternRoute { kFormula, kDense, kSparse };
 PatternRoute pattern_route(const mc_dgraph *g, int pattern);
-constexpr int kDenseMax = 1024;
 int motif_count(mc_dgraph *g, int pattern, uint64_t *out);
 int dense_count(mc_dgraph *g, int pattern, uint64_t *out);
 int dense_triangles(mc_dgraph *g, bool check);

@@ -1159,50 +1159,23 @@ int launch_pairs(mc_dgraph *g, const MotifArgs &a, int64_t longest, int big_grid
 
 }  // namespace
 
-// The route of a whole count.  Not the motif sums: above the degree at which
-// the reference's 32-bit products could wrap (its counts are then no subgraph
-// counts), with columns in host memory (the pairs stage reads rows once per
-// two-path), and when the environment asks for another route or its forms.
-//
-// By size (measured on a B200, whole calls, formula / bit rows / sparse, ms):
-//  - bit rows take P2 and P5 up to 512 vertices (RMAT scale 8, edge factor 8:
-//    1.39 / 0.14 / 0.41 and 0.32 / 0.14 / 0.41; at 1,024 vertices the two
-//    differ by -15% to +50%), and every pattern up to 64, where the sparse
-//    stages are launches alone (RMAT 6, P6: 0.068 / 0.055 / 0.079);
-//  - the per-edge formulas, one launch against five or more, keep P4 to P8
-//    on small graphs of low degree (the limits below), where every set of an
-//    edge is a warp or two: Chung-Lu of 10,001 vertices, mean 4, cap 40 (39,942
-//    entries, degree 61), P4 to P8: 0.094, 0.093, 0.081, 0.081 and 0.094 against
-//    0.122, 0.139, 0.096, 0.091 and 0.091 sparse; of 30,001 (119,934 entries):
-//    0.172, 0.167, 0.146, 0.132 and 0.170 against 0.165, 0.165, 0.107, 0.097 and
-//    0.097.  Hubs turn it: 3,001 vertices, mean 4, cap 200 (11,186 entries,
-//    degree 165), P5 to P8: 0.52, 1.20, 0.33 and 0.71 against 0.37, 0.10, 0.09
-//    and 0.09.
+// The route of a whole count: by sizes (routes.h), unless the environment asks
+// for another route or its forms; never the motif sums with columns in host
+// memory (the pairs stage reads rows once per two-path).
 PatternRoute pattern_route(const mc_dgraph *g, int pattern) {
-  if (g->n == 0 || g->nnz == 0 || g->batch.gid || g->col_host) return PatternRoute::kFormula;
-  if (g->max_degree > 46340 || g->nnz > (int64_t(1) << 30)) return PatternRoute::kFormula;
+  if (!motif_sums_apply(g->n, g->nnz, g->max_degree) || g->batch.gid || g->col_host)
+    return PatternRoute::kFormula;
   for (const char *name : {"MERCURY_PATTERN_KERNEL", "MERCURY_CLIQUE_ROUTE", "MERCURY_PATTERN_SETS",
                            "MERCURY_PATTERN_SLICE", "MERCURY_HUB_P1", "MERCURY_HOP_ROWS"})
     if (std::getenv(name)) return PatternRoute::kFormula;
-  const bool few = g->n <= kDenseMax;
   // MERCURY_MOTIF_ROUTE=formula|dense|sparse (tests and timing comparisons).
   if (const char *env = std::getenv("MERCURY_MOTIF_ROUTE")) {
     if (std::strcmp(env, "formula") == 0) return PatternRoute::kFormula;
-    if (std::strcmp(env, "dense") == 0) return few ? PatternRoute::kDense : PatternRoute::kSparse;
+    if (std::strcmp(env, "dense") == 0)
+      return g->n <= kDenseMax ? PatternRoute::kDense : PatternRoute::kSparse;
     if (std::strcmp(env, "sparse") == 0) return PatternRoute::kSparse;
   }
-  if (g->n <= 64 && pattern != 4) return PatternRoute::kDense;
-  if (g->n <= 512 && (pattern == 2 || pattern == 5)) return PatternRoute::kDense;
-  struct Limit {
-    int64_t degree, entries;
-  };
-  constexpr Limit kFormulaUpTo[] = {{100, 65536}, {80, 98304}, {72, 49152}, {80, 65536}, {64, 16384}};
-  if (pattern >= 4) {
-    const Limit &up = kFormulaUpTo[pattern - 4];
-    if (g->max_degree <= up.degree && g->nnz <= up.entries) return PatternRoute::kFormula;
-    if (pattern == 4 && g->nnz <= 12288) return PatternRoute::kFormula;
-  }
-  return PatternRoute::kSparse;
+  return pattern_route_by_size(g->n, g->nnz, g->max_degree, pattern);
 }
 
 int motif_triangles(mc_dgraph *g, uint64_t *out) {

@@ -1,0 +1,81 @@
+// The route of a whole count by its graph's sizes alone.  Plain C++, so that the
+// CPU tests compile it; the settings that force a route are read by the callers
+// (dgraph.cu, motifs.cu).
+#pragma once
+#include <cstdint>
+
+namespace mc {
+
+constexpr int kDenseMax = 1024;  // vertices of a graph that bit rows take
+
+// The stages of the motif sums and the pairs of up neighbours walk vertices and
+// entries in 32-bit loops of up to kMotifStride (4,096 blocks of 8 warps, or
+// fewer, larger ones) past the last one.
+constexpr int64_t kMotifMax = int64_t(1) << 30;
+constexpr int64_t kMotifStride = int64_t(1) << 20;
+static_assert(kMotifMax + kMotifStride <= INT32_MAX, "32-bit loops end");
+inline bool motif_range(int64_t n, int64_t nnz) {
+  return n > 0 && nnz > 0 && n <= kMotifMax && nnz <= kMotifMax;
+}
+
+// How a whole triangle count runs: over the DAG's tasks; on small graphs from
+// bit rows, or from pairs of up neighbours in three launches.
+enum class TriangleRoute { kDag, kBits, kPairs };
+// Whole calls on a B200, us, bits / pairs / DAG: RMAT scale 10, edge factor 16:
+// 74 / 49 / 144; scale 13, 16 (203,886 entries): - / 144 / 189; scale 13, 32
+// (365,688): - / 336 / 195; Chung-Lu of 100,000, mean 5 (499,200): - / 78 / 190;
+// mean 20 (1,960,194): - / 323 / 284.  The pairs grow with the square of the
+// out-degrees, so beyond 2^18 entries they keep sparse graphs only.
+// Bits win while one pass over the CSR is all there is (RMAT 8, edge factors 4,
+// 16 and 64: 37 / 46 / 98, 47 / 45 / 135 and 62 / 47 / 137).
+constexpr int64_t kBitVertices = 256, kBitEntries = 4096;
+inline bool pairs_pay(int64_t n, int64_t nnz) {
+  return motif_range(n, nnz) && (nnz <= 1 << 18 || (nnz <= 1 << 19 && nnz <= 16 * n));
+}
+inline TriangleRoute triangle_route_by_size(int64_t n, int64_t nnz) {
+  if (n > kDenseMax && !pairs_pay(n, nnz)) return TriangleRoute::kDag;
+  if (n <= kBitVertices && nnz <= kBitEntries) return TriangleRoute::kBits;
+  return pairs_pay(n, nnz) ? TriangleRoute::kPairs : TriangleRoute::kBits;
+}
+
+// P1..P8 from motif sums (over sparse stages, or, for graphs of at most
+// kDenseMax vertices, from bit rows), or the per-edge formulas.  No motif sums
+// above the degree at which the reference's 32-bit products could wrap (its
+// counts are then no subgraph counts).
+//
+// By size (measured on a B200, whole calls, formula / bit rows / sparse, ms):
+//  - bit rows take P2 and P5 up to 512 vertices (RMAT scale 8, edge factor 8:
+//    1.39 / 0.14 / 0.41 and 0.32 / 0.14 / 0.41; at 1,024 vertices the two
+//    differ by -15% to +50%), and every pattern up to 64, where the sparse
+//    stages are launches alone (RMAT 6, P6: 0.068 / 0.055 / 0.079);
+//  - the per-edge formulas, one launch against five or more, keep P4 to P8
+//    on small graphs of low degree (the limits below), where every set of an
+//    edge is a warp or two: Chung-Lu of 10,001 vertices, mean 4, cap 40 (39,942
+//    entries, degree 61), P4 to P8: 0.094, 0.093, 0.081, 0.081 and 0.094 against
+//    0.122, 0.139, 0.096, 0.091 and 0.091 sparse; of 30,001 (119,934 entries):
+//    0.172, 0.167, 0.146, 0.132 and 0.170 against 0.165, 0.165, 0.107, 0.097 and
+//    0.097.  Hubs turn it: 3,001 vertices, mean 4, cap 200 (11,186 entries,
+//    degree 165), P5 to P8: 0.52, 1.20, 0.33 and 0.71 against 0.37, 0.10, 0.09
+//    and 0.09.
+enum class PatternRoute { kFormula, kDense, kSparse };
+inline bool motif_sums_apply(int64_t n, int64_t nnz, int64_t max_degree) {
+  return motif_range(n, nnz) && max_degree <= 46340;
+}
+inline PatternRoute pattern_route_by_size(int64_t n, int64_t nnz, int64_t max_degree,
+                                          int pattern) {
+  if (!motif_sums_apply(n, nnz, max_degree)) return PatternRoute::kFormula;
+  if (n <= 64 && pattern != 4) return PatternRoute::kDense;
+  if (n <= 512 && (pattern == 2 || pattern == 5)) return PatternRoute::kDense;
+  struct Limit {
+    int64_t degree, entries;
+  };
+  constexpr Limit kFormulaUpTo[] = {{100, 65536}, {80, 98304}, {72, 49152}, {80, 65536}, {64, 16384}};
+  if (pattern >= 4) {
+    const Limit &up = kFormulaUpTo[pattern - 4];
+    if (max_degree <= up.degree && nnz <= up.entries) return PatternRoute::kFormula;
+    if (pattern == 4 && nnz <= 12288) return PatternRoute::kFormula;
+  }
+  return PatternRoute::kSparse;
+}
+
+}  // namespace mc

@@ -1,0 +1,49 @@
+"""The routes of whole counts by size (mercury_b200/csrc/routes.h), compiled for
+the CPU (tests/routes.cpp)."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+DAG, BITS, PAIRS = range(3)
+FORMULA, DENSE, SPARSE = range(3)
+
+
+@pytest.fixture(scope="module")
+def routes():
+    out = os.path.join(HERE, "_build", "libroutes.so")
+    src = [os.path.join(HERE, "routes.cpp"),
+           os.path.join(HERE, "..", "mercury_b200", "csrc", "routes.h")]
+    if not os.path.exists(out) or os.path.getmtime(out) < max(map(os.path.getmtime, src)):
+        os.makedirs(os.path.dirname(out), exist_ok=True)
+        subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", src[0], "-o", out],
+                       check=True)
+    lib = C.CDLL(out)
+
+    class Routes:
+        @staticmethod
+        def triangle(n, nnz):
+            return lib.triangle_route(C.c_int64(n), C.c_int64(nnz))
+
+        @staticmethod
+        def pattern(n, nnz, max_degree, k):
+            return lib.pattern_route(C.c_int64(n), C.c_int64(nnz), C.c_int64(max_degree), k)
+
+    return Routes
+
+
+@pytest.mark.parametrize("n", [2**30 + 1, 2**31 - 32768, 2**31 - 2])
+def test_vertices_beyond_32_bit_loops_keep_the_64_bit_routes(routes, n):
+    """The largest graphs a handle takes have more vertices than a 32-bit
+    grid-stride loop can step past."""
+    assert routes.triangle(n, 1000) == DAG
+    assert all(routes.pattern(n, 1000, 40, k) == FORMULA for k in range(1, 9))
+
+
+def test_at_the_largest_size_of_the_32_bit_loops(routes):
+    assert routes.triangle(2**30, 1000) == PAIRS
+    assert routes.pattern(2**30, 1000, 40, 1) == SPARSE
+    assert routes.pattern(2**30, 2**30 + 1, 40, 1) == FORMULA
+    assert routes.pattern(1000, 90000, 46341, 1) == FORMULA
