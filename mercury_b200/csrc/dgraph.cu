@@ -483,9 +483,8 @@ namespace {
 // launches are what the others save, so a setting of the hub kernel or the
 // orientation that a caller wants to see at work keeps the DAG.
 TriangleRoute triangle_route(const mc_dgraph *g) {
-  const TriangleRoute by_size = triangle_route_by_size(g->n, g->nnz);
   if (!motif_range(g->n, g->nnz) || g->col_host || g->dag_host) return TriangleRoute::kDag;
-  if (g->n > kDenseMax && by_size == TriangleRoute::kDag) return TriangleRoute::kDag;
+  if (g->n > kDenseMax && !pairs_pay(g->n, g->nnz)) return TriangleRoute::kDag;
   for (const char *name : {"MERCURY_TC_TABLE_LOG2_MAX", "MERCURY_TC_BITMAP_BITS",
                            "MERCURY_TC_DENSE_FACTOR", "MERCURY_TC_CORE_RANKS", "MERCURY_TC_TMA",
                            "MERCURY_TC_ROW_STAGE", "MERCURY_TC_SHORT_RANGES",
@@ -495,7 +494,7 @@ TriangleRoute triangle_route(const mc_dgraph *g) {
     return std::strcmp(env, "bits") == 0 && g->n <= kDenseMax ? TriangleRoute::kBits
            : std::strcmp(env, "pairs") == 0                   ? TriangleRoute::kPairs
                                                               : TriangleRoute::kDag;
-  return by_size;
+  return triangle_route_by_size(g->n, g->nnz);
 }
 
 // The triangle count of a handle; upload (host memory, or null) streams the

@@ -33,6 +33,7 @@ inline bool pairs_pay(int64_t n, int64_t nnz) {
   return motif_range(n, nnz) && (nnz <= 1 << 18 || (nnz <= 1 << 19 && nnz <= 16 * n));
 }
 inline TriangleRoute triangle_route_by_size(int64_t n, int64_t nnz) {
+  if (!motif_range(n, nnz)) return TriangleRoute::kDag;
   if (n > kDenseMax && !pairs_pay(n, nnz)) return TriangleRoute::kDag;
   if (n <= kBitVertices && nnz <= kBitEntries) return TriangleRoute::kBits;
   return pairs_pay(n, nnz) ? TriangleRoute::kPairs : TriangleRoute::kBits;

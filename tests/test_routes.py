@@ -47,3 +47,10 @@ def test_at_the_largest_size_of_the_32_bit_loops(routes):
     assert routes.pattern(2**30, 1000, 40, 1) == SPARSE
     assert routes.pattern(2**30, 2**30 + 1, 40, 1) == FORMULA
     assert routes.pattern(1000, 90000, 46341, 1) == FORMULA
+
+
+@pytest.mark.parametrize("nnz", [2**31 + 5, 2**32 + 5])
+def test_entry_counts_beyond_32_bits_are_no_bit_rows(routes, nnz):
+    """Unchecked host arrays may claim any number of entries; the bit rows hold
+    row offsets in 32 bits, where such a number would pass for a small one."""
+    assert routes.triangle(1000, nnz) == DAG
