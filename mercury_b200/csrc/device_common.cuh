@@ -59,6 +59,11 @@ struct NvtxRange {
 // synchronisation, and the next allocation maps it again), so repeated
 // calls reuse their buffers. The pool stays private to this process.
 void retain_pool_memory(int device);
+// Device memory an allocation can still have: what the driver reports free,
+// what the pool holds unused, and the kept scratch blocks.  (The driver's figure
+// alone falls with every block the pool has ever held.)  MERCURY_DEVICE_BYTES
+// replaces the figure (tests reach the fallbacks with it on small graphs).
+int device_bytes_available(int device, int64_t *avail);
 
 cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s);
 inline void dev_free(void *p, cudaStream_t s) { cudaFreeAsync(p, s); }

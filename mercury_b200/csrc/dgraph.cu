@@ -61,30 +61,6 @@ void release(mc_dgraph *g) {
   delete g;
 }
 
-// Free device memory for the placement decision: what the driver reports
-// plus what this process's pool holds unused. MERCURY_DEVICE_BYTES replaces
-// the figure (tests reach the host-column fallback with it on small graphs).
-int device_bytes_available(int device, int64_t *avail) {
-  size_t free_b = 0, total_b = 0;
-  MC_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-  int64_t a = (int64_t)free_b;
-  cudaMemPool_t pool;
-  if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
-    uint64_t reserved = 0, used = 0;
-    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
-        reserved > used)
-      a += (int64_t)(reserved - used);
-  }
-  a += (int64_t)scratch_kept(device);
-  if (const char *env = std::getenv("MERCURY_DEVICE_BYTES")) {
-    const long long v = std::atoll(env);
-    if (v > 0) a = v;
-  }
-  *avail = a;
-  return MC_OK;
-}
-
 // Where a graph's column array goes. In device memory when the device can
 // hold it together with the triangle-count scratch (and a margin);
 // otherwise, or when the caller asks, in pinned host memory that the
@@ -228,6 +204,27 @@ bool is_pageable(const void *p) {
 thread_local HostCache t_cache;
 
 }  // namespace
+
+int device_bytes_available(int device, int64_t *avail) {
+  size_t free_b = 0, total_b = 0;
+  MC_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+  int64_t a = (int64_t)free_b;
+  cudaMemPool_t pool;
+  if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
+    uint64_t reserved = 0, used = 0;
+    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+        reserved > used)
+      a += (int64_t)(reserved - used);
+  }
+  a += (int64_t)scratch_kept(device);
+  if (const char *env = std::getenv("MERCURY_DEVICE_BYTES")) {
+    const long long v = std::atoll(env);
+    if (v > 0) a = v;
+  }
+  *avail = a;
+  return MC_OK;
+}
 
 void set_last_cuda_error(cudaError_t e) { t_last_cuda = e; }
 cudaError_t last_cuda_error() { return t_last_cuda; }

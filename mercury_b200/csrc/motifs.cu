@@ -1295,13 +1295,20 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
     Carver size;
     lay_out(size);
     Carver c;
-    // Large scratch leaves half of the free memory alone; the caller then
-    // takes a formula route, as it does when the allocation fails.
+    // Large scratch leaves half of the free memory alone: first with lists
+    // sized by a counting pass, then the caller takes a formula route, as it
+    // does when the allocation fails.
     const size_t counters_b = pairs && !table_shared ? pair_grid * table_b : 0;
     if (size.used + counters_b > size_t(1) << 30) {
-      size_t free_b = 0, total_b = 0;
-      MC_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-      if (size.used + counters_b > free_b / 2) return MC_ERR_OOM;
+      int64_t avail = 0;
+      const int arc = device_bytes_available(g->device, &avail);
+      if (arc != MC_OK) return arc;
+      if ((int64_t)(size.used + counters_b) > avail / 2) {
+        if (counted) return MC_ERR_OOM;
+        counted = true;
+        list_cap = std::min<int64_t>(list_cap, 4 * (int64_t)nnz);
+        continue;
+      }
     }
     size_t got = 0, got_counters = 0;
     MC_CUDA_TRY(scratch_take(reinterpret_cast<void **>(&c.base), size.used, &got, g->device, s));

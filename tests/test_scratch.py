@@ -53,3 +53,33 @@ def test_triangle_counts_of_different_table_sizes_in_threads(monkeypatch):
     with ThreadPoolExecutor(2) as pool:
         for got, w in zip(pool.map(work, [0, 1]), want):
             assert set(got) == {w}
+
+
+def test_route_does_not_depend_on_earlier_counts():
+    """Scratch that an earlier count gave back to the pool is free memory: with
+    room for it twice, but not four times, the same count takes the motif sums
+    every time."""
+    import torch
+    g = Graph.chung_lu(1000000, 2.1, 9.0, 100.0, seed=6)
+    with DeviceGraph(g) as d:
+        free = torch.cuda.mem_get_info()[0]
+        scratch = 4 * 64 * d.nnz + 40 * d.nnz  # lists at the first guess, and the rest
+        fill = torch.empty(max(0, free - int(2.4 * scratch)), dtype=torch.uint8, device="cuda")
+        try:
+            seen = [(d.pattern_count(1), d.last_timing.launches) for _ in range(3)]
+        finally:
+            del fill
+            torch.cuda.empty_cache()
+        assert seen == [(d.pattern_count(1), d.last_timing.launches)] * 3
+
+
+def test_lists_that_do_not_fit_are_counted_first(monkeypatch):
+    """Half of the memory holds the lists' true size but not their first guess:
+    a counting pass sizes them (two more launches) before any other route."""
+    g = Graph.chung_lu(1000000, 2.1, 9.0, 100.0, seed=6)
+    with DeviceGraph(g) as d:
+        want, launches = d.pattern_count(7), d.last_timing.launches
+        monkeypatch.setenv("MERCURY_DEVICE_BYTES", str(2 * 200 * d.nnz))
+        assert (d.pattern_count(7), d.last_timing.launches) == (want, launches + 2)
+        monkeypatch.setenv("MERCURY_DEVICE_BYTES", str(1 << 20))
+        assert d.pattern_count(7) == want
