@@ -199,9 +199,10 @@ int mc_csr_build(const int32_t *src, const int32_t *dst, int64_t num_edges,
                  int64_t n, unsigned flags, void *stream, mc_graph_t **out,
                  mc_timing_t *timing);
 /* Same build, but the CSR stays on the device as a graph handle ready for
- * mc_tc_count / mc_pattern_count, with no host round trip. flags may also
- * hold MC_VALIDATE_SYMMETRY (the handle's contract check runs as in
- * mc_dgraph_create). timing->total_ms includes the handle's check. */
+ * mc_tc_count / mc_pattern_count, with no host round trip.  The build's output
+ * keeps the contract, so no check reads it again; with MC_VALIDATE_SYMMETRY in
+ * flags the handle's contract check runs as in mc_dgraph_create, and
+ * timing->total_ms includes it. */
 int mc_dgraph_from_edges(const int32_t *src, const int32_t *dst,
                          int64_t num_edges, int64_t n, unsigned flags,
                          void *stream, mc_dgraph_t **out,

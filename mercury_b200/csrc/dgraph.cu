@@ -405,8 +405,12 @@ int mc_dgraph_from_edges(const int32_t *src, const int32_t *dst, int64_t num_edg
   mc::csr_build_free(b);
   // The built CSR keeps the contract by construction (distinct entries in
   // sorted rows, both directions of every pair, ids checked on the way in), so
-  // no check reads it again (0.35 ms at RMAT scale 20).
-  if (rc == MC_OK && cudaMemsetAsync(g->err, 0, sizeof(unsigned), g->stream) != cudaSuccess)
+  // nothing reads it again (0.35 ms at RMAT scale 20) unless the caller asks
+  // for the check.
+  const bool check = (flags & MC_VALIDATE_SYMMETRY) != 0;
+  g->launches = 0;
+  if (rc == MC_OK && check) rc = mc::validate_graph(g, MC_VALIDATE_SYMMETRY);
+  if (rc == MC_OK && !check && cudaMemsetAsync(g->err, 0, sizeof(unsigned), g->stream) != cudaSuccess)
     rc = MC_ERR_CUDA;
   if (rc != MC_OK) {
     release(g);
@@ -419,7 +423,7 @@ int mc_dgraph_from_edges(const int32_t *src, const int32_t *dst, int64_t num_edg
     timing->h2d_ms = mc::elapsed(g->ev[0], g->ev[1]);
     timing->count_ms = mc::elapsed(g->ev[1], g->ev[2]);
     timing->total_ms = mc::elapsed(g->ev[0], g->ev[3]);
-    timing->launches = launches;
+    timing->launches = launches + g->launches;
   }
   return MC_OK;
 }
