@@ -748,7 +748,7 @@ int mc_tc_count_host(const int64_t *rowptr, const int32_t *col, int64_t n, int64
   int64_t validate_launches = 0;
   if (bit_rows) {
     // Small graphs: offsets and entries checked and counted by one kernel
-    // (scale 8: 300 -> 60 us per call).
+    // (scale 8: 300 -> 75 us per call).
     auto whole = [&]() -> int {
       if (nnz > 0)
         MC_CUDA_TRY(cudaMemcpyAsync(g->col, col, sizeof(int32_t) * (size_t)nnz,

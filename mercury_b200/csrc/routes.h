@@ -25,18 +25,24 @@ enum class TriangleRoute { kDag, kBits, kPairs };
 // 74 / 49 / 144; scale 13, 16 (203,886 entries): - / 144 / 189; scale 13, 32
 // (365,688): - / 336 / 195; Chung-Lu of 100,000, mean 5 (499,200): - / 78 / 190;
 // mean 20 (1,960,194): - / 323 / 284.  The pairs grow with the square of the
-// out-degrees, so beyond 2^18 entries they keep sparse graphs only.
+// out-degrees, so beyond 2^18 entries they keep sparse graphs only, and none where
+// the entries times the mean degree exceed 2^25 (pairs / DAG: complete graphs of
+// 300, 400 and 512 vertices, 27, 64 and 134 million: 147 / 139, 364 / 157 and 798
+// / 170; random ones of 1,200, 700 and 1,000 vertices, 29, 42 and 250 million: 171 /
+// 137, 253 / 137 and 1,228 / 220; 64 x 2,000 complete bipartite, 32: 109 / 128).
 // Bits win while one pass over the CSR is all there is (RMAT 8, edge factors 4,
-// 16 and 64: 37 / 46 / 98, 47 / 45 / 135 and 62 / 47 / 137).
+// 16 and 64: 37 / 46 / 98, 47 / 45 / 135 and 62 / 47 / 137); each of their CTAs
+// reads every entry, so dense graphs lose there too (complete graphs of 512 and
+// 1,000: 358 and 1,307).
 constexpr int64_t kBitVertices = 256, kBitEntries = 4096;
 inline bool pairs_pay(int64_t n, int64_t nnz) {
-  return motif_range(n, nnz) && (nnz <= 1 << 18 || (nnz <= 1 << 19 && nnz <= 16 * n));
+  return motif_range(n, nnz) && nnz <= 1 << 19 && (nnz <= 1 << 18 || nnz <= 16 * n) &&
+         nnz * nnz <= (n << 25);
 }
 inline TriangleRoute triangle_route_by_size(int64_t n, int64_t nnz) {
   if (!motif_range(n, nnz)) return TriangleRoute::kDag;
-  if (n > kDenseMax && !pairs_pay(n, nnz)) return TriangleRoute::kDag;
   if (n <= kBitVertices && nnz <= kBitEntries) return TriangleRoute::kBits;
-  return pairs_pay(n, nnz) ? TriangleRoute::kPairs : TriangleRoute::kBits;
+  return pairs_pay(n, nnz) ? TriangleRoute::kPairs : TriangleRoute::kDag;
 }
 
 // P1..P8 from motif sums (over sparse stages, or, for graphs of at most

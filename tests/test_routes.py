@@ -54,3 +54,20 @@ def test_entry_counts_beyond_32_bits_are_no_bit_rows(routes, nnz):
     """Unchecked host arrays may claim any number of entries; the bit rows hold
     row offsets in 32 bits, where such a number would pass for a small one."""
     assert routes.triangle(1000, nnz) == DAG
+
+
+def complete(n):
+    return n, n * (n - 1)
+
+
+def test_triangles_of_dense_graphs_keep_the_dag(routes):
+    """Pairs of up neighbours and bit rows both lose to the DAG where most
+    vertices see most others, whatever the number of entries."""
+    for n in (400, 512, 600, 1000, 1024):
+        assert routes.triangle(*complete(n)) == DAG
+    for n, nnz in [(600, 180000), (600, 179886), (1000, 499968), (1000, 500000), (700, 172052)]:
+        assert routes.triangle(n, nnz) == DAG
+    assert [routes.triangle(*complete(n)) for n in (32, 64, 100, 300)] == [BITS, BITS, PAIRS, PAIRS]
+    # Sparse ones, hubs or not, keep the pairs.
+    for n, nnz in [(1024, 12014), (8192, 204044), (2048, 177992), (100000, 499200), (2064, 256000)]:
+        assert routes.triangle(n, nnz) == PAIRS
