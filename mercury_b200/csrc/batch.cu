@@ -264,13 +264,14 @@ using mc::batch_release;
 namespace mc {
 
 // Builds a batch from a union CSR held in host memory (device_csr false) or
-// device memory (true), with each graph's largest degree and entry count
-// given by the caller (gmaxdeg, gnnz); with do_capture the count sequence is
-// captured as a CUDA graph, otherwise every count launches it directly.
+// device memory (true), with each graph's largest degree, entry count and sum of
+// squared degrees given by the caller (gmaxdeg, gnnz, gsquares); with do_capture
+// the count sequence is captured as a CUDA graph, otherwise every count launches
+// it directly.
 int batch_create(const int64_t *rowptr, const int32_t *col, bool device_csr, int64_t n,
                  int64_t nnz, const int64_t *graph_vptr, int num_graphs, const int32_t *jobs,
-                 const int64_t *gmaxdeg, const int64_t *gnnz_of, void *stream, bool do_capture,
-                 mc_batch_t **out) {
+                 const int64_t *gmaxdeg, const int64_t *gnnz_of, const int64_t *gsquares,
+                 void *stream, bool do_capture, mc_batch_t **out) {
   if (!out || !rowptr || !graph_vptr || !jobs || num_graphs < 1 || n < 0 || nnz < 0)
     return MC_ERR_ARG;
   *out = nullptr;
@@ -315,6 +316,16 @@ int batch_create(const int64_t *rowptr, const int32_t *col, bool device_csr, int
   std::vector<uint8_t> is_dense(G, 0);
   const char *route = std::getenv("MERCURY_MOTIF_ROUTE");
   const bool use_dense = !(route && std::strcmp(route, "formula") == 0);
+  auto takes_bits = [&](int i) {
+    if (!use_dense || jobs[i] == 0) return false;
+    const int64_t gn = graph_vptr[i + 1] - graph_vptr[i];
+    if (route && std::strcmp(route, "dense") == 0) return gn <= kDenseMax;
+    return batch_takes_bits(gn, gnnz_of[i], gmaxdeg[i], gsquares[i], jobs[i]);
+  };
+  int64_t dense_total = 0;
+  for (int i = 0; i < G; ++i)
+    if (takes_bits(i))
+      dense_total += dense_work(graph_vptr[i + 1] - graph_vptr[i], gnnz_of[i], gmaxdeg[i]);
   for (int i = 0; i < G; ++i) {
     const int64_t md = gmaxdeg[i];
     const int64_t gnnz = gnnz_of[i];
@@ -322,9 +333,9 @@ int batch_create(const int64_t *rowptr, const int32_t *col, bool device_csr, int
       b->has_tc = true;
       b->bucket[i] = degree_bucket(md);
       b->dplus_bound[i] = std::min<int64_t>(md, (int64_t)std::sqrt((double)gnnz) + 1);
-    } else if (use_dense && graph_vptr[i + 1] - graph_vptr[i] <= kDenseMax) {
+    } else if (takes_bits(i)) {
       const int gn = (int)(graph_vptr[i + 1] - graph_vptr[i]);
-      const int parts = dense_parts(gn, gnnz, md);
+      const int parts = dense_parts(gn, gnnz, md, dense_total, g->num_sms);
       for (int p = 0; p < parts; ++p)
         dense.push_back(DenseTask{graph_vptr[i], gn, i, jobs[i], p, parts});
       is_dense[i] = 1;
@@ -450,15 +461,18 @@ int mc_batch_create(const int64_t *rowptr, const int32_t *col, int64_t n, int64_
   if (graph_vptr[0] != 0 || graph_vptr[num_graphs] != n) return MC_ERR_ARG;
   for (int i = 0; i < num_graphs; ++i)
     if (graph_vptr[i + 1] < graph_vptr[i]) return MC_ERR_ARG;
-  // Per-graph largest degree and entry count from the host arrays.
-  std::vector<int64_t> md(num_graphs, 0), gnnz(num_graphs, 0);
+  // Per-graph largest degree, entry count and squared degrees from the host arrays.
+  std::vector<int64_t> md(num_graphs, 0), gnnz(num_graphs, 0), squares(num_graphs, 0);
   for (int i = 0; i < num_graphs; ++i) {
-    for (int64_t v = graph_vptr[i]; v < graph_vptr[i + 1]; ++v)
-      md[i] = std::max<int64_t>(md[i], rowptr[v + 1] - rowptr[v]);
+    for (int64_t v = graph_vptr[i]; v < graph_vptr[i + 1]; ++v) {
+      const int64_t deg = rowptr[v + 1] - rowptr[v];
+      md[i] = std::max<int64_t>(md[i], deg);
+      squares[i] += deg * deg;
+    }
     gnnz[i] = rowptr[graph_vptr[i + 1]] - rowptr[graph_vptr[i]];
   }
   return mc::batch_create(rowptr, col, false, n, nnz, graph_vptr, num_graphs, jobs, md.data(),
-                          gnnz.data(), stream, true, out);
+                          gnnz.data(), squares.data(), stream, true, out);
 }
 
 int mc_batch_count(mc_batch_t *b, uint64_t *counts, mc_timing_t *timing) {

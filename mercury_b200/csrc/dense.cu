@@ -33,14 +33,10 @@ struct DenseGraph {
   int64_t nnz = 0;  // entries the caller gave (checked loads only)
 };
 
-// Rows of W words (1, 2, 4, 8 or above 256 vertices what n takes: the loops
-// over a row's words are unrolled up to 8) at an odd stride, so that lanes
-// reading the same word of consecutive rows hit distinct banks; then n + 1 row
-// offsets.
-__host__ __device__ constexpr int dense_words(int n) {
-  return n <= 32 ? 1 : n <= 64 ? 2 : n <= 128 ? 4 : n <= 256 ? 8 : (n + 31) / 32;
-}
-__host__ __device__ constexpr int dense_stride(int n) { return dense_words(n) | 1; }
+// Rows of W words (bit_words: the loops over a row's words are unrolled up to 8)
+// at an odd stride, so that lanes reading the same word of consecutive rows hit
+// distinct banks; then n + 1 row offsets.
+__host__ __device__ constexpr int dense_stride(int n) { return bit_words(n) | 1; }
 size_t dense_bytes(int n) { return sizeof(int) * ((size_t)n * dense_stride(n) + n + 1); }
 
 // The last row starting at or before entry e.
@@ -104,7 +100,7 @@ __device__ __forceinline__ bool load_matrix(const DenseGraph &g, unsigned *bits,
 template <unsigned need, int kW>
 __device__ __forceinline__ void dense_sums(const DenseGraph &g, int part, int parts, unsigned *smem,
                                            const BlockSums &bs) {
-  const int n = g.n, W = kW > 0 ? kW : dense_words(n), P = W | 1;
+  const int n = g.n, W = kW > 0 ? kW : bit_words(n), P = W | 1;
   unsigned *bits = smem;
   int *off = reinterpret_cast<int *>(smem + (size_t)n * P);
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
@@ -278,7 +274,7 @@ __device__ __forceinline__ void dense_sums(const DenseGraph &g, int part, int pa
 template <unsigned need>
 __device__ __forceinline__ void dense_words_of(const DenseGraph &g, int part, int parts,
                                                unsigned *smem, const BlockSums &bs) {
-  switch (dense_words(g.n)) {
+  switch (bit_words(g.n)) {
     case 1: return dense_sums<need, 1>(g, part, parts, smem, bs);
     case 2: return dense_sums<need, 2>(g, part, parts, smem, bs);
     case 4: return dense_sums<need, 4>(g, part, parts, smem, bs);
@@ -330,7 +326,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_triangles_kernel(DenseGra
   extern __shared__ unsigned smem[];
   __shared__ u64 s_total;
   if (threadIdx.x == 0) s_total = 0;
-  const int n = g.n, W = dense_words(n), P = W | 1;
+  const int n = g.n, W = bit_words(n), P = W | 1;
   int *off = reinterpret_cast<int *>(smem + (size_t)n * P);
   if (!load_matrix<kCheck>(g, smem, off, P, err)) return;
   const int nnz = off[n];
@@ -362,7 +358,7 @@ int dense_triangles(mc_dgraph *g, bool check) {
   if (smem > (size_t(40) << 10))
     MC_CUDA_TRY(allow_smem((const void *)kern, smem));
   // About 2^16 row words per CTA: each builds the matrix for itself.
-  const int64_t words = g->nnz * dense_words(n) / 2;
+  const int64_t words = g->nnz * bit_words(n) / 2;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(g->num_sms, words >> 16));
   kern<<<grid, kDenseThreads, smem, s>>>(DenseGraph{g->rowptr, g->col, 0, n, g->nnz}, g->counters,
                                          reinterpret_cast<unsigned *>(g->counters + 1));
@@ -381,7 +377,7 @@ int dense_count(mc_dgraph *g, int pattern, uint64_t *out) {
   MC_CUDA_TRY(allow_smem((const void *)dense_kernel, smem));
   // A CTA per SM at most: each builds the matrix, which costs as much as
   // its share of the tasks.
-  const int tasks = n * dense_words(n), warps = kDenseThreads / kWarp;
+  const int tasks = n * bit_words(n), warps = kDenseThreads / kWarp;
   dense_kernel<<<std::min(g->num_sms, (tasks + warps - 1) / warps), kDenseThreads, smem, s>>>(
       DenseGraph{g->rowptr, g->col, 0, n}, pattern, acc);
   MC_CUDA_TRY(cudaGetLastError());
@@ -394,15 +390,27 @@ int dense_count(mc_dgraph *g, int pattern, uint64_t *out) {
   return MC_OK;
 }
 
-// Parts of one graph of a batch: about 1 M row words each (pairs, and three
-// rows per two-path, bounded through the largest degree), so that a batch's
-// largest graphs do not end it on one SM, while few CTAs build a matrix again.
-// 512 graphs (57 triangle jobs, 455 patterns on RMAT scale 5 to 8), whole
-// batch: 1.50, 1.42, 1.33, 1.28, 1.24 and 1.23 ms at 2^15 to 2^20 words, 2.8 ms
-// with one part per graph.
-int dense_parts(int64_t n, int64_t nnz, int64_t max_degree) {
-  const int64_t words = dense_words((int)n) * (n * n / 2 + 3 * nnz * max_degree / 2);
-  return (int)std::max<int64_t>(1, std::min<int64_t>(64, words >> 20));
+// Row words of one graph of a batch: pairs, and three rows per two-path, bounded
+// through the largest degree.
+int64_t dense_work(int64_t n, int64_t nnz, int64_t max_degree) {
+  return bit_words((int)n) * (n * n / 2 + 3 * nnz * max_degree / 2);
+}
+
+// Its parts: about 1 M words each, so that a batch's largest graphs do not end it
+// on one SM, while few CTAs build a matrix again.  512 graphs (57 triangle jobs,
+// 455 patterns on RMAT scale 5 to 8), whole batch: 1.50, 1.42, 1.33, 1.28, 1.24 and
+// 1.23 ms at 2^15 to 2^20 words, 2.8 ms with one part per graph.  A batch whose
+// words (total: of all its graphs) are fewer than that on every SM takes smaller
+// parts, down to four times the matrix that each of them builds: a complete graph
+// of 100 vertices alone took 5.3 ms in P5 on its one CTA, 1.2 so.  One that fills
+// the SMs sixteen times over takes larger ones: 40 random graphs of 1,000
+// vertices, 100,000 entries each, took 25 ms in P7 at 2^20, 9.6 in 64 parts.
+int dense_parts(int64_t n, int64_t nnz, int64_t max_degree, int64_t total, int num_sms) {
+  const int64_t own = 4 * n * bit_words((int)n);
+  const int64_t share = std::max({std::min<int64_t>(total / num_sms, 1 << 20),
+                                  total / (16 * num_sms), own, int64_t(1)});
+  return (int)std::max<int64_t>(
+      1, std::min<int64_t>(num_sms, dense_work(n, nnz, max_degree) / share));
 }
 
 int dense_batch_launch(const int64_t *rp, const int32_t *ci, const DenseTask *tasks, int num_tasks,

@@ -190,7 +190,8 @@ struct DenseTask {
 };
 // acc: the motif sums of every batch graph (zeroed by the caller); largest:
 // the most vertices among the tasks' graphs.
-int dense_parts(int64_t n, int64_t nnz, int64_t max_degree);
+int64_t dense_work(int64_t n, int64_t nnz, int64_t max_degree);
+int dense_parts(int64_t n, int64_t nnz, int64_t max_degree, int64_t total, int num_sms);
 int dense_batch_launch(const int64_t *rp, const int32_t *ci, const DenseTask *tasks, int num_tasks,
                        int largest, unsigned long long *acc, cudaStream_t s);
 // Contract checks of the row offsets alone; sets max_degree.
@@ -232,8 +233,8 @@ int batch_pattern_launch(const BatchPatternArgs &b, int grid, cudaStream_t s);
 // batch.cu: a batch over a host (device_csr false) or device union CSR.
 int batch_create(const int64_t *rowptr, const int32_t *col, bool device_csr, int64_t n,
                  int64_t nnz, const int64_t *graph_vptr, int num_graphs, const int32_t *jobs,
-                 const int64_t *gmaxdeg, const int64_t *gnnz_of, void *stream, bool do_capture,
-                 mc_batch_t **out);
+                 const int64_t *gmaxdeg, const int64_t *gnnz_of, const int64_t *gsquares,
+                 void *stream, bool do_capture, mc_batch_t **out);
 // Blocks of the batch pattern kernel whose frontier lists fit the scratch
 // budget; *warps receives the resident warp count.
 int batch_pattern_grid(int num_sms, int64_t cap, int64_t *warps);

@@ -4,6 +4,12 @@
 #pragma once
 #include <cstdint>
 
+#ifdef __CUDACC__
+#define MC_HOST_DEVICE __host__ __device__
+#else
+#define MC_HOST_DEVICE
+#endif
+
 namespace mc {
 
 constexpr int kDenseMax = 1024;  // vertices of a graph that bit rows take
@@ -83,6 +89,33 @@ inline PatternRoute pattern_route_by_size(int64_t n, int64_t nnz, int64_t max_de
     if (pattern == 4 && nnz <= 12288) return PatternRoute::kFormula;
   }
   return PatternRoute::kSparse;
+}
+
+
+// A batch's pattern job (P1..P8) by bit rows, or by the persistent per-edge
+// kernel: whichever is shorter on a full GPU, in ns per graph.  The bit rows take
+// the ANDs of all vertex pairs; the formulas some ns per entry and, by pattern, a
+// part of the sum of squared degrees (and, of P1, of the largest one: a hub's star
+// is one warp's).  Fitted to 40 copies of one graph, us per graph, formulas / bit
+// rows: a path of 1,000 vertices, P4 and P7: 2 / 28 and 1.5 / 10; random graphs of
+// 1,000 vertices, 10,034 entries, P2, P4, P7: 82 / 33, 13 / 32, 8 / 17; of 500,
+// 12,418 entries: 320 / 14, 23 / 8, 10 / 8; a star of 1,000, P1, P4, P8: 130 / 15,
+// 12 / 28, 50 / 15; complete graphs of 100, P2 to P4 (no two neighbours of an edge
+// apart, which the sizes do not show otherwise): 25 / 150, 16 / 142, 14 / 21.
+MC_HOST_DEVICE constexpr int bit_words(int64_t n) {
+  return n <= 32 ? 1 : n <= 64 ? 2 : n <= 128 ? 4 : n <= 256 ? 8 : (int)((n + 31) / 32);
+}
+inline bool batch_takes_bits(int64_t n, int64_t nnz, int64_t max_degree, int64_t degree_squares,
+                             int pattern) {
+  if (n > kDenseMax) return false;
+  if (pattern >= 2 && pattern <= 4 && n >= 24 && 10 * nnz >= 9 * n * (n - 1)) return false;
+  const double pairs = 0.5 * (double)n * (double)n * bit_words(n);
+  const double bits = pairs * (pattern == 1 || pattern >= 7 ? 0.0011 : 0.002);
+  constexpr double kPerSquare[] = {0.013, 0.75, 0.57, 0.012, 0.06, 0.01, 0.002, 0.04};
+  double formula = (pattern == 7 ? 0.8 : 1.1) * (double)nnz +
+                   kPerSquare[pattern - 1] * (double)degree_squares;
+  if (pattern == 1) formula += 0.13 * (double)max_degree * (double)max_degree;
+  return bits <= formula;
 }
 
 }  // namespace mc

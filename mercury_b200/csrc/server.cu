@@ -187,7 +187,7 @@ void run_batch(mc_server *s, std::vector<std::shared_ptr<Request>> &batch, int64
   };
   std::vector<Upload> uploads;  // keyed graphs uploaded by this batch
   std::vector<uint64_t> pinned;  // cache entries this batch pinned
-  std::vector<int64_t> vptr(G + 1, 0), maxdeg(G), gnnz(G);
+  std::vector<int64_t> vptr(G + 1, 0), maxdeg(G), gnnz(G), squares(G);
   std::vector<int32_t> jobs(G);
   std::vector<uint64_t> counts(G, 0);
   int status = MC_OK;
@@ -213,6 +213,7 @@ void run_batch(mc_server *s, std::vector<std::shared_ptr<Request>> &batch, int64
         r.n = it->second.n;
         r.nnz = it->second.nnz;
         r.max_degree = it->second.max_degree;
+        r.sumsq = it->second.sumsq;
         if (!r.prepinned) ++it->second.pins;  // a prepinned request holds its pin already
         pinned.push_back(r.key);
         cached = true;
@@ -246,6 +247,7 @@ void run_batch(mc_server *s, std::vector<std::shared_ptr<Request>> &batch, int64
     e_total += r.nnz;
     maxdeg[i] = r.max_degree;
     gnnz[i] = r.nnz;
+    squares[i] = r.sumsq;
     jobs[i] = r.job;
   }
   const int64_t n = vptr[G];
@@ -293,7 +295,7 @@ void run_batch(mc_server *s, std::vector<std::shared_ptr<Request>> &batch, int64
     }
     if (status == MC_OK) {
       status = batch_create(urp, ucol, true, n, e_total, vptr.data(), G, jobs.data(), maxdeg.data(),
-                            gnnz.data(), stream, false, &b);
+                            gnnz.data(), squares.data(), stream, false, &b);
       if (status == MC_OK) status = mc_batch_count(b, counts.data(), nullptr);
     }
   }

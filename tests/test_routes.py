@@ -31,6 +31,12 @@ def routes():
         def pattern(n, nnz, max_degree, k):
             return lib.pattern_route(C.c_int64(n), C.c_int64(nnz), C.c_int64(max_degree), k)
 
+        @staticmethod
+        def batch_bits(degrees, k):
+            n, nnz = len(degrees), sum(degrees)
+            return bool(lib.batch_bits(C.c_int64(n), C.c_int64(nnz), C.c_int64(max(degrees)),
+                                       C.c_int64(sum(d * d for d in degrees)), k))
+
     return Routes
 
 
@@ -71,3 +77,20 @@ def test_triangles_of_dense_graphs_keep_the_dag(routes):
     # Sparse ones, hubs or not, keep the pairs.
     for n, nnz in [(1024, 12014), (8192, 204044), (2048, 177992), (100000, 499200), (2064, 256000)]:
         assert routes.triangle(n, nnz) == PAIRS
+
+
+def test_batch_jobs_take_bit_rows_where_they_pay(routes):
+    """Pattern jobs of a batch: all vertex pairs of a sparse graph of 1,000 vertices
+    cost more than its few entries, unless a hub makes the formulas dear; complete
+    graphs leave P2 to P4 nothing to test."""
+    takes = lambda degrees: [k for k in range(1, 9) if routes.batch_bits(degrees, k)]
+    every = list(range(1, 9))
+    assert takes([2] * 1000) == []
+    assert takes([3] * 1000) == []
+    assert takes([10] * 1000) == [2, 3]
+    assert takes([100] * 1000) == every
+    assert takes([999] + [1] * 999) == [1, 2, 3, 5, 8]
+    assert takes([2] * 100) == takes([25] * 500) == takes([10] * 256) == every
+    assert takes([99] * 100) == [1, 5, 6, 7, 8]
+    assert takes([15] * 16) == every
+    assert takes([50] * 1025) == []
