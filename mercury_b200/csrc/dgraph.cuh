@@ -177,7 +177,9 @@ int clique_launch(mc_dgraph *g, int pattern, int64_t dag_edges, int shard, int n
 // returns MC_ERR_OOM when its scratch does not fit: the formula routes need
 // less.
 PatternRoute pattern_route(const mc_dgraph *g, int pattern);
-int motif_count(mc_dgraph *g, int pattern, uint64_t *out);
+// estimates: stop where the formulas turn out to be the shorter way (*elsewhere,
+// count not written); otherwise count whatever it costs.
+int motif_count(mc_dgraph *g, int pattern, bool estimates, uint64_t *out, bool *elsewhere);
 int dense_count(mc_dgraph *g, int pattern, uint64_t *out);
 int dense_triangles(mc_dgraph *g, bool check);
 // Triangles from pairs of up neighbours (motifs.cu): three launches.

@@ -62,6 +62,7 @@ struct MotifArgs {
   const int64_t *__restrict__ rp;
   const int32_t *__restrict__ ci;
   int n, nnz;
+  int pattern;
   unsigned need;
   int32_t *deg;    // n
   int32_t *dp;     // n: |N+(v)|
@@ -78,6 +79,9 @@ struct MotifArgs {
   int32_t *list;   // common-neighbour lists
   int64_t list_cap;
   u64 *pool;       // list entries handed out (above list_cap: all later stages stop)
+  u64 *probe;      // two-paths sampled, and the closed ones among them
+  int probe_percent;  // closed from here on: every stage stops (0: no samples)
+  bool early;      // motif_outweighs is asked before the tau stage
   u64 *acc;        // kSums
   // Vertices too large for one warp.  pair_mid: the two hash classes, from the
   // front and from the back of its n entries; pair_big: tables over all
@@ -121,6 +125,8 @@ constexpr u64 kFewWalk = 64;
 constexpr int kFewVertices = 16384;
 constexpr int kHashSlots = 1024;  // of a warp
 constexpr int kWheelDeg = 512;    // warp form of the wheel stage
+constexpr int kProbeBlocks = 4;   // samples: a thread each
+constexpr int kEarlyOut = 400;    // bound on d+ above which a^2 is summed before tau (7 us at 1 M entries)
 
 // (degree, id) order.
 __device__ __forceinline__ bool lower(int du, int u, int dv, int v) {
@@ -189,6 +195,13 @@ struct RowLanes {
 __device__ __forceinline__ bool lists_overrun(const MotifArgs &a) {
   return *a.pool > (u64)a.list_cap;
 }
+constexpr u64 kClosed = ~0ull;  // in *pool: the samples sent the count elsewhere
+
+// The stages that a^2 drives: not for lists that overran, nor where the formulas
+// are the shorter way.
+__device__ __forceinline__ bool stops_here(const MotifArgs &a) {
+  return lists_overrun(a) || ((a.need & kNeedWork) && motif_outweighs(a.pattern, a.acc));
+}
 
 // Offsets of the lists of this lane's up entry e and its reverse, `len` entries
 // each (0: none); one atomic per warp.
@@ -209,14 +222,39 @@ __device__ __forceinline__ void take_lists(const MotifArgs &a, int e, int r, int
 }
 
 // ---- rows, up ---------------------------------------------------------------
-// Warp per row: src, deg, and the sums of degrees alone.
-__global__ void __launch_bounds__(kThreads) motif_rows_kernel(MotifArgs a) {
+// A sample of two-paths u - v - w per thread (from a random entry u -> v on),
+// counted, and the closed ones among them.
+__device__ void sample_two_paths(const MotifArgs &a, unsigned sample, int lane) {
+  u64 r = (u64)(sample + 1) * 0x9e3779b97f4a7c15ull;
+  r = (r ^ (r >> 30)) * 0xbf58476d1ce4e5b9ull;
+  r ^= r >> 31;
+  const int e = (int)((r & 0xffffffffu) % (unsigned)a.nnz);
+  const int u = (int)upper_row(a.rp, 0, a.n - 1, e), v = __ldg(a.ci + e);
+  const int b = (int)__ldg(a.rp + v), d = (int)__ldg(a.rp + v + 1) - b;
+  const int w = d > 0 ? __ldg(a.ci + b + (int)((unsigned)(r >> 32) % (unsigned)d)) : u;
+  const bool path = w != u;
+  const bool closed =
+      path && find_entry(a.ci, (int)__ldg(a.rp + u), (int)__ldg(a.rp + u + 1), w) >= 0;
+  const unsigned paths = __ballot_sync(kFull, path), hits = __ballot_sync(kFull, closed);
+  if (lane == 0) {
+    if (paths) atomicAdd(a.probe, (u64)__popc(paths));
+    if (hits) atomicAdd(a.probe + 1, (u64)__popc(hits));
+  }
+}
+
+// Warp per row: src, deg, and the sums of degrees alone.  The blocks from
+// row_blocks on take the samples beside them.
+__global__ void __launch_bounds__(kThreads) motif_rows_kernel(MotifArgs a, int row_blocks) {
   __shared__ u64 sm[kSums];
   const BlockSums bs{sm};
   bs.init();
   const int lane = threadIdx.x & (kWarp - 1);
+  if ((int)blockIdx.x >= row_blocks) {
+    sample_two_paths(a, (blockIdx.x - row_blocks) * kThreads + threadIdx.x, lane);
+    return;
+  }
   u64 d3 = 0, d4 = 0;
-  const int stride = gridDim.x * kWarps;
+  const int stride = row_blocks * kWarps;
   for (int v = blockIdx.x * kWarps + threadIdx.x / kWarp; v < a.n; v += stride) {
     const int b = (int)__ldg(a.rp + v), e = (int)__ldg(a.rp + v + 1);
     for (int i = b + lane; i < e; i += kWarp) a.src[i] = v;
@@ -237,6 +275,11 @@ __global__ void __launch_bounds__(kThreads) motif_rows_kernel(MotifArgs a) {
 __global__ void __launch_bounds__(kThreads) motif_up_kernel(MotifArgs a) {
   const int lane = threadIdx.x & (kWarp - 1);
   const int64_t e64 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  if (a.probe_percent > 0 && a.probe[0] > 0 &&
+      100 * a.probe[1] >= (u64)a.probe_percent * a.probe[0]) {
+    if (e64 == 0) *a.pool = kClosed;
+    return;
+  }
   const bool in = e64 < a.nnz;
   const int e = in ? (int)e64 : a.nnz - 1;
   const int u = a.src[e], v = __ldg(a.ci + e);
@@ -281,6 +324,7 @@ __global__ void __launch_bounds__(kThreads) motif_up_kernel(MotifArgs a) {
 
 // With counts: exactly sized lists.
 __global__ void __launch_bounds__(kThreads) motif_lists_kernel(MotifArgs a) {
+  if (*a.pool == kClosed) return;
   const int64_t e64 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   const int e = (int)(e64 < a.nnz ? e64 : 0);
   const bool up = e64 < a.nnz && a.pos1[e];
@@ -436,6 +480,23 @@ __global__ void __launch_bounds__(kThreads) tri_pairs_kernel(MotifArgs a, int pe
 }
 
 // ---- triangles with their common neighbours -----------------------------------
+// The sum of a^2 ahead of the tau stage, thread per entry, where a graph's up lists
+// may be long: K5 can then take that stage as long as the wheels and X7 take later
+// (a complete graph of 512 vertices beside a path, P3: 75 ms of 450 in tau).
+__global__ void __launch_bounds__(kThreads) motif_squares_kernel(MotifArgs a) {
+  __shared__ u64 sm[kSums];
+  const BlockSums bs{sm};
+  bs.init();
+  if (lists_overrun(a)) return;
+  u64 a2 = 0;
+  for (int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x; e < a.nnz;
+       e += (int64_t)gridDim.x * kThreads)
+    if (a.pos1[e]) a2 += (u64)a.a[e] * (u64)a.a[e];  // an edge once, at its up entry
+  __syncwarp();
+  bs.add(kA2, a2);
+  bs.flush(a.acc);
+}
+
 struct TauSums {
   u64 D = 0, C3 = 0, p4 = 0, fork = 0, dart = 0, vt2 = 0;
   u64 cricket = 0, bull = 0, lolli = 0, kite = 0, gem = 0, kd = 0, ka = 0, kk = 0, K4 = 0, K5 = 0;
@@ -612,8 +673,6 @@ __device__ void tau_large(const MotifArgs &a, TauSums &t, unsigned *s_rows, int 
   }
 }
 
-// Both forms in one launch while the large form's rows leave the SM full of
-// CTAs, else one launch each.
 // Between the sum of all walks and the pairs stage: the walks to take in parts
 // leave the list of the huge ones (-1).
 __device__ __forceinline__ void split_walks(const MotifArgs &a) {
@@ -632,6 +691,8 @@ __device__ __forceinline__ void split_walks(const MotifArgs &a) {
   }
 }
 
+// Both forms in one launch while the large form's rows leave the SM full of
+// CTAs, else one launch each.
 template <bool kLarge, bool kSmall>
 __global__ void __launch_bounds__(kThreads) motif_tau_kernel(MotifArgs a, int smem_words) {
   extern __shared__ unsigned s_rows[];
@@ -641,7 +702,7 @@ __global__ void __launch_bounds__(kThreads) motif_tau_kernel(MotifArgs a, int sm
   __shared__ int s_u;
   const BlockSums bs{sm};
   bs.init();
-  if (lists_overrun(a)) return;
+  if (a.early ? stops_here(a) : lists_overrun(a)) return;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   TauSums t;
   if (kLarge && a.split_cap > 0) split_walks(a);
@@ -855,7 +916,7 @@ __global__ void __launch_bounds__(kThreads) motif_pairs_kernel(MotifArgs a) {
   __shared__ u64 sm[kSums];
   const BlockSums bs{sm};
   bs.init();
-  if (lists_overrun(a)) return;
+  if (stops_here(a)) return;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   int *mine = s_tab + warp * (kHashSlots + kHashSlots / 2);
   HashTable tab{mine, reinterpret_cast<unsigned *>(mine + kHashSlots), 10};
@@ -886,7 +947,7 @@ __global__ void __launch_bounds__(kT) motif_pairs_hash_kernel(MotifArgs a) {
   __shared__ int s_s;
   const BlockSums bs{sm};
   bs.init();
-  if (lists_overrun(a)) return;
+  if (stops_here(a)) return;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   HashTable tab{s_tab, reinterpret_cast<unsigned *>(s_tab + (1 << kLg)), kLg};
   PairSums ps;
@@ -937,7 +998,7 @@ __global__ void __launch_bounds__(kPairThreads) motif_pairs_big_kernel(MotifArgs
   __shared__ int s_range[2];
   const BlockSums bs{sm};
   bs.init();
-  if (lists_overrun(a)) return;
+  if (stops_here(a)) return;
   const int words = (a.n + 1) >> 1;
   unsigned *cnt = kShared ? reinterpret_cast<unsigned *>(s_tab)
                           : counters + (int64_t)blockIdx.x * words;
@@ -1016,7 +1077,7 @@ __global__ void __launch_bounds__(kThreads) motif_wheel_kernel(MotifArgs a, int 
   __shared__ unsigned s_cnt[kWarps][kWheelDeg];
   const BlockSums bs{sm};
   bs.init();
-  if (lists_overrun(a)) return;
+  if (stops_here(a)) return;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   unsigned *cnt = s_cnt[warp];
   for (int i = lane; i < kWheelDeg; i += kWarp) cnt[i] = 0;
@@ -1059,7 +1120,7 @@ __global__ void __launch_bounds__(kThreads) motif_wheel_big_kernel(MotifArgs a, 
   __shared__ int s_e[kThreads], s_n;
   const BlockSums bs{sm};
   bs.init();
-  if (lists_overrun(a)) return;
+  if (stops_here(a)) return;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   for (int i = threadIdx.x; i < table; i += kThreads) s_cnt[i] = 0;
   u64 w4 = 0;
@@ -1204,7 +1265,8 @@ int motif_triangles(mc_dgraph *g, uint64_t *out) {
   u64 total = 0;
   auto run = [&]() -> int {
     MC_CUDA_TRY(cudaMemsetAsync(c.base, 0, zeroed, s));
-    motif_rows_kernel<<<std::min(blocks(n, kWarps), 4096u), kThreads, 0, s>>>(a);
+    const unsigned row_blocks = std::min(blocks(n, kWarps), 4096u);
+    motif_rows_kernel<<<row_blocks, kThreads, 0, s>>>(a, (int)row_blocks);
     MC_CUDA_TRY(cudaGetLastError());
     tri_up_kernel<<<blocks(nnz, kThreads), kThreads, 0, s>>>(a);
     MC_CUDA_TRY(cudaGetLastError());
@@ -1224,11 +1286,13 @@ int motif_triangles(mc_dgraph *g, uint64_t *out) {
   return rc;
 }
 
-int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
+int motif_count(mc_dgraph *g, int pattern, bool estimates, uint64_t *out, bool *elsewhere) {
   NvtxRange range("motif_count");
   cudaStream_t s = g->stream;
   const int n = (int)g->n, nnz = (int)g->nnz;
-  const unsigned need = motif_needs(pattern);
+  const bool asked_for = estimates && n > kEstimateAbove;
+  const unsigned need = motif_needs(pattern) & (asked_for ? ~0u : ~(unsigned)kNeedWork);
+  *elsewhere = false;
   const bool pairs = need & (kNeedC4 | kNeedPairs), ordered = need & kNeedC4;
   const bool wheel = need & kNeedW4;
   // Shared-memory tables of the pairs stage: 16 bits per vertex.
@@ -1257,7 +1321,10 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
     a.ci = g->col;
     a.n = n;
     a.nnz = nnz;
+    a.pattern = pattern;
     a.need = need;
+    a.probe_percent = estimates ? probe_percent(n, nnz, g->max_degree, pattern) : 0;
+    a.early = (need & kNeedWork) && std::min(g->max_degree, root) > kEarlyOut;
     a.list_cap = list_cap;
     a.slice_words = slice_words;
     // Few vertices: a CTA for all but the shortest walks.
@@ -1269,9 +1336,10 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
     // The same layout for every pattern (so that each finds the last one's block).
     auto lay_out = [&](Carver &c) {
       // Zeroed before the first kernel.
-      a.acc = c.take<u64>(kSums + 2);
+      a.acc = c.take<u64>(kSums + 4);
       a.pool = a.acc + kSums;
       a.walk_total = a.pool + 1;
+      a.probe = a.walk_total + 1;
       a.counts = c.take<unsigned>(kCounts);
       a.dp = c.take<int32_t>(n);
       a.d2 = c.take<u64>(n);
@@ -1326,7 +1394,9 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
       const unsigned tri_grid = blocks(std::max<int64_t>(n, ((int64_t)nnz + per - 1) / per * kWarp),
                                        kThreads);
       MC_CUDA_TRY(cudaMemsetAsync(c.base, 0, zeroed, s));
-      motif_rows_kernel<<<std::min(blocks(n, kWarps), 4096u), kThreads, 0, s>>>(a);
+      const unsigned row_blocks = std::min(blocks(n, kWarps), 4096u);
+      motif_rows_kernel<<<row_blocks + (a.probe_percent > 0 ? kProbeBlocks : 0), kThreads, 0, s>>>(
+          a, (int)row_blocks);
       MC_CUDA_TRY(cudaGetLastError());
       motif_up_kernel<<<blocks(nnz, kThreads), kThreads, 0, s>>>(a);
       MC_CUDA_TRY(cudaGetLastError());
@@ -1339,6 +1409,12 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
       }
       motif_tri_kernel<false><<<tri_grid, kThreads, 0, s>>>(a, per);
       MC_CUDA_TRY(cudaGetLastError());
+      if (a.early) {
+        motif_squares_kernel<<<std::min(blocks(nnz, kThreads), (unsigned)(8 * g->num_sms)), kThreads,
+                               0, s>>>(a);
+        MC_CUDA_TRY(cudaGetLastError());
+        g->launches += 1;
+      }
       const unsigned tau_small_grid = std::min(blocks(n, kWarps), (unsigned)(8 * g->num_sms));
       if (slice_words * 4 <= kTauBoth) {
         motif_tau_kernel<true, true><<<tau_small_grid, kThreads, slice_words * 4, s>>>(
@@ -1387,6 +1463,11 @@ int motif_count(mc_dgraph *g, int pattern, uint64_t *out) {
     }
     scratch_give(c.base, got, g->device, s);
     scratch_give(counters, got_counters, g->device, s);
+    if (h[kSums] == kClosed || (h[kSums] <= (u64)list_cap && (need & kNeedWork) &&
+                                motif_outweighs(pattern, h))) {
+      *elsewhere = true;
+      return MC_OK;
+    }
     const int64_t asked = (int64_t)h[kSums];
     if (asked <= list_cap) {
       *out = motif_combine(pattern, h);

@@ -15,6 +15,7 @@ enum Sum : int {
   kT, kCricket, kBull, kLolli, kKite, kGem,  // triangles
   kKd, kKa, kKk, kK4, kK5,                 // with common neighbours; cliques
   kC4, kC4d, kC4a, kX7, kW4, kK23,         // 4-cycles and beyond
+  kA2,                                     // edges: a^2, where it is taken ahead of kD
   kSums
 };
 
@@ -27,14 +28,15 @@ enum Need : unsigned {
   kNeedPairs = 16u, // every pair's common neighbours (C4 counted twice)
   kNeedW4 = 32u,
   kNeedK23 = 64u,   // with kNeedPairs: K2,3 and degrees on 4-cycles
+  kNeedWork = 128u, // motif_outweighs is asked
 };
 
 __host__ __device__ constexpr unsigned motif_needs(int pattern) {
   return pattern == 1   ? 0u
-         : pattern == 2 ? kNeedTau | kNeedD2 | kNeedT | kNeedPairs | kNeedW4 | kNeedK23
-         : pattern == 3 ? kNeedTau | kNeedT | kNeedW4
+         : pattern == 2 ? kNeedTau | kNeedD2 | kNeedT | kNeedPairs | kNeedW4 | kNeedK23 | kNeedWork
+         : pattern == 3 ? kNeedTau | kNeedT | kNeedW4 | kNeedWork
          : pattern == 4 ? kNeedC4
-         : pattern == 5 ? kNeedTau | kNeedPairs | kNeedW4
+         : pattern == 5 ? kNeedTau | kNeedPairs | kNeedW4 | kNeedWork
          : pattern == 6 ? kNeedTau | kNeedW4
                         : (unsigned)kNeedTau;
 }
@@ -52,6 +54,34 @@ __device__ __forceinline__ u64 c4(long long x) {
 __device__ __forceinline__ unsigned above(int j, int w) {
   const int s = j + 1 - 32 * w;
   return s <= 0 ? kFull : (s >= 32 ? 0u : kFull << s);
+}
+
+// P2, P3 and P5 above 512 vertices, known once the triangles are: the wheel stage
+// and X7 visit the sum of a^2 over the entries, some cliques' whole cost, while the
+// per-edge formulas test the neighbours that an edge's ends do not share (x and y
+// of them), next to none in a clique.  True where the formulas are the shorter
+// way, by the sums of a^2, a, x^2 and a x over the entries, which follow from those
+// of the vertices (an entry of v has x = d - 1 - a, and a adds up to 2 t along v's
+// row).  The weights, in ps, are fitted to whole calls (formulas / sums, ms): three
+// complete graphs of 400 vertices, P2, P3, P5: 10 / 864, 1.3 / 395, 109 / 868; one of
+// 300 beside the Chung-Lu graph of 100,000: 34 / 445, 10 / 73, 25 / 436; a random
+// graph of 800 vertices with 70% of all edges: 645 / 1,069, 542 / 251, above 2,500 /
+// 1,066; 2,000 vertices, 10%: 56 / 4.4, 23 / 2.0, 96 / 4.3; the Chung-Lu graph of
+// 20,000 with hubs of 5,000: above 2,500 / 140, 24 and 138.
+constexpr u64 kOutweighFloor = 20000000;  // some 0.1 ms
+__host__ __device__ inline bool motif_outweighs(int pattern, const u64 *s) {
+  const u64 a = 6 * s[kT], a2 = s[kA2] ? 2 * s[kA2] : 4 * s[kD] + a;
+  if (a2 < kOutweighFloor) return false;
+  const u64 da = 2 * (s[kVtd] - 3 * s[kT]);  // sum of (d - 1) a
+  const u64 d3 = 6 * s[kVd3] + a2;           // of (d - 1)^2 + a^2, but for sum of d (d - 1)
+  const u64 q = (d3 > 2 * da ? d3 - 2 * da : 0) >> 6, m = (da > a2 ? da - a2 : 0) >> 6;
+  const u64 e = a >> 6, w = a2 >> 6;
+  switch (pattern) {
+    case 2: return 15 * w > 5 * q + 19 * m + 80 * e;
+    case 3: return 6 * w > q + 16 * m + 8 * e;
+    case 5: return 20 * w > 2 * q + 200 * m + 500 * e;
+    default: return false;
+  }
 }
 
 // Per-block totals of the sums a kernel adds to.

@@ -2173,13 +2173,18 @@ int pattern_count_body(mc_dgraph *g, int pattern, uint64_t *out, uint64_t *c12,
   // counters stay with the routes below.
   const PatternRoute route = num_shards == 1 && budget_ms <= 0 && !c12 ? pattern_route(g, pattern)
                                                                         : PatternRoute::kFormula;
+  const int64_t launches_before = g->launches;
+  bool started = false;  // ev[0] marks the start of this count
   if (route != PatternRoute::kFormula) {
-    const int64_t launches = g->launches;
     MC_CUDA_TRY(cudaEventRecord(g->ev[0], g->stream));
-    const int rc = route == PatternRoute::kDense ? dense_count(g, pattern, out)
-                                                 : motif_count(g, pattern, out);
+    started = true;
+    // A route that the environment asks for is taken to its end.
+    bool elsewhere = false;
+    const int rc = route == PatternRoute::kDense
+                       ? dense_count(g, pattern, out)
+                       : motif_count(g, pattern, !std::getenv("MERCURY_MOTIF_ROUTE"), out, &elsewhere);
     if (rc != MC_OK && rc != MC_ERR_OOM) return rc;
-    if (rc == MC_OK) {
+    if (rc == MC_OK && !elsewhere) {
       if (progress) *progress = 1.0;
       if (timing) {
         std::memset(timing, 0, sizeof(*timing));
@@ -2187,18 +2192,20 @@ int pattern_count_body(mc_dgraph *g, int pattern, uint64_t *out, uint64_t *c12,
         cudaEventElapsedTime(&ms, g->ev[0], g->ev[3]);
         timing->count_ms = ms;
         timing->total_ms = ms;
-        timing->launches = g->launches - launches;
+        timing->launches = g->launches - launches_before;
       }
       return MC_OK;
     }
-    cudaGetLastError();  // a failed allocation: the routes below need less scratch
+    // Cliques, where the formulas are the shorter way; or a failed allocation:
+    // the routes below need less scratch.
+    cudaGetLastError();
   }
   // P7 and P8 on graphs with hubs: by clique counts over the degree-ordered
   // DAG (cliques.cu), which is built first; its time counts as the pattern's.
   bool cliques = false;
   int64_t dag_edges = 0;
   if (pattern == 7 || pattern == 8) {
-    MC_CUDA_TRY(cudaEventRecord(g->ev[0], g->stream));
+    if (!started) MC_CUDA_TRY(cudaEventRecord(g->ev[0], g->stream));
     const int rc = clique_prepare(g, pattern, &cliques, &dag_edges);
     if (rc != MC_OK) return rc;
   }
@@ -2212,7 +2219,6 @@ int pattern_count_body(mc_dgraph *g, int pattern, uint64_t *out, uint64_t *c12,
   if (const char *env = std::getenv("MERCURY_PATTERN_SLICE_MS")) sl.target_ms = std::max(0.01, std::atof(env));
   sl.trace = std::getenv("MERCURY_TRACE_SLICES") != nullptr;
   cudaStream_t s = g->stream;
-  const int64_t launches_before = g->launches;
   MC_CUDA_TRY(cudaMemsetAsync(g->counters, 0, sizeof(unsigned long long) * 8, s));
   // The frontier lists hold at most max_degree vertices.
   const int64_t cap = std::max<int64_t>(g->max_degree, 1);
@@ -2241,7 +2247,7 @@ int pattern_count_body(mc_dgraph *g, int pattern, uint64_t *out, uint64_t *c12,
     g->h_counters[6] = 0;
   }
   if (const char *env = std::getenv("MERCURY_PATTERN_SETS")) a.use_sets = std::atoi(env) != 0;
-  if (!cliques) MC_CUDA_TRY(cudaEventRecord(g->ev[0], s));
+  if (!cliques && !started) MC_CUDA_TRY(cudaEventRecord(g->ev[0], s));
   int rc = MC_OK;
   if (cliques) {
     rc = clique_launch(g, pattern, dag_edges, shard, num_shards, a.deadline, a.stop_flag);

@@ -70,6 +70,12 @@ inline TriangleRoute triangle_route_by_size(int64_t n, int64_t nnz) {
 //    0.097.  Hubs turn it: 3,001 vertices, mean 4, cap 200 (11,186 entries,
 //    degree 165), P5 to P8: 0.52, 1.20, 0.33 and 0.71 against 0.37, 0.10, 0.09
 //    and 0.09.
+//  - the formulas keep near-complete graphs (formula / default without them:
+//    complete graphs of 100, 200 and 512 vertices, P1: 0.23 / 0.33, 0.70 / 0.53,
+//    1.3 / 5.4; P2: 0.86 / 1.5, 3.8 / 6.3, 5.7 / 74; P3: 0.23 / 1.7, 0.64 / 9.0, 1.07 /
+//    431; P4 of 128: 0.07 / 0.45; P5, P6 and P8 of 64: 0.21, 0.25 and 0.17 / 0.52; 90%
+//    of all edges, 400 vertices, P1 to P4: 0.77 / 2.1, 17 / 24, 13 / 91, 2.7 / 2.3).
+//    Cliques in larger graphs show on the way (probe_percent, motif_outweighs).
 enum class PatternRoute { kFormula, kDense, kSparse };
 inline bool motif_sums_apply(int64_t n, int64_t nnz, int64_t max_degree) {
   return motif_range(n, nnz) && max_degree <= 46340;
@@ -77,6 +83,32 @@ inline bool motif_sums_apply(int64_t n, int64_t nnz, int64_t max_degree) {
 inline PatternRoute pattern_route_by_size(int64_t n, int64_t nnz, int64_t max_degree,
                                           int pattern) {
   if (!motif_sums_apply(n, nnz, max_degree)) return PatternRoute::kFormula;
+  // In percent of all entries: near-complete graphs, where the ends of an edge share
+  // almost every neighbour and the formulas have next to nothing to test.
+  const auto filled = [&](int percent) {
+    return 100.0 * (double)nnz >= percent * (double)n * (double)(n - 1);
+  };
+  switch (pattern) {
+    case 1:
+      if ((n >= 256 && filled(78)) || (n > 64 && n <= 140 && filled(95)))
+        return PatternRoute::kFormula;
+      break;
+    case 2:
+      if ((n >= 64 && filled(97)) || (n >= 300 && filled(88))) return PatternRoute::kFormula;
+      break;
+    case 3:
+      if ((n >= 32 && filled(88)) || (n >= 300 && filled(75))) return PatternRoute::kFormula;
+      break;
+    case 4:
+      if (filled(93)) return PatternRoute::kFormula;
+      break;
+    case 6:
+      if (n >= 32 && n <= 128 && filled(93)) return PatternRoute::kFormula;
+      break;
+    case 7: break;
+    default:  // 5, 8
+      if (n >= 32 && n <= 140 && filled(97)) return PatternRoute::kFormula;
+  }
   if (n <= 64 && pattern != 4) return PatternRoute::kDense;
   if (n <= 512 && (pattern == 2 || pattern == 5)) return PatternRoute::kDense;
   struct Limit {
@@ -91,6 +123,19 @@ inline PatternRoute pattern_route_by_size(int64_t n, int64_t nnz, int64_t max_de
   return PatternRoute::kSparse;
 }
 
+// Graphs above 256 vertices that may be unions of cliques, by sizes: P1 to P4 then
+// sample two-paths beside the first stage, and go to the formulas when this many
+// percent of them are closed; 0: no samples.  Formula / sums, ms: 20 complete
+// graphs of 128 vertices, P1 to P4: 0.39 / 1.3, 1.6 / 47, 0.36 / 24, 0.44 / 1.5; 20
+// random ones of 150 with 80% of all edges: 0.88 / 1.3, 11 / 29, 7.4 / 14.5, 1.3 /
+// 1.5; with 50%: 0.39 / 0.45, 4.5 / 4.8, 2.6 / 2.0, 0.87 / 0.54; one of 800, 80%, P4:
+// 31 / 11, 98%: 6.4 / 18; 2,000 complete graphs of 20, P1 to P4: 0.21 / 0.32, 0.74 /
+// 1.8, 0.18 / 1.2, 0.60 / 0.36.
+inline int probe_percent(int64_t n, int64_t nnz, int64_t max_degree, int pattern) {
+  if (pattern > 4 || n <= 256 || max_degree * n > 8 * nnz) return 0;
+  return pattern == 4 ? (nnz >= 32 * n ? 88 : 0) : (nnz >= 16 * n ? 78 : 0);
+}
+constexpr int64_t kEstimateAbove = 512;  // vertices from which motif_outweighs is asked
 
 // A batch's pattern job (P1..P8) by bit rows, or by the persistent per-edge
 // kernel: whichever is shorter on a full GPU, in ns per graph.  The bit rows take

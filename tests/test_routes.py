@@ -32,6 +32,10 @@ def routes():
             return lib.pattern_route(C.c_int64(n), C.c_int64(nnz), C.c_int64(max_degree), k)
 
         @staticmethod
+        def samples(n, nnz, max_degree, k):
+            return lib.samples(C.c_int64(n), C.c_int64(nnz), C.c_int64(max_degree), k)
+
+        @staticmethod
         def batch_bits(degrees, k):
             n, nnz = len(degrees), sum(degrees)
             return bool(lib.batch_bits(C.c_int64(n), C.c_int64(nnz), C.c_int64(max(degrees)),
@@ -94,3 +98,22 @@ def test_batch_jobs_take_bit_rows_where_they_pay(routes):
     assert takes([99] * 100) == [1, 5, 6, 7, 8]
     assert takes([15] * 16) == every
     assert takes([50] * 1025) == []
+
+
+def test_patterns_of_near_complete_graphs_keep_the_formulas(routes):
+    def formulas(n, percent):
+        nnz = n * (n - 1) * percent // 100
+        return [k for k in range(1, 9) if routes.pattern(n, nnz, n - 1, k) == FORMULA]
+
+    assert formulas(100, 100) == [1, 2, 3, 4, 5, 6, 8]
+    assert formulas(64, 100) == [2, 3, 4, 5, 6, 8]
+    assert formulas(200, 100) == formulas(512, 100)[1:] == [2, 3, 4]
+    assert formulas(512, 100) == formulas(1000, 100) == [1, 2, 3, 4]
+    assert formulas(400, 80) == [1, 3] and formulas(400, 50) == []
+
+
+def test_samples_are_for_graphs_that_may_be_unions_of_cliques(routes):
+    assert [routes.samples(2560, 325120, 127, k) for k in range(1, 9)] == [78] * 3 + [88] + [0] * 4
+    assert routes.samples(200, 39800, 199, 1) == 0        # by size
+    assert routes.samples(100000, 996680, 200, 1) == 0   # mean 10
+    assert routes.samples(60000, 1100000, 17215, 1) == 0  # hubs
