@@ -301,7 +301,7 @@ int mc_pattern_count_shard(mc_dgraph_t *g, int pattern, int shard,
  * once the slices have used more than budget_ms of device time the count
  * stops between two slices and returns MC_ERR_TIMEOUT (count not written).
  * progress (optional) receives the fraction of the tasks done.  Graphs with
- * a maximum degree above 4,096 are counted in slices by the formulas of mc_pattern_count too
+ * a maximum degree above 4,096 are counted in slices by mc_pattern_count too
  * (no budget): a hub edge alone can take seconds.  The reference has no
  * budget; its kernels run to the end (subgraph_matching/sm_multigpu.cu:
  * 150-200). */

@@ -49,13 +49,16 @@
 #include "device_common.cuh"
 #include "dgraph.cuh"
 #include "motifs.cuh"
+#include "slices.cuh"
 
 namespace mc {
 namespace {
 
 // Words of MotifArgs::counts: list lengths, then queue positions.
 enum Count : int {
-  kTauN, kMidN, kHashN, kHugeN, kBigN, kSplitN, kTauQueue, kMidQueue, kHashQueue, kBigQueue, kCounts
+  kTauN, kMidN, kHashN, kHugeN, kBigN, kSplitN, kTauQueue, kMidQueue, kHashQueue, kUnused,
+  kBigQueue,  // 64 bits (run_slices clears it)
+  kCounts = kBigQueue + 2
 };
 
 struct MotifArgs {
@@ -988,10 +991,11 @@ __device__ int row_at(const int64_t *__restrict__ rp, int n, int64_t e) {
 
 // CTA per larger s (longest walks first): 16-bit counters over all vertices,
 // two to a word, in shared memory when n of them fit, else one slice of
-// `counters` per CTA.
+// `counters` per CTA.  Items [begin, end) of the list (ordered walks, with their
+// parts in front: all).
 template <bool kOrdered, bool kShared>
-__global__ void __launch_bounds__(kPairThreads) motif_pairs_big_kernel(MotifArgs a,
-                                                                       unsigned *counters) {
+__global__ void __launch_bounds__(kPairThreads) motif_pairs_big_kernel(MotifArgs a, unsigned *counters,
+                                                                       unsigned begin, unsigned end) {
   extern __shared__ __align__(16) int s_tab[];
   __shared__ u64 sm[kSums];
   __shared__ int2 s_item;
@@ -1009,7 +1013,7 @@ __global__ void __launch_bounds__(kPairThreads) motif_pairs_big_kernel(MotifArgs
   const int splits = kOrdered ? (int)min(a.counts[kSplitN], (unsigned)a.split_cap) : 0;
   for (;;) {
     if (threadIdx.x == 0) {
-      unsigned i = atomicAdd(a.counts + kBigQueue, 1u);
+      unsigned i = begin + atomicAdd(a.counts + kBigQueue, 1u);
       const unsigned huge = a.counts[kHugeN], big = a.counts[kBigN];
       int4 item = make_int4(kEnd, 0, 1, 0);
       if ((int)i < splits) {
@@ -1017,7 +1021,7 @@ __global__ void __launch_bounds__(kPairThreads) motif_pairs_big_kernel(MotifArgs
         // Parts of about the same number of entries: t's place in the CSR.
         for (int k = 0; k < 2; ++k)
           s_range[k] = row_at(a.rp, a.n, (int64_t)a.nnz * (item.y + k) / item.z);
-      } else if (i - (unsigned)splits < huge + big) {
+      } else if (i < end && i - (unsigned)splits < huge + big) {
         i -= (unsigned)splits;
         item.x = i < huge ? a.pair_big[i] : a.pair_big[a.n - 1 - (i - huge)];
       }
@@ -1113,8 +1117,10 @@ __global__ void __launch_bounds__(kThreads) motif_wheel_kernel(MotifArgs a, int 
   bs.flush(a.acc);
 }
 
-// CTA per entry of a longer row: warp per y, lanes over y's list.
-__global__ void __launch_bounds__(kThreads) motif_wheel_big_kernel(MotifArgs a, int table) {
+// CTA per entry of a longer row: warp per y, lanes over y's list; entries [begin,
+// end), a CTA looking at `per` of them at a time.
+__global__ void __launch_bounds__(kThreads) motif_wheel_big_kernel(MotifArgs a, int table, int64_t begin,
+                                                                   int64_t end, int per) {
   extern __shared__ unsigned s_cnt[];
   __shared__ u64 sm[kSums];
   __shared__ int s_e[kThreads], s_n;
@@ -1124,12 +1130,12 @@ __global__ void __launch_bounds__(kThreads) motif_wheel_big_kernel(MotifArgs a, 
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   for (int i = threadIdx.x; i < table; i += kThreads) s_cnt[i] = 0;
   u64 w4 = 0;
-  const int64_t stride = (int64_t)gridDim.x * kThreads;
-  for (int64_t base = (int64_t)blockIdx.x * kThreads; base < a.nnz; base += stride) {
+  const int64_t stride = (int64_t)gridDim.x * per;
+  for (int64_t base = begin + (int64_t)blockIdx.x * per; base < end; base += stride) {
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
     const int64_t e64 = base + threadIdx.x;
-    if (e64 < a.nnz && a.a[e64] >= 2 && a.deg[a.src[e64]] > kWheelDeg)
+    if ((int)threadIdx.x < per && e64 < end && a.a[e64] >= 2 && a.deg[a.src[e64]] > kWheelDeg)
       s_e[atomicAdd(&s_n, 1)] = (int)e64;
     __syncthreads();
     for (int i = 0; i < s_n; ++i) {
@@ -1190,7 +1196,7 @@ struct Carver {
 // The pairs stage's classes that walks up to `longest` reach.
 template <bool kOrdered>
 int launch_pairs(mc_dgraph *g, const MotifArgs &a, int64_t longest, int big_grid, bool shared,
-                 size_t table_b, unsigned *counters) {
+                 size_t table_b, unsigned *counters, Slicer &sl) {
   cudaStream_t s = g->stream;
   auto launch = [&](auto kern, int threads, size_t smem, int64_t items) -> int {
     MC_CUDA_TRY(allow_smem((const void *)kern, smem));
@@ -1212,10 +1218,22 @@ int launch_pairs(mc_dgraph *g, const MotifArgs &a, int64_t longest, int big_grid
   auto big = shared ? motif_pairs_big_kernel<kOrdered, true> : motif_pairs_big_kernel<kOrdered, false>;
   const size_t smem = shared ? table_b : 0;
   MC_CUDA_TRY(allow_smem((const void *)big, smem));
-  big<<<big_grid, kPairThreads, smem, s>>>(a, counters);
-  MC_CUDA_TRY(cudaGetLastError());
-  g->launches += 1;
-  return MC_OK;
+  // In slices the walks of all pairs, of hubs seconds in all (ordered ones are
+  // bounded by the edges' smaller degrees).
+  unsigned n_items[kCounts] = {};
+  if (sl.on && !kOrdered) {
+    MC_CUDA_TRY(cudaMemcpyAsync(n_items, a.counts, sizeof(n_items), cudaMemcpyDeviceToHost, s));
+    MC_CUDA_TRY(cudaStreamSynchronize(s));
+  }
+  auto run = [&](int64_t b, int64_t e) -> int {
+    big<<<big_grid, kPairThreads, smem, s>>>(a, counters, (unsigned)b, e < 0 ? ~0u : (unsigned)e);
+    MC_CUDA_TRY(cudaGetLastError());
+    g->launches += 1;
+    return MC_OK;
+  };
+  if (kOrdered) return run(0, -1);
+  return run_slices(g, sl, "pairs", (int64_t)n_items[kHugeN] + n_items[kBigN], big_grid,
+                    reinterpret_cast<u64 *>(a.counts + kBigQueue), run);
 }
 
 }  // namespace
@@ -1389,6 +1407,7 @@ int motif_count(mc_dgraph *g, int pattern, bool estimates, uint64_t *out, bool *
       MC_CUDA_TRY(e);
     }
     u64 h[kSums + 1];
+    Slicer sl(g, -1.0);
     auto run = [&]() -> int {
       const int per = spread(nnz, g->num_sms);
       const unsigned tri_grid = blocks(std::max<int64_t>(n, ((int64_t)nnz + per - 1) / per * kWarp),
@@ -1430,8 +1449,8 @@ int motif_count(mc_dgraph *g, int pattern, bool estimates, uint64_t *out, bool *
         g->launches += 5;
       }
       if (pairs) {
-        const int rcp = ordered ? launch_pairs<true>(g, a, longest, pair_grid, table_shared, table_b, counters)
-                                : launch_pairs<false>(g, a, longest, pair_grid, table_shared, table_b, counters);
+        const int rcp = ordered ? launch_pairs<true>(g, a, longest, pair_grid, table_shared, table_b, counters, sl)
+                                : launch_pairs<false>(g, a, longest, pair_grid, table_shared, table_b, counters, sl);
         if (rcp != MC_OK) return rcp;
       }
       if (wheel) {
@@ -1444,10 +1463,16 @@ int motif_count(mc_dgraph *g, int pattern, bool estimates, uint64_t *out, bool *
           const size_t smem = sizeof(unsigned) * (size_t)table;
           MC_CUDA_TRY(allow_smem((const void *)motif_wheel_big_kernel, smem));
           const int per_sm = resident((const void *)motif_wheel_big_kernel, kThreads, smem);
-          motif_wheel_big_kernel<<<std::min(blocks(nnz, kThreads), (unsigned)(per_sm * g->num_sms)),
-                                   kThreads, smem, s>>>(a, table);
-          MC_CUDA_TRY(cudaGetLastError());
-          g->launches += 1;
+          const int64_t ctas = std::min(blocks(nnz, kThreads), (unsigned)(per_sm * g->num_sms));
+          const int rcw = run_slices(g, sl, "wheels", nnz, 4 * ctas, nullptr, [&](int64_t b, int64_t e) {
+            if (e < 0) e = nnz;
+            const int each = (int)std::max<int64_t>(1, std::min<int64_t>(kThreads, (e - b) / ctas));
+            motif_wheel_big_kernel<<<(unsigned)ctas, kThreads, smem, s>>>(a, table, b, e, each);
+            MC_CUDA_TRY(cudaGetLastError());
+            g->launches += 1;
+            return MC_OK;
+          });
+          if (rcw != MC_OK) return rcw;
         }
       }
       MC_CUDA_TRY(cudaEventRecord(g->ev[3], s));
