@@ -489,7 +489,7 @@ TriangleRoute triangle_route(const mc_dgraph *g) {
   for (const char *name : {"MERCURY_TC_TABLE_LOG2_MAX", "MERCURY_TC_BITMAP_BITS",
                            "MERCURY_TC_DENSE_FACTOR", "MERCURY_TC_CORE_RANKS", "MERCURY_TC_TMA",
                            "MERCURY_TC_ROW_STAGE", "MERCURY_TC_SHORT_RANGES",
-                           "MERCURY_TC_LONG_CLASSES", "MERCURY_DAG_STAGE", "MERCURY_STAGE_EDGES"})
+                           "MERCURY_TC_LONG_CLASSES", "MERCURY_STAGE_EDGES"})
     if (std::getenv(name)) return TriangleRoute::kDag;
   if (const char *env = std::getenv("MERCURY_TC_ROUTE"))  // dag, bits or pairs
     return std::strcmp(env, "bits") == 0 && g->n <= kDenseMax ? TriangleRoute::kBits
