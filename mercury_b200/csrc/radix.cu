@@ -259,7 +259,11 @@ cudaError_t sort_passes(u64 *keys, u64 *alt, int64_t count, int begin_bit, int p
   cudaError_t e = cudaMemsetAsync(work, 0, head_bytes() + (at_once ? one * passes : 0), s);
   if (e != cudaSuccess) return e;
   const size_t hist_smem = sizeof(int) * ((size_t)passes << kBits);
-  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(tiles, 148 * 8));
+  int device = 0, num_sms = 0;
+  e = cudaGetDevice(&device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device);
+  if (e != cudaSuccess) return e;
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(tiles, 8 * num_sms));
   radix_hist_kernel<kBits><<<(unsigned)blocks, kSortThreads, hist_smem, s>>>(keys, count, begin_bit,
                                                                            passes, hist);
   e = cudaGetLastError();
