@@ -112,17 +112,6 @@ __device__ __forceinline__ int64_t upper_row(const int64_t *__restrict__ a, int6
   return lo;
 }
 
-// Smallest r in [lo, hi] with a[r] >= key (a[hi] >= key).
-__device__ __forceinline__ int64_t lower_row(const int64_t *__restrict__ a, int64_t lo,
-                                             int64_t hi, int64_t key) {
-  while (lo < hi) {
-    int64_t mid = lo + ((hi - lo) >> 1);
-    if (__ldg(a + mid) >= key) hi = mid;
-    else lo = mid + 1;
-  }
-  return lo;
-}
-
 // Multiplicative (Fibonacci) hash of a vertex id to `bits` bits.
 __device__ __forceinline__ unsigned hash_slot(int key, int shift) {
   return ((unsigned)key * 2654435769u) >> shift;

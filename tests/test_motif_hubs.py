@@ -61,3 +61,17 @@ def test_long_stages_run_in_slices(monkeypatch):
     assert [c for c, _ in seen["0.02"]] == [c for c, _ in seen["250"]] == \
         [c for c, _ in seen["100000"]]
     assert all(short > long for (_, short), (_, long) in zip(seen["0.02"], seen["100000"]))
+
+
+@pytest.mark.gpu
+def test_walks_in_parts_beyond_the_shared_counters():
+    """A hub whose ordered walk goes in parts on a graph of more vertices than the
+    shared counters hold (102,400): counters per CTA in global memory."""
+    n, spokes = 110000, 30000
+    rng = np.random.default_rng(5)
+    ends = rng.integers(1, spokes + 1, (90000, 2))
+    hub = np.stack([np.zeros(spokes, dtype=np.int64), np.arange(1, spokes + 1)], 1)
+    tail = np.stack([np.arange(spokes + 1, n - 1), np.arange(spokes + 2, n)], 1)
+    rp, col = csr_from_edges(n, np.concatenate([hub, ends[ends[:, 0] != ends[:, 1]], tail]))
+    with DeviceGraph(rp, col) as d:
+        assert d.pattern_count(4) == orc.pattern_fast(rp, col, 4)
