@@ -625,10 +625,14 @@ int64_t stage_capacity(int64_t nnz, bool col_host) {
 // Ranks with core bitmaps: kCoreRanks, on small graphs a sixteenth of the
 // vertices (clearing 67 MB of bitmaps and filling them cost more than the hub
 // kernel gained there: 521 -> 499 us per count at RMAT scale 16, 0.944 -> 0.933
-// ms at 18), or MERCURY_TC_CORE_RANKS (0 turns them off; tests move the
-// boundary with it), at most n.
-int core_rank_count(int64_t n) {
-  int64_t k = std::min<int64_t>(kCoreRanks, n / 16);
+// ms at 18), and one per 512 entries where those are more: dense graphs live on
+// them (hub kernel, n / 16 ranks against this, ms: complete graph of 2,500 vertices
+// 1.57 / 0.42; random ones of 5,000 with 30%, of 8,000 with 10% and of 20,000 with
+// 7.7% of all edges 1.44 / 0.45, 0.75 / 0.37 and, with 8,192 ranks, 3.9 / 2.3).  Or
+// MERCURY_TC_CORE_RANKS (0 turns them off; tests move the boundary with it), at
+// most n.
+int core_rank_count(int64_t n, int64_t nnz) {
+  int64_t k = std::min<int64_t>(kCoreRanks, std::max<int64_t>(n / 16, nnz / 512));
   if (const char *env = std::getenv("MERCURY_TC_CORE_RANKS")) {
     const long long v = std::atoll(env);
     if (v >= 0) k = std::min<long long>(v, 1 << 18);
@@ -646,7 +650,7 @@ int64_t tc_device_bytes(int64_t n, int64_t nnz, bool col_host, bool dag_host) {
   return (n + 1) * (8 + 16 + 8 + 4 + 4 + 16) + n / 8 + 3 * 8 * tasks +
          (dag_host ? 0 : 2 * 4 * (dag_capacity(nnz, col_host) + 4)) +
          tiles * (2 * kTileThreads + 28) +
-         (int64_t)radix_work_bytes(n, 32) + scan + staging + 4 * core_offset(core_rank_count(n));
+         (int64_t)radix_work_bytes(n, 32) + scan + staging + 4 * core_offset(core_rank_count(n, nnz));
 }
 
 int tc_alloc(mc_dgraph *g) {
@@ -689,7 +693,7 @@ int tc_alloc(mc_dgraph *g) {
     MC_CUDA_TRY(dag_alloc(&g->dag_rank, &g->dag_rank_h));
     MC_ALLOC(g->rank_keys, 2 * n + 2);
     MC_CUDA_TRY(dev_alloc(&g->rank_work, radix_work_bytes(n, 32), g->stream));
-    g->core_ranks = core_rank_count(n);
+    g->core_ranks = core_rank_count(n, g->nnz);
     if (g->core_ranks > 0) MC_ALLOC(g->core_bits, core_offset(g->core_ranks));
   }
   // Chunked column passes (host columns, or a streamed upload of a single
@@ -867,7 +871,7 @@ int tc_orient(mc_dgraph *g, const int32_t *upload) {
   // A handle reused for a smaller graph keeps its capacity: only the ranks
   // of this graph get core bitmaps.
   if (g->core_bits && ranked) {
-    g->core_used = std::min(g->core_ranks, core_rank_count(n));
+    g->core_used = std::min(g->core_ranks, core_rank_count(n, nnz));
     MC_CUDA_TRY(cudaMemsetAsync(g->core_bits, 0, sizeof(unsigned) * core_offset(g->core_used), s));
     core_bits_kernel<<<grid_for((int64_t)g->core_used * kWarp, 256), 256, 0, s>>>(
         g->rank_sorted, n, g->core_used, g->dag_rowptr, g->dag_rank, g->core_bits, g->err);
