@@ -124,7 +124,7 @@ struct mc_dgraph {
   int64_t pin_entries = 0;
   cudaEvent_t pin_done[2] = {nullptr, nullptr};
   int32_t *deg = nullptr;         // n      degrees alone
-  int64_t *list_len = nullptr;    // 3      lengths of the hub, leaf and mega lists
+  int64_t *list_len = nullptr;    // 4      lengths of the hub, leaf and mega lists; not complete
   unsigned long long *task_status = nullptr;  // chained scans of the task lists
   uint64_t *hub_tasks = nullptr, *leaf_tasks = nullptr, *mega_tasks = nullptr;  // capacity
   int64_t task_capacity = 0;

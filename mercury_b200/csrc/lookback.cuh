@@ -5,8 +5,7 @@
 // waits are bounded all the same.  One that gives up raises kErrScanTimeout and
 // goes on within its arrays; what the launch wrote is then not complete, and
 // every later kernel that takes an index from it returns at its start.  (The
-// bit is raised by chained scans alone, so no kernel that tests it can see it
-// change.)
+// bit is raised by chained scans alone, so it stands still in those kernels.)
 #pragma once
 #include "device_common.cuh"
 
@@ -24,7 +23,8 @@ int wait_polls();
 // one word per tile, zero before the launch; max_polls: wait_polls().
 __device__ __forceinline__ unsigned long long tile_prefix(volatile unsigned long long *status,
                                                           int64_t tile, unsigned long long sum,
-                                                          int lane, int max_polls, unsigned *err) {
+                                                          int lane, int max_polls, unsigned *err,
+                                                          bool *gave_up) {
   if (lane == 0) status[tile] = (tile == 0 ? kTileTotal : kTileSum) | sum;
   unsigned long long prefix = 0;
   for (int64_t t = tile - 1; t >= 0; t -= kWarp) {
@@ -42,6 +42,7 @@ __device__ __forceinline__ unsigned long long tile_prefix(volatile unsigned long
     }
     if (!ready) {
       if (lane == 0) atomicOr(err, (unsigned)kErrScanTimeout);
+      *gave_up = true;
       break;
     }
     const unsigned total = __ballot_sync(kFull, (s & ~kTileValue) == kTileTotal);

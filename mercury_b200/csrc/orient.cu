@@ -384,9 +384,13 @@ __global__ void core_bits_kernel(const unsigned long long *__restrict__ sorted, 
 // The first `words` words of status are cleared (words <= n + 4), and so are
 // the waits that gave up in an earlier orientation or count.
 __global__ void init_key_kernel(const int64_t *rowptr, int64_t n, int2 *key, int32_t *deg,
-                                unsigned long long *status, int64_t words, unsigned *err) {
+                                unsigned long long *status, int64_t words, int64_t *lists_bad,
+                                unsigned *err) {
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v == 0) atomicAnd(err, ~(unsigned)(kErrScanTimeout | kErrWaitTimeout));
+  if (v == 0) {
+    atomicAnd(err, ~(unsigned)(kErrScanTimeout | kErrWaitTimeout));
+    *lists_bad = 0;
+  }
   if (v < words) status[v] = 0;
   if (v < n) {
     const int d = (int)(rowptr[v + 1] - rowptr[v]);
@@ -397,6 +401,7 @@ __global__ void init_key_kernel(const int64_t *rowptr, int64_t n, int2 *key, int
 
 struct TaskLists {
   int64_t *hub_end, *leaf_end, *mega_end;  // receive the lists' lengths
+  int64_t *bad;                            // set: the ranks or the lists are not complete
   uint64_t *hub, *leaf, *mega;
   // One running sum per list and block (kTaskThreads x kTaskItems vertices), a
   // ticket; cleared by init_key_kernel.
@@ -470,9 +475,13 @@ __global__ void __launch_bounds__(kTaskThreads) partner_tasks_kernel(
   if (warp < 3) {  // warp k: list k
     unsigned long long sum = 0;
     for (int w = 0; w < kW; ++w) sum += (unsigned)s_warp[warp][w];
+    bool gave_up = false;
     const unsigned long long before =
-        tile_prefix(t.status + warp * t.blocks, block, sum, lane, max_polls, err);
+        tile_prefix(t.status + warp * t.blocks, block, sum, lane, max_polls, err, &gave_up);
+    // (The rank sort's waits are over before this launch.)
+    if (lane == 0 && block == 0 && warp == 0) gave_up = (*err & kErrScanTimeout) != 0;
     if (lane == 0) {
+      if (gave_up) *t.bad = 1;
       s_base[warp] = (int64_t)before;
       if (block == t.blocks - 1)
         *(warp == 0 ? t.hub_end : warp == 1 ? t.leaf_end : t.mega_end) = (int64_t)(before + sum);
@@ -683,7 +692,7 @@ int tc_alloc(mc_dgraph *g) {
   MC_ALLOC(g->tile_offsets, tiles + 1);
   MC_ALLOC(g->tile_rows, 2 * tiles);
   MC_ALLOC(g->deg, n + 1);
-  MC_ALLOC(g->list_len, 3);
+  MC_ALLOC(g->list_len, 4);
   MC_ALLOC(g->task_status, n / kTaskThreads + 4);  // at least 3 per block of 1,024, and a ticket
   MC_ALLOC(g->hub_tasks, g->task_capacity);
   MC_ALLOC(g->leaf_tasks, g->task_capacity);
@@ -821,7 +830,7 @@ int tc_orient(mc_dgraph *g, const int32_t *upload) {
   g->ranked = ranked;
   const int64_t task_blocks = (n + kTaskThreads * kTaskItems - 1) / (kTaskThreads * kTaskItems);
   init_key_kernel<<<grid_for(n + 4, 256), 256, 0, s>>>(g->rowptr, n, g->key, deg, g->task_status,
-                                                       3 * task_blocks + 1, g->err);
+                                                       3 * task_blocks + 1, g->list_len + 3, g->err);
   MC_CUDA_TRY(cudaGetLastError());
   g->launches += 1;
   if (ranked) {
@@ -880,7 +889,7 @@ int tc_orient(mc_dgraph *g, const int32_t *upload) {
   }
   partner_tasks_kernel<<<(unsigned)task_blocks, kTaskThreads, 0, s>>>(
       g->key, ranked ? g->rank : nullptr, g->dag_rowptr, n, g->pinfo,
-      TaskLists{g->list_len, g->list_len + 1, g->list_len + 2, g->hub_tasks, g->leaf_tasks,
+      TaskLists{g->list_len, g->list_len + 1, g->list_len + 2, g->list_len + 3, g->hub_tasks, g->leaf_tasks,
                 g->mega_tasks, g->task_status, task_blocks},
       g->counters + 3, g->batch, wait_polls(), g->err);
   MC_CUDA_TRY(cudaGetLastError());
