@@ -57,8 +57,9 @@ namespace {
 // Words of MotifArgs::counts: list lengths, then queue positions.
 enum Count : int {
   kTauN, kMidN, kHashN, kHugeN, kBigN, kSplitN, kTauQueue, kMidQueue, kHashQueue, kUnused,
-  kBigQueue,  // 64 bits (run_slices clears it)
-  kCounts = kBigQueue + 2
+  kBigQueue,                   // 64 bits each: run_slices clears them
+  kWheelQueue = kBigQueue + 2,
+  kCounts = kWheelQueue + 2
 };
 
 struct MotifArgs {
@@ -128,6 +129,7 @@ constexpr u64 kFewWalk = 64;
 constexpr int kFewVertices = 16384;
 constexpr int kHashSlots = 1024;  // of a warp
 constexpr int kWheelDeg = 512;    // warp form of the wheel stage
+constexpr int kWheelClaim = 32;   // entries a CTA claims at once in the other
 constexpr int kProbeBlocks = 4;   // samples: a thread each
 constexpr int kEarlyOut = 400;    // bound on d+ above which a^2 is summed before tau (7 us at 1 M entries)
 
@@ -1118,22 +1120,30 @@ __global__ void __launch_bounds__(kThreads) motif_wheel_kernel(MotifArgs a, int 
 }
 
 // CTA per entry of a longer row: warp per y, lanes over y's list; entries [begin,
-// end), a CTA looking at `per` of them at a time.
+// end), claimed `per` at a time: the hubs' entries lie together, and with fixed
+// shares the slices of the Chung-Lu graph of 10^6 vertices (cap 50,000) took 13.7 s
+// in P3 where one launch took 5.6.
 __global__ void __launch_bounds__(kThreads) motif_wheel_big_kernel(MotifArgs a, int table, int64_t begin,
                                                                    int64_t end, int per) {
   extern __shared__ unsigned s_cnt[];
   __shared__ u64 sm[kSums];
   __shared__ int s_e[kThreads], s_n;
+  __shared__ int64_t s_base;
   const BlockSums bs{sm};
   bs.init();
   if (stops_here(a)) return;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   for (int i = threadIdx.x; i < table; i += kThreads) s_cnt[i] = 0;
+  u64 *queue = reinterpret_cast<u64 *>(a.counts + kWheelQueue);
   u64 w4 = 0;
-  const int64_t stride = (int64_t)gridDim.x * per;
-  for (int64_t base = begin + (int64_t)blockIdx.x * per; base < end; base += stride) {
-    if (threadIdx.x == 0) s_n = 0;
+  for (;;) {
+    if (threadIdx.x == 0) {
+      s_n = 0;
+      s_base = begin + (int64_t)(atomicAdd(queue, 1ull) * (u64)per);
+    }
     __syncthreads();
+    const int64_t base = s_base;
+    if (base >= end) break;
     const int64_t e64 = base + threadIdx.x;
     if ((int)threadIdx.x < per && e64 < end && a.a[e64] >= 2 && a.deg[a.src[e64]] > kWheelDeg)
       s_e[atomicAdd(&s_n, 1)] = (int)e64;
@@ -1464,9 +1474,10 @@ int motif_count(mc_dgraph *g, int pattern, bool estimates, uint64_t *out, bool *
           MC_CUDA_TRY(allow_smem((const void *)motif_wheel_big_kernel, smem));
           const int per_sm = resident((const void *)motif_wheel_big_kernel, kThreads, smem);
           const int64_t ctas = std::min(blocks(nnz, kThreads), (unsigned)(per_sm * g->num_sms));
-          const int rcw = run_slices(g, sl, "wheels", nnz, 4 * ctas, nullptr, [&](int64_t b, int64_t e) {
+          u64 *queue = reinterpret_cast<u64 *>(a.counts + kWheelQueue);
+          const int rcw = run_slices(g, sl, "wheels", nnz, 4 * ctas, queue, [&](int64_t b, int64_t e) {
             if (e < 0) e = nnz;
-            const int each = (int)std::max<int64_t>(1, std::min<int64_t>(kThreads, (e - b) / ctas));
+            const int each = (int)std::max<int64_t>(1, std::min<int64_t>(kWheelClaim, (e - b) / (4 * ctas)));
             motif_wheel_big_kernel<<<(unsigned)ctas, kThreads, smem, s>>>(a, table, b, e, each);
             MC_CUDA_TRY(cudaGetLastError());
             g->launches += 1;
