@@ -92,7 +92,8 @@ struct MotifArgs {
   // vertices, the longest walks from the front, so that they start first.
   int32_t *tau_big, *pair_mid, *pair_big;
   unsigned *counts;  // see Count
-  // Parts of the longest walks: split_cap entries (s, part, parts) at most (0:
+  // Parts of the longest walks (ordered), or those walks themselves (all pairs):
+  // split_cap entries (s, part, parts) at most (0:
   // none); num_sms and the sum of walk place the line.
   int4 *split;
   int split_cap, num_sms;
@@ -125,6 +126,11 @@ constexpr u64 kHugeWalk = 1 << 15;
 // stage cost 0.04 ms at 1 M entries.
 constexpr u64 kSplitWalk = 1 << 16;
 constexpr int kSplitMax = 1024;
+// Of all pairs, the walks of vertices above this degree (whose X7 outlasts any walk)
+// stand in front and run in the first slice, beside one another: in the order of
+// their arrival, slices of 250 ms waited for one hub each (P5 at n = 500,000, cap
+// 50,000: 6.5 to 7.1 s against 6.0 in one launch).
+constexpr int kGiantDegree = 1024;
 constexpr u64 kFewWalk = 64;
 constexpr int kFewVertices = 16384;
 constexpr int kHashSlots = 1024;  // of a warp
@@ -350,7 +356,7 @@ __global__ void __launch_bounds__(kThreads) motif_tri_kernel(MotifArgs a, int pe
   const int lane = threadIdx.x & (kWarp - 1);
   if (!kCount && lists_overrun(a)) return;  // the host makes room and starts over
   const int64_t s64 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (!kCount && a.split_cap > 0 && s64 - lane < a.n) {
+  if (!kCount && a.split_cap > 0 && (a.need & kNeedC4) && s64 - lane < a.n) {
     const u64 w = warp_sum_u64(s64 < a.n ? a.walk[s64] : 0);
     if (lane == 0 && w) atomicAdd(a.walk_total, w);
   }
@@ -360,7 +366,11 @@ __global__ void __launch_bounds__(kThreads) motif_tri_kernel(MotifArgs a, int pe
     if (p > kTauOut || (p >= 2 && d > kTauDeg)) a.tau_big[atomicAdd(a.counts + kTauN, 1u)] = v;
     if (a.need & (kNeedC4 | kNeedPairs)) {
       const u64 w = a.walk[v];
-      if (w > kHugeWalk) a.pair_big[atomicAdd(a.counts + kHugeN, 1u)] = v;
+      unsigned front = kSplitMax;
+      if (w > kHashWalk && d > kGiantDegree && a.split_cap > 0 && !(a.need & kNeedC4))
+        front = atomicAdd(a.counts + kSplitN, 1u);
+      if (front < (unsigned)kSplitMax) a.split[front] = make_int4(v, 0, 1, 0);
+      else if (w > kHugeWalk) a.pair_big[atomicAdd(a.counts + kHugeN, 1u)] = v;
       else if (w > kHashWalk) a.pair_big[a.n - 1 - atomicAdd(a.counts + kBigN, 1u)] = v;
       else if (w > a.mid_walk) a.pair_mid[a.n - 1 - atomicAdd(a.counts + kHashN, 1u)] = v;
       else if (w > a.warp_walk) a.pair_mid[atomicAdd(a.counts + kMidN, 1u)] = v;
@@ -710,7 +720,7 @@ __global__ void __launch_bounds__(kThreads) motif_tau_kernel(MotifArgs a, int sm
   if (a.early ? stops_here(a) : lists_overrun(a)) return;
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   TauSums t;
-  if (kLarge && a.split_cap > 0) split_walks(a);
+  if (kLarge && a.split_cap > 0 && (a.need & kNeedC4)) split_walks(a);
   if (kLarge) tau_large(a, t, s_rows, smem_words, &s_u, lane, warp);
   if (kSmall) tau_small(a, t, s_r[kSmall ? warp : 0], s_m[kSmall ? warp : 0], lane);
   t.flush(bs, a.need & kNeedTau);
@@ -1012,13 +1022,13 @@ __global__ void __launch_bounds__(kPairThreads) motif_pairs_big_kernel(MotifArgs
   constexpr int kEnd = -2;
   bool clean = false;  // the counters are zero
   PairSums ps;
-  const int splits = kOrdered ? (int)min(a.counts[kSplitN], (unsigned)a.split_cap) : 0;
+  const int splits = (int)min(a.counts[kSplitN], (unsigned)a.split_cap);
   for (;;) {
     if (threadIdx.x == 0) {
       unsigned i = begin + atomicAdd(a.counts + kBigQueue, 1u);
       const unsigned huge = a.counts[kHugeN], big = a.counts[kBigN];
       int4 item = make_int4(kEnd, 0, 1, 0);
-      if ((int)i < splits) {
+      if (i < end && (int)i < splits) {
         item = a.split[i];
         // Parts of about the same number of entries: t's place in the CSR.
         for (int k = 0; k < 2; ++k)
@@ -1242,7 +1252,8 @@ int launch_pairs(mc_dgraph *g, const MotifArgs &a, int64_t longest, int big_grid
     return MC_OK;
   };
   if (kOrdered) return run(0, -1);
-  return run_slices(g, sl, "pairs", (int64_t)n_items[kHugeN] + n_items[kBigN], big_grid,
+  const int64_t giants = std::min<unsigned>(n_items[kSplitN], (unsigned)a.split_cap);
+  return run_slices(g, sl, "pairs", giants + n_items[kHugeN] + n_items[kBigN], giants + big_grid,
                     reinterpret_cast<u64 *>(a.counts + kBigQueue), run);
 }
 
@@ -1359,7 +1370,10 @@ int motif_count(mc_dgraph *g, int pattern, bool estimates, uint64_t *out, bool *
     a.warp_walk = n <= kFewVertices ? kFewWalk : kWarpWalk;
     a.mid_walk = kMidWalk;
     a.num_sms = g->num_sms;
-    a.split_cap = ordered && longest > (int64_t)kSplitWalk ? kSplitMax : 0;
+    a.split_cap = (ordered && longest > (int64_t)kSplitWalk) ||
+                          (pairs && !ordered && g->max_degree > kGiantDegree)
+                      ? kSplitMax
+                      : 0;
     size_t zeroed = 0;
     // The same layout for every pattern (so that each finds the last one's block).
     auto lay_out = [&](Carver &c) {
