@@ -72,8 +72,13 @@ typedef struct mc_timing {
   double count_ms;    /* counting kernels                                    */
   double d2h_ms;      /* device->host copy of the result                     */
   double total_ms;    /* first to last event of the call                     */
-  double hub_ms;      /* share of count_ms spent in the hash (hub) kernel    */
-  double leaf_ms;     /* share of count_ms spent in the warp (leaf) kernel   */
+  /* Shares of count_ms: up to the end of the hash (hub) kernel, and from there
+   * to the end of the warp (leaf) kernel.  Up to 2^24 entries the leaf kernel
+   * starts where the hub kernel leaves the SMs idle, so hub_ms then holds a
+   * part of its work and leaf_ms what is left; above, each is its kernel's own
+   * time.  Both are 0 where a count needs no DAG. */
+  double hub_ms;
+  double leaf_ms;
   int64_t launches;   /* kernels this call launched                          */
 } mc_timing_t;
 
@@ -271,7 +276,8 @@ int mc_dgraph_export_dag(const mc_dgraph_t *g, int64_t *rowptr_out,
  * sm_multigpu.cu:206-232): the same quantities over all 2m directed edges,
  * bit-exact, without MPI.  Whole counts come from sums over vertices,
  * edges, triangles and vertex pairs wherever those apply and are faster
- * (MERCURY_MOTIF_ROUTE=formula / dense / sparse forces a route); otherwise
+ * (MERCURY_MOTIF_ROUTE=formula / dense / sparse forces a route; a count of
+ * a graph made of cliques may change to the formulas on the way); otherwise
  * the formulas are evaluated edge by edge, with per-warp frontier scratch of
  * max_degree entries per list.  Scratch is taken for the call and shared by
  * the device's handles.  Shards and budgets of P7 and P8
