@@ -64,6 +64,9 @@ void retain_pool_memory(int device);
 // alone falls with every block the pool has ever held.)  MERCURY_DEVICE_BYTES
 // replaces the figure (tests reach the fallbacks with it on small graphs).
 int device_bytes_available(int device, int64_t *avail);
+// Whether that is at least `bytes`, by the driver's figure alone where that says so
+// (asking the pool took 0.6 ms in a process that had counted some hundred graphs).
+int device_bytes_hold(int device, int64_t bytes, bool *holds);
 
 cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s);
 inline void dev_free(void *p, cudaStream_t s) { cudaFreeAsync(p, s); }

@@ -226,6 +226,17 @@ int device_bytes_available(int device, int64_t *avail) {
   return MC_OK;
 }
 
+int device_bytes_hold(int device, int64_t bytes, bool *holds) {
+  size_t free_b = 0, total_b = 0;
+  MC_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+  *holds = (int64_t)free_b >= bytes && !std::getenv("MERCURY_DEVICE_BYTES");
+  if (*holds) return MC_OK;
+  int64_t avail = 0;
+  const int rc = device_bytes_available(device, &avail);
+  *holds = rc == MC_OK && avail >= bytes;
+  return rc;
+}
+
 void set_last_cuda_error(cudaError_t e) { t_last_cuda = e; }
 cudaError_t last_cuda_error() { return t_last_cuda; }
 

@@ -1410,10 +1410,11 @@ int motif_count(mc_dgraph *g, int pattern, bool estimates, uint64_t *out, bool *
     // does when the allocation fails.
     const size_t counters_b = pairs && !table_shared ? pair_grid * table_b : 0;
     if (size.used + counters_b > size_t(1) << 30) {
-      int64_t avail = 0;
-      const int arc = device_bytes_available(g->device, &avail);
+      const int64_t wanted = (int64_t)(size.used + counters_b);
+      bool fits = false;
+      const int arc = device_bytes_hold(g->device, 2 * wanted, &fits);
       if (arc != MC_OK) return arc;
-      if ((int64_t)(size.used + counters_b) > avail / 2) {
+      if (!fits) {
         if (counted) return MC_ERR_OOM;
         counted = true;
         list_cap = std::min<int64_t>(list_cap, 4 * (int64_t)nnz);
@@ -1472,11 +1473,23 @@ int motif_count(mc_dgraph *g, int pattern, bool estimates, uint64_t *out, bool *
         MC_CUDA_TRY(cudaGetLastError());
         g->launches += 5;
       }
+      // Slices are for stages that last: 2^30 of a^2 are some 7 ms of wheels and 30 of
+      // X7, 2^32 two-paths some 20 (a star of 5,000, P3: 77 us in one launch, 163 in
+      // slices).
+      bool long_lists = false, long_walks = false;
+      if (sl.on && !ordered && (pairs || wheel)) {
+        MC_CUDA_TRY(cudaMemcpyAsync(h, a.acc, sizeof(h), cudaMemcpyDeviceToHost, s));
+        MC_CUDA_TRY(cudaStreamSynchronize(s));
+        long_lists = 4 * h[kD] + 6 * h[kT] > u64(1) << 30;
+        long_walks = long_lists || (int64_t)nnz * g->max_degree > int64_t(1) << 33;
+      }
       if (pairs) {
+        sl.on = long_walks;
         const int rcp = ordered ? launch_pairs<true>(g, a, longest, pair_grid, table_shared, table_b, counters, sl)
                                 : launch_pairs<false>(g, a, longest, pair_grid, table_shared, table_b, counters, sl);
         if (rcp != MC_OK) return rcp;
       }
+      sl.on = long_lists;
       if (wheel) {
         motif_wheel_kernel<<<std::min(blocks(nnz, kWarps * per), (unsigned)(8 * g->num_sms)), kThreads,
                              0, s>>>(a, per);

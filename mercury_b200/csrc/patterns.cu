@@ -1735,11 +1735,13 @@ int launch_center(mc_dgraph *g, const CenterArgs &a, int num_sms, int64_t total,
     // fit build their rows per edge.
     const int64_t groups = (int64_t)grid * (kPatThreads / kWarp / G);
     const int64_t need = hop_group_words(a.hop_walk, W);
-    int64_t avail = 0;
-    const int arc = device_bytes_available(g->device, &avail);
+    constexpr int64_t kHopCap = int64_t(4) << 30;
+    int64_t avail = 4 * kHopCap;
+    bool plenty = false;
+    int arc = device_bytes_hold(g->device, avail, &plenty);
+    if (arc == MC_OK && !plenty) arc = device_bytes_available(g->device, &avail);
     if (arc != MC_OK) return arc;
-    const int64_t cap_words =
-        std::min<int64_t>(int64_t(4) << 30, avail / 4) / (int64_t)sizeof(unsigned);
+    const int64_t cap_words = std::min<int64_t>(kHopCap, avail / 4) / (int64_t)sizeof(unsigned);
     int64_t per_group = std::min<int64_t>(need, cap_words / groups);
     // MERCURY_HOP_WORDS lowers the share (tests use it to send the larger
     // centers to the per-edge rows).
