@@ -308,7 +308,8 @@ int mc_pattern_count_shard(mc_dgraph_t *g, int pattern, int shard,
  * stops between two slices and returns MC_ERR_TIMEOUT (count not written).
  * progress (optional) receives the fraction of the tasks done.  Graphs with
  * a maximum degree above 4,096 are counted in slices by mc_pattern_count too
- * (no budget): a hub edge alone can take seconds.  The reference has no
+ * (no budget): a hub edge alone can take seconds.  (By the formulas; of
+ * the motif sums, the stages that last.)  The reference has no
  * budget; its kernels run to the end (subgraph_matching/sm_multigpu.cu:
  * 150-200). */
 int mc_pattern_count_budget(mc_dgraph_t *g, int pattern, double budget_ms,
